@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_prompt_tc(const AttnRowsAr
         if (t + 1 < n_tiles) { load_tile(t + 1, buf ^ 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
         fence_proxy_async_smem();
         __syncthreads();
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             tc_fence_after_sync();
             const uint32_t kb = s_base + kAtOffK + buf * kAtKVBytes;
 #pragma unroll
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_prompt_tc(const AttnRowsAr
         fence_proxy_async_smem();
         tc_fence_before_sync();
         __syncthreads();
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             tc_fence_after_sync();
             const uint32_t vb = s_base + kAtOffV + buf * kAtKVBytes;
             // V as stored: 16-byte groups of 8 head dimensions, 1024 bytes apart along the head dimension (MN), 8 positions = 128
@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_band_tc(const BandArgs a) 
     auto load_k = [&](int i) { load_tile(i, s_base + L.k + (i & 1) * kAtKT * dkp * 2, kc, k_row, kgr); };
     auto load_v = [&](int i) { load_tile(i, s_base + L.v + (i & 1) * kAtKT * dvp * 2, vc, v_row, vgr); };
     const uint32_t idesc_s = idesc_bf16(128, kAtKT, false), idesc_o = idesc_bf16(128, dvp, true);
-    auto issue_s = [&](int i) {                                // thread 0: scores of tile i
+    auto issue_s = [&](int i) {                                // one thread of warp 0: scores of tile i
         const uint32_t kb = s_base + L.k + (i & 1) * kAtKT * dkp * 2, d = tmem + (i & 1) * kAtKT;
         for (int term = 0; term < 2; term++) {
             const uint32_t qb = s_base + (term ? L.qlo : 0);
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_band_tc(const BandArgs a) 
         cp_async_wait<2>();
         fence_proxy_async_smem();
         __syncthreads();
-        if (tid == 0) { tc_fence_after_sync(); issue_s(0); }
+        if (warp == 0 && elect_one()) { tc_fence_after_sync(); issue_s(0); }
     }
 #pragma unroll 1
     for (int i = 0; i < n_t; i++) {
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_band_tc(const BandArgs a) 
         tc_fence_before_sync();
         if (__syncthreads_or(failed ? 1 : 0)) { failed = true; break; }      // the tensor core never answered: give up, together
         tc_fence_after_sync();
-        if (tid == 0 && i + 1 < n_t) issue_s(i + 1);
+        if (i + 1 < n_t && warp == 0 && elect_one()) issue_s(i + 1);
 
         // ---- softmax of this thread's row over its 32 keys of the tile
         float s[32];
@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_band_tc(const BandArgs a) 
         fence_proxy_async_smem();
         tc_fence_before_sync();
         __syncthreads();
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             tc_fence_after_sync();
             const uint32_t vb = s_base + L.v + (i & 1) * kAtKT * dvp * 2;
 #pragma unroll

@@ -115,6 +115,16 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* p, uint32_t bytes) 
 }
 
 // ---- 5th-generation tensor core (tcgen05) and tensor memory ----------------------------------------
+// One thread of the (converged) warp, the same one every time.  Every tcgen05.mma / commit and bulk copy that one thread issues is
+// guarded by this and not by a comparison of the lane: behind `lane == 0` the compiler does not know that a single thread is left, and the
+// code it then makes of an instruction with operands in uniform registers takes 60 clocks to issue whatever the instruction's size.
+// Measured, clocks per tcgen05.mma of M 128, K 32 bytes, back to back (branch on the lane / elected): kind::f16 with A in tensor memory
+// 62 / 17 at N 32, 62 / 33 at N 64, 65 / 65 at N 128; kind::i8 from shared memory 52 / 45 at N 48.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 // Shared-memory operand descriptor for a K-major operand without swizzling: the operand is a grid of "core matrices"
 // of 8 rows x 16 bytes, each stored as 128 contiguous bytes (row stride 16 B).  `lbo` is the byte distance between the
 // two core matrices that cover K = 32 bytes of the same 8 rows, `sbo` the distance between consecutive groups of 8 rows.

@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(kDmThreads, 1) dense_gemm_tc(const DenseArgs a
     const int KC0 = a.seg[0].chunks, KC = KC0 + (a.nk > 1 ? a.seg[1].chunks : 0);
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t it = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(kDmThreads, 1) dense_gemm_tc(const DenseArgs a
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t it = 0;
             int ti = 0;
             bool ok = true;

@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
 
     if (warp == kGmCvtWarps) {
         // ---------------------------------------------------------------- activation producer: one lane, one 32 KiB copy per stage
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t xi = 0;
             bool ok = true;
             for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
     }
     if (warp == kGmCvtWarps + 1) {
         // ---------------------------------------------------------------- tensor-core warp: one lane issues
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t xi = 0, ci = 0, ic = 0;
             bool ok = true;
             // 128 activation rows per chunk: hi x1, hi x2, lo x1 as three instructions of N = 128 into one accumulator.  Fewer rows:
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(kGsThreads, 1) q8_gemm_tc_staged(const GemmArg
     }
     if (warp == kGsCvtWarps) {
         // ---------------------------------------------------------------- activation producer: one lane, one 32 KiB copy per stage
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t xi = 0;
             bool ok = true;
             for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(kGsThreads, 1) q8_gemm_tc_staged(const GemmArg
     }
     if (warp == kGsCvtWarps + 1) {
         // ---------------------------------------------------------------- tensor-core warp: one lane issues
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t xi = 0, ci = 0, ic = 0;
             bool ok = true;
             // hi x [x1 | x2] is ONE instruction of N = 2 nc (its two halves of the accumulator are added when it is stored), lo x x1

@@ -101,14 +101,14 @@ __global__ void __launch_bounds__(kGemvThreads, 1) q8_gemv_stream(const GemvArgs
 
     if (warp == kProducerWarp) {
         // producer: the weight stream does not depend on the previous kernel, so it starts at once
-        if (lane == 0) {
+        if (elect_one()) {
             ProducerRing pr{0, 0u, 0};
             if (!gemv_produce(a, plan, g, pr, (int)blockIdx.x, (int)gridDim.x, a.job_ctr, a.status)) gemv_producer_drain(g, pr, a.status);
         }
         return;
     }
     if (warp == kMmaWarp) {
-        if (lane == 0) {
+        if (elect_one()) {
             MmaRing mr{0, 0u, 0u, 0u, 0u};
             gemv_mma_issue(a, plan, g, mr, tmem, a.status);
         }

@@ -792,8 +792,8 @@ __device__ __forceinline__ void gemv_producer_drain(const GemvSmem& g, const Pro
 // memory (tile i of the fill at column 64 i), overwritten — and has "accumulators written" signalled when they retire.
 // Lane (8 b + r) of tile t, column 3 b + l is the exact integer dot product of row r's block b with level l of the
 // matching activation block; the other 45 columns of a lane pair the weights with other blocks' activations and are
-// never read.  Measured on B200: an instruction of this shape occupies the tensor pipe for about 73 cycles whatever
-// N is, and tcgen05.ld issued while instructions are in flight completes only after they retire — so the fill's
+// never read.  Measured on B200: an instruction of this shape occupies the tensor pipe for 40 (N 16) to 45 (N 48)
+// cycles, and tcgen05.ld issued while instructions are in flight completes only after they retire — so the fill's
 // instructions are issued back to back and the read-back follows as one burst, the two strictly alternating.
 __device__ __forceinline__ bool gemv_mma_issue(const GemvArgs& a, const GemvPlan& p, const GemvSmem& g, MmaRing& r, uint32_t tmem, uint32_t* status) {
     const int S = g.stages;
@@ -827,8 +827,7 @@ __device__ __forceinline__ bool gemv_mma_issue(const GemvArgs& a, const GemvPlan
             uint32_t b_lo = xq_lo + (uint32_t)c0 * (kXqTileBytes >> 4);
             tc_fence_after_sync();
             if (nt == kFillTiles && !wrap) {
-                // the common case, straight-line: the tensor pipe takes ~60 cycles per instruction and the issuing thread
-                // is held that long, so every other instruction in between adds to the burst
+                // the common case, straight-line: eight instructions, 45 cycles of the tensor pipe each
 #pragma unroll
                 for (int i = 0; i < kFillTiles; i++)
                     umma_s8_ss_split(tmem + (uint32_t)(64 * i), a_lo + (uint32_t)i * (kTileBytes >> 4), b_lo + (uint32_t)i * (kXqTileBytes >> 4), hi, idesc);
@@ -1011,7 +1010,7 @@ __device__ __forceinline__ uint32_t gemv_cta_begin(const GemvSmem& g, int tid, v
 // gemv_mma_end(), which waits (bounded) for the last instruction it issued, then for the draining warps, and frees tensor memory.
 __device__ __forceinline__ void gemv_consumers_done() { tc_fence_before_sync(); named_arrive(4, kConsumers + 32); }
 __device__ __forceinline__ void gemv_mma_end(const GemvSmem& g, uint32_t tmem, int lane, uint32_t* status) {
-    if (lane == 0) {
+    if (elect_one()) {
         umma_commit(g.fin);
         if (!mbar_wait(g.fin, 0u)) atomicOr(status, LUM_ST_WAIT_TMEM);
     }

@@ -171,11 +171,11 @@ __global__ void __launch_bounds__(kGemvThreads, 1) decode_mega(const MegaArgs a)
             if (cta == 0 && tid == 0) a.job_ctr[(pseq + kJobCtrRing / 2) % kJobCtrRing] = 0u;
             pseq++;
             if (is_producer) {
-                if (streams && lane == 0 && producing) {
+                if (streams && elect_one() && producing) {
                     producing = gemv_produce(ga, plan, g, pring, cta, ncta, ctr, a.status);
                 }
             } else if (is_mma) {
-                if (streams && lane == 0 && issuing) issuing = gemv_mma_issue(ga, plan, g, mring, tmem, a.status);
+                if (streams && elect_one() && issuing) issuing = gemv_mma_issue(ga, plan, g, mring, tmem, a.status);
             } else if (!streams) {
                 // RoPE + cache append + attention
                 if (!s_abort) attn_phase<HD, GM, BF16>(a, L, (unsigned char*)g.xq, pos, tid);
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) decode_mega(const MegaArgs a)
     }
 
     if (is_producer) {
-        if (lane == 0 && (s_abort || !producing)) gemv_producer_drain(g, pring, a.status);
+        if (elect_one() && (s_abort || !producing)) gemv_producer_drain(g, pring, a.status);
         return;
     }
     if (is_mma) {
