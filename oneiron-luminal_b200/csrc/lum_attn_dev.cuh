@@ -450,4 +450,23 @@ __device__ __forceinline__ void attn_decode_body(const AttnArgs& a, unsigned cha
     if (tid == 0) a.counters[kvh] = 0u;
 }
 
+// ---- Products of attention on m16n8k16 tensor-core instructions (bf16 operands, f32 sums) without giving up f32 operands: K and V are bf16
+// already; an f32 query or softmax weight is the sum of THREE bf16 terms (24 bits: all of it), and the terms take the rows of the first
+// operand that a group of four query heads leaves free: row h holds head h's first term, row 4 + h its second, row 8 + h its third.
+// The three rows' results are added.
+__device__ __forceinline__ void attn_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Two neighbouring elements for this thread's two rows, g = lane / 4 and g + 8: the first and the third terms of head g (g < 4), or the second
+// terms of head g - 4 and nothing
+__device__ __forceinline__ void attn_terms(float x0, float x1, bool second, uint32_t* lo_row, uint32_t* hi_row) {
+    const __nv_bfloat162 t1 = __floats2bfloat162_rn(x0, x1);
+    const float r0 = x0 - __low2float(t1), r1 = x1 - __high2float(t1);
+    const __nv_bfloat162 t2 = __floats2bfloat162_rn(r0, r1);
+    const __nv_bfloat162 t3 = __floats2bfloat162_rn(r0 - __low2float(t2), r1 - __high2float(t2));
+    *lo_row = second ? *(const uint32_t*)&t2 : *(const uint32_t*)&t1;
+    *hi_row = second ? 0u : *(const uint32_t*)&t3;
+}
+
 }  // namespace lum

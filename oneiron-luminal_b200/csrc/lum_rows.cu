@@ -203,172 +203,222 @@ __global__ void __launch_bounds__(256) attn_rows(const AttnRowsArgs a) {
     }
 }
 
-// The same attention for rows of a bfloat16 cache, reorganised so that no dot product needs a shuffle: used for batched decode
-// (every row its own sequence with a long context), where the kernel above — one warp per key, five shuffles per key and query head
-// — runs at a fifth of the memory rate.  One CTA per (KV head, row, split of the cached positions), 4 warps; a warp takes 32 keys at
-// a time:
-//   scores  : lane = key.  The lane reads its key's row (16-byte loads) and multiplies it with the group's queries from shared
-//             memory (the same address in every lane: a broadcast).
-//   softmax : per warp and query head, one max-reduction per 32 keys; the weights go to shared memory.
-//   values  : lane = HD / 32 head dimensions.  The 32 value rows are read coalesced, each weighted by its key's weight from shared
-//             memory (a broadcast again).
-// The warps' (max, sum, output) triples are merged in shared memory; with more than one split the CTA writes its triple to global
-// memory and attn_rows_merge folds the splits.
-template <int HD, int GM>
+// The same attention for rows of a bfloat16 cache: batched decode (every row its own sequence with a long context), and the rows of a
+// prompt that do not take the tcgen05 kernel.  Bound by the cache's bytes.  What counts is how many of them are on their way and how
+// few instructions a key costs:
+//   * a cluster of CTAs per (KV head, row), one CTA per split of the cached positions, four warps per CTA.  Warps do not wait for
+//     each other: each takes 16 keys at a time and fetches their K and V (cp.async, coalesced 16-byte pieces, rows swizzled so that
+//     ldmatrix reads them without bank conflicts) into its own ring in shared memory, ar_stages - 1 tiles ahead.
+//   * both products are tensor-core instructions over three bf16 terms of the f32 operand (attn_terms): nothing is rounded to fewer bits
+//     than the plain evaluation keeps.
+//   * warps merge in shared memory, splits through the cluster's distributed shared memory: no partial results in global memory and no
+//     second kernel.
+// Measured (32 sequences x 2049 keys, 8 KV heads x 4 query heads, head dimension 128; 268 MB of cache): 53 us.  The form before it, with
+// a lane per key and the products on CUDA cores (1700 instructions per warp and 32 keys, 16-byte loads 2 KiB apart), took 147 us and
+// 6 us more to merge.
+__device__ __forceinline__ void ar_ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ar_ldsm4_t(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ar_cp16(uint32_t dst, const void* src, uint32_t src_bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+}
+constexpr int kArTile = 16;                                        // keys per warp and step
+__host__ __device__ constexpr int ar_stages(int hd) { return hd == 128 ? 2 : 3; }
+__host__ __device__ constexpr int ar_smem(int hd) { return 4 * ar_stages(hd) * 2 * kArTile * hd * 2; }
+
+// MT: groups of four query heads (G <= 4 MT)
+template <int HD, int MT>
 __global__ void __launch_bounds__(128) attn_rows_split(const AttnRowsArgs a, int n_splits) {
-    constexpr int DPL = HD / 32, NW = 4;
-    __shared__ __align__(16) float s_q[GM][HD];
-    __shared__ float s_p[NW][GM][32];
-    __shared__ float s_m[NW][GM], s_l[NW][GM];
-    __shared__ float s_o[NW][GM][HD];
+    constexpr int NW = 4, NT = HD / 8, KS = HD / 16, CH = HD / 8, GM = 4 * MT, NS = ar_stages(HD);
+    constexpr int kSide = kArTile * HD * 2, kStage = 2 * kSide;     // bytes of one tile's K (or V); of both
+    extern __shared__ __align__(128) unsigned char ar_sm[];
+    static_assert((NW * GM * HD + GM * HD + 2 * NW * GM + 2 * GM) * 4 <= ar_smem(HD), "the merge reuses the ring");
     const int kvh = blockIdx.x, m = blockIdx.y, sp = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int g = lane >> 2, t = lane & 3;                           // row and column group of the fragments
+    const bool second = g >= 4;
     const int G = a.n_q / a.n_kv;
     const int pos = a.row_pos[m];
     const int seq = a.row_seq ? a.row_seq[m] : a.seq0;
-    if (pos < 0 || pos >= a.max_seq || seq < 0 || seq >= a.max_batch) return;       // flagged by the append kernel
+    if (pos < 0 || pos >= a.max_seq || seq < 0 || seq >= a.max_batch) return;       // flagged by the append kernel (the whole cluster returns)
     const int n_keys = pos + 1;
-    const int per = ((n_keys + n_splits - 1) / n_splits + 31) & ~31;                // keys per split, whole 32-key tiles
+    const int per = ((n_keys + n_splits - 1) / n_splits + 63) & ~63;                // keys per split, whole steps of the four warps
     const int k0 = sp * per, k1 = min(n_keys, k0 + per);
     const size_t row_elems = (size_t)a.n_kv * HD;
-    const __nv_bfloat16* kc0 = (const __nv_bfloat16*)a.k_cache + (size_t)kvh * HD;
-    const __nv_bfloat16* vc0 = (const __nv_bfloat16*)a.v_cache + (size_t)kvh * HD;
+    const __nv_bfloat16* kc = (const __nv_bfloat16*)a.k_cache + (size_t)kvh * HD;
+    const __nv_bfloat16* vc = (const __nv_bfloat16*)a.v_cache + (size_t)kvh * HD;
     const float scale = 1.0f / sqrtf((float)HD);
-    for (int i = tid; i < GM * HD; i += 128) {
-        const int g = i / HD, e = i - g * HD;
-        s_q[g][e] = g < G ? a.q_rot[(size_t)m * a.n_q * HD + ((size_t)kvh * G + g) * HD + e] : 0.0f;
-    }
-    __syncthreads();
-    float o[GM][DPL], mx[GM], l[GM];
+    const uint32_t ring = smem_u32(ar_sm) + (uint32_t)warp * (NS * kStage);
+    const int j_first = k0 + warp * kArTile;
+    const int n_it = j_first < k1 ? (k1 - j_first + 63) / 64 : 0;
+
+    auto load = [&](int i) {
+        if (i < n_it) {
+            const int j0 = j_first + 64 * i;
+            // the tile's 16 keys start on a multiple of 16: one sequence slot or one page holds them all
+            const size_t base = kv_phys_row(a.pg, seq, a.max_seq, j0);
+            const uint32_t dst = ring + (uint32_t)(i % NS) * kStage;
 #pragma unroll
-    for (int g = 0; g < GM; g++) {
-        mx[g] = -INFINITY; l[g] = 0.0f;
+            for (int x = 0; x < kArTile * CH / 32; x++) {
+                const int r = (x * 32 + lane) / CH, c = (x * 32 + lane) % CH;
+                const bool in = j0 + r < k1;                          // rows past the end read as zeros
+                const size_t off = (base + (in ? r : 0)) * row_elems + c * 8;
+                const uint32_t d = dst + (uint32_t)(r * HD * 2 + ((c ^ (r & 7)) << 4));
+                ar_cp16(d, kc + off, in ? 16u : 0u);
+                ar_cp16(d + kSide, vc + off, in ? 16u : 0u);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
 #pragma unroll
-        for (int i = 0; i < DPL; i++) o[g][i] = 0.0f;
+    for (int i = 0; i < NS - 1; i++) load(i);
+
+    uint32_t qa[MT][KS][4];
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++) {
+        const int h = mt * 4 + (g & 3);
+        const float* q = a.q_rot + (size_t)m * a.n_q * HD + ((size_t)kvh * G + h) * HD + 2 * t;
+#pragma unroll
+        for (int ks = 0; ks < KS; ks++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const float2 v = h < G ? *(const float2*)(q + ks * 16 + e * 8) : make_float2(0.0f, 0.0f);
+                attn_terms(v.x, v.y, second, &qa[mt][ks][2 * e], &qa[mt][ks][2 * e + 1]);
+            }
     }
+    float o[MT][NT][4], mx[MT], l[MT];
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++) {
+        mx[mt] = -INFINITY; l[mt] = 0.0f;
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) o[mt][n][e] = 0.0f;
+    }
+    const int kkey = ((lane >> 4) << 3) + (lane & 7), kch = (lane >> 3) & 1;       // this lane's row and 16-byte group in a ldmatrix of K ...
+    const int vkey = (((lane >> 3) & 1) << 3) + (lane & 7), vch = lane >> 4;        // ... and of V
 #pragma unroll 1
-    for (int j0 = k0 + warp * 32; j0 < k1; j0 += NW * 32) {
-        const int j = j0 + lane;
-        const bool live = j < k1;
-        // the tile's 32 keys start on a multiple of 32: one sequence slot or one page holds them all
-        const size_t tile_off = (kv_phys_row(a.pg, seq, a.max_seq, j0) - (size_t)j0) * row_elems;
-        const __nv_bfloat16* kc = kc0 + tile_off;
-        const __nv_bfloat16* vc = vc0 + tile_off;
-        // ---- scores of this lane's key
-        float sc[GM];
-#pragma unroll
-        for (int g = 0; g < GM; g++) sc[g] = 0.0f;
-        const uint4* krow = (const uint4*)(kc + (size_t)(live ? j : k0) * row_elems);
-#pragma unroll 4
-        for (int c = 0; c < HD / 8; c++) {
-            const uint4 raw = krow[c];
-            const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-            float kf[8];
-#pragma unroll
-            for (int t = 0; t < 4; t++) { kf[2 * t] = __uint_as_float(w[t] << 16); kf[2 * t + 1] = __uint_as_float(w[t] & 0xffff0000u); }
-#pragma unroll
-            for (int g = 0; g < GM; g++) {
-                const float4 q0 = *(const float4*)&s_q[g][c * 8], q1 = *(const float4*)&s_q[g][c * 8 + 4];
-                sc[g] = fmaf(q0.x, kf[0], sc[g]); sc[g] = fmaf(q0.y, kf[1], sc[g]); sc[g] = fmaf(q0.z, kf[2], sc[g]); sc[g] = fmaf(q0.w, kf[3], sc[g]);
-                sc[g] = fmaf(q1.x, kf[4], sc[g]); sc[g] = fmaf(q1.y, kf[5], sc[g]); sc[g] = fmaf(q1.z, kf[6], sc[g]); sc[g] = fmaf(q1.w, kf[7], sc[g]);
-            }
-        }
-        // ---- softmax bookkeeping per query head; weights to shared memory
-        float corr[GM];
-#pragma unroll
-        for (int g = 0; g < GM; g++) {
-            const float logit = live ? sc[g] * scale : -INFINITY;
-            float tm = logit;
-#pragma unroll
-            for (int of = 16; of > 0; of >>= 1) tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, of));
-            const float mn = fmaxf(mx[g], tm);                       // finite: a tile always holds at least one live key
-            corr[g] = (mx[g] == -INFINITY) ? 0.0f : expf(mx[g] - mn);
-            const float p = live ? expf(logit - mn) : 0.0f;
-            l[g] = l[g] * corr[g] + p;                               // per-lane partial sums, folded at the end
-            mx[g] = mn;
-            s_p[warp][g][lane] = p;
-        }
+    for (int i = 0; i < n_it; i++) {
+        load(i + NS - 1);
+        asm volatile("cp.async.wait_group %0;" ::"n"(NS - 1) : "memory");
         __syncwarp();
-        // ---- weighted values: lane = DPL head dimensions
+        const uint32_t kb = ring + (uint32_t)(i % NS) * kStage, vb = kb + kSide;
+        float s[MT][2][4];
 #pragma unroll
-        for (int g = 0; g < GM; g++)
+        for (int mt = 0; mt < MT; mt++)
 #pragma unroll
-            for (int i = 0; i < DPL; i++) o[g][i] *= corr[g];
-        const int nk = min(32, k1 - j0);
-#pragma unroll 4
-        for (int t = 0; t < nk; t++) {
-            const __nv_bfloat16* vrow = vc + (size_t)(j0 + t) * row_elems + lane * DPL;
-            float vf[DPL];
-            if (DPL == 4) {
-                const uint2 raw = *(const uint2*)vrow;
-                vf[0] = __uint_as_float(raw.x << 16); vf[1] = __uint_as_float(raw.x & 0xffff0000u);
-                vf[2 % DPL] = __uint_as_float(raw.y << 16); vf[3 % DPL] = __uint_as_float(raw.y & 0xffff0000u);
-            } else {
-                const uint32_t raw = *(const uint32_t*)vrow;
-                vf[0] = __uint_as_float(raw << 16); vf[1] = __uint_as_float(raw & 0xffff0000u);
+            for (int e = 0; e < 4; e++) s[mt][0][e] = s[mt][1][e] = 0.0f;
+#pragma unroll
+        for (int ks = 0; ks < KS; ks++) {
+            uint32_t b[4];
+            ar_ldsm4(kb + (uint32_t)(kkey * HD * 2 + (((ks * 2 + kch) ^ (kkey & 7)) << 4)), b);
+#pragma unroll
+            for (int mt = 0; mt < MT; mt++) { attn_mma(s[mt][0], qa[mt][ks], b[0], b[1]); attn_mma(s[mt][1], qa[mt][ks], b[2], b[3]); }
+        }
+        const int j = j_first + 64 * i + 2 * t;                       // this thread's keys: j, j + 1, j + 8, j + 9
+        uint32_t pa[MT][4];
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++) {
+            float v[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                float x = s[mt][e >> 1][e & 1] + s[mt][e >> 1][2 + (e & 1)];       // rows g and g + 8
+                x += __shfl_xor_sync(0xffffffffu, x, 16);                          // and the second terms' row
+                v[e] = j + (e >> 1) * 8 + (e & 1) < k1 ? x * scale : -INFINITY;
             }
+            float tm = fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3]));
+            tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 1));
+            tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 2));
+            const float mn = fmaxf(mx[mt], tm);                       // a tile always holds at least one live key
+            const float corr = mx[mt] == -INFINITY ? 0.0f : expf(mx[mt] - mn);
+            mx[mt] = mn;
+            float ps = 0.0f;
 #pragma unroll
-            for (int g = 0; g < GM; g++) {
-                const float p = s_p[warp][g][t];
+            for (int e = 0; e < 4; e++) { v[e] = v[e] == -INFINITY ? 0.0f : expf(v[e] - mn); ps += v[e]; }
+            l[mt] = l[mt] * corr + ps;                                // per-lane partial sums, folded at the end
+            attn_terms(v[0], v[1], second, &pa[mt][0], &pa[mt][1]);
+            attn_terms(v[2], v[3], second, &pa[mt][2], &pa[mt][3]);
+            if (__any_sync(0xffffffffu, corr != 1.0f)) {
 #pragma unroll
-                for (int i = 0; i < DPL; i++) o[g][i] = fmaf(p, vf[i], o[g][i]);
+                for (int n = 0; n < NT; n++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) o[mt][n][e] *= corr;
             }
+        }
+#pragma unroll
+        for (int np = 0; np < NT / 2; np++) {
+            uint32_t b[4];
+            ar_ldsm4_t(vb + (uint32_t)(vkey * HD * 2 + (((np * 2 + vch) ^ (vkey & 7)) << 4)), b);
+#pragma unroll
+            for (int mt = 0; mt < MT; mt++) { attn_mma(o[mt][2 * np], pa[mt], b[0], b[1]); attn_mma(o[mt][2 * np + 1], pa[mt], b[2], b[3]); }
         }
         __syncwarp();
     }
-    // ---- fold the lanes' sums, then the warps
+    // ---- add up the terms' rows and the lanes' sums, then the warps
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    float* s_o = (float*)ar_sm;                    // [NW][GM][HD]
+    float* s_f = s_o + NW * GM * HD;               // [GM][HD]: this CTA's split
+    float* s_m = s_f + GM * HD;                    // [NW][GM]
+    float* s_l = s_m + NW * GM;                    // [NW][GM]
+    float* s_fm = s_l + NW * GM;                   // [GM]
+    float* s_fl = s_fm + GM;                       // [GM]
 #pragma unroll
-    for (int g = 0; g < GM; g++) {
-        float lt = l[g];
+    for (int mt = 0; mt < MT; mt++) {
+        const int h = mt * 4 + (g & 3);
+        float lt = l[mt];
+        lt += __shfl_xor_sync(0xffffffffu, lt, 1);
+        lt += __shfl_xor_sync(0xffffffffu, lt, 2);
+        if (t == 0 && !second) { s_m[warp * GM + h] = mx[mt]; s_l[warp * GM + h] = lt; }
 #pragma unroll
-        for (int of = 16; of > 0; of >>= 1) lt += __shfl_xor_sync(0xffffffffu, lt, of);
-        if (lane == 0) { s_m[warp][g] = mx[g]; s_l[warp][g] = lt; }
-#pragma unroll
-        for (int i = 0; i < DPL; i++) s_o[warp][g][lane * DPL + i] = o[g][i];
+        for (int n = 0; n < NT; n++) {
+            float x0 = o[mt][n][0] + o[mt][n][2], x1 = o[mt][n][1] + o[mt][n][3];
+            x0 += __shfl_xor_sync(0xffffffffu, x0, 16);
+            x1 += __shfl_xor_sync(0xffffffffu, x1, 16);
+            if (!second) *(float2*)(s_o + (warp * GM + h) * HD + n * 8 + 2 * t) = make_float2(x0, x1);
+        }
     }
     __syncthreads();
+    float* out = a.out + ((size_t)m * a.n_q + (size_t)kvh * G) * HD;
     for (int idx = tid; idx < G * HD; idx += 128) {
-        const int g = idx / HD, e = idx - g * HD;
+        const int h = idx / HD;
         float M = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < NW; w++) M = fmaxf(M, s_m[w][g]);
+        for (int w = 0; w < NW; w++) M = fmaxf(M, s_m[w * GM + h]);
         float L = 0.0f, O = 0.0f;
 #pragma unroll
         for (int w = 0; w < NW; w++) {
-            const float c = (s_m[w][g] == -INFINITY) ? 0.0f : expf(s_m[w][g] - M);
-            L = fmaf(s_l[w][g], c, L);
-            O = fmaf(s_o[w][g][e], c, O);
+            const float c = s_m[w * GM + h] == -INFINITY ? 0.0f : expf(s_m[w * GM + h] - M);
+            L = fmaf(s_l[w * GM + h], c, L);
+            O = fmaf(s_o[w * GM * HD + idx], c, O);
         }
-        const size_t head = (size_t)m * a.n_q + (size_t)kvh * G + g;
-        if (n_splits == 1) {
-            a.out[head * HD + e] = O * (1.0f / L);
-        } else {
-            float* pp = a.part + (head * n_splits + sp) * (HD + 2);
-            pp[e] = O;
-            if (e == 0) { pp[HD] = M; pp[HD + 1] = L; }                // a split without keys leaves M = -inf, L = 0
+        if (n_splits == 1) out[idx] = O * (1.0f / L);
+        else {
+            s_f[idx] = O;
+            if (idx % HD == 0) { s_fm[h] = M; s_fl[h] = L; }            // a split without keys leaves M = -inf, L = 0
         }
     }
-}
-
-template <int HD>
-__global__ void __launch_bounds__(HD) attn_rows_merge(const AttnRowsArgs a, int n_splits) {
-    const int head = blockIdx.x, m = blockIdx.y, e = threadIdx.x;
-    const int pos = a.row_pos[m];
-    const int seq = a.row_seq ? a.row_seq[m] : a.seq0;
-    if (pos < 0 || pos >= a.max_seq || seq < 0 || seq >= a.max_batch) return;
-    const float* pp = a.part + (((size_t)m * a.n_q + head) * n_splits) * (HD + 2);
-    float M = -INFINITY;
-    for (int s = 0; s < n_splits; s++) M = fmaxf(M, pp[(size_t)s * (HD + 2) + HD]);
-    float L = 0.0f, O = 0.0f;
-    for (int s = 0; s < n_splits; s++) {
-        const float ms = pp[(size_t)s * (HD + 2) + HD];
-        const float c = (ms == -INFINITY) ? 0.0f : expf(ms - M);
-        L = fmaf(pp[(size_t)s * (HD + 2) + HD + 1], c, L);
-        O = fmaf(pp[(size_t)s * (HD + 2) + e], c, O);
+    if (n_splits == 1) return;
+    cluster_arrive_release();
+    cluster_wait_acquire();
+    for (int idx = sp * 128 + tid; idx < G * HD; idx += n_splits * 128) {
+        const int h = idx / HD;
+        float M = -INFINITY;
+        for (int r = 0; r < n_splits; r++) M = fmaxf(M, cluster_ld_f32(cluster_map(smem_u32(s_fm + h), (uint32_t)r)));
+        float L = 0.0f, O = 0.0f;
+        for (int r = 0; r < n_splits; r++) {
+            const float ms = cluster_ld_f32(cluster_map(smem_u32(s_fm + h), (uint32_t)r));
+            const float c = ms == -INFINITY ? 0.0f : expf(ms - M);
+            L = fmaf(cluster_ld_f32(cluster_map(smem_u32(s_fl + h), (uint32_t)r)), c, L);
+            O = fmaf(cluster_ld_f32(cluster_map(smem_u32(s_f + idx), (uint32_t)r)), c, O);
+        }
+        out[idx] = O * (1.0f / L);
     }
-    a.out[((size_t)m * a.n_q + head) * HD + e] = O * (1.0f / L);
+    cluster_arrive_release();                       // nobody leaves while another CTA may still read its shared memory
+    cluster_wait_acquire();
 }
-
-size_t attn_rows_part_floats(int rows, int n_q, int hd) { return (size_t)rows * n_q * kAttnRowsMaxSplits * (hd + 2); }
 
 // ---------------------------------------------------------------------------------------------------- greedy sample per row
 // One CTA per row: logits[m][:] = sum of the vocabulary projection's partial planes (written back to plane 0), the greedy
@@ -440,21 +490,34 @@ cudaError_t launch_attn_rows(const AttnRowsArgs& a, cudaStream_t st) {
     static const int env_split = [] { const char* e = getenv("LUM_ATTN_ROWS_SPLIT"); return e ? atoi(e) : 1; }();
     if (env_split && a.kv_bf16 && a.window == 0 && (a.hd == 128 || a.hd == 64) && G >= 1 && G <= 8 && (((uintptr_t)a.k_cache | (uintptr_t)a.v_cache) & 15) == 0 &&
         ((size_t)a.n_kv * a.hd * 2) % 16 == 0) {
-        // enough CTAs for a few waves over the SMs; a split is at least 64 keys long only when the context is (the kernel handles empty splits)
+        const void* fn = a.hd == 128 ? (G <= 4 ? (const void*)attn_rows_split<128, 1> : (const void*)attn_rows_split<128, 2>)
+                                     : (G <= 4 ? (const void*)attn_rows_split<64, 1> : (const void*)attn_rows_split<64, 2>);
+        const size_t smem = (size_t)ar_smem(a.hd);
+        if (smem > 48 * 1024) {
+            cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return e;
+        }
+        // Splits per (KV head, row): rounds of resident CTAs (three per SM) times the keys of one, plus what a CTA costs beside its keys —
+        // about the time of 100 of them.  The positions are on the device, so a context of middling length (1024 keys) stands for all.
+        const long long pairs = (long long)a.n_kv * a.M, slots = 3 * 148;
         int splits = 1;
-        if (a.part && a.M <= a.part_rows) {
-            splits = (4 * 148 + a.n_kv * a.M - 1) / (a.n_kv * a.M);
-            if (splits > kAttnRowsMaxSplits) splits = kAttnRowsMaxSplits;
-            if (splits < 1) splits = 1;
+        for (int s = 2; s <= kAttnRowsMaxSplits; s++) {
+            auto cost = [&](int n) { return (double)((pairs * n + slots - 1) / slots) * (1024.0 / n + 100.0); };
+            if (cost(s) < cost(splits)) splits = s;
         }
         AttnRowsArgs b = a;
         void* params[] = {&b, &splits};
-        const void* fn = a.hd == 128 ? (G <= 4 ? (const void*)attn_rows_split<128, 4> : (const void*)attn_rows_split<128, 8>)
-                                     : (G <= 4 ? (const void*)attn_rows_split<64, 4> : (const void*)attn_rows_split<64, 8>);
-        cudaError_t e = cudaLaunchKernel(fn, dim3(a.n_kv, a.M, splits), dim3(128), params, 0, st);
-        if (e != cudaSuccess || splits == 1) return e;
-        const void* fm = a.hd == 128 ? (const void*)attn_rows_merge<128> : (const void*)attn_rows_merge<64>;
-        return cudaLaunchKernel(fm, dim3(a.n_q, a.M), dim3(a.hd), params, 0, st);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(a.n_kv, a.M, splits);
+        cfg.blockDim = dim3(128);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = (unsigned)splits;
+        cfg.attrs = at;
+        cfg.numAttrs = splits > 1 ? 1 : 0;
+        return cudaLaunchKernelExC(&cfg, fn, params);
     }
     const void* fn = nullptr;
     const bool bf = a.kv_bf16 != 0;
