@@ -78,98 +78,118 @@ __device__ __forceinline__ float block_max(float v, float* scratch, int tid, int
 
 // activation operand: [chunk][K / 32 slices][4 groups of 8 columns][kGmXTerms terms][chunk rows][16 bytes]: within a column group the
 // rows of the first term are followed by the rows of the second, so ONE operand descriptor of 2 x chunk rows covers both terms
-__global__ void __launch_bounds__(256) rows_quantize(const RowsArgs a) {
-    extern __shared__ __align__(16) float rowbuf[];          // K floats + 8 words of reduction scratch
-    const int m = blockIdx.x, tid = threadIdx.x;
+//
+// A cluster of C CTAs forms one row, each K / C of its columns (whole 32-column slices); the sum of squares and the largest magnitude go
+// round through distributed shared memory.  With few rows this kernel is bound by its chain of trips to L2 and by how many loads are
+// on their way, so a row is spread over as many SMs as there are.  Measured (32 rows, the four of a Llama-3-8B layer, K 4096 and
+// 14336): 70 us a layer with one CTA per row, 31 us with eight.
+constexpr int kRqMaxCluster = 8;
+__global__ void __launch_bounds__(256) rows_quantize(const RowsArgs a, const int C) {
+    extern __shared__ __align__(16) float rowbuf[];          // this CTA's columns
+    __shared__ float scratch[8], s_x[2];
+    const int m = blockIdx.x / C, part = blockIdx.x - m * C, tid = threadIdx.x;
     const int K = a.K, nb = K >> 5;
-    float* scratch = rowbuf + K;
+    const int s0 = (int)((long long)nb * part / C), s1 = (int)((long long)nb * (part + 1) / C);     // this CTA's slices
+    const int k0 = s0 << 5, n4 = (s1 - s0) << 3;             // its first column, its float4
     if (a.use_pdl) { pdl_launch_dependents(); pdl_grid_wait(); }
     const int nc = gemm_chunk_rows(a.M);
     const size_t slice_bytes = (size_t)kGmXTerms * 4 * nc * 16;
     unsigned char* xq_chunk = (unsigned char*)a.xq + (size_t)(m / nc) * nb * slice_bytes;
     const int ml = m % nc;
     if (m >= a.M) {
-        // padding row of the last chunk: zeros
-        for (int ch = tid; ch < nb * kGmXTerms * 4; ch += 256) {
+        // padding row of the last chunk: zeros (the whole cluster returns)
+        for (int ch = s0 * kGmXTerms * 4 + tid; ch < s1 * kGmXTerms * 4; ch += 256) {
             const int s = ch / (kGmXTerms * 4), tc = ch - s * (kGmXTerms * 4);           // (column group, term) of slice s
             *(uint4*)(xq_chunk + (size_t)s * slice_bytes + (size_t)tc * nc * 16 + ml * 16) = make_uint4(0u, 0u, 0u, 0u);
         }
-        if (tid == 0) a.sx[m] = 0.0f;
+        if (tid == 0 && part == 0) a.sx[m] = 0.0f;
         return;
     }
     float ss = 0.0f;
-    for (int f4 = tid; f4 < (K >> 2); f4 += 256) {
+    for (int f4 = tid; f4 < n4; f4 += 256) {
+        const size_t at = (size_t)m * a.ld + k0 + f4 * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f), u = v;
+#pragma unroll 4
         for (int p = 0; p < a.n_parts; p++) {
-            const float4 t = __ldcg((const float4*)(a.a + p * a.part_stride + (size_t)m * a.ld) + f4);
+            const float4 t = __ldcg((const float4*)(a.a + p * a.part_stride + at));
             v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
             if (a.b) {
-                const float4 s = __ldcg((const float4*)(a.b + p * a.part_stride + (size_t)m * a.ld) + f4);
+                const float4 s = __ldcg((const float4*)(a.b + p * a.part_stride + at));
                 u.x += s.x; u.y += s.y; u.z += s.z; u.w += s.w;
             }
         }
         if (a.b) { v.x = swiglu(v.x, u.x); v.y = swiglu(v.y, u.y); v.z = swiglu(v.z, u.z); v.w = swiglu(v.w, u.w); }
         if (a.resid) {
-            const float4 r = __ldcg((const float4*)(a.resid + (size_t)m * a.resid_ld) + f4);
+            const float4 r = __ldcg((const float4*)(a.resid + (size_t)m * a.resid_ld + k0) + f4);
             v.x = r.x + v.x; v.y = r.y + v.y; v.z = r.z + v.z; v.w = r.w + v.w;
         }
-        if (a.out) ((float4*)(a.out + (size_t)m * a.out_ld))[f4] = v;
+        if (a.out) ((float4*)(a.out + (size_t)m * a.out_ld + k0))[f4] = v;
         ((float4*)rowbuf)[f4] = v;
         ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss); ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
     }
+    // one number per CTA -> the cluster's, combined in the order of its CTAs
+    auto exchange = [&](float v, int slot, bool maximum) -> float {
+        if (C == 1) return v;
+        if (tid == 0) s_x[slot] = v;
+        cluster_arrive_release();
+        cluster_wait_acquire();
+        float t = cluster_ld_f32(cluster_map(smem_u32(&s_x[slot]), 0u));
+        for (int r = 1; r < C; r++) {
+            const float x = cluster_ld_f32(cluster_map(smem_u32(&s_x[slot]), (uint32_t)r));
+            t = maximum ? fmaxf(t, x) : t + x;
+        }
+        return t;
+    };
     float inv = 1.0f;
     if (a.gain) {
-        ss = block_sum(ss, scratch, tid, 256, 1);
+        ss = exchange(block_sum(ss, scratch, tid, 256, 1), 0, false);
         inv = 1.0f / sqrtf(ss * (1.0f / (float)K) + a.eps);
     } else {
         __syncthreads();
     }
     // the normalised row, and its largest magnitude
     float amax = 0.0f;
-    for (int f4 = tid; f4 < (K >> 2); f4 += 256) {          // each thread revisits the elements it wrote
+    for (int f4 = tid; f4 < n4; f4 += 256) {                // each thread revisits the elements it wrote
         float4 v = ((const float4*)rowbuf)[f4];
         if (a.gain) {
-            v.x = (inv * v.x) * load_gain(a.gain, a.gain_kind, f4 * 4);
-            v.y = (inv * v.y) * load_gain(a.gain, a.gain_kind, f4 * 4 + 1);
-            v.z = (inv * v.z) * load_gain(a.gain, a.gain_kind, f4 * 4 + 2);
-            v.w = (inv * v.w) * load_gain(a.gain, a.gain_kind, f4 * 4 + 3);
+            v.x = (inv * v.x) * load_gain(a.gain, a.gain_kind, k0 + f4 * 4);
+            v.y = (inv * v.y) * load_gain(a.gain, a.gain_kind, k0 + f4 * 4 + 1);
+            v.z = (inv * v.z) * load_gain(a.gain, a.gain_kind, k0 + f4 * 4 + 2);
+            v.w = (inv * v.w) * load_gain(a.gain, a.gain_kind, k0 + f4 * 4 + 3);
             ((float4*)rowbuf)[f4] = v;
         }
         amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
     }
-    amax = block_max(amax, scratch, tid, 256, 1);           // (its barriers also publish the row to the other threads)
+    amax = exchange(block_max(amax, scratch, tid, 256, 1), 1, true);       // (its barriers also publish the row to the other threads)
+    if (C > 1) cluster_arrive_release();                    // waited for at the end: nobody leaves while its s_x may still be read
     // power of two that puts the maximum in [2^13, 2^14); a zero (or non-finite) row keeps factor 1
     int ex = 0;
     if (amax > 0.0f && amax < INFINITY) frexpf(amax, &ex);
     else ex = 14;
     const float up = ldexpf(1.0f, 14 - ex);
-    if (tid == 0) a.sx[m] = ldexpf(1.0f, ex - 14 - kGmWExp);       // undoes this factor and the weights' 2^10
-    for (int c8 = tid; c8 < (K >> 3); c8 += 256) {
+    if (tid == 0 && part == 0) a.sx[m] = ldexpf(1.0f, ex - 14 - kGmWExp);       // undoes this factor and the weights' 2^10
+    for (int c8 = tid; c8 < (n4 >> 1); c8 += 256) {
         const float4 v0 = ((const float4*)rowbuf)[2 * c8], v1 = ((const float4*)rowbuf)[2 * c8 + 1];
         const float e[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-        uint32_t t1[4], t2[4], t3[4];
+        uint32_t t1[4], t2[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            __half h[2][3];
+            __half h[2][2];
 #pragma unroll
             for (int q = 0; q < 2; q++) {
                 const float x = e[2 * j + q] * up;                       // exact: a power of two
                 h[q][0] = __float2half_rn(x);
-                const float r1 = x - __half2float(h[q][0]);              // exact in f32
-                h[q][1] = __float2half_rn(r1);
-                const float r2 = r1 - __half2float(h[q][1]);
-                h[q][2] = __float2half_rn(r2);
+                h[q][1] = __float2half_rn(x - __half2float(h[q][0]));   // (the difference is exact in f32)
             }
             t1[j] = (uint32_t)__half_as_ushort(h[0][0]) | ((uint32_t)__half_as_ushort(h[1][0]) << 16);
             t2[j] = (uint32_t)__half_as_ushort(h[0][1]) | ((uint32_t)__half_as_ushort(h[1][1]) << 16);
-            t3[j] = (uint32_t)__half_as_ushort(h[0][2]) | ((uint32_t)__half_as_ushort(h[1][2]) << 16);
         }
-        const int s = c8 >> 2, cg = c8 & 3;
+        const int s = s0 + (c8 >> 2), cg = c8 & 3;
         unsigned char* dst = xq_chunk + (size_t)s * slice_bytes + (size_t)cg * kGmXTerms * nc * 16 + ml * 16;
         *(uint4*)(dst) = make_uint4(t1[0], t1[1], t1[2], t1[3]);
         *(uint4*)(dst + (size_t)nc * 16) = make_uint4(t2[0], t2[1], t2[2], t2[3]);
-        if (kGmXTerms > 2) *(uint4*)(dst + (size_t)2 * nc * 16) = make_uint4(t3[0], t3[1], t3[2], t3[3]);
     }
+    if (C > 1) cluster_wait_acquire();
 }
 
 struct GemmItem { int seg, rg0, n_rg, mc, t0, t1, ks; };
@@ -255,7 +275,9 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
     tc_fence_after_sync();
     uint32_t tmem;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
-    if (a.use_pdl) { pdl_launch_dependents(); pdl_grid_wait(); }     // the activation operand comes from the previous kernel
+    // The weights do not depend on the previous kernel: they are on their way while it still runs.  Its results are waited for where they
+    // are read (activation copies, row factors) or where what it may still read is overwritten (the sums).
+    if (a.use_pdl) pdl_launch_dependents();
 
     const int tpr = a.K / kTileK, nb = a.K >> 5;
     const int nc = a.nc;                                   // activation rows per chunk
@@ -273,6 +295,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
         if (elect_one()) {
             uint32_t xi = 0;
             bool ok = true;
+            if (a.use_pdl) pdl_grid_wait();
             for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
                 const GemmItem it = gemm_item(a, item, tpr);
                 for (int t = it.t0; t < it.t1 && ok; t++) {
@@ -436,6 +459,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
             if (!ok) break;
             // ---- the item's K range is done: store the accumulators (lane = weight row, columns = activation rows)
             if (!mbar_wait_abortable(afull, ic & 1u, abort)) { fail(LUM_ST_WAIT_TMEM); ok = false; break; }
+            if (a.use_pdl) pdl_grid_wait();              // (long over: the sums are there)
             tc_fence_after_sync();
             const GemmSeg& sg = a.seg[it.seg];
             const int half_rows = nc >> 1;
@@ -524,7 +548,9 @@ __global__ void __launch_bounds__(kGsThreads, 1) q8_gemm_tc_staged(const GemmArg
     tc_fence_after_sync();
     uint32_t tmem;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
-    if (a.use_pdl) { pdl_launch_dependents(); pdl_grid_wait(); }     // the activation operand comes from the previous kernel
+    // The weights do not depend on the previous kernel: they are on their way while it still runs.  Its results are waited for where they
+    // are read (activation copies, row factors) or where what it may still read is overwritten (the sums).
+    if (a.use_pdl) pdl_launch_dependents();
 
     const int tpr = a.K / kTileK, nb = a.K >> 5;
     const int nc = a.nc;                                   // activation rows per chunk
@@ -574,6 +600,7 @@ __global__ void __launch_bounds__(kGsThreads, 1) q8_gemm_tc_staged(const GemmArg
         if (elect_one()) {
             uint32_t xi = 0;
             bool ok = true;
+            if (a.use_pdl) pdl_grid_wait();
             for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
                 const GemmItem it = gemm_item(a, item, tpr, kGsRows);
                 for (int t = it.t0; t < it.t1 && ok; t++) {
@@ -714,6 +741,7 @@ __global__ void __launch_bounds__(kGsThreads, 1) q8_gemm_tc_staged(const GemmArg
             if (!ok) break;
             // ---- the item's K range is done: store the accumulator (lane = weight row, columns = activation rows)
             if (!mbar_wait_abortable(afull, ic & 1u, abort)) { fail(LUM_ST_WAIT_TMEM); ok = false; break; }
+            if (a.use_pdl) pdl_grid_wait();              // (long over: the sums are there)
             tc_fence_after_sync();
             const GemmSeg& sg = a.seg[it.seg];
             const int half_rows = nc >> 1;
@@ -777,7 +805,13 @@ int gemm_pick_ksplit(int n_rows_total, int M, int K, int sm_count) {
 cudaError_t launch_rows_quantize(const RowsArgs& a_in, cudaStream_t st) {
     RowsArgs a = a_in;
     if (a.M <= 0 || a.K <= 0 || (a.K % 32) || a.n_parts < 1) return cudaErrorInvalidValue;
-    const size_t smem = (size_t)a.K * 4 + 64;
+    const int nc = gemm_chunk_rows(a.M);
+    const int rows = (a.M + nc - 1) / nc * nc;            // padding rows of the last chunk are zeroed by their own CTAs
+    // CTAs per row: up to eight while the rows alone leave SMs idle, of at least eight slices each
+    int C = 1;
+    while (C < kRqMaxCluster && rows * C * 2 <= 4 * 148 && (a.K >> 5) / (C * 2) >= 8) C *= 2;
+    const size_t smem = (size_t)(((a.K >> 5) + C - 1) / C) * 128;
+    if (smem > 200 * 1024) return cudaErrorInvalidValue;
     if (smem > 48 * 1024) {
         static bool set = false;
         if (!set) {
@@ -785,20 +819,27 @@ cudaError_t launch_rows_quantize(const RowsArgs& a_in, cudaStream_t st) {
             if (e != cudaSuccess) return e;
             set = true;
         }
-        if (smem > 200 * 1024) return cudaErrorInvalidValue;
     }
-    const int nc = gemm_chunk_rows(a.M);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((a.M + nc - 1) / nc * nc);      // padding rows of the last chunk are zeroed by their own CTAs
+    cfg.gridDim = dim3(rows * C);
     cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2];
+    int n_at = 0;
+    if (C > 1) {
+        at[n_at].id = cudaLaunchAttributeClusterDimension;
+        at[n_at].val.clusterDim.x = (unsigned)C; at[n_at].val.clusterDim.y = 1; at[n_at].val.clusterDim.z = 1;
+        n_at++;
+    }
+    if (a.use_pdl) {
+        at[n_at].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n_at].val.programmaticStreamSerializationAllowed = 1;
+        n_at++;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = a.use_pdl ? 1 : 0;
-    void* params[] = {&a};
+    cfg.numAttrs = n_at;
+    void* params[] = {&a, &C};
     return cudaLaunchKernelExC(&cfg, (const void*)rows_quantize, params);
 }
 

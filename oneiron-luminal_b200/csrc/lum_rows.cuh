@@ -52,6 +52,7 @@ struct RopeRowsArgs {
     int M, n_q, n_kv, hd, kv_bf16, rope_style, max_seq, max_batch;
     float c_inv_d, c_ln_theta, c_log2e, c_half_pi, theta;
     uint32_t* status;
+    int use_pdl;
 };
 struct AttnRowsArgs {
     const float* q_rot;        // [M][n_q * hd]
@@ -61,6 +62,7 @@ struct AttnRowsArgs {
     float* out;                // [M][n_q * hd]
     int M, n_q, n_kv, hd, kv_bf16, window, max_seq, max_batch;
     uint32_t* status;
+    int use_pdl;
 };
 struct ArgmaxRowsArgs {
     float* logits;             // [n_parts][M][vocab]; the sums end up in plane 0
@@ -69,6 +71,7 @@ struct ArgmaxRowsArgs {
     int* best;                 // optional [M]: the samples
     int* row_tok; int* row_pos;     // optional: batched decode state, advanced in place
     int* log; const int* step; int max_steps;   // optional: log[*step][m] = sample
+    int use_pdl;
 };
 
 size_t gemm_xq_bytes(int M, int K);

@@ -1203,7 +1203,7 @@ int batch_sample(lum_rt* rt, int M, int* d_tok, int* d_pos, const int* d_seq, in
     lum_rt::Rows& b = rt->rows;
     const int V = rt->vocab_l;
     ArgmaxRowsArgs x{};
-    x.logits = b.logits; x.n_parts = n_parts; x.part_stride = (size_t)M * V; x.M = M; x.vocab = V;
+    x.logits = b.logits; x.n_parts = n_parts; x.part_stride = (size_t)M * V; x.M = M; x.vocab = V; x.use_pdl = rt->cfg.use_pdl != 0;
     if (!rt->sampling) { x.row_tok = d_tok; x.row_pos = d_pos; x.log = rt->b_log; x.step = rt->b_step; x.max_steps = rt->d.max_new_tokens; }
     CU(rt, launch_argmax_rows(x, rt->stream));          // with a sampler set it only adds up the partial planes
     if (rt->sampling) {
@@ -1389,15 +1389,15 @@ int run_rows(lum_rt* rt, int M, int* d_tok, int* d_pos, const int* d_seq, int se
     const lum_model_desc& d = rt->d;
     lum_rt::Rows& b = rt->rows;
     const int H = d.hidden, hd = d.head_dim, qd = rt->nq_l * hd, kvd = rt->nkv_l * hd, W = qd + 2 * kvd, F = rt->ffn_l;
-    const int gk = kind_of(d.embed_dtype), sms = rt->sm_count;
+    const int gk = kind_of(d.embed_dtype), sms = rt->sm_count, pdl = rt->cfg.use_pdl != 0;
     cudaStream_t st = rt->stream;
     const int ks_qkv = gemm_pick_ksplit(W, M, H, sms), ks_o = gemm_pick_ksplit(H, M, qd, sms), ks_gu = gemm_pick_ksplit(2 * F, M, H, sms),
               ks_dn = gemm_pick_ksplit(H, M, F, sms);
     CU(rt, launch_embed_rows(rt->embed.w, rt->embed.kind, H, d.vocab, d_tok, b.xr, M, rt->status, st));
     uint64_t launches = 1;
-    auto quant = [&](RowsArgs& r, int K) -> cudaError_t { r.M = M; r.K = K; r.xq = b.xq; r.sx = b.sx; launches++; return launch_rows_quantize(r, st); };
+    auto quant = [&](RowsArgs& r, int K) -> cudaError_t { r.M = M; r.K = K; r.xq = b.xq; r.sx = b.sx; r.use_pdl = pdl; launches++; return launch_rows_quantize(r, st); };
     auto gemm = [&](GemmArgs& g, int K, int ks, float* y, int ldy) -> cudaError_t {
-        g.K = K; g.xq = b.xq; g.sx = b.sx; g.M = M; g.ksplit = ks; g.y = y; g.ldy = ldy; g.part_stride = (size_t)M * ldy; g.status = rt->status;
+        g.K = K; g.xq = b.xq; g.sx = b.sx; g.M = M; g.ksplit = ks; g.y = y; g.ldy = ldy; g.part_stride = (size_t)M * ldy; g.status = rt->status; g.use_pdl = pdl;
         launches++;
         return launch_gemm(g, sms, st);
     };
@@ -1424,12 +1424,12 @@ int run_rows(lum_rt* rt, int M, int* d_tok, int* d_pos, const int* d_seq, int se
             t.M = M; t.n_q = rt->nq_l; t.n_kv = rt->nkv_l; t.hd = hd; t.kv_bf16 = d.kv_dtype == LUM_BF16; t.rope_style = d.rope_style;
             t.max_seq = d.max_seq; t.max_batch = rt->max_batch;
             t.c_inv_d = rt->c_inv_d; t.c_ln_theta = rt->c_ln_theta; t.c_log2e = rt->c_log2e; t.c_half_pi = rt->c_half_pi; t.theta = d.rope_theta;
-            t.status = rt->status;
+            t.status = rt->status; t.use_pdl = pdl;
             CU(rt, launch_rope_append_rows(t, st));
             AttnRowsArgs a{};
             a.q_rot = b.q_rot; a.k_cache = w.kc; a.v_cache = w.vc; a.pg = kv_pages(rt); a.row_pos = d_pos; a.row_seq = d_seq; a.seq0 = seq0; a.out = b.attn;
             a.M = M; a.n_q = rt->nq_l; a.n_kv = rt->nkv_l; a.hd = hd; a.kv_bf16 = t.kv_bf16; a.window = 0; a.max_seq = d.max_seq; a.max_batch = rt->max_batch;
-            a.status = rt->status;
+            a.status = rt->status; a.use_pdl = pdl;
             // many rows of one sequence (a prompt): the tensor-core kernel; few rows, or rows of different sequences: one CTA per row
             static const int env_tc = [] { const char* e = getenv("LUM_ATTN_TC"); return e ? atoi(e) : 1; }();
             if (env_tc && M >= 16 && attn_prompt_tc_supported(a)) CU(rt, launch_attn_prompt_tc(a, st));
