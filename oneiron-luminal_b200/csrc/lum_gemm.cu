@@ -45,7 +45,7 @@ namespace lum {
 
 constexpr int kGmHB = 2;                            // tensor-core tiles (128 weight rows) per work item; they share every activation slice
 constexpr int kGmRows = 128 * kGmHB;                // weight rows per work item
-constexpr int kGmMaxChunk = 128;                    // activation rows per chunk: 32, 64 or 128 (gemm_chunk_rows)
+constexpr int kGmMaxChunk = 128;                    // activation rows per chunk: 16, 32, 64 or 128 (gemm_chunk_rows)
 constexpr int kGmXTerms = 2;                        // binary16 terms per activation element
 constexpr int kGmStep = 2;                          // 32-column slices per hand-over between the warps (every hand-over costs each single-threaded role
                                                     // several hundred cycles of its own, whatever the amount of work behind it)
@@ -63,7 +63,7 @@ constexpr uint32_t kGmTmemCols = 512;               // one accumulator of 128 co
 constexpr uint32_t kGmCvtCol0 = 128 * kGmHB;
 
 // activation rows per chunk for a product of M rows
-__host__ __device__ inline int gemm_chunk_rows(int M) { return M <= 32 ? 32 : M <= 64 ? 64 : 128; }
+__host__ __device__ inline int gemm_chunk_rows(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128; }
 
 __device__ __forceinline__ float block_max(float v, float* scratch, int tid, int nthreads, int bar_id) {
 #pragma unroll
@@ -493,49 +493,84 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
 }
 
 
-// ===== The kernel for fewer than 128 activation rows per chunk (batched decode) =====
-// Same arithmetic and roles, but the regime is the other one: the weights are the stream that matters (HBM-bound), so they are
-// staged through shared memory by bulk copies of whole 4352-byte tiles (contiguous 4 KiB reads: the 16-byte-per-row reads of the
-// kernel above cost a third of the HBM rate here — measured: vocabulary projection at 32 rows 422 against 324 us), work items are
-// 128 weight rows, and a hand-over covers four 32-column slices.
-constexpr int kGsHB = 1;                            // tensor-core tiles (128 weight rows) per work item; they share every activation slice
-constexpr int kGsRows = 128 * kGsHB;                // weight rows per work item
-constexpr int kGsRG = kGsRows / kTileRows;
-// A weight stage is a whole K-tile of the item's row groups: one bulk copy of 4352 bytes per row group.  (Measured: a bulk copy
-// costs the SM's copy engine about 50 ns whatever its size, so stages cut into halves or quarters of a K-tile — two small copies
-// per row group each — bound the kernel at 5 to 17 copies per 32-column slice; whole tiles are 2 copies per slice.)
-constexpr int kGsPartSlices = 16;                   // 32-column slices per weight stage
+// ===== The kernel for up to 64 activation rows (batched decode, short prompts) =====
+// Same arithmetic, but the regime is the other one: the weights are the stream that matters (HBM-bound), and everything else has to
+// keep up with 23 bytes of them per SM and clock, which is 187 clocks per 32-column slice of 128 weight rows.
+//   * Work items are runs of up to 32 row groups of 8 weight rows, over the concatenated matrices, times a range of K-tiles: the row groups
+//     are dealt out evenly (gemm_plan), so that all SMs finish together and few K ranges (planes of partial sums) are needed.  An item of
+//     more than 16 row groups is two tensor-core tiles that take turns on each K-tile and share its activation slices in shared memory.
+//   * Weights are staged by bulk copies of whole 4352-byte tiles, half an item's row groups of one K-tile per stage, two stages.
+//   * 16 warps convert: four per quarter of the tensor-memory lanes, each one slice of the four of a hand-over (two loads, 32 weights in
+//     registers, two stores of 16 columns).  With 8 warps of half a slice the loads' and stores' latencies were exposed.
+//   * Tensor core: per 16 columns of K two instructions, hi x [x1 | x2] of N = 2 nc (its two halves are added when the sums are stored) and
+//     lo x x1 of N = nc: 33 + 17 clocks at nc = 32.  lo x x1 joins the half of hi x x2, whose values are as small: every addition to an
+//     accumulator is cut to 24 bits, so the large half takes one per 16 columns and not two (whole-model error against 64 bits 3.8e-5
+//     with both in the large half).
+//   * Activations: a chunk is 16, 32 or 64 rows, whichever holds the step; a slice is 128 bytes per row, and with 32 rows a CTA reads as many
+//     bytes of them from L2 as of weights from HBM if it has one tensor-core tile, half as many if it has two.
+// Measured, alone, back to back over weights that L2 does not hold (us at 32 rows / 5 rows; before: q8_gemm_tc_layer_shapes of the profiles, a chunk
+// of 32 rows for both): qkv 6144 x 4096 39.5 -> 16.6 / 15.5, gate|up 28672 x 4096 111.3 -> 43.3 / 41.1, down 4096 x 14336 68.8 -> 26.8 / 22.7,
+// vocabulary 128256 x 4096 323.1 -> 152.7 / 139.5 (3.7 and 4.0 TB/s of weights).  What is left is latency: set-up and first copies, about 5 us
+// that a dependent launch hides, and hand-overs of about 800 clocks per four slices where the conversion's issue slots are 440.
+constexpr int kGsRG = 16;                           // row groups per tensor-core tile
 constexpr int kGsWRow = kTileBytes;                 // 4352: one tile, quants then scales, as streamed
-constexpr int kGsWStage = kGsRG * kGsWRow;          // 69632 per 128 weight rows
-constexpr int kGsStep = 2;                          // 32-column slices per hand-over at 64 / 128 rows per chunk (4 at 32: GemmArgs::step) between the warps (every hand-over costs each single-threaded role
-                                                    // several hundred cycles of its own, whatever the amount of work behind it)
-constexpr int kGsXStageMax = kGsStep * kGmXTerms * kGmMaxChunk * 32 * 2;   // 32768: the activation terms of one step of a 128-row chunk
-constexpr int kGsWStages = 2, kGsCvtBufs = 4, kGsXStages = 2;
-constexpr uint32_t kGsCvtCols1 = 32 * kGsHB;                 // tensor-memory columns of one converted slice: per 128-row tile hi (16: 32 binary16 per row) | lo (16)
-constexpr int kGsCvtWarps = 8;
+constexpr int kGsWStage = kGsRG * kGsWRow;          // 69632
+constexpr int kGsStep = 4;                          // 32-column slices per hand-over between the warps
+constexpr int kGsXStage = 16384;                    // one activation stage: 16384 / (128 nc) slices
+constexpr int kGsWStages = 2, kGsCvtBufs = 3, kGsXStages = 4;
+constexpr uint32_t kGsSliceCols = 32;               // tensor-memory columns of one converted slice: hi (16: 32 binary16 per row) | lo (16)
+constexpr uint32_t kGsCvtCols = kGsStep * kGsSliceCols;
+constexpr int kGsCvtWarps = 16;
 constexpr int kGsThreads = (kGsCvtWarps + 3) * 32;   // + activation producer warp + tensor-core warp + weight producer warp
-constexpr int kGsBarBytes = 512;
-constexpr size_t kGsSmem = kGsBarBytes + 128 + (size_t)kGsWStages * kGsWStage + (size_t)kGsXStages * kGsXStageMax;
-constexpr uint32_t kGsTmemCols = 512;               // one accumulator of up to 128 columns per 128-row tile, then the four converted-weight buffers
-constexpr uint32_t kGsCvtCol0 = 256;
+constexpr int kGsBarBytes = 256;
+constexpr double kGsCvtUs = 1.5;                    // measured: one K-tile (16 slices) of one tensor-core tile through the converting warps
+constexpr size_t kGsSmem = kGsBarBytes + 128 + (size_t)kGsWStages * kGsWStage + (size_t)kGsXStages * kGsXStage;
+constexpr uint32_t kGsTmemCols = 512;
+constexpr uint32_t kGsAccCols = 64, kGsCvtCol0 = 128;   // accumulators: 2 nc <= 64 columns per tile, or (nc = 64, one tile) 128
 
-__global__ void __launch_bounds__(kGsThreads, 1) q8_gemm_tc_staged(const GemmArgs a) {
+// item -> row groups [g0, g0 + n) of the concatenated matrices, K-tiles [t0, t1), part of the sums
+struct SkinnyItem { int g0, n, t0, t1, ks; };
+__device__ __forceinline__ SkinnyItem skinny_item(const GemmArgs& a, int item, int tpr, int groups) {
+    SkinnyItem it;
+    it.ks = item % a.ksplit;
+    const int c = item / a.ksplit;
+    it.g0 = (int)((long long)c * groups / a.row_chunks);
+    it.n = (int)((long long)(c + 1) * groups / a.row_chunks) - it.g0;
+    it.t0 = (int)((long long)it.ks * tpr / a.ksplit);
+    it.t1 = (int)((long long)(it.ks + 1) * tpr / a.ksplit);
+    return it;
+}
+// matrix and row group inside it of row group g of the concatenation
+__device__ __forceinline__ int skinny_seg(const GemmArgs& a, int& g) {
+    int s = 0;
+    while (s < a.nseg - 1 && g >= a.seg[s].rows / kTileRows) { g -= a.seg[s].rows / kTileRows; s++; }
+    return s;
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
+                 "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]),
+                 "r"(v[14]), "r"(v[15])
+                 : "memory");
+}
+__device__ __forceinline__ uint32_t h2_neg(uint32_t a) { uint32_t d; asm("neg.f16x2 %0, %1;" : "=r"(d) : "r"(a)); return d; }
+
+// NC: activation rows of the chunk (a compile-time number: with the index arithmetic done at run time the issuing thread took 86 clocks per
+// instruction)
+template <int NC>
+__global__ void __launch_bounds__(kGsThreads, 1) q8_gemm_tc_skinny(const GemmArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t bars = smem_u32(smem);
-    const uint32_t wfull = bars, wempty = bars + 16, xfull = bars + 32, xempty = bars + 96, cfull = bars + 160, cempty = bars + 224,
-                   afull = bars + 288, aempty = bars + 296, fin = bars + 304, tmem_slot = bars + 312;
-    static_assert(kGsXStages <= 8 && kGsCvtBufs <= 8 && kGsCvtCol0 + kGsCvtBufs * kGsCvtCols1 * kGsStep <= kGsTmemCols && kGmXTerms == 2 &&
-                  kGsHB * 2 * kGmMaxChunk <= (int)kGsCvtCol0, "barrier area / tensor memory");
+    const uint32_t wfull = bars, wempty = bars + 16, xfull = bars + 32, xempty = bars + 64, cfull = bars + 96, cempty = bars + 128,
+                   afull = bars + 160, aempty = bars + 168, fin = bars + 176, tmem_slot = bars + 184;
+    static_assert(kGsXStages <= 4 && kGsCvtBufs <= 4 && kGsCvtCol0 + kGsCvtBufs * kGsCvtCols <= kGsTmemCols && kGmXTerms == 2, "barrier area / tensor memory");
     unsigned char* wst = (unsigned char*)(((uintptr_t)smem + kGsBarBytes + 127) & ~(uintptr_t)127);
     unsigned char* xst = wst + (size_t)kGsWStages * kGsWStage;
     volatile int* abort = &s_abort;
     if (tid == 0) {
         s_abort = 0;
-        for (int i = 0; i < 2; i++) {
-            mbar_init(wfull + 8u * i, 1); mbar_init(wempty + 8u * i, kGsCvtWarps);
-        }
+        for (int i = 0; i < kGsWStages; i++) { mbar_init(wfull + 8u * i, 1); mbar_init(wempty + 8u * i, kGsCvtWarps); }
         mbar_init(afull, 1); mbar_init(aempty, kGsCvtWarps);
         for (int i = 0; i < kGsCvtBufs; i++) { mbar_init(cfull + 8u * i, kGsCvtWarps); mbar_init(cempty + 8u * i, 1); }
         for (int i = 0; i < kGsXStages; i++) { mbar_init(xfull + 8u * i, 1); mbar_init(xempty + 8u * i, 1); }
@@ -552,121 +587,121 @@ __global__ void __launch_bounds__(kGsThreads, 1) q8_gemm_tc_staged(const GemmArg
     // are read (activation copies, row factors) or where what it may still read is overwritten (the sums).
     if (a.use_pdl) pdl_launch_dependents();
 
-    const int tpr = a.K / kTileK, nb = a.K >> 5;
-    const int nc = a.nc;                                   // activation rows per chunk
-    const uint32_t x_term = (uint32_t)nc * 64u;            // bytes of one term of one slice: 4 column groups x nc rows x 16
-    const uint32_t x_slice = (uint32_t)kGmXTerms * x_term;
-    const uint32_t ncb = (uint32_t)a.cvt_bufs, nxs = (uint32_t)a.x_stages;
-    const int step = a.step;                               // slices per hand-over
-    const uint32_t cvt_cols = kGsCvtCols1 * (uint32_t)step;
-    const int sps = kGsStep * kGmMaxChunk / nc;            // slices per activation stage: a stage is always one 32 KiB copy
-    int tiles = 0;
-    for (int s = 0; s < a.nseg; s++) tiles += (a.seg[s].rows + kGsRows - 1) / kGsRows;
-    const int n_items = tiles * a.ksplit * a.m_chunks;
+    const int tpr = a.K / kTileK;
+    constexpr int nc = NC;
+    constexpr uint32_t x_cg = (uint32_t)kGmXTerms * (uint32_t)nc * 16u;      // bytes of one column group of a slice: both terms' rows
+    constexpr uint32_t x_slice = 4u * x_cg;
+    constexpr int sps = kGsXStage / (int)x_slice;          // slices per activation stage: 8, 4 or 2
+    int groups = 0;
+    for (int s = 0; s < a.nseg; s++) groups += a.seg[s].rows / kTileRows;
+    const int n_items = a.row_chunks * a.ksplit;
     auto fail = [&](uint32_t code) { if (!*abort) { atomicOr(a.status, code); *abort = 1; } };
+    // row groups of tensor-core tile hb of an item of n: all of them, or halves
+    auto tiles_of = [](int n) { return n > kGsRG ? 2 : 1; };
+    auto first_of = [](int n, int hb) { return hb ? (n + 1) / 2 : 0; };
+    auto count_of = [](int n, int hb) { return n <= kGsRG ? n : hb ? n / 2 : (n + 1) / 2; };
 
     if (warp == kGsCvtWarps + 2) {
-        // ---------------------------------------------------------------- weight producer warp
-        // Lane 0 waits for a free stage and arms its barrier; the 16 tile copies of a stage are then issued by 16 lanes side by side
-        // (a bulk copy costs the copy engine about 50 ns whatever its size; one lane issuing them one after the other is slower
-        // still).  A warp of its own: in one warp with the activation copies, the next weight stage was only asked for after the
-        // current K-tile's last activation stage had found a free slot — a third of the converters' time went into waiting for it.
+        // ---------------------------------------------------------------- weight producer warp: lane = row group
         uint32_t wi = 0;
         int ok = 1;
         for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-            const GemmItem it = gemm_item(a, item, tpr, kGsRows);
-            const unsigned char* wseg = a.seg[it.seg].w;
+            const SkinnyItem it = skinny_item(a, item, tpr, groups);
+            const int hbs = tiles_of(it.n);
+            const unsigned char* src[2];                   // this lane's row group of each tensor-core tile
+#pragma unroll
+            for (int hb = 0; hb < 2; hb++) {
+                int g = it.g0 + first_of(it.n, hb) + (lane < count_of(it.n, hb) ? lane : 0);
+                if (hb >= hbs) g = it.g0;
+                const int sg = skinny_seg(a, g);
+                src[hb] = a.seg[sg].w + (size_t)g * tpr * kTileBytes;
+            }
             for (int t = it.t0; t < it.t1 && ok; t++) {
-                const uint32_t ws = wi & 1u;
-                if (lane == 0) {
-                    if (!mbar_wait_abortable(wempty + 8u * ws, ((wi >> 1) & 1u) ^ 1u, abort)) { fail(LUM_ST_WAIT_EMPTY); ok = 0; }
-                    else mbar_arrive_expect_tx(wfull + 8u * ws, (uint32_t)it.n_rg * kGsWRow);
+                for (int hb = 0; hb < hbs; hb++) {
+                    const uint32_t ws = wi % kGsWStages;
+                    const int cnt = count_of(it.n, hb);
+                    if (lane == 0) {
+                        if (!mbar_wait_abortable(wempty + 8u * ws, ((wi / kGsWStages) & 1u) ^ 1u, abort)) { fail(LUM_ST_WAIT_EMPTY); ok = 0; }
+                        else mbar_arrive_expect_tx(wfull + 8u * ws, (uint32_t)cnt * kGsWRow);
+                    }
+                    ok = __shfl_sync(0xffffffffu, ok, 0);
+                    if (!ok) break;
+                    if (lane < cnt)
+                        bulk_g2s(smem_u32(wst + (size_t)ws * kGsWStage + (size_t)lane * kGsWRow), (hb ? src[1] : src[0]) + (size_t)t * kTileBytes, kTileBytes, wfull + 8u * ws);
+                    wi++;
                 }
-                ok = __shfl_sync(0xffffffffu, ok, 0);
-                if (!ok) break;
-                for (int j = lane; j < it.n_rg; j += 32)
-                    bulk_g2s(smem_u32(wst + (size_t)ws * kGsWStage + (size_t)j * kGsWRow), wseg + ((size_t)(it.rg0 + j) * tpr + t) * kTileBytes, kTileBytes,
-                             wfull + 8u * ws);
-                wi++;
             }
         }
         // never leave while a copy into this CTA's shared memory may be in flight: wait (bounded) for what was armed
         if (!ok && lane == 0)
-            for (uint32_t k = 0; k < 2 && k < wi; k++) { const uint32_t i = wi - 1 - k; mbar_wait(wfull + 8u * (i & 1u), (i >> 1) & 1u); }
+            for (uint32_t k = 0; k < kGsWStages && k < wi; k++) { const uint32_t i = wi - 1 - k; mbar_wait(wfull + 8u * (i % kGsWStages), (i / kGsWStages) & 1u); }
         return;
     }
     if (warp == kGsCvtWarps) {
-        // ---------------------------------------------------------------- activation producer: one lane, one 32 KiB copy per stage
+        // ---------------------------------------------------------------- activation producer: one lane, one copy per stage
         if (elect_one()) {
             uint32_t xi = 0;
             bool ok = true;
             if (a.use_pdl) pdl_grid_wait();
             for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                const GemmItem it = gemm_item(a, item, tpr, kGsRows);
-                for (int t = it.t0; t < it.t1 && ok; t++) {
-                    for (int s = 0; s < kGsPartSlices; s += sps) {
-                        const uint32_t xs = xi % nxs;
-                        if (!mbar_wait_abortable(xempty + 8u * xs, ((xi / nxs) & 1u) ^ 1u, abort)) { fail(LUM_ST_WAIT_EMPTY); ok = false; break; }
-                        mbar_arrive_expect_tx(xfull + 8u * xs, x_slice * (uint32_t)sps);
-                        bulk_g2s(smem_u32(xst + (size_t)xs * kGsXStageMax), (const unsigned char*)a.xq + ((size_t)it.mc * nb + (size_t)t * 16 + s) * x_slice,
-                                 x_slice * (uint32_t)sps, xfull + 8u * xs);
-                        xi++;
-                    }
+                const SkinnyItem it = skinny_item(a, item, tpr, groups);
+                for (int s = it.t0 * 16; s < it.t1 * 16; s += sps) {
+                    const uint32_t xs = xi % kGsXStages;
+                    if (!mbar_wait_abortable(xempty + 8u * xs, ((xi / kGsXStages) & 1u) ^ 1u, abort)) { fail(LUM_ST_WAIT_EMPTY); ok = false; break; }
+                    mbar_arrive_expect_tx(xfull + 8u * xs, kGsXStage);
+                    bulk_g2s(smem_u32(xst + (size_t)xs * kGsXStage), (const unsigned char*)a.xq + (size_t)s * x_slice, kGsXStage, xfull + 8u * xs);
+                    xi++;
                 }
             }
             if (!ok)
-                for (uint32_t k = 0; k < nxs && k < xi; k++) { const uint32_t i = xi - 1 - k; mbar_wait(xfull + 8u * (i % nxs), (i / nxs) & 1u); }
+                for (uint32_t k = 0; k < kGsXStages && k < xi; k++) { const uint32_t i = xi - 1 - k; mbar_wait(xfull + 8u * (i % kGsXStages), (i / kGsXStages) & 1u); }
         }
         return;
     }
     if (warp == kGsCvtWarps + 1) {
-        // ---------------------------------------------------------------- tensor-core warp: one lane issues
+        // ---------------------------------------------------------------- tensor-core warp: one thread issues
         if (elect_one()) {
-            uint32_t xi = 0, ci = 0, ic = 0;
+            uint32_t x0 = 0, ci = 0, ic = 0;               // x0: activation stages before the current K-tile
             bool ok = true;
-            // hi x [x1 | x2] is ONE instruction of N = 2 nc (its two halves of the accumulator are added when it is stored), lo x x1
-            // one of N = nc into the first half: two instructions per 16 columns of K instead of three (an instruction costs its
-            // issuing thread about 80 cycles whatever its N: at nc = 32 that, not the tensor core, bounds the kernel)
-            const uint32_t idesc2 = umma_idesc_f16(128, 2 * nc), idesc1 = umma_idesc_f16(128, nc);
-            // activation operand descriptors: start address in the low 14 bits; column groups 2 nc * 16 bytes apart, 8-row groups 128
-            const uint32_t x_cg = (uint32_t)kGmXTerms * (uint32_t)nc * 16u;
-            const uint32_t x_lo = ((x_cg >> 4) & 0x3fffu) << 16, x_hi = umma_desc_hi(128u), x_base = smem_u32(xst);
+            constexpr uint32_t idesc2 = umma_idesc_f16(128, 2 * nc), idesc1 = umma_idesc_f16(128, nc);
+            // activation operand descriptors: start address in the low 14 bits; column groups x_cg bytes apart, 8-row groups 128
+            constexpr uint32_t x_lo = ((x_cg >> 4) & 0x3fffu) << 16, x_hi = umma_desc_hi(128u);
+            const uint32_t x_base = smem_u32(xst);
+            constexpr int spt = 16 / sps;                  // activation stages per K-tile
             for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ic++) {
-                const GemmItem it = gemm_item(a, item, tpr, kGsRows);
+                const SkinnyItem it = skinny_item(a, item, tpr, groups);
+                const int hbs = tiles_of(it.n);
                 if (!mbar_wait_abortable(aempty, (ic & 1u) ^ 1u, abort)) { fail(LUM_ST_WAIT_TMEM); break; }      // the previous item's sums were stored
                 tc_fence_after_sync();
-                uint32_t started = 0;
-                for (int t = it.t0; t < it.t1 && ok; t++) {
-                    for (int s = 0; s < 16; s += step) {
-                        const uint32_t cb = ci % ncb, xs = xi % nxs;
-                        const int sub = s % sps;                  // first slice of the step inside the activation stage
-                        if (!mbar_wait_abortable(cfull + 8u * cb, (ci / ncb) & 1u, abort) ||
-                            (sub == 0 && !mbar_wait_abortable(xfull + 8u * xs, (xi / nxs) & 1u, abort))) {
-                            fail(LUM_ST_WAIT_FULL); ok = false; break;
-                        }
-                        tc_fence_after_sync();
-                        const uint32_t wt = tmem + kGsCvtCol0 + cb * cvt_cols;
-                        const uint32_t xb = x_base + xs * (uint32_t)kGsXStageMax + (uint32_t)sub * x_slice;
-                        if (!(a.debug & 2)) {
-#pragma unroll 4
-                            for (int kk = 0; kk < 2 * step; kk++) {     // K = 16 per instruction: two per 32-column slice
-                                // weights: tensor memory, 8 columns (16 binary16) per instruction; activations: shared memory,
-                                // [column group of 8][row][16 bytes], an instruction reads two adjacent column groups
-                                const uint32_t xo = xb + (uint32_t)(kk >> 1) * x_slice + (uint32_t)(kk & 1) * 2u * x_cg;
-                                const uint32_t x12 = x_lo | ((xo >> 4) & 0x3fffu);
+                for (int t = it.t0; t < it.t1 && ok; t++, x0 += (uint32_t)spt) {
+                    for (int hb = 0; hb < hbs && ok; hb++) {
+                        const uint32_t acc = tmem + (uint32_t)hb * kGsAccCols;
 #pragma unroll
-                                for (int hb = 0; hb < kGsHB; hb++) {      // the 128-row tiles of the item
-                                    const uint32_t acc = tmem + (uint32_t)hb * 2u * (uint32_t)kGmMaxChunk;
-                                    const uint32_t hi = wt + (uint32_t)(kk >> 1) * 32u * kGsHB + (uint32_t)hb * 32u + (uint32_t)(kk & 1) * 8u, lo = hi + 16u;
-                                    umma_f16_ts2(acc, hi, x12, x_hi, idesc2, started);
-                                    umma_f16_ts2(acc, lo, x12, x_hi, idesc1, 1u);
+                        for (int s = 0; s < 16; s += kGsStep, ci++) {
+                            const uint32_t cb = ci % kGsCvtBufs;
+                            if (!mbar_wait_abortable(cfull + 8u * cb, (ci / kGsCvtBufs) & 1u, abort)) { fail(LUM_ST_WAIT_FULL); ok = false; break; }
+                            tc_fence_after_sync();
+                            const uint32_t wt = tmem + kGsCvtCol0 + cb * kGsCvtCols;
+#pragma unroll
+                            for (int ss = 0; ss < kGsStep; ss++) {
+                                const int sub = (s + ss) % sps;               // the slice inside its activation stage
+                                const uint32_t xi = x0 + (uint32_t)((s + ss) / sps), xs = xi % kGsXStages;
+                                if (sub == 0 && hb == 0 && !mbar_wait_abortable(xfull + 8u * xs, (xi / kGsXStages) & 1u, abort)) { fail(LUM_ST_WAIT_FULL); ok = false; break; }
+                                const uint32_t xb = x_base + xs * (uint32_t)kGsXStage + (uint32_t)sub * x_slice;
+#pragma unroll
+                                for (int kk = 0; kk < 2; kk++) {      // K = 16 per instruction: two per 32-column slice
+                                    // weights: tensor memory, 8 columns (16 binary16) per instruction; activations: shared memory,
+                                    // [column group of 8][term][row][16 bytes], an instruction reads two adjacent column groups
+                                    const uint32_t x12 = x_lo | (((xb + (uint32_t)kk * 2u * x_cg) >> 4) & 0x3fffu);
+                                    const uint32_t hi = wt + (uint32_t)ss * kGsSliceCols + (uint32_t)kk * 8u;
+                                    umma_f16_ts2(acc, hi, x12, x_hi, idesc2, (t > it.t0 || s + ss + kk > 0) ? 1u : 0u);
+                                    umma_f16_ts2(acc + (uint32_t)nc, hi + 16u, x12, x_hi, idesc1, 1u);
                                 }
-                                started = 1u;
+                                if (sub == sps - 1 && hb == hbs - 1) umma_commit(xempty + 8u * xs);       // the tile that reads it last has done so
                             }
+                            if (!ok) break;
+                            umma_commit(cempty + 8u * cb);        // arrive when the instructions that read these operands have retired
                         }
-                        umma_commit(cempty + 8u * cb);        // arrive when the instructions that read these operands have retired
-                        ci++;
-                        if (sub + step == sps) { umma_commit(xempty + 8u * xs); xi++; }
                     }
                 }
                 if (ok) umma_commit(afull);
@@ -683,83 +718,87 @@ __global__ void __launch_bounds__(kGsThreads, 1) q8_gemm_tc_staged(const GemmArg
 
     // -------------------------------------------------------------------- converting / storing warps
     {
-        // a warp reaches the 32 tensor-memory lanes of its quarter: thread = weight row of the item (lane of tensor memory); warps
-        // 0-3 take columns 0-15 of every 32-block, warps 4-7 columns 16-31 (and, for the store, the two halves of the chunk's rows)
-        const int q = warp & 3, h = warp >> 2, ch = h;
-        const int n = (q << 5) + lane, r = n & 7;                    // row inside a 128-row tile
+        // a warp reaches the 32 tensor-memory lanes of its quarter: thread = weight row of the tile (lane of tensor memory); of a
+        // hand-over's four slices it converts number z (and stores columns 16 z .. of the sums)
+        const int q = warp & 3, z = warp >> 2;
+        const int n = (q << 5) + lane, g = n >> 3, r = n & 7;        // row, row group inside the tile, row inside that
         const uint32_t lane_addr = (uint32_t)(q << 5) << 16;
         uint32_t wi = 0, ci = 0, ic = 0;
         bool ok = true;
         for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ic++) {
-            const GemmItem it = gemm_item(a, item, tpr, kGsRows);
+            const SkinnyItem it = skinny_item(a, item, tpr, groups);
+            const int hbs = tiles_of(it.n);
             for (int t = it.t0; t < it.t1 && ok; t++) {
-                const uint32_t ws = wi & 1u;
-                if (!mbar_wait_abortable(wfull + 8u * ws, (wi >> 1) & 1u, abort)) { fail(LUM_ST_WAIT_FULL); ok = false; break; }
-#pragma unroll 1
-                for (int s0 = 0; s0 < kGsPartSlices; s0 += step) {
-                    const uint32_t cb = ci % ncb;
-                    if (!mbar_wait_abortable(cempty + 8u * cb, ((ci / ncb) & 1u) ^ 1u, abort)) { fail(LUM_ST_WAIT_EMPTY); ok = false; break; }
-                    tc_fence_after_sync();
-                    if (a.debug & 1) { __syncwarp(); if (lane == 0) mbar_arrive(cfull + 8u * cb); ci++; continue; }
-#pragma unroll 2
-                 for (int ss = 0; ss < step; ss++) {
-                  const int s = s0 + ss;
-#pragma unroll
-                  for (int hb = 0; hb < kGsHB; hb++) {
-                    const int g = (n >> 3) + hb * 16;
+                for (int hb = 0; hb < hbs && ok; hb++) {
+                    const uint32_t ws = wi % kGsWStages;
+                    if (!mbar_wait_abortable(wfull + 8u * ws, (wi / kGsWStages) & 1u, abort)) { fail(LUM_ST_WAIT_FULL); ok = false; break; }
+                    // a quarter without rows converts nothing (its lanes' sums are never stored); lanes past the last row read stale bytes
+                    // of the stage, for the same reason
+                    const bool live = q * 4 < count_of(it.n, hb);
                     const unsigned char* tile = wst + (size_t)ws * kGsWStage + (size_t)g * kGsWRow;
-                    const bool live = g < it.n_rg;                   // row groups past the matrix's end contribute zeros
-                    const uint4 raw = *(const uint4*)(tile + s * 256 + h * 128 + r * 16);
-                    const uint32_t d16 = live ? (uint32_t)*(const unsigned short*)(tile + kTileQ + (s * 8 + r) * 2) : 0u;
-                    const uint32_t dd = h2_mul(d16 | (d16 << 16), 0x64006400u);            // 1024 d, exact
-                    const uint32_t w4[4] = {raw.x ^ 0x80808080u, raw.y ^ 0x80808080u, raw.z ^ 0x80808080u, raw.w ^ 0x80808080u};
-                    uint32_t hi[8], lo[8];
+#pragma unroll 2
+                    for (int s0 = 0; s0 < 16; s0 += kGsStep, ci++) {
+                        const uint32_t cb = ci % kGsCvtBufs;
+                        const int s = s0 + z;
+                        // converted before the buffer is waited for: the wait then costs no arithmetic
+                        uint32_t hi[16], lo[16];
+                        if (live) {
+                            const uint4 raw0 = *(const uint4*)(tile + s * 256 + r * 16), raw1 = *(const uint4*)(tile + s * 256 + 128 + r * 16);
+                            const uint32_t d16 = (uint32_t)*(const unsigned short*)(tile + kTileQ + (s * 8 + r) * 2);
+                            const uint32_t dd = h2_mul(d16 | (d16 << 16), 0x64006400u);            // 1024 d, exact
+                            const uint32_t w8[8] = {raw0.x, raw0.y, raw0.z, raw0.w, raw1.x, raw1.y, raw1.z, raw1.w};
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        // bytes (q + 128) into the mantissas of 1024 + (q + 128), two at a time; minus 1152 leaves q, exactly
-                        const uint32_t q0 = h2_sub(__byte_perm(w4[j], 0x64646464u, 0x4140), 0x64806480u);
-                        const uint32_t q1 = h2_sub(__byte_perm(w4[j], 0x64646464u, 0x4342), 0x64806480u);
-                        hi[2 * j] = h2_mul(q0, dd); hi[2 * j + 1] = h2_mul(q1, dd);
-                        lo[2 * j] = h2_fma(q0, dd, hi[2 * j] ^ 0x80008000u);             // q d' - hi: the rounding error of hi, exactly
-                        lo[2 * j + 1] = h2_fma(q1, dd, hi[2 * j + 1] ^ 0x80008000u);
+                            for (int j = 0; j < 8; j++) {
+                                // bytes (q + 128) into the mantissas of 1024 + (q + 128), two at a time; minus 1152 leaves q, exactly
+                                const uint32_t w = w8[j] ^ 0x80808080u;
+                                const uint32_t q0 = h2_sub(__byte_perm(w, 0x64646464u, 0x4140), 0x64806480u);
+                                const uint32_t q1 = h2_sub(__byte_perm(w, 0x64646464u, 0x4342), 0x64806480u);
+                                hi[2 * j] = h2_mul(q0, dd); hi[2 * j + 1] = h2_mul(q1, dd);
+                                lo[2 * j] = h2_fma(q0, dd, h2_neg(hi[2 * j]));             // q d' - hi: the rounding error of hi, exactly
+                                lo[2 * j + 1] = h2_fma(q1, dd, h2_neg(hi[2 * j + 1]));
+                            }
+                        }
+                        if (!mbar_wait_abortable(cempty + 8u * cb, ((ci / kGsCvtBufs) & 1u) ^ 1u, abort)) { fail(LUM_ST_WAIT_EMPTY); ok = false; break; }
+                        tc_fence_after_sync();
+                        if (live) {
+                            const uint32_t wt = tmem + lane_addr + kGsCvtCol0 + cb * kGsCvtCols + (uint32_t)z * kGsSliceCols;
+                            tmem_st16(wt, hi);
+                            tmem_st16(wt + 16u, lo);
+                            tmem_st_wait();
+                        }
+                        tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(cfull + 8u * cb);
                     }
-                    const uint32_t wt = tmem + lane_addr + kGsCvtCol0 + cb * cvt_cols + (uint32_t)ss * 32u * kGsHB + (uint32_t)hb * 32u + (uint32_t)h * 8u;
-                    tmem_st8(wt, hi);
-                    tmem_st8(wt + 16u, lo);
-                  }
-                 }
-                    tmem_st_wait();
-                    tc_fence_before_sync();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(cfull + 8u * cb);
-                    ci++;
+                    if (lane == 0) mbar_arrive(wempty + 8u * ws);
+                    wi++;
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(wempty + 8u * ws);
-                wi++;
             }
             if (!ok) break;
-            // ---- the item's K range is done: store the accumulator (lane = weight row, columns = activation rows)
+            // ---- the item's K range is done: store the accumulators (lane = weight row, columns = activation rows)
             if (!mbar_wait_abortable(afull, ic & 1u, abort)) { fail(LUM_ST_WAIT_TMEM); ok = false; break; }
             if (a.use_pdl) pdl_grid_wait();              // (long over: the sums are there)
             tc_fence_after_sync();
-            const GemmSeg& sg = a.seg[it.seg];
-            const int half_rows = nc >> 1;
+            if (16 * z < nc && 16 * z < a.M) {
+                // one request per warp: every CTA wants the same few bytes at the same time (a load per row and warp cost 2 us at 32 rows)
+                const float sx_lane = __ldcg(a.sx + 16 * z + (lane & 15));
 #pragma unroll 1
-            for (int hb = 0; hb < kGsHB; hb++) {
-                const int n_st = hb * 128 + n;
-                const bool row_live = (n_st >> 3) < it.n_rg;
-                float* yp = a.y + (size_t)it.ks * a.part_stride + sg.col0 + it.rg0 * kTileRows + n_st;
-                for (int c0 = 0; c0 < half_rows; c0 += 16) {
+                for (int hb = 0; hb < hbs; hb++) {
+                    const bool row_live = g < count_of(it.n, hb);
+                    int rg = it.g0 + first_of(it.n, hb) + (row_live ? g : 0);
+                    const int sg = skinny_seg(a, rg);
+                    float* yp = a.y + (size_t)it.ks * a.part_stride + a.seg[sg].col0 + rg * kTileRows + r;
                     uint32_t v[16], v2[16];
-                    const uint32_t col = tmem + lane_addr + (uint32_t)hb * 2u * (uint32_t)kGmMaxChunk + (uint32_t)(ch * half_rows + c0);
+                    const uint32_t col = tmem + lane_addr + (uint32_t)hb * kGsAccCols + (uint32_t)(16 * z);
                     tmem_ld16(col, v);
                     tmem_ld16(col + (uint32_t)nc, v2);              // the x2 half of the accumulator
                     tmem_ld_wait();
 #pragma unroll
                     for (int i = 0; i < 16; i++) {
-                        const int m = it.mc * nc + ch * half_rows + c0 + i;
-                        if (row_live && m < a.M) yp[(size_t)m * a.ldy] = (__uint_as_float(v[i]) + __uint_as_float(v2[i])) * __ldg(a.sx + m);
+                        const int m = 16 * z + i;
+                        const float sum = (__uint_as_float(v[i]) + __uint_as_float(v2[i])) * __shfl_sync(0xffffffffu, sx_lane, i);
+                        if (row_live && m < a.M) yp[(size_t)m * a.ldy] = sum;
                     }
                 }
             }
@@ -778,18 +817,44 @@ __global__ void __launch_bounds__(kGsThreads, 1) q8_gemm_tc_staged(const GemmArg
 size_t gemm_xq_bytes(int M, int K) { const int nc = gemm_chunk_rows(M); return (size_t)((M + nc - 1) / nc) * nc * K * 2 * kGmXTerms; }
 size_t gemm_sx_bytes(int M, int K) { (void)K; const int nc = gemm_chunk_rows(M); return (size_t)((M + nc - 1) / nc) * nc * 4; }
 
-// K ranges per product.  Work items are equal, so a product takes ceil(items / SMs) rounds of one item each: with few items per SM
+// Up to 64 rows: K ranges and runs of row groups of a product.  An SM's time for one K-tile of n row groups is the largest of: its
+// share of HBM (4352 n bytes at 44 GB/s), the conversion (kGsCvtUs per tensor-core tile), and what comes
+// in from L2 and HBM together (90 GB/s); an item costs about 2.5 us beside that, a plane of partial sums its write and read at the copy rate.  Everything depends on the rows' class (nc) and not on their number, so that a plan holds for the class.
+struct SkinnyPlan { int ks, chunks; };
+static SkinnyPlan gemm_plan(int groups, int nc, int K, int sms) {
+    const int tpr = K / kTileK, most = nc == 64 ? kGsRG : 2 * kGsRG;       // two tiles share activation slices that are all resident
+    SkinnyPlan best{1, (groups + most - 1) / most};
+    double best_t = 1e30;
+    for (int ks = 1; ks <= 8 && ks <= tpr; ks++) {
+        const double plane_us = (double)nc * groups * kTileRows * 8.0 / 6.5e6;
+        for (int p = 1; p <= 64; p++) {                                     // items per SM
+            int chunks = (int)((long long)sms * p / ks);
+            if (chunks < 1) continue;
+            if (chunks > groups) chunks = groups;
+            const int n = (groups + chunks - 1) / chunks;
+            if (n > most) continue;
+            const double hbm = 4352.0 * n / 44e3, cvt = kGsCvtUs * (n > kGsRG ? 2 : 1), in = (4352.0 * n + 16.0 * 128.0 * nc) / 90e3;
+            const double tile_us = hbm > cvt ? (hbm > in ? hbm : in) : (cvt > in ? cvt : in);
+            const int rounds = (int)(((long long)chunks * ks + sms - 1) / sms);
+            const double t = rounds * ((double)((tpr + ks - 1) / ks) * tile_us + 2.5) + (ks - 1) * plane_us;
+            if (t < best_t * 0.98) { best_t = t; best = {ks, chunks}; }
+            if (chunks == groups) break;
+        }
+    }
+    return best;
+}
+
+// More rows: K ranges per product.  Work items are equal, so a product takes ceil(items / SMs) rounds of one item each: with few items per SM
 // the last, partly filled round is a large share of the time (224 tiles over 148 SMs: 2 rounds for 1.5 rounds of work).  Cutting K
 // makes the rounds shorter and the loss smaller, but every item pays its own pipeline fill and store, and every extra range
 // writes (and the consumer reads) another plane of partial sums.  The estimate below weighs the three; its constants are
-// measured orders of magnitude (a K-tile of one item: 4 us at 32 rows per chunk, 14 us at 128 rows and 256 weight rows; an item's own cost: a third of a
+// measured orders of magnitude (a K-tile of one item: 14 us at 256 weight rows; an item's own cost: a third of a
 // tile; plane traffic at the HBM copy rate), not a fit.
 int gemm_pick_ksplit(int n_rows_total, int M, int K, int sm_count) {
     const int nc = gemm_chunk_rows(M);
-    const bool wide = nc == kGmMaxChunk;                                          // 256-row items (q8_gemm_tc) or 128-row items (q8_gemm_tc_staged)
-    const int rows_per_item = wide ? kGmRows : kGsRows;
-    const int tiles = (n_rows_total + rows_per_item - 1) / rows_per_item, mc = (M + nc - 1) / nc, tpr = K / kTileK;
-    const double t_tile = wide ? 14.4 : 16.0 * (0.16 + 0.43 * nc / 128.0);       // us per K-tile of one item
+    if (nc < kGmMaxChunk) return gemm_plan(n_rows_total / kTileRows, nc, K, sm_count).ks;
+    const int tiles = (n_rows_total + kGmRows - 1) / kGmRows, mc = (M + nc - 1) / nc, tpr = K / kTileK;
+    const double t_tile = 14.4;                                                   // us per K-tile of one item
     const double plane_us = (double)M * n_rows_total * 8.0 / 6.5e6;               // write + read of one plane of partial sums
     int best = 1;
     double best_t = 1e30;
@@ -857,27 +922,31 @@ cudaError_t launch_gemm(const GemmArgs& a_in, int sm_count, cudaStream_t st) {
     a.debug = env_debug;
     a.m_chunks = (a.M + a.nc - 1) / a.nc;
     if (!gemm_supported(a)) return cudaErrorInvalidValue;
-    // 128 activation rows per chunk (prompts): the tensor core is the resource; fewer (batched decode): the weight stream is
+    // more than 64 rows (prompts): the tensor core is the resource; fewer (batched decode): the weight stream is
     const bool wide = a.nc == kGmMaxChunk;
-    const void* fn = wide ? (const void*)q8_gemm_tc : (const void*)q8_gemm_tc_staged;
+    const void* fn = wide ? (const void*)q8_gemm_tc : a.nc == 16 ? (const void*)q8_gemm_tc_skinny<16> : a.nc == 32 ? (const void*)q8_gemm_tc_skinny<32> : (const void*)q8_gemm_tc_skinny<64>;
     const size_t smem = wide ? kGmSmem : kGsSmem;
-    const int rows_per_item = wide ? kGmRows : kGsRows, threads = wide ? kGmThreads : kGsThreads;
-    if (wide) { a.cvt_bufs = kGmCvtBufs; a.x_stages = kGmXStages; a.step = kGmStep; }
-    else {
-        a.step = a.nc == 32 ? 4 : kGsStep;
-        int bufs = 256 / (32 * kGsHB * a.step);                    // converted-weight buffers that fit the 256 columns behind the accumulators
-        a.cvt_bufs = bufs > kGsCvtBufs ? kGsCvtBufs : bufs;
-        a.x_stages = kGsXStages;
-    }
-    static bool set[2] = {false, false};
-    if (!set[wide ? 1 : 0]) {
+    const int threads = wide ? kGmThreads : kGsThreads;
+    static bool set[4] = {false, false, false, false};
+    const int which = wide ? 3 : a.nc / 32;
+    if (!set[which]) {
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        set[wide ? 1 : 0] = true;
+        set[which] = true;
     }
-    int tiles = 0;
-    for (int s = 0; s < a.nseg; s++) tiles += (a.seg[s].rows + rows_per_item - 1) / rows_per_item;
-    const long long items = (long long)tiles * a.ksplit * a.m_chunks;
+    long long items = 0;
+    if (wide) {
+        for (int s = 0; s < a.nseg; s++) items += (a.seg[s].rows + kGmRows - 1) / kGmRows;
+        items *= (long long)a.ksplit * a.m_chunks;
+    } else {
+        // the row groups of one K range over the SMs it has, in as many rounds as the plan takes (the split itself was the caller's choice)
+        int groups = 0;
+        for (int s = 0; s < a.nseg; s++) groups += a.seg[s].rows / kTileRows;
+        const SkinnyPlan p = gemm_plan(groups, a.nc, a.K, sm_count);
+        const int most = a.nc == 64 ? kGsRG : 2 * kGsRG;
+        a.row_chunks = p.ks == a.ksplit ? p.chunks : (groups + most - 1) / most;
+        items = (long long)a.row_chunks * a.ksplit;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(items < sm_count ? items : sm_count));
     cfg.blockDim = dim3(threads);

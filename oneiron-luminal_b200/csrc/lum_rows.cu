@@ -514,10 +514,9 @@ cudaError_t launch_rope_append_rows(const RopeRowsArgs& a, cudaStream_t st) {
 cudaError_t launch_attn_rows(const AttnRowsArgs& a, cudaStream_t st) {
     const int G = a.n_kv > 0 ? a.n_q / a.n_kv : 0;
     static const int env_split = [] { const char* e = getenv("LUM_ATTN_ROWS_SPLIT"); return e ? atoi(e) : 1; }();
-    if (env_split && a.kv_bf16 && a.window == 0 && (a.hd == 128 || a.hd == 64) && G >= 1 && G <= 8 && (((uintptr_t)a.k_cache | (uintptr_t)a.v_cache) & 15) == 0 &&
+    if (env_split && a.kv_bf16 && a.window == 0 && (a.hd == 128 || a.hd == 64) && G >= 1 && G <= (a.hd == 128 ? 4 : 8) && (((uintptr_t)a.k_cache | (uintptr_t)a.v_cache) & 15) == 0 &&
         ((size_t)a.n_kv * a.hd * 2) % 16 == 0) {
-        const void* fn = a.hd == 128 ? (G <= 4 ? (const void*)attn_rows_split<128, 1> : (const void*)attn_rows_split<128, 2>)
-                                     : (G <= 4 ? (const void*)attn_rows_split<64, 1> : (const void*)attn_rows_split<64, 2>);
+        const void* fn = a.hd == 128 ? (const void*)attn_rows_split<128, 1> : (G <= 4 ? (const void*)attn_rows_split<64, 1> : (const void*)attn_rows_split<64, 2>);
         const size_t smem = (size_t)ar_smem(a.hd);
         if (smem > 48 * 1024) {
             cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

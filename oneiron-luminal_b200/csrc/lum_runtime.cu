@@ -1122,8 +1122,7 @@ bool rows_supported(const lum_rt* rt) {
 // floats the K-split partial planes of a product with n_out outputs per row can need, over every row count up to cap
 size_t rows_parts_floats(const lum_rt* rt, int n_out, int K, int cap) {
     size_t worst = 0;
-    for (int M = 32; M <= ((cap + 31) / 32) * 32; M += 32) {
-        const int m = M < cap ? M : cap;
+    for (int m = 1; m <= cap; m++) {
         const size_t need = (size_t)gemm_pick_ksplit(n_out, m, K, rt->sm_count) * m * n_out;
         if (need > worst) worst = need;
     }

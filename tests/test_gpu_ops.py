@@ -279,6 +279,8 @@ GEMM_KAT = [
     (1024, 4096, 32, "random"),       # the batched-decode shape class (k/v projection)
     (4096, 4096, 40, "random"),
     (512, 14336, 17, "random"),       # down-projection K: 28 K-tiles
+    (1288, 1536, 16, "random"),       # 161 row groups, a chunk of 16 rows, three K-tiles
+    (2176, 2048, 31, "integers"),     # 272 row groups: runs of one and of two tensor-core tiles
     (384, 2560, 64, "random"),        # K = 5 tiles (Qwen hidden)
     (2048, 512, 200, "random"),       # many activation chunks per weight tile
 ]
