@@ -28,11 +28,14 @@
 //    ops.rs:135-146 are fused here), writes the two terms in tensor-core operand order and the row's output factor.
 //  * q8_gemm_tc — 128 activation rows per chunk (prompts).  Persistent CTAs over work items (256 weight rows = two tensor-core tiles
 //    that share every activation slice, one chunk, one K range).  One lane fills a ring of six 32 KiB activation stages with bulk
-//    copies; 8 warps read their rows' weights straight from global memory (16 bytes per row and slice, eight slices ahead, in
+//    copies; 16 warps read their rows' weights straight from global memory (32 bytes per row and slice, two steps ahead, in
 //    registers), turn them into the hi / lo operands and store those to tensor memory (the A operand is read from there: shared
 //    memory and its bandwidth belong to the activation operand); one thread issues the tensor-core instructions (24 of N = 128 per
-//    step of two 32-column slices) and commits the buffers free; the 8 warps store the two accumulators when the K range is done.
-//  * q8_gemm_tc_staged — 32 or 64 rows per chunk (batched decode): see its own header further down.
+//    step of two 32-column slices) and commits the buffers free; the 16 warps store the two accumulators when the K range is done.
+//    Bound by the tensor core, if everything else keeps up: 24 instructions of 65 clocks a step.  Measured, alone (issued TFLOP/s, 6 per
+//    weight and row; 8 warps that converted after the wait for their buffer / 16 that convert before it): 28672 x 4096 at 512 rows
+//    909 -> 1342, at 4096 rows 1177 -> 1649 (constant operands; a prompt's run into the power limit), 128 rows 771 -> 1188.
+//  * q8_gemm_tc_skinny — up to 64 rows (batched decode): see its own header further down.
 //    Outputs are plain f32 stores of K-split partial planes; whoever consumes them (the next rows_quantize) adds them up.
 #include <cstdlib>
 
@@ -49,12 +52,12 @@ constexpr int kGmMaxChunk = 128;                    // activation rows per chunk
 constexpr int kGmXTerms = 2;                        // binary16 terms per activation element
 constexpr int kGmStep = 2;                          // 32-column slices per hand-over between the warps (every hand-over costs each single-threaded role
                                                     // several hundred cycles of its own, whatever the amount of work behind it)
-constexpr int kGmAhead = 8;                         // slices of weights a converter thread has on their way from global memory
+constexpr int kGmAhead = 2;                         // steps whose weights a converter thread has on their way from global memory
 constexpr int kGmXStageMax = kGmStep * kGmXTerms * kGmMaxChunk * 32 * 2;   // 32768: one activation stage (the terms of one step of a 128-row chunk)
 constexpr int kGmCvtBufs = 2, kGmXStages = 6;
 constexpr uint32_t kGmCvtCols = 32 * kGmHB * kGmStep;        // tensor-memory columns of one converted step: per slice and 128-row tile hi (16 columns: 32 binary16
                                                              // per row) | lo (16)
-constexpr int kGmCvtWarps = 8;
+constexpr int kGmCvtWarps = 16;
 constexpr int kGmThreads = (kGmCvtWarps + 2) * 32;   // + activation producer warp + tensor-core warp
 constexpr int kGmBarBytes = 512;
 constexpr size_t kGmSmem = kGmBarBytes + 128 + (size_t)kGmXStages * kGmXStageMax;
@@ -242,12 +245,14 @@ __device__ __forceinline__ void umma_f16_ts2(uint32_t tmem_d, uint32_t tmem_a, u
         ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// whole warp: 8 consecutive 32-bit columns of this thread's lane
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
-                 "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+// whole warp: 16 consecutive 32-bit columns of this thread's lane
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
+                 "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]),
+                 "r"(v[14]), "r"(v[15])
                  : "memory");
 }
+__device__ __forceinline__ uint32_t h2_neg(uint32_t a) { uint32_t d; asm("neg.f16x2 %0, %1;" : "=r"(d) : "r"(a)); return d; }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
@@ -258,7 +263,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
     const uint32_t xfull = bars, xempty = bars + 64, cfull = bars + 128, cempty = bars + 160, afull = bars + 192, aempty = bars + 200,
                    fin = bars + 208, tmem_slot = bars + 216;
     static_assert(kGmXStages <= 8 && kGmCvtBufs <= 4 && kGmCvtCol0 + kGmCvtBufs * kGmCvtCols <= kGmTmemCols && kGmXTerms == 2 && kGmStep == 2 &&
-                  kGmAhead % kGmStep == 0 && 16 % kGmAhead == 0, "barrier area / tensor memory / the converter's unrolled loop");
+                  kGmHB == 2 && 16 % (kGmAhead * kGmStep) == 0, "barrier area / tensor memory / the converter's unrolled loop");
     unsigned char* xst = (unsigned char*)(((uintptr_t)smem + kGmBarBytes + 127) & ~(uintptr_t)127);
     volatile int* abort = &s_abort;
     if (tid == 0) {
@@ -280,11 +285,11 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
     if (a.use_pdl) pdl_launch_dependents();
 
     const int tpr = a.K / kTileK, nb = a.K >> 5;
-    const int nc = a.nc;                                   // activation rows per chunk
-    const uint32_t x_cg = (uint32_t)kGmXTerms * (uint32_t)nc * 16u;      // bytes of one column group of a slice: both terms' rows
-    const uint32_t x_slice = 4u * x_cg;
+    constexpr int nc = kGmMaxChunk;                        // activation rows per chunk
+    constexpr uint32_t x_cg = (uint32_t)kGmXTerms * (uint32_t)nc * 16u;      // bytes of one column group of a slice: both terms' rows
+    constexpr uint32_t x_slice = 4u * x_cg;
     constexpr uint32_t ncb = kGmCvtBufs, nxs = kGmXStages;
-    const int sps = kGmStep * kGmMaxChunk / nc;            // slices per activation stage: a stage is always one 32 KiB copy
+    constexpr int sps = kGmStep;                           // slices per activation stage: one step, one 32 KiB copy
     int tiles = 0;
     for (int s = 0; s < a.nseg; s++) tiles += (a.seg[s].rows + kGmRows - 1) / kGmRows;
     const int n_items = tiles * a.ksplit * a.m_chunks;
@@ -320,14 +325,11 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
         if (elect_one()) {
             uint32_t xi = 0, ci = 0, ic = 0;
             bool ok = true;
-            // 128 activation rows per chunk: hi x1, hi x2, lo x1 as three instructions of N = 128 into one accumulator.  Fewer rows:
-            // hi x [x1 | x2] is ONE instruction of N = 2 nc (its two halves of the accumulator are added when it is stored) and lo x1 one
-            // of N = nc into the first half — an instruction occupies the tensor pipe about 80 cycles whatever its N, and at few rows
-            // the instruction count is what bounds the kernel.
-            const bool wide = nc == kGmMaxChunk;
-            const uint32_t idesc_a = umma_idesc_f16(128, wide ? nc : 2 * nc), idesc_b = umma_idesc_f16(128, nc);
+            // hi x1, hi x2, lo x1 as three instructions of N = 128 into one accumulator
+            constexpr uint32_t idesc = umma_idesc_f16(128, nc);
             // activation operand descriptors: start address in the low 14 bits; column groups x_cg bytes apart, 8-row groups 128
-            const uint32_t x_lo = ((x_cg >> 4) & 0x3fffu) << 16, x_hi = umma_desc_hi(128u), x_base = smem_u32(xst);
+            constexpr uint32_t x_lo = ((x_cg >> 4) & 0x3fffu) << 16, x_hi = umma_desc_hi(128u);
+            const uint32_t x_base = smem_u32(xst);
             for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ic++) {
                 const GemmItem it = gemm_item(a, item, tpr);
                 if (!mbar_wait_abortable(aempty, (ic & 1u) ^ 1u, abort)) { fail(LUM_ST_WAIT_TMEM); break; }      // the previous item's sums were stored
@@ -336,35 +338,32 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
                 for (int t = it.t0; t < it.t1 && ok; t++) {
                     for (int s = 0; s < 16; s += kGmStep) {
                         const uint32_t cb = ci % ncb, xs = xi % nxs;
-                        const int sub = s % sps;                  // first slice of the step inside the activation stage
-                        if (!mbar_wait_abortable(cfull + 8u * cb, (ci / ncb) & 1u, abort) ||
-                            (sub == 0 && !mbar_wait_abortable(xfull + 8u * xs, (xi / nxs) & 1u, abort))) {
+                        if (!mbar_wait_abortable(cfull + 8u * cb, (ci / ncb) & 1u, abort) || !mbar_wait_abortable(xfull + 8u * xs, (xi / nxs) & 1u, abort)) {
                             fail(LUM_ST_WAIT_FULL); ok = false; break;
                         }
                         tc_fence_after_sync();
                         const uint32_t wt = tmem + kGmCvtCol0 + cb * kGmCvtCols;
-                        const uint32_t xb = x_base + xs * (uint32_t)kGmXStageMax + (uint32_t)sub * x_slice;
-                        if (!(a.debug & 2)) {
+                        const uint32_t xb = x_base + xs * (uint32_t)kGmXStageMax;
 #pragma unroll
-                            for (int kk = 0; kk < 2 * kGmStep; kk++) {     // K = 16 per instruction: two per 32-column slice
-                                // weights: tensor memory, 8 columns (16 binary16) per instruction; activations: shared memory,
-                                // [column group of 8][term][row][16 bytes], an instruction reads two adjacent column groups
-                                const uint32_t xo = xb + (uint32_t)(kk >> 1) * x_slice + (uint32_t)(kk & 1) * 2u * x_cg;
-                                const uint32_t x1 = x_lo | ((xo >> 4) & 0x3fffu), x2 = x_lo | (((xo + (uint32_t)nc * 16u) >> 4) & 0x3fffu);
+                        for (int kk = 0; kk < 2 * kGmStep; kk++) {     // K = 16 per instruction: two per 32-column slice
+                            // weights: tensor memory, 8 columns (16 binary16) per instruction; activations: shared memory,
+                            // [column group of 8][term][row][16 bytes], an instruction reads two adjacent column groups
+                            const uint32_t xo = xb + (uint32_t)(kk >> 1) * x_slice + (uint32_t)(kk & 1) * 2u * x_cg;
+                            const uint32_t x1 = x_lo | ((xo >> 4) & 0x3fffu), x2 = x_lo | (((xo + (uint32_t)nc * 16u) >> 4) & 0x3fffu);
 #pragma unroll
-                                for (int hb = 0; hb < kGmHB; hb++) {      // the 128-row tiles of the item
-                                    const uint32_t acc = tmem + (uint32_t)hb * 128u;
-                                    const uint32_t hi = wt + (uint32_t)(kk >> 1) * 32u * kGmHB + (uint32_t)hb * 32u + (uint32_t)(kk & 1) * 8u, lo = hi + 16u;
-                                    umma_f16_ts2(acc, hi, x1, x_hi, idesc_a, started);
-                                    if (wide) umma_f16_ts2(acc, hi, x2, x_hi, idesc_b, 1u);
-                                    umma_f16_ts2(acc, lo, x1, x_hi, idesc_b, 1u);
-                                }
-                                started = 1u;
+                            for (int hb = 0; hb < kGmHB; hb++) {      // the 128-row tiles of the item
+                                const uint32_t acc = tmem + (uint32_t)hb * 128u;
+                                const uint32_t hi = wt + (uint32_t)((kk >> 1) * kGmHB + hb) * 32u + (uint32_t)(kk & 1) * 8u;
+                                umma_f16_ts2(acc, hi, x1, x_hi, idesc, kk > 0 ? 1u : started);
+                                umma_f16_ts2(acc, hi, x2, x_hi, idesc, 1u);
+                                umma_f16_ts2(acc, hi + 16u, x1, x_hi, idesc, 1u);
                             }
                         }
+                        started = 1u;
                         umma_commit(cempty + 8u * cb);        // arrive when the instructions that read these operands have retired
+                        umma_commit(xempty + 8u * xs);
                         ci++;
-                        if (sub + kGmStep == sps) { umma_commit(xempty + 8u * xs); xi++; }
+                        xi++;
                     }
                 }
                 if (ok) umma_commit(afull);
@@ -381,74 +380,57 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
 
     // -------------------------------------------------------------------- converting / storing warps
     {
-        // A warp reaches the 32 tensor-memory lanes of its quarter: thread = weight row of a 128-row tile (lane of tensor memory); warps
-        // 0-3 take columns 0-15 of every 32-block, warps 4-7 columns 16-31 (and, for the store, the two halves of the chunk's rows).
-        // The weights come straight from global memory: a thread's 16 bytes of a slice are 16 consecutive columns of its row in the
-        // tile stream (8 rows x 16 bytes of a tile are contiguous: full 32-byte sectors), kGmAhead slices ahead of their use, in
-        // registers — no shared-memory staging, no copy engine, and the 139 KiB a staged K-tile of 256 rows would take go to the
-        // activation stages instead.
-        const int q = warp & 3, h = warp >> 2, ch = h;
+        // A warp reaches the 32 tensor-memory lanes of its quarter: thread = weight row of a 128-row tile; of a step's four operands (two
+        // slices of two tiles) it converts slice ss of tile hb (and stores half of that tile's sums).  The weights come straight from global
+        // memory: a thread's 2 x 16 bytes of a slice are the columns of its row in the tile stream (8 rows x 16 bytes of a tile are
+        // contiguous: full 32-byte sectors), kGmAhead steps ahead of their use, in registers — no shared-memory staging, no copy engine, and
+        // the 139 KiB a staged K-tile of 256 rows would take go to the activation stages instead.  A step is converted before its
+        // buffer is waited for: between "the tensor core has let go of it" and "it is full again" lie only the stores.
+        const int q = warp & 3, z = warp >> 2, hb = z >> 1, ss = z & 1;
         const int n = (q << 5) + lane, r = n & 7;                    // row inside a 128-row tile
         const uint32_t lane_addr = (uint32_t)(q << 5) << 16;
         uint32_t ci = 0, ic = 0;
         bool ok = true;
         for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ic++) {
             const GemmItem it = gemm_item(a, item, tpr);
-            const unsigned char* wseg = a.seg[it.seg].w;
-            const unsigned char* base[kGmHB];
-            bool live[kGmHB];
-#pragma unroll
-            for (int hb = 0; hb < kGmHB; hb++) {
-                const int g = (n >> 3) + hb * 16;
-                live[hb] = g < it.n_rg;                              // row groups past the matrix's end contribute zeros (and are never read)
-                base[hb] = wseg + (size_t)(it.rg0 + (live[hb] ? g : 0)) * tpr * kTileBytes;
-            }
-            uint4 rq[kGmAhead][kGmHB];
-            uint32_t rs[kGmAhead][kGmHB];
-            const int si0 = it.t0 * 16, si1 = it.t1 * 16;
-            auto fetch = [&](int si, uint4 (&dq)[kGmHB], uint32_t (&ds)[kGmHB]) {
-#pragma unroll
-                for (int hb = 0; hb < kGmHB; hb++) {
-                    const unsigned char* tile = base[hb] + (size_t)(si >> 4) * kTileBytes;
-                    dq[hb] = live[hb] ? __ldg((const uint4*)(tile + (si & 15) * 256 + h * 128 + r * 16)) : make_uint4(0u, 0u, 0u, 0u);
-                    ds[hb] = live[hb] ? (uint32_t)__ldg((const unsigned short*)(tile + kTileQ + ((si & 15) * 8 + r) * 2)) : 0u;
-                }
+            const int g = (n >> 3) + hb * 16;
+            const bool live = g < it.n_rg;                           // row groups past the matrix's end contribute zeros (and are never read)
+            const unsigned char* base = a.seg[it.seg].w + (size_t)(it.rg0 + (live ? g : 0)) * tpr * kTileBytes;
+            uint4 rq[kGmAhead][2];
+            uint32_t rs[kGmAhead];
+            const int si0 = it.t0 * 16 + ss, si1 = it.t1 * 16;
+            auto fetch = [&](int si, uint4 (&dq)[2], uint32_t& ds) {
+                const unsigned char* tile = base + (size_t)(si >> 4) * kTileBytes;
+                dq[0] = live ? __ldg((const uint4*)(tile + (si & 15) * 256 + r * 16)) : make_uint4(0u, 0u, 0u, 0u);
+                dq[1] = live ? __ldg((const uint4*)(tile + (si & 15) * 256 + 128 + r * 16)) : make_uint4(0u, 0u, 0u, 0u);
+                ds = live ? (uint32_t)__ldg((const unsigned short*)(tile + kTileQ + ((si & 15) * 8 + r) * 2)) : 0u;
             };
 #pragma unroll
-            for (int d = 0; d < kGmAhead; d++) fetch(si0 + d, rq[d], rs[d]);          // (an item holds whole K-tiles: at least 16 slices)
+            for (int d = 0; d < kGmAhead; d++) fetch(si0 + d * kGmStep, rq[d], rs[d]);          // (an item holds whole K-tiles: at least 16 slices)
 #pragma unroll 1
-            for (int si = si0; si < si1 && ok; si += kGmAhead) {
+            for (int si = si0; si < si1 && ok; si += kGmAhead * kGmStep) {
 #pragma unroll
-                for (int half = 0; half < kGmAhead / kGmStep; half++) {
+                for (int d = 0; d < kGmAhead; d++) {
                     const uint32_t cb = ci % ncb;
+                    const uint32_t dd = h2_mul(rs[d] | (rs[d] << 16), 0x64006400u);            // 1024 d, exact
+                    const uint32_t w8[8] = {rq[d][0].x, rq[d][0].y, rq[d][0].z, rq[d][0].w, rq[d][1].x, rq[d][1].y, rq[d][1].z, rq[d][1].w};
+                    uint32_t hi[16], lo[16];
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        // bytes (q + 128) into the mantissas of 1024 + (q + 128), two at a time; minus 1152 leaves q, exactly
+                        const uint32_t w = w8[j] ^ 0x80808080u;
+                        const uint32_t q0 = h2_sub(__byte_perm(w, 0x64646464u, 0x4140), 0x64806480u);
+                        const uint32_t q1 = h2_sub(__byte_perm(w, 0x64646464u, 0x4342), 0x64806480u);
+                        hi[2 * j] = h2_mul(q0, dd); hi[2 * j + 1] = h2_mul(q1, dd);
+                        lo[2 * j] = h2_fma(q0, dd, h2_neg(hi[2 * j]));             // q d' - hi: the rounding error of hi, exactly
+                        lo[2 * j + 1] = h2_fma(q1, dd, h2_neg(hi[2 * j + 1]));
+                    }
+                    if (si + (d + kGmAhead) * kGmStep < si1) fetch(si + (d + kGmAhead) * kGmStep, rq[d], rs[d]);     // this slot's next step
                     if (!mbar_wait_abortable(cempty + 8u * cb, ((ci / ncb) & 1u) ^ 1u, abort)) { fail(LUM_ST_WAIT_EMPTY); ok = false; break; }
                     tc_fence_after_sync();
-#pragma unroll
-                    for (int ss = 0; ss < kGmStep; ss++) {
-                        const int d = half * kGmStep + ss;
-                        if (!(a.debug & 1)) {
-#pragma unroll
-                            for (int hb = 0; hb < kGmHB; hb++) {
-                                const uint32_t d16 = rs[d][hb];
-                                const uint32_t dd = h2_mul(d16 | (d16 << 16), 0x64006400u);            // 1024 d, exact
-                                const uint32_t w4[4] = {rq[d][hb].x ^ 0x80808080u, rq[d][hb].y ^ 0x80808080u, rq[d][hb].z ^ 0x80808080u, rq[d][hb].w ^ 0x80808080u};
-                                uint32_t hi[8], lo[8];
-#pragma unroll
-                                for (int j = 0; j < 4; j++) {
-                                    // bytes (q + 128) into the mantissas of 1024 + (q + 128), two at a time; minus 1152 leaves q, exactly
-                                    const uint32_t q0 = h2_sub(__byte_perm(w4[j], 0x64646464u, 0x4140), 0x64806480u);
-                                    const uint32_t q1 = h2_sub(__byte_perm(w4[j], 0x64646464u, 0x4342), 0x64806480u);
-                                    hi[2 * j] = h2_mul(q0, dd); hi[2 * j + 1] = h2_mul(q1, dd);
-                                    lo[2 * j] = h2_fma(q0, dd, hi[2 * j] ^ 0x80008000u);             // q d' - hi: the rounding error of hi, exactly
-                                    lo[2 * j + 1] = h2_fma(q1, dd, hi[2 * j + 1] ^ 0x80008000u);
-                                }
-                                const uint32_t wt = tmem + lane_addr + kGmCvtCol0 + cb * kGmCvtCols + (uint32_t)ss * 32u * kGmHB + (uint32_t)hb * 32u + (uint32_t)h * 8u;
-                                tmem_st8(wt, hi);
-                                tmem_st8(wt + 16u, lo);
-                            }
-                        }
-                        if (si + d + kGmAhead < si1) fetch(si + d + kGmAhead, rq[d], rs[d]);     // this slot's next slice
-                    }
+                    const uint32_t wt = tmem + lane_addr + kGmCvtCol0 + cb * kGmCvtCols + (uint32_t)(ss * kGmHB + hb) * 32u;
+                    tmem_st16(wt, hi);
+                    tmem_st16(wt + 16u, lo);
                     tmem_st_wait();
                     tc_fence_before_sync();
                     __syncwarp();
@@ -462,24 +444,21 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
             if (a.use_pdl) pdl_grid_wait();              // (long over: the sums are there)
             tc_fence_after_sync();
             const GemmSeg& sg = a.seg[it.seg];
-            const int half_rows = nc >> 1;
-            const bool wide = nc == kGmMaxChunk;
-#pragma unroll 1
-            for (int hb = 0; hb < kGmHB; hb++) {
-                const int n_st = hb * 128 + n;
+            {
+                const int n_st = hb * 128 + n, m0 = it.mc * nc + ss * (nc / 2);      // this warp's half of the chunk's rows
                 const bool row_live = (n_st >> 3) < it.n_rg;
                 float* yp = a.y + (size_t)it.ks * a.part_stride + sg.col0 + it.rg0 * kTileRows + n_st;
-                for (int c0 = 0; c0 < half_rows; c0 += 16) {
-                    uint32_t v[16], v2[16];
-                    const uint32_t col = tmem + lane_addr + (uint32_t)hb * 128u + (uint32_t)(ch * half_rows + c0);
-                    tmem_ld16(col, v);
-                    if (!wide) tmem_ld16(col + (uint32_t)nc, v2);   // the x2 half of the accumulator
+#pragma unroll 1
+                for (int c0 = 0; c0 < nc / 2; c0 += 16) {
+                    uint32_t v[16];
+                    const float sx_lane = __ldcg(a.sx + m0 + c0 + (lane & 15));
+                    tmem_ld16(tmem + lane_addr + (uint32_t)hb * 128u + (uint32_t)(ss * (nc / 2) + c0), v);
                     tmem_ld_wait();
 #pragma unroll
                     for (int i = 0; i < 16; i++) {
-                        const int m = it.mc * nc + ch * half_rows + c0 + i;
-                        const float sum = wide ? __uint_as_float(v[i]) : __uint_as_float(v[i]) + __uint_as_float(v2[i]);
-                        if (row_live && m < a.M) yp[(size_t)m * a.ldy] = sum * __ldg(a.sx + m);
+                        const int m = m0 + c0 + i;
+                        const float sum = __uint_as_float(v[i]) * __shfl_sync(0xffffffffu, sx_lane, i);
+                        if (row_live && m < a.M) yp[(size_t)m * a.ldy] = sum;
                     }
                 }
             }
@@ -546,14 +525,6 @@ __device__ __forceinline__ int skinny_seg(const GemmArgs& a, int& g) {
     while (s < a.nseg - 1 && g >= a.seg[s].rows / kTileRows) { g -= a.seg[s].rows / kTileRows; s++; }
     return s;
 }
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
-                 "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]),
-                 "r"(v[14]), "r"(v[15])
-                 : "memory");
-}
-__device__ __forceinline__ uint32_t h2_neg(uint32_t a) { uint32_t d; asm("neg.f16x2 %0, %1;" : "=r"(d) : "r"(a)); return d; }
-
 // NC: activation rows of the chunk (a compile-time number: with the index arithmetic done at run time the issuing thread took 86 clocks per
 // instruction)
 template <int NC>
@@ -918,8 +889,6 @@ bool gemm_supported(const GemmArgs& a) {
 cudaError_t launch_gemm(const GemmArgs& a_in, int sm_count, cudaStream_t st) {
     GemmArgs a = a_in;
     a.nc = gemm_chunk_rows(a.M);
-    static const int env_debug = [] { const char* e = getenv("LUM_GEMM_DEBUG"); return e ? atoi(e) : 0; }();
-    a.debug = env_debug;
     a.m_chunks = (a.M + a.nc - 1) / a.nc;
     if (!gemm_supported(a)) return cudaErrorInvalidValue;
     // more than 64 rows (prompts): the tensor core is the resource; fewer (batched decode): the weight stream is

@@ -15,7 +15,6 @@ struct GemmArgs {
     const float* sx;         // [rows]: the power-of-two factor that turns a row's accumulators into its outputs
     int M, m_chunks, nc;     // nc: activation rows per chunk (set by the launcher)
     int row_chunks;          // up to 64 rows: runs of row groups (set by the launcher)
-    int debug;               // timing experiments only (LUM_GEMM_DEBUG): 1 = skip the weight conversion, 2 = skip the tensor-core instructions
     int ksplit;              // K ranges (whole K-tiles each); part i of the sums goes to y + i * part_stride
     float* y;
     int ldy;
