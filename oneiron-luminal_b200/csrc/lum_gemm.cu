@@ -26,11 +26,11 @@
 //  * rows_quantize — one CTA per activation row.  Forms the row (sum of the previous product's K-split partials, residual
 //    add, SwiGLU), optionally RMS-normalises it (`RowRMSNorm`, ops.rs:519-566; `RowSwishMul`, ops.rs:303-325; `RowAdd`,
 //    ops.rs:135-146 are fused here), writes the two terms in tensor-core operand order and the row's output factor.
-//  * q8_gemm_tc — 128 activation rows per chunk (prompts).  Persistent CTAs over work items (256 weight rows = two tensor-core tiles
+//  * q8_gemm_tc — 80 to 128 activation rows per chunk (prompts).  Persistent CTAs over work items (256 weight rows = two tensor-core tiles
 //    that share every activation slice, one chunk, one K range).  One lane fills a ring of six 32 KiB activation stages with bulk
 //    copies; 16 warps read their rows' weights straight from global memory (32 bytes per row and slice, two steps ahead, in
 //    registers), turn them into the hi / lo operands and store those to tensor memory (the A operand is read from there: shared
-//    memory and its bandwidth belong to the activation operand); one thread issues the tensor-core instructions (24 of N = 128 per
+//    memory and its bandwidth belong to the activation operand); one thread issues the tensor-core instructions (24 of N = chunk rows per
 //    step of two 32-column slices) and commits the buffers free; the 16 warps store the two accumulators when the K range is done.
 //    Bound by the tensor core, if everything else keeps up: 24 instructions of 65 clocks a step.  Measured, alone (issued TFLOP/s, 6 per
 //    weight and row; 8 warps that converted after the wait for their buffer / 16 that convert before it): 28672 x 4096 at 512 rows
@@ -48,7 +48,7 @@ namespace lum {
 
 constexpr int kGmHB = 2;                            // tensor-core tiles (128 weight rows) per work item; they share every activation slice
 constexpr int kGmRows = 128 * kGmHB;                // weight rows per work item
-constexpr int kGmMaxChunk = 128;                    // activation rows per chunk: 16, 32, 64 or 128 (gemm_chunk_rows)
+constexpr int kGmMaxChunk = 128;                    // activation rows per chunk: 16, 32 or 64, or (q8_gemm_tc) 80 .. 128 (gemm_shape)
 constexpr int kGmXTerms = 2;                        // binary16 terms per activation element
 constexpr int kGmStep = 2;                          // 32-column slices per hand-over between the warps (every hand-over costs each single-threaded role
                                                     // several hundred cycles of its own, whatever the amount of work behind it)
@@ -64,9 +64,6 @@ constexpr size_t kGmSmem = kGmBarBytes + 128 + (size_t)kGmXStages * kGmXStageMax
 constexpr int kGmWExp = 10;                         // weights enter as 2^10 w
 constexpr uint32_t kGmTmemCols = 512;               // one accumulator of 128 columns per 128-row tile, then the converted-weight buffers
 constexpr uint32_t kGmCvtCol0 = 128 * kGmHB;
-
-// activation rows per chunk for a product of M rows
-__host__ __device__ inline int gemm_chunk_rows(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128; }
 
 __device__ __forceinline__ float block_max(float v, float* scratch, int tid, int nthreads, int bar_id) {
 #pragma unroll
@@ -95,7 +92,7 @@ __global__ void __launch_bounds__(256) rows_quantize(const RowsArgs a, const int
     const int s0 = (int)((long long)nb * part / C), s1 = (int)((long long)nb * (part + 1) / C);     // this CTA's slices
     const int k0 = s0 << 5, n4 = (s1 - s0) << 3;             // its first column, its float4
     if (a.use_pdl) { pdl_launch_dependents(); pdl_grid_wait(); }
-    const int nc = gemm_chunk_rows(a.M);
+    const int nc = a.nc;
     const size_t slice_bytes = (size_t)kGmXTerms * 4 * nc * 16;
     unsigned char* xq_chunk = (unsigned char*)a.xq + (size_t)(m / nc) * nb * slice_bytes;
     const int ml = m % nc;
@@ -285,9 +282,9 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
     if (a.use_pdl) pdl_launch_dependents();
 
     const int tpr = a.K / kTileK, nb = a.K >> 5;
-    constexpr int nc = kGmMaxChunk;                        // activation rows per chunk
-    constexpr uint32_t x_cg = (uint32_t)kGmXTerms * (uint32_t)nc * 16u;      // bytes of one column group of a slice: both terms' rows
-    constexpr uint32_t x_slice = 4u * x_cg;
+    const int nc = a.nc;                                   // activation rows per chunk
+    const uint32_t x_cg = (uint32_t)kGmXTerms * (uint32_t)nc * 16u;      // bytes of one column group of a slice: both terms' rows
+    const uint32_t x_slice = 4u * x_cg;
     constexpr uint32_t ncb = kGmCvtBufs, nxs = kGmXStages;
     constexpr int sps = kGmStep;                           // slices per activation stage: one step, one 32 KiB copy
     int tiles = 0;
@@ -325,11 +322,11 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
         if (elect_one()) {
             uint32_t xi = 0, ci = 0, ic = 0;
             bool ok = true;
-            // hi x1, hi x2, lo x1 as three instructions of N = 128 into one accumulator
-            constexpr uint32_t idesc = umma_idesc_f16(128, nc);
+            // hi x1, hi x2, lo x1 as three instructions of N = nc into one accumulator
+            const uint32_t idesc = umma_idesc_f16(128, nc);
             // activation operand descriptors: start address in the low 14 bits; column groups x_cg bytes apart, 8-row groups 128
-            constexpr uint32_t x_lo = ((x_cg >> 4) & 0x3fffu) << 16, x_hi = umma_desc_hi(128u);
-            const uint32_t x_base = smem_u32(xst);
+            const uint32_t x_lo = ((x_cg >> 4) & 0x3fffu) << 16, x_base = smem_u32(xst);
+            constexpr uint32_t x_hi = umma_desc_hi(128u);
             for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ic++) {
                 const GemmItem it = gemm_item(a, item, tpr);
                 if (!mbar_wait_abortable(aempty, (ic & 1u) ^ 1u, abort)) { fail(LUM_ST_WAIT_TMEM); break; }      // the previous item's sums were stored
@@ -445,14 +442,14 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
             tc_fence_after_sync();
             const GemmSeg& sg = a.seg[it.seg];
             {
-                const int n_st = hb * 128 + n, m0 = it.mc * nc + ss * (nc / 2);      // this warp's half of the chunk's rows
+                const int n_st = hb * 128 + n, m0 = it.mc * nc;          // this warp's half of the chunk's rows: every second block of 16
                 const bool row_live = (n_st >> 3) < it.n_rg;
                 float* yp = a.y + (size_t)it.ks * a.part_stride + sg.col0 + it.rg0 * kTileRows + n_st;
 #pragma unroll 1
-                for (int c0 = 0; c0 < nc / 2; c0 += 16) {
+                for (int c0 = 16 * ss; c0 < nc; c0 += 32) {
                     uint32_t v[16];
                     const float sx_lane = __ldcg(a.sx + m0 + c0 + (lane & 15));
-                    tmem_ld16(tmem + lane_addr + (uint32_t)hb * 128u + (uint32_t)(ss * (nc / 2) + c0), v);
+                    tmem_ld16(tmem + lane_addr + (uint32_t)hb * 128u + (uint32_t)c0, v);
                     tmem_ld_wait();
 #pragma unroll
                     for (int i = 0; i < 16; i++) {
@@ -785,8 +782,10 @@ __global__ void __launch_bounds__(kGsThreads, 1) q8_gemm_tc_skinny(const GemmArg
 
 // ---------------------------------------------------------------------------------------------------------- host side
 
-size_t gemm_xq_bytes(int M, int K) { const int nc = gemm_chunk_rows(M); return (size_t)((M + nc - 1) / nc) * nc * K * 2 * kGmXTerms; }
-size_t gemm_sx_bytes(int M, int K) { (void)K; const int nc = gemm_chunk_rows(M); return (size_t)((M + nc - 1) / nc) * nc * 4; }
+// rows of the activation operand: M and what fills the last chunk, whatever the chunk
+static int gemm_padded_rows(int M) { return M <= 64 ? 64 : M + kGmMaxChunk - 1; }
+size_t gemm_xq_bytes(int M, int K) { return (size_t)gemm_padded_rows(M) * K * 2 * kGmXTerms; }
+size_t gemm_sx_bytes(int M, int K) { (void)K; return (size_t)gemm_padded_rows(M) * 4; }
 
 // Up to 64 rows: K ranges and runs of row groups of a product.  An SM's time for one K-tile of n row groups is the largest of: its
 // share of HBM (4352 n bytes at 44 GB/s), the conversion (kGsCvtUs per tensor-core tile), and what comes
@@ -815,33 +814,51 @@ static SkinnyPlan gemm_plan(int groups, int nc, int K, int sms) {
     return best;
 }
 
-// More rows: K ranges per product.  Work items are equal, so a product takes ceil(items / SMs) rounds of one item each: with few items per SM
-// the last, partly filled round is a large share of the time (224 tiles over 148 SMs: 2 rounds for 1.5 rounds of work).  Cutting K
-// makes the rounds shorter and the loss smaller, but every item pays its own pipeline fill and store, and every extra range
-// writes (and the consumer reads) another plane of partial sums.  The estimate below weighs the three; its constants are
-// measured orders of magnitude (a K-tile of one item: 14 us at 256 weight rows; an item's own cost: a third of a
-// tile; plane traffic at the HBM copy rate), not a fit.
-int gemm_pick_ksplit(int n_rows_total, int M, int K, int sm_count) {
-    const int nc = gemm_chunk_rows(M);
-    if (nc < kGmMaxChunk) return gemm_plan(n_rows_total / kTileRows, nc, K, sm_count).ks;
-    const int tiles = (n_rows_total + kGmRows - 1) / kGmRows, mc = (M + nc - 1) / nc, tpr = K / kTileK;
-    const double t_tile = 14.4;                                                   // us per K-tile of one item
+// More rows: rows per chunk and K ranges per product.  Work items are equal, so a product takes ceil(items / SMs) rounds of one item each: with few
+// items per SM the last, partly filled round is a large share of the time (448 items over 148 SMs: 4 rounds for 3.03 rounds of work), and so are the
+// rows that fill up the last chunk (387 rows in chunks of 128: a quarter).  Smaller chunks and more K ranges make both finer, but every item pays
+// its own pipeline fill and store, every extra range writes (and the consumer reads) another plane of partial sums, and the
+// converting warps set a floor.  Constants: measured, us per K-tile of one item (28672 x 4096 in chunks of 80 / 112 / 128 rows: 6.6 / 8.1 / 8.75),
+// an item's own cost a third of that, planes at the HBM copy rate.  An
+// accumulator's additions are cut to 24 bits, so longer ranges cost accuracy: the split that the first estimate gives (chunks of 128, items of 14 us
+// per K-tile) is never undercut.
+// Measured, alone, us (chunks of 128 / as chosen): 28672 x 4096 at 65 rows 74 / 58, 129 rows 143 / 109, 387 rows 264 / 231, 1000 rows 487 / 449.
+static GemmShape gemm_shape_wide(int n_rows_total, int M, int K, int sm_count) {
+    const int tiles = (n_rows_total + kGmRows - 1) / kGmRows, tpr = K / kTileK;
     const double plane_us = (double)M * n_rows_total * 8.0 / 6.5e6;               // write + read of one plane of partial sums
-    int best = 1;
-    double best_t = 1e30;
-    for (int ks = 1; ks <= 8 && ks <= tpr; ks++) {
-        const long long items = (long long)tiles * mc * ks;
+    auto cost = [&](int nc, int ks, double t_tile) {
+        const long long items = (long long)tiles * ((M + nc - 1) / nc) * ks;
         const long long rounds = (items + sm_count - 1) / sm_count;
-        const double t = (double)rounds * ((double)tpr / ks + 0.33) * t_tile + (ks - 1) * plane_us;
-        if (t < best_t * 0.97) { best_t = t; best = ks; }                         // a larger split has to pay for itself
+        return (double)rounds * ((double)((tpr + ks - 1) / ks) * t_tile + 0.33 * t_tile) + (ks - 1) * plane_us;
+    };
+    int least = 1;
+    for (int ks = 2; ks <= 8 && ks <= tpr; ks++) {
+        auto first = [&](int k) {
+            const long long rounds = ((long long)tiles * ((M + kGmMaxChunk - 1) / kGmMaxChunk) * k + sm_count - 1) / sm_count;
+            return (double)rounds * ((double)tpr / k + 0.33) * 14.4 + (k - 1) * plane_us;
+        };
+        if (first(ks) < first(least) * 0.97) least = ks;                          // a larger split has to pay for itself
     }
+    GemmShape best{kGmMaxChunk, least};
+    auto tile = [](int nc) { return 2.9 + 5.85 * nc / kGmMaxChunk; };
+    double best_t = cost(kGmMaxChunk, least, tile(kGmMaxChunk));
+    for (int nc = kGmMaxChunk; nc >= 80; nc -= 16)
+        for (int ks = least; ks <= 8 && ks <= tpr; ks++) {
+            const double t = cost(nc, ks, tile(nc));
+            if (t < best_t * 0.98) { best_t = t; best = {nc, ks}; }
+        }
     return best;
+}
+GemmShape gemm_shape(int n_rows_total, int M, int K, int sm_count) {
+    if (M > 64) return gemm_shape_wide(n_rows_total, M, K, sm_count);
+    const int nc = M <= 16 ? 16 : M <= 32 ? 32 : 64;
+    return {nc, gemm_plan(n_rows_total / kTileRows, nc, K, sm_count).ks};
 }
 
 cudaError_t launch_rows_quantize(const RowsArgs& a_in, cudaStream_t st) {
     RowsArgs a = a_in;
-    if (a.M <= 0 || a.K <= 0 || (a.K % 32) || a.n_parts < 1) return cudaErrorInvalidValue;
-    const int nc = gemm_chunk_rows(a.M);
+    if (a.M <= 0 || a.K <= 0 || (a.K % 32) || a.n_parts < 1 || a.nc < 16 || a.nc > kGmMaxChunk || a.nc % 16) return cudaErrorInvalidValue;
+    const int nc = a.nc;
     const int rows = (a.M + nc - 1) / nc * nc;            // padding rows of the last chunk are zeroed by their own CTAs
     // CTAs per row: up to eight while the rows alone leave SMs idle, of at least eight slices each
     int C = 1;
@@ -888,11 +905,11 @@ bool gemm_supported(const GemmArgs& a) {
 
 cudaError_t launch_gemm(const GemmArgs& a_in, int sm_count, cudaStream_t st) {
     GemmArgs a = a_in;
-    a.nc = gemm_chunk_rows(a.M);
+    if (a.M <= 0 || (a.M <= 64 ? a.nc != 16 && a.nc != 32 && a.nc != 64 : a.nc < 80) || a.nc > kGmMaxChunk || a.nc % 16 || (a.M <= 64 && a.nc < a.M)) return cudaErrorInvalidValue;
     a.m_chunks = (a.M + a.nc - 1) / a.nc;
     if (!gemm_supported(a)) return cudaErrorInvalidValue;
     // more than 64 rows (prompts): the tensor core is the resource; fewer (batched decode): the weight stream is
-    const bool wide = a.nc == kGmMaxChunk;
+    const bool wide = a.nc > 64;
     const void* fn = wide ? (const void*)q8_gemm_tc : a.nc == 16 ? (const void*)q8_gemm_tc_skinny<16> : a.nc == 32 ? (const void*)q8_gemm_tc_skinny<32> : (const void*)q8_gemm_tc_skinny<64>;
     const size_t smem = wide ? kGmSmem : kGsSmem;
     const int threads = wide ? kGmThreads : kGsThreads;
@@ -946,7 +963,7 @@ __global__ void gemm_sum_parts(const float* parts, int n_parts, size_t part_stri
 extern "C" size_t lum_op_gemm_q8_0_workspace(int32_t n, int32_t k, int32_t m) {
     using namespace lum;
     if (n <= 0 || k <= 0 || m <= 0 || k % kTileK || n % kTileRows) return 0;
-    const int ks = gemm_pick_ksplit(n, m, k, 148);
+    const int ks = gemm_shape(n, m, k, 148).ks;
     return gemm_xq_bytes(m, k) + gemm_sx_bytes(m, k) + (size_t)ks * m * n * 4 + 1024;
 }
 
@@ -973,12 +990,13 @@ extern "C" int32_t lum_op_gemm_q8_0_packed(const void* packed, int32_t n, int32_
         if (cudaMalloc((void**)&status[dev], 4) != cudaSuccess) { set_op_error("gemm_q8_0_packed: status word"); return -5; }
         cudaMemset(status[dev], 0, 4);
     }
+    const GemmShape shape = gemm_shape(n, m, k, 148);
     RowsArgs r{};
-    r.a = x; r.n_parts = 1; r.part_stride = 0; r.ld = k; r.M = m; r.K = k; r.xq = xq; r.sx = sx;
+    r.nc = shape.nc; r.a = x; r.n_parts = 1; r.part_stride = 0; r.ld = k; r.M = m; r.K = k; r.xq = xq; r.sx = sx;
     cudaError_t e = launch_rows_quantize(r, st);
     GemmArgs g{};
     g.nseg = 1; g.seg[0] = {(const unsigned char*)packed, n, 0}; g.K = k; g.xq = xq; g.sx = sx; g.M = m;
-    g.ksplit = gemm_pick_ksplit(n, m, k, 148);
+    g.nc = shape.nc; g.ksplit = shape.ks;
     g.y = g.ksplit > 1 ? parts : y; g.ldy = n; g.part_stride = (size_t)m * n; g.status = status[dev];
     if (e == cudaSuccess) e = launch_gemm(g, sms, st);
     if (e == cudaSuccess && g.ksplit > 1) {

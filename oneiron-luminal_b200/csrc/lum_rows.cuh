@@ -13,7 +13,7 @@ struct GemmArgs {
     int K;
     const int8_t* xq;        // activation operand as rows_quantize writes it: three binary16 terms per element, tensor-core order
     const float* sx;         // [rows]: the power-of-two factor that turns a row's accumulators into its outputs
-    int M, m_chunks, nc;     // nc: activation rows per chunk (set by the launcher)
+    int M, nc, m_chunks;     // nc: activation rows per chunk, as the rows were written (gemm_shape); m_chunks is set by the launcher
     int row_chunks;          // up to 64 rows: runs of row groups (set by the launcher)
     int ksplit;              // K ranges (whole K-tiles each); part i of the sums goes to y + i * part_stride
     float* y;
@@ -31,7 +31,7 @@ struct RowsArgs {
     const float* resid; int resid_ld;
     float* out; int out_ld;                          // optional: the formed rows (the new residual stream), before the norm
     const void* gain; int gain_kind; float eps;      // RMSNorm gains (null: none)
-    int M, K;
+    int M, K, nc;                                    // nc: rows per chunk of the operand (gemm_shape of the product that reads it)
     int8_t* xq; float* sx;
     int use_pdl;
 };
@@ -75,7 +75,8 @@ struct ArgmaxRowsArgs {
 
 size_t gemm_xq_bytes(int M, int K);
 size_t gemm_sx_bytes(int M, int K);
-int gemm_pick_ksplit(int n_rows_total, int M, int K, int sm_count);
+struct GemmShape { int nc, ks; };                // activation rows per chunk, K ranges
+GemmShape gemm_shape(int n_rows_total, int M, int K, int sm_count);
 bool gemm_supported(const GemmArgs& a);
 cudaError_t launch_rows_quantize(const RowsArgs& a, cudaStream_t st);
 cudaError_t launch_gemm(const GemmArgs& a, int sm_count, cudaStream_t st);

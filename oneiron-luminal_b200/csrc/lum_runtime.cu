@@ -1123,7 +1123,7 @@ bool rows_supported(const lum_rt* rt) {
 size_t rows_parts_floats(const lum_rt* rt, int n_out, int K, int cap) {
     size_t worst = 0;
     for (int m = 1; m <= cap; m++) {
-        const size_t need = (size_t)gemm_pick_ksplit(n_out, m, K, rt->sm_count) * m * n_out;
+        const size_t need = (size_t)gemm_shape(n_out, m, K, rt->sm_count).ks * m * n_out;
         if (need > worst) worst = need;
     }
     return worst;
@@ -1390,13 +1390,13 @@ int run_rows(lum_rt* rt, int M, int* d_tok, int* d_pos, const int* d_seq, int se
     const int H = d.hidden, hd = d.head_dim, qd = rt->nq_l * hd, kvd = rt->nkv_l * hd, W = qd + 2 * kvd, F = rt->ffn_l;
     const int gk = kind_of(d.embed_dtype), sms = rt->sm_count, pdl = rt->cfg.use_pdl != 0;
     cudaStream_t st = rt->stream;
-    const int ks_qkv = gemm_pick_ksplit(W, M, H, sms), ks_o = gemm_pick_ksplit(H, M, qd, sms), ks_gu = gemm_pick_ksplit(2 * F, M, H, sms),
-              ks_dn = gemm_pick_ksplit(H, M, F, sms);
+    const GemmShape g_qkv = gemm_shape(W, M, H, sms), g_o = gemm_shape(H, M, qd, sms), g_gu = gemm_shape(2 * F, M, H, sms), g_dn = gemm_shape(H, M, F, sms);
+    const int ks_qkv = g_qkv.ks, ks_o = g_o.ks, ks_gu = g_gu.ks, ks_dn = g_dn.ks;
     CU(rt, launch_embed_rows(rt->embed.w, rt->embed.kind, H, d.vocab, d_tok, b.xr, M, rt->status, st));
     uint64_t launches = 1;
-    auto quant = [&](RowsArgs& r, int K) -> cudaError_t { r.M = M; r.K = K; r.xq = b.xq; r.sx = b.sx; r.use_pdl = pdl; launches++; return launch_rows_quantize(r, st); };
-    auto gemm = [&](GemmArgs& g, int K, int ks, float* y, int ldy) -> cudaError_t {
-        g.K = K; g.xq = b.xq; g.sx = b.sx; g.M = M; g.ksplit = ks; g.y = y; g.ldy = ldy; g.part_stride = (size_t)M * ldy; g.status = rt->status; g.use_pdl = pdl;
+    auto quant = [&](RowsArgs& r, int K, GemmShape gs) -> cudaError_t { r.M = M; r.K = K; r.nc = gs.nc; r.xq = b.xq; r.sx = b.sx; r.use_pdl = pdl; launches++; return launch_rows_quantize(r, st); };
+    auto gemm = [&](GemmArgs& g, int K, GemmShape gs, float* y, int ldy) -> cudaError_t {
+        g.K = K; g.xq = b.xq; g.sx = b.sx; g.M = M; g.nc = gs.nc; g.ksplit = gs.ks; g.y = y; g.ldy = ldy; g.part_stride = (size_t)M * ldy; g.status = rt->status; g.use_pdl = pdl;
         launches++;
         return launch_gemm(g, sms, st);
     };
@@ -1407,13 +1407,13 @@ int run_rows(lum_rt* rt, int M, int* d_tok, int* d_pos, const int* d_seq, int se
             if (l == 0) { r.a = b.xr; r.n_parts = 1; r.ld = H; }
             else { r.a = b.down; r.n_parts = ks_dn; r.part_stride = (size_t)M * H; r.ld = H; r.resid = b.xr; r.resid_ld = H; r.out = b.xr; r.out_ld = H; }
             r.gain = w.attn_norm.w; r.gain_kind = gk; r.eps = rt->eps6;
-            CU(rt, quant(r, H));
+            CU(rt, quant(r, H, g_qkv));
             GemmArgs g{};
             g.nseg = 3;
             g.seg[0] = {(const unsigned char*)w.q.w, (int)w.q.rows, 0};
             g.seg[1] = {(const unsigned char*)w.k.w, (int)w.k.rows, qd};
             g.seg[2] = {(const unsigned char*)w.v.w, (int)w.v.rows, qd + kvd};
-            CU(rt, gemm(g, H, ks_qkv, b.qkv, W));
+            CU(rt, gemm(g, H, g_qkv, b.qkv, W));
         }
         {
             RopeRowsArgs t{};
@@ -1438,29 +1438,29 @@ int run_rows(lum_rt* rt, int M, int* d_tok, int* d_pos, const int* d_seq, int se
         {   // attention output -> operand of the o projection
             RowsArgs r{};
             r.a = b.attn; r.n_parts = 1; r.ld = qd;
-            CU(rt, quant(r, qd));
+            CU(rt, quant(r, qd, g_o));
             GemmArgs g{};
             g.nseg = 1; g.seg[0] = {(const unsigned char*)w.o.w, (int)w.o.rows, 0};
-            CU(rt, gemm(g, qd, ks_o, b.o, H));
+            CU(rt, gemm(g, qd, g_o, b.o, H));
         }
         {   // residual add -> RMSNorm -> operand of gate | up
             RowsArgs r{};
             r.a = b.o; r.n_parts = ks_o; r.part_stride = (size_t)M * H; r.ld = H; r.resid = b.xr; r.resid_ld = H; r.out = b.xr; r.out_ld = H;
             r.gain = w.mlp_norm.w; r.gain_kind = gk; r.eps = rt->eps6;
-            CU(rt, quant(r, H));
+            CU(rt, quant(r, H, g_gu));
             GemmArgs g{};
             g.nseg = 2;
             g.seg[0] = {(const unsigned char*)w.gate.w, (int)w.gate.rows, 0};
             g.seg[1] = {(const unsigned char*)w.up.w, (int)w.up.rows, F};
-            CU(rt, gemm(g, H, ks_gu, b.gu, 2 * F));
+            CU(rt, gemm(g, H, g_gu, b.gu, 2 * F));
         }
         {   // SwiGLU -> operand of the down projection
             RowsArgs r{};
             r.a = b.gu; r.b = b.gu + F; r.n_parts = ks_gu; r.part_stride = (size_t)M * 2 * F; r.ld = 2 * F;
-            CU(rt, quant(r, F));
+            CU(rt, quant(r, F, g_dn));
             GemmArgs g{};
             g.nseg = 1; g.seg[0] = {(const unsigned char*)w.down.w, (int)w.down.rows, 0};
-            CU(rt, gemm(g, F, ks_dn, b.down, H));
+            CU(rt, gemm(g, F, g_dn, b.down, H));
         }
     }
     if (head == 1) {
@@ -1488,12 +1488,13 @@ int run_rows(lum_rt* rt, int M, int* d_tok, int* d_pos, const int* d_seq, int se
         RowsArgs r{};
         r.a = b.down; r.n_parts = ks_dn; r.part_stride = (size_t)M * H; r.ld = H; r.resid = b.xr; r.resid_ld = H; r.out = b.xr; r.out_ld = H;
         r.gain = rt->final_norm.w; r.gain_kind = gk; r.eps = rt->eps6;
-        CU(rt, quant(r, H));
-        const int V = rt->vocab_l, ks_v = gemm_pick_ksplit(V, M, H, sms);
+        const int V = rt->vocab_l;
+        const GemmShape g_v = gemm_shape(V, M, H, sms);
+        CU(rt, quant(r, H, g_v));
         GemmArgs g{};
         g.nseg = 1; g.seg[0] = {(const unsigned char*)rt->lm_head.w, V, 0};
-        CU(rt, gemm(g, H, ks_v, b.logits, V));
-        if (int r2 = batch_sample(rt, M, d_tok, d_pos, d_seq, ks_v, &launches)) return r2;
+        CU(rt, gemm(g, H, g_v, b.logits, V));
+        if (int r2 = batch_sample(rt, M, d_tok, d_pos, d_seq, g_v.ks, &launches)) return r2;
     }
     rt->n_launches += launches;
     return 0;
@@ -1511,7 +1512,7 @@ int want_row(lum_rt* rt, int m, int M, size_t slot) {
     a.nseg = 1; a.seg[0] = {hw.w, hw.s, (int)hw.rows, hw.kc};
     a.K = H; a.epi = EPI_STORE; a.gain = rt->final_norm.w; a.y = rt->want_logits + slot * rt->vocab_l;
     a.x = b.xr + (size_t)m * H;
-    a.parts = b.down + (size_t)m * H; a.n_parts = gemm_pick_ksplit(H, M, rt->ffn_l, rt->sm_count); a.part_stride = M * H;
+    a.parts = b.down + (size_t)m * H; a.n_parts = gemm_shape(H, M, rt->ffn_l, rt->sm_count).ks; a.part_stride = M * H;
     CU(rt, launch_gemv(a, rt->sm_count, rt->stream));
     rt->n_launches++;
     return 0;

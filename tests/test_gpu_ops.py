@@ -283,6 +283,8 @@ GEMM_KAT = [
     (2176, 2048, 31, "integers"),     # 272 row groups: runs of one and of two tensor-core tiles
     (384, 2560, 64, "random"),        # K = 5 tiles (Qwen hidden)
     (2048, 512, 200, "random"),       # many activation chunks per weight tile
+    (7936, 1024, 65, "random"),       # the smallest chunk of the prompt kernel: 80 rows, 15 of them padding
+    (2304, 2048, 387, "integers"),    # chunks that are not a multiple of 32
 ]
 
 
