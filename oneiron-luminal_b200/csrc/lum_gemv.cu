@@ -15,7 +15,7 @@
 //    The weight stream does not depend on the activations, so under programmatic dependent launch the producer
 //    starts filling the ring while the previous kernel is still running; only the other warps wait for the
 //    grid dependency.
-//  * gemv_direct — any K, f32 / bf16 / Q8_0 weights, one warp per row with plain vector loads.
+//  * gemv_direct — any K, f32 / bf16 / Q8_0 weights, plain vector loads, one warp per row (bf16: per four rows).
 //    Used for the small all-f32 model and for shapes the streaming kernel does not take.
 //
 // Both fuse the RMSNorm that precedes the projection (`RowRMSNorm`, ops.rs:519-566; math per
@@ -132,6 +132,37 @@ __global__ void __launch_bounds__(kGemvThreads, 1) q8_gemv_stream(const GemvArgs
 
 // ------------------------------------------------------------------------------ direct kernel
 
+// N bf16 rows of 8 n8 elements (per lane; the caller folds the lanes).  A vocabulary-sized bf16 matrix (a head tied to the embedding) is hundreds
+// of megabytes per token and must stream: 2 N 16-byte loads in flight per lane, and the activations' reads from shared memory — twice the
+// bytes of a row's weights, which for one row at a time is what binds the SM — shared by the N rows.
+template <int N>
+__device__ __forceinline__ void bf16_rows_dot(const uint4* const (&w)[N], int n8, const float* xs, int lane, float (&acc)[N]) {
+    auto dot8 = [](uint4 a, float4 x0, float4 x1, float s) {
+        s = fmaf(__uint_as_float(a.x << 16), x0.x, s); s = fmaf(__uint_as_float(a.x & 0xffff0000u), x0.y, s);
+        s = fmaf(__uint_as_float(a.y << 16), x0.z, s); s = fmaf(__uint_as_float(a.y & 0xffff0000u), x0.w, s);
+        s = fmaf(__uint_as_float(a.z << 16), x1.x, s); s = fmaf(__uint_as_float(a.z & 0xffff0000u), x1.y, s);
+        s = fmaf(__uint_as_float(a.w << 16), x1.z, s); s = fmaf(__uint_as_float(a.w & 0xffff0000u), x1.w, s);
+        return s;
+    };
+    int i = lane;
+    for (; i + 32 < n8; i += 64) {
+        uint4 a[N], b[N];
+#pragma unroll
+        for (int r = 0; r < N; r++) { a[r] = __ldcs(w[r] + i); b[r] = __ldcs(w[r] + i + 32); }
+        float4 x0 = *(const float4*)(xs + (size_t)i * 8), x1 = *(const float4*)(xs + (size_t)i * 8 + 4);
+#pragma unroll
+        for (int r = 0; r < N; r++) acc[r] = dot8(a[r], x0, x1, acc[r]);
+        x0 = *(const float4*)(xs + (size_t)(i + 32) * 8); x1 = *(const float4*)(xs + (size_t)(i + 32) * 8 + 4);
+#pragma unroll
+        for (int r = 0; r < N; r++) acc[r] = dot8(b[r], x0, x1, acc[r]);
+    }
+    if (i < n8) {
+        const float4 x0 = *(const float4*)(xs + (size_t)i * 8), x1 = *(const float4*)(xs + (size_t)i * 8 + 4);
+#pragma unroll
+        for (int r = 0; r < N; r++) acc[r] = dot8(__ldcs(w[r] + i), x0, x1, acc[r]);
+    }
+}
+
 template <int WK>
 __device__ __forceinline__ float row_dot(const GemvSeg& sg, int row, int K, const float* xs, int lane) {
     float acc = 0.0f;
@@ -179,25 +210,10 @@ __device__ __forceinline__ float row_dot(const GemvSeg& sg, int row, int K, cons
     } else {
         const uint16_t* w = (const uint16_t*)sg.w + (size_t)row * K;
         if ((K & 7) == 0) {
-            // 16-byte loads (8 weights), two in flight per lane: a vocabulary-sized bf16 matrix (a head tied to the embedding) is
-            // hundreds of megabytes per token and must stream
-            const uint4* w8 = (const uint4*)w;
-            const int n8 = K >> 3;
-            auto dot8 = [&](uint4 a, int i, float s) {
-                const float4 x0 = *(const float4*)(xs + (size_t)i * 8), x1 = *(const float4*)(xs + (size_t)i * 8 + 4);
-                s = fmaf(__uint_as_float(a.x << 16), x0.x, s); s = fmaf(__uint_as_float(a.x & 0xffff0000u), x0.y, s);
-                s = fmaf(__uint_as_float(a.y << 16), x0.z, s); s = fmaf(__uint_as_float(a.y & 0xffff0000u), x0.w, s);
-                s = fmaf(__uint_as_float(a.z << 16), x1.x, s); s = fmaf(__uint_as_float(a.z & 0xffff0000u), x1.y, s);
-                s = fmaf(__uint_as_float(a.w << 16), x1.z, s); s = fmaf(__uint_as_float(a.w & 0xffff0000u), x1.w, s);
-                return s;
-            };
-            int i = lane;
-            for (; i + 32 < n8; i += 64) {
-                const uint4 a = __ldcs(w8 + i), b = __ldcs(w8 + i + 32);
-                acc = dot8(a, i, acc);
-                acc = dot8(b, i + 32, acc);
-            }
-            if (i < n8) acc = dot8(__ldcs(w8 + i), i, acc);
+            const uint4* const w8[1] = {(const uint4*)w};
+            float r[1] = {0.0f};
+            bf16_rows_dot<1>(w8, K >> 3, xs, lane, r);
+            acc = r[0];
         } else {
             for (int i = lane; i < K; i += 32) acc = fmaf(bf16_bits_to_f32(w[i]), xs[i], acc);
         }
@@ -205,8 +221,9 @@ __device__ __forceinline__ float row_dot(const GemvSeg& sg, int row, int K, cons
     return warp_sum(acc);
 }
 
+constexpr int kDirectBf16Ctas = 3;                     // resident CTAs per SM of the bf16 form (four rows' loads in registers)
 template <int WK>
-__global__ void __launch_bounds__(256) gemv_direct(const GemvArgs a) {
+__global__ void __launch_bounds__(256, WK == WK_BF16 ? kDirectBf16Ctas : 0) gemv_direct(const GemvArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const bool paired = a.epi == EPI_SWIGLU;
@@ -226,13 +243,40 @@ __global__ void __launch_bounds__(256) gemv_direct(const GemvArgs a) {
     gemv_load_x(a, xs, tid, 256, scratch, 1);
 
     const int sub = paired ? 2 : 1;
-    for (int i = warp; i < n * sub; i += 8) {
-        const int h = i / n, r = i - h * n;
-        int row = row0 + r, sg = 0;
-        if (paired) sg = h;
-        else while (sg < a.nseg - 1 && row >= a.seg[sg].rows) { row -= a.seg[sg].rows; sg++; }
-        const float v = row_dot<WK>(a.seg[sg], row, a.K, xs, lane);
-        if (lane == 0) vals[i] = v;
+    auto row_of = [&](int i, int* sg) {
+        const int h = i / n;
+        int row = row0 + i - h * n;
+        *sg = 0;
+        if (paired) *sg = h;
+        else while (*sg < a.nseg - 1 && row >= a.seg[*sg].rows) { row -= a.seg[*sg].rows; (*sg)++; }
+        return row;
+    };
+    if (WK == WK_BF16 && (a.K & 7) == 0) {
+        // four rows at a time: vocabulary projection of 151936 x 2560 (778 MB) 222 us with one, 125 us = 6.2 TB/s with four
+        for (int i0 = warp * 4; i0 < n * sub; i0 += 32) {
+            const uint4* w[4];
+            float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                int sg;
+                const int row = row_of(min(i0 + r, n * sub - 1), &sg);         // (rows past the end: the last one again, not stored)
+                w[r] = (const uint4*)((const uint16_t*)a.seg[sg].w + (size_t)row * a.K);
+            }
+            const uint4* const (&wc)[4] = w;
+            bf16_rows_dot<4>(wc, a.K >> 3, xs, lane, v);
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const float t = warp_sum(v[r]);
+                if (lane == 0 && i0 + r < n * sub) vals[i0 + r] = t;
+            }
+        }
+    } else {
+        for (int i = warp; i < n * sub; i += 8) {
+            int sg;
+            const int row = row_of(i, &sg);
+            const float v = row_dot<WK>(a.seg[sg], row, a.K, xs, lane);
+            if (lane == 0) vals[i] = v;
+        }
     }
     named_sync(1, 256);
     ArgBest best{-INFINITY, -1};
@@ -332,7 +376,7 @@ cudaError_t launch_gemv(const GemvArgs& a_in, int sm_count, cudaStream_t st) {
     if (a.ksplit == 2) return cudaErrorInvalidValue;     // the caller's consumer expects two partial vectors: only the streaming kernel makes them
     // direct kernel: a few CTAs per SM's worth of rows, at least 8 rows per CTA; a large bf16 / f32 matrix gets as many CTAs as
     // an SM can hold, so that enough loads are in flight to keep HBM busy
-    int grid = sm_count * (a.wkind != WK_Q8 && (long long)rows_total * a.K >= (1ll << 24) ? 8 : 2);
+    int grid = sm_count * (a.wkind != WK_Q8 && (long long)rows_total * a.K >= (1ll << 24) ? (a.wkind == WK_BF16 ? kDirectBf16Ctas : 8) : 2);
     if (grid > (rows_total + 7) / 8) grid = (rows_total + 7) / 8;
     if (a.epi == EPI_ARGMAX && grid > kArgmaxSlots) grid = kArgmaxSlots;       // one best-logit slot per CTA
     if (grid < 1) grid = 1;
