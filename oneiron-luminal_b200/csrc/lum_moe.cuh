@@ -21,6 +21,7 @@ struct MoeArgs {
     float* sw;                                // [n_tokens][top_k][ffn] scratch: the gated activations
     float* out; float* out_add; int out_ld;   // out_add != null: += into the residual stream; else out = this rank's share
     float limit;
+    uint32_t* status;
     int use_pdl;
 };
 

@@ -695,7 +695,7 @@ int issue_step(lum_rt* rt, bool with_head, bool pdl, int* n_launch) {
             m.expert0 = rt->ep_rank * (d.n_experts / rt->ep_size); m.n_local = d.n_experts / rt->ep_size;
             m.gu_q = (const int8_t*)w.exp_gu.w; m.gu_s = w.exp_gu.s; m.gu_bias = w.exp_gu_b.w;
             m.dn_q = (const int8_t*)w.exp_dn.w; m.dn_s = w.exp_dn.s; m.dn_bias = w.exp_dn_b.w;
-            m.sw = rt->moe_sw; m.limit = d.swiglu_limit; m.use_pdl = pdl; m.out_ld = H;
+            m.sw = rt->moe_sw; m.limit = d.swiglu_limit; m.status = rt->status; m.use_pdl = pdl; m.out_ld = H;
             CU(rt, launch_moe_route(m, 1, st)); n++;
             if (rt->ep_size > 1) {
                 const int T = rt->ep_size;
