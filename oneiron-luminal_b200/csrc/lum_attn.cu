@@ -19,12 +19,8 @@
 
 namespace lum {
 
-// One (kv head, split) per CTA.
-template <int HD, int GM, bool BF16, bool CL, int RS>
-__global__ void __launch_bounds__(kAttnThreads, 1) attn_decode(const AttnArgs a) {
-    extern __shared__ __align__(16) unsigned char attn_smem[];
-    if (a.use_pdl) pdl_launch_dependents();
-    // L2 warm-up for the kernels that follow: this CTA's share of each range, in 16 KiB requests (one per thread)
+// L2 warm-up for the kernels that follow: this CTA's share of each range, in 16 KiB requests (one per thread)
+__device__ __forceinline__ void attn_warm_l2(const AttnArgs& a, int threads) {
     {
         const unsigned int cta = blockIdx.y * gridDim.x + blockIdx.x, n_cta = gridDim.x * gridDim.y;
         constexpr unsigned long long kReq = 16384;
@@ -33,7 +29,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_decode(const AttnArgs a)
             const unsigned long long total = a.l2_pf_bytes[i];
             if (total) {
                 const unsigned long long n_req = (total + kReq - 1) / kReq;
-                for (unsigned long long r = (unsigned long long)threadIdx.x * n_cta + cta; r < n_req; r += (unsigned long long)n_cta * kAttnThreads) {
+                for (unsigned long long r = (unsigned long long)threadIdx.x * n_cta + cta; r < n_req; r += (unsigned long long)n_cta * threads) {
                     const unsigned long long off = r * kReq;
                     const unsigned long long len = total - off < kReq ? (total - off) & ~15ull : kReq;
                     if (len) bulk_prefetch_l2((const unsigned char*)a.l2_pf_ptr[i] + off, (uint32_t)len);
@@ -41,11 +37,19 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_decode(const AttnArgs a)
             }
         }
     }
+}
+
+// One (kv head, split) per CTA.
+template <int HD, int GM, bool BF16, bool CL, int RS>
+__global__ void __launch_bounds__(kAttnThreads, 1) attn_decode(const AttnArgs a) {
+    extern __shared__ __align__(16) unsigned char attn_smem[];
+    if (a.use_pdl) pdl_launch_dependents();
+    attn_warm_l2(a, kAttnThreads);
     // The position was settled by the previous step's sampler, several kernels back in stream order (the step's first
     // kernel waits for that step in full), so the rotation table can be worked out while the projections still run.
     const int p = a.state->pos;
     const bool ok = p >= 0 && p < a.max_seq;
-    if (ok) attn_fill_rope<HD, RS>(a, attn_smem, p, (int)threadIdx.x);
+    if (ok) attn_fill_rope<HD, RS>(a, attn_rope_table(attn_smem, HD), p, (int)threadIdx.x);
     if (ok && a.kv_prefetch) attn_prefetch_rows<HD, BF16>(a, (int)blockIdx.x, (int)blockIdx.y, p, (int)threadIdx.x);
     if (a.use_pdl) pdl_grid_wait();
     if (!ok) {                                  // the same for every CTA of the grid: no cluster barrier is left half attended
@@ -55,8 +59,51 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_decode(const AttnArgs a)
     attn_decode_body<HD, GM, BF16, CL>(a, attn_smem, (int)blockIdx.x, (int)blockIdx.y, p, (int)threadIdx.x, 2, true);
 }
 
+// The same on the tensor core (bf16 cache, heads that fit: attn_tc_fits)
+template <int HD, int MT, bool CL, int RS>
+__global__ void __launch_bounds__(kAttnTcThreads, 2) attn_decode_tc(const AttnArgs a) {
+    extern __shared__ __align__(16) unsigned char attn_smem[];
+    if (a.use_pdl) pdl_launch_dependents();
+    attn_warm_l2(a, kAttnTcThreads);
+    const int p = a.state->pos;                 // settled several kernels back, like every cached row: see attn_decode
+    const bool ok = p >= 0 && p < a.max_seq;
+    AttnTile<HD> f;
+    AttnPre<HD> pre;
+    if (ok) {
+        const int lane = threadIdx.x & 31, kvh = blockIdx.x;
+        int r0, r1;
+        attn_tc_range(a, blockIdx.y, p, &r0, &r1);
+        const int j0 = r0 + (threadIdx.x >> 5) * kAttnTcTile;
+        attn_tc_load_k<HD>(a, f, kvh, j0, r1, lane);
+        attn_tc_load_v<HD>(a, f, kvh, j0, r1, lane);
+        attn_tc_pre<HD>(a, pre, kvh, (int)blockIdx.y, (int)threadIdx.x >> 5, lane);
+        if (a.kv_prefetch) {
+            // one request per 128-byte line of the rows behind the first tiles
+            constexpr int kLines = HD * 2 / 128;
+            const int nc = r1 - r0 - kAttnTcWarps * kAttnTcTile;
+            for (int i = threadIdx.x; i < nc * 2 * kLines; i += kAttnTcThreads) {
+                const int r = r1 - nc + i / (2 * kLines), w = i % (2 * kLines);
+                const char* base = (const char*)(w < kLines ? a.k_cache : a.v_cache) + (kv_phys_row(a.pg, 0, 0, r) * a.n_kv + kvh) * (HD * 2) + (w % kLines) * 128;
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(base));
+            }
+        }
+        attn_fill_rope<HD, RS>(a, attn_rope_table(attn_smem, HD, kAttnTcWarps + 1), p, (int)threadIdx.x);
+    }
+    if (a.use_pdl) pdl_grid_wait();
+    if (!ok) {                                  // the same for every CTA of the grid: no cluster barrier is left half attended
+        if (threadIdx.x == 0) atomicOr(a.status, LUM_ST_BAD_POS);
+        return;
+    }
+    attn_tc_body<HD, MT, CL>(a, attn_smem, f, pre, (int)blockIdx.x, (int)blockIdx.y, p, (int)threadIdx.x, 2, true);
+}
+
 template <int HD, int GM, int RS>
 static const void* attn_fn(bool bf16, bool cl) {
+    constexpr int MT = GM / 4;
+    if constexpr (attn_tc_fits(HD, GM)) {
+        if (bf16) return cl ? (const void*)attn_decode_tc<HD, MT, true, RS> : (const void*)attn_decode_tc<HD, MT, false, RS>;
+        return cl ? (const void*)attn_decode<HD, GM, false, true, RS> : (const void*)attn_decode<HD, GM, false, false, RS>;
+    }
     if (cl) return bf16 ? (const void*)attn_decode<HD, GM, true, true, RS> : (const void*)attn_decode<HD, GM, false, true, RS>;
     return bf16 ? (const void*)attn_decode<HD, GM, true, false, RS> : (const void*)attn_decode<HD, GM, false, false, RS>;
 }
@@ -70,11 +117,13 @@ static const void* attn_fn_for(int hd, int G, bool bf16, bool cl, int rope_style
     return rope_style == 0 ? attn_fn_rs<0>(hd, G, bf16, cl) : attn_fn_rs<1>(hd, G, bf16, cl);
 }
 
+static bool attn_tc(const AttnArgs& a, int G) { return a.kv_bf16 && attn_tc_fits(a.hd, G <= 4 ? 4 : 8); }
+static size_t attn_smem_for(const AttnArgs& a, int G) { return attn_tc(a, G) ? attn_tc_smem_bytes(a.hd, G) : attn_smem_bytes(a.hd, G); }
 static void attn_fill_config(const AttnArgs& a, int G, bool cl, cudaStream_t st, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at) {
     *cfg = cudaLaunchConfig_t{};
     cfg->gridDim = dim3(a.n_kv, a.n_splits);
-    cfg->blockDim = dim3(kAttnThreads);
-    cfg->dynamicSmemBytes = attn_smem_bytes(a.hd, G);
+    cfg->blockDim = dim3(attn_tc(a, G) ? kAttnTcThreads : kAttnThreads);
+    cfg->dynamicSmemBytes = attn_smem_for(a, G);
     cfg->stream = st;
     int n = 0;
     if (a.use_pdl) {
@@ -97,7 +146,7 @@ bool attn_cluster_supported(const AttnArgs& a) {
     if (a.n_splits < 2 || a.n_splits > kMaxClusterSplits || G < 1 || G > 8) return false;
     const void* fn = attn_fn_for(a.hd, G, a.kv_bf16 != 0, true, a.rope_style);
     if (!fn) return false;
-    const size_t smem = attn_smem_bytes(a.hd, G);
+    const size_t smem = attn_smem_for(a, G);
     if (smem > 48 * 1024 && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) { cudaGetLastError(); return false; }
     if (a.n_splits > 8 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) { cudaGetLastError(); return false; }
     cudaLaunchConfig_t cfg;
@@ -118,7 +167,7 @@ cudaError_t launch_attn_decode(const AttnArgs& a_in, cudaStream_t st) {
     if (cl && (a.n_splits < 2 || a.n_splits > kMaxClusterSplits)) return cudaErrorInvalidValue;
     const void* fn = attn_fn_for(a.hd, G, a.kv_bf16 != 0, cl, a.rope_style);
     if (!fn) return cudaErrorInvalidValue;
-    const size_t smem = attn_smem_bytes(a.hd, G);
+    const size_t smem = attn_smem_for(a, G);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;

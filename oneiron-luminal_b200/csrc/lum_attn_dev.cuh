@@ -89,12 +89,11 @@ constexpr int kMaxClusterSplits = 16;      // largest cluster the hardware sched
 __host__ __device__ inline size_t attn_smem_bytes(int HD, int G) {
     return (size_t)(9 * HD + HD + 2 * kAttnWarps * 8 + 4 + HD) * 4 + (size_t)kAttnWarps * G * HD * 4;
 }
-// where the rotation table (cos, sin per dimension pair) lives in the attention scratch
-__device__ __forceinline__ float* attn_rope_table(unsigned char* smem, int HD) { return (float*)smem + 9 * HD + HD + 2 * kAttnWarps * 8 + 4; }
+// where the rotation table (cos, sin per dimension pair) lives in the attention scratch (`states`: partial states merged in the CTA)
+__device__ __forceinline__ float* attn_rope_table(unsigned char* smem, int HD, int states = kAttnWarps) { return (float*)smem + 9 * HD + HD + 2 * states * 8 + 4; }
 // The table depends only on the position: a kernel can fill it while it still waits for the projections (threads 0 .. HD/2-1).
 template <int HD, int RS = -1>
-__device__ __forceinline__ void attn_fill_rope(const AttnArgs& a, unsigned char* smem, int p, int tid) {
-    float* tab = attn_rope_table(smem, HD);
+__device__ __forceinline__ void attn_fill_rope(const AttnArgs& a, float* tab, int p, int tid) {
     if (tid < HD / 2) {
         float cs, sn;
         rope_cs<RS>(a, tid, p, &cs, &sn);
@@ -165,6 +164,56 @@ __device__ __forceinline__ void attn_prefetch_rows(const AttnArgs& a, int kvh, i
     }
 }
 
+// Merging the splits of a KV head from a.part, called by all T threads of every CTA that holds one: the last CTA to arrive does it.
+template <int HD>
+__device__ __forceinline__ void attn_merge_ticket(const AttnArgs& a, int* s_last, int kvh, int G, int tid, int T, int bar_id) {
+    __threadfence();
+    named_sync(bar_id, T);
+    if (tid == 0) {
+        const unsigned int t = atomicAdd(&a.counters[kvh], 1u);
+        *s_last = (t == (unsigned int)a.n_splits - 1u) ? 1 : 0;
+    }
+    named_sync(bar_id, T);
+    if (!*s_last) return;
+    __threadfence();
+    // The partials were written by other CTAs: read them through L2 (ld.cg).  All loads of a batch of 8 splits
+    // are issued before any is used, so a batch costs one round trip; batches fold into a running (max, sum, out).
+    constexpr int kBatch = 8;
+#pragma unroll 1
+    for (int idx = tid; idx < G * HD; idx += T) {
+        const int g = idx / HD, e = idx - g * HD;
+        const float* src = a.part + ((size_t)kvh * a.n_splits * G + g) * (HD + 2);
+        const size_t sstride = (size_t)G * (HD + 2);
+        float M = -INFINITY, L = 0.0f, O = 0.0f;
+#pragma unroll 1
+        for (int s0 = 0; s0 < a.n_splits; s0 += kBatch) {
+            float mv[kBatch], lv[kBatch], ov[kBatch];
+#pragma unroll
+            for (int j = 0; j < kBatch; j++) {
+                const bool in = s0 + j < a.n_splits;
+                const float* q2 = src + (size_t)(in ? s0 + j : 0) * sstride;
+                mv[j] = in ? __ldcg(q2 + HD) : -INFINITY;
+                lv[j] = __ldcg(q2 + HD + 1);
+                ov[j] = __ldcg(q2 + e);
+            }
+            float Mb = M;
+#pragma unroll
+            for (int j = 0; j < kBatch; j++) Mb = fmaxf(Mb, mv[j]);
+            const float c0 = (M == -INFINITY) ? 0.0f : expf(M - Mb);
+            L *= c0; O *= c0;
+#pragma unroll
+            for (int j = 0; j < kBatch; j++) {
+                const float c = (mv[j] == -INFINITY) ? 0.0f : expf(mv[j] - Mb);
+                L = fmaf(lv[j], c, L);
+                O = fmaf(ov[j], c, O);
+            }
+            M = Mb;
+        }
+        a.out[((size_t)kvh * G + g) * HD + e] = attn_finish(O, M, L, a.sinks, a.gain_kind, kvh * G + g);
+    }
+    if (tid == 0) a.counters[kvh] = 0u;
+}
+
 // Runs on exactly kAttnThreads threads (tid 0..511) that synchronise on named barrier `bar_id`.
 // p = position of the token being processed (rows [.., p) are cached, row p is this step's own).
 // smem: attn_smem_bytes(HD, G) bytes, 16-byte aligned.
@@ -215,7 +264,7 @@ __device__ __forceinline__ void attn_decode_body(const AttnArgs& a, unsigned cha
             if (a.v_bias) v = v + gain_at(a.v_bias, a.gain_kind, kvh * HD + e);
             s_v[e] = v;
         }
-    if (!rope_ready) attn_fill_rope<HD>(a, smem, p, tid);
+    if (!rope_ready) attn_fill_rope<HD>(a, s_rope, p, tid);
     sync();
     if (a.q_gain || a.k_gain) {
         // per-head RMSNorm: x * 1/sqrt(mean(x^2) + eps) * g   (one warp per head)
@@ -402,52 +451,7 @@ __device__ __forceinline__ void attn_decode_body(const AttnArgs& a, unsigned cha
     }
     if (a.n_splits == 1) return;
 
-    // last CTA of this KV head merges the splits
-    __threadfence();
-    sync();
-    if (tid == 0) {
-        const unsigned int t = atomicAdd(&a.counters[kvh], 1u);
-        s_last = (t == (unsigned int)a.n_splits - 1u) ? 1 : 0;
-    }
-    sync();
-    if (!s_last) return;
-    __threadfence();
-    // The partials were written by other CTAs: read them through L2 (ld.cg).  All loads of a batch of 8 splits
-    // are issued before any is used, so a batch costs one round trip; batches fold into a running (max, sum, out).
-    constexpr int kBatch = 8;
-#pragma unroll 1
-    for (int idx = tid; idx < G * HD; idx += kAttnThreads) {
-        const int g = idx / HD, e = idx - g * HD;
-        const float* src = a.part + ((size_t)kvh * a.n_splits * G + g) * (HD + 2);
-        const size_t sstride = (size_t)G * (HD + 2);
-        float M = -INFINITY, L = 0.0f, O = 0.0f;
-#pragma unroll 1
-        for (int s0 = 0; s0 < a.n_splits; s0 += kBatch) {
-            float mv[kBatch], lv[kBatch], ov[kBatch];
-#pragma unroll
-            for (int j = 0; j < kBatch; j++) {
-                const bool in = s0 + j < a.n_splits;
-                const float* q2 = src + (size_t)(in ? s0 + j : 0) * sstride;
-                mv[j] = in ? __ldcg(q2 + HD) : -INFINITY;
-                lv[j] = __ldcg(q2 + HD + 1);
-                ov[j] = __ldcg(q2 + e);
-            }
-            float Mb = M;
-#pragma unroll
-            for (int j = 0; j < kBatch; j++) Mb = fmaxf(Mb, mv[j]);
-            const float c0 = (M == -INFINITY) ? 0.0f : expf(M - Mb);
-            L *= c0; O *= c0;
-#pragma unroll
-            for (int j = 0; j < kBatch; j++) {
-                const float c = (mv[j] == -INFINITY) ? 0.0f : expf(mv[j] - Mb);
-                L = fmaf(lv[j], c, L);
-                O = fmaf(ov[j], c, O);
-            }
-            M = Mb;
-        }
-        a.out[((size_t)kvh * G + g) * HD + e] = attn_finish(O, M, L, a.sinks, a.gain_kind, kvh * G + g);
-    }
-    if (tid == 0) a.counters[kvh] = 0u;
+    attn_merge_ticket<HD>(a, &s_last, kvh, G, tid, kAttnThreads, bar_id);
 }
 
 // ---- Products of attention on m16n8k16 tensor-core instructions (bf16 operands, f32 sums) without giving up f32 operands: K and V are bf16
@@ -467,6 +471,350 @@ __device__ __forceinline__ void attn_terms(float x0, float x1, bool second, uint
     const __nv_bfloat162 t3 = __floats2bfloat162_rn(r0 - __low2float(t2), r1 - __high2float(t2));
     *lo_row = second ? *(const uint32_t*)&t2 : *(const uint32_t*)&t1;
     *hi_row = second ? 0u : *(const uint32_t*)&t3;
+}
+
+// ---- Single-token attention over a bf16 cache on the tensor core: the form every decode step takes whose heads fit it (up to four query heads
+// of 128 dimensions or eight of 64 per KV head; others, and f32 caches, take the form above).
+//
+// Bound by latency, not by bytes (2 to 12 MB a layer): what counts is the chain of trips to memory, barriers and shuffles.
+//   * 128 threads; a warp takes 16 keys at a time and holds their K and V in registers exactly as the tensor core reads them — no shared
+//     memory, no barrier.  The contraction does not care about the order of the dimensions, so a thread's 16-byte load of a K row is
+//     four pairs of two consecutive K = 16 steps; the outputs' order is free too, so a 16-byte load of a V row serves eight column tiles.
+//   * The cached rows were written by earlier steps: the first 16 keys of every warp are requested before the grid dependency is waited for, the
+//     rest is prefetched into L2, and inside the loop a tile's K is replaced while its softmax runs, its V right after use.
+//   * The step's own row never passes through memory: one warp of the CTA that owns it adds it as one more partial state.
+//   * In a cluster every CTA stores its results straight into the shared memory of the CTA that finishes them: one barrier, no trip back.
+// Measured, whole decode steps (this form against the one above): 36 layers of 32 / 8 heads of 128 behind 3000 rows 2.48 -> 2.28 ms a token, 32 such
+// layers behind 512 rows 2.265 -> 2.232 ms, 24 layers of 64 / 8 heads of 64 behind 700 rows (half of them with a window of 128) 2.14 -> 2.12 ms.
+// The plain form takes a warp per key, five shuffles and two exponentials per key and head in a chain.  Tried: the cluster's results fetched by their
+// readers instead of pushed (two barriers and a trip: 3 % of a step behind 512 rows); 64 registers in the projections, so that a CTA of this
+// kernel fits beside theirs (their prologue spills: 48 against 36 ms for 16 tokens).
+constexpr int kAttnTcThreads = 128, kAttnTcWarps = kAttnTcThreads / 32, kAttnTcTile = 16;
+__host__ __device__ constexpr bool attn_tc_fits(int HD, int G) { return HD * ((G + 3) / 4) <= 128; }
+__host__ __device__ inline size_t attn_tc_smem_bytes(int HD, int G) {
+    return (size_t)(9 * HD + HD + 2 * (kAttnTcWarps + 1) * 8 + 4 + HD + (G + 3) / 4 * (HD / 16) * 128) * 4 + (size_t)(kAttnTcWarps + 1) * G * HD * 4 +
+           (size_t)(G * HD + kMaxClusterSplits) * 16;
+}
+// cached rows of a split: [r0, r1), whole tiles except at the end
+__device__ __forceinline__ void attn_tc_range(const AttnArgs& a, int split, int p, int* r0, int* r1) {
+    const int lo = (a.window > 0 && p + 1 > a.window) ? p + 1 - a.window : 0;
+    const int per = ((p - lo + a.n_splits - 1) / a.n_splits + kAttnTcTile - 1) / kAttnTcTile * kAttnTcTile;
+    *r0 = min(p, lo + split * per);
+    *r1 = min(p, *r0 + per);
+}
+template <int HD> struct AttnTile { uint4 k[2][HD / 32], v[4][HD / 64]; };
+template <int HD>
+__device__ __forceinline__ void attn_tc_load_k(const AttnArgs& a, AttnTile<HD>& f, int kvh, int j0, int r1, int lane) {
+#pragma unroll
+    for (int x = 0; x < 2; x++) {
+        const int row = j0 + 8 * x + (lane >> 2);
+        const bool in = row < r1;
+        const uint4* p = (const uint4*)((const __nv_bfloat16*)a.k_cache + (kv_phys_row(a.pg, 0, 0, in ? row : 0) * a.n_kv + kvh) * HD) + (lane & 3);
+#pragma unroll
+        for (int j = 0; j < HD / 32; j++) f.k[x][j] = in ? __ldcg(p + 4 * j) : make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+template <int HD>
+__device__ __forceinline__ void attn_tc_load_v(const AttnArgs& a, AttnTile<HD>& f, int kvh, int j0, int r1, int lane) {
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+        const int row = j0 + 8 * (x >> 1) + 2 * (lane & 3) + (x & 1);
+        const bool in = row < r1;
+        const uint4* p = (const uint4*)((const __nv_bfloat16*)a.v_cache + (kv_phys_row(a.pg, 0, 0, in ? row : 0) * a.n_kv + kvh) * HD) + (lane >> 2);
+#pragma unroll
+        for (int j = 0; j < HD / 64; j++) f.v[x][j] = in ? __ldcg(p + 8 * j) : make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+// Gains and biases of the heads this warp prepares (warp, warp + 4, ..: the group's queries, then the step's own key and value): they do not depend
+// on the previous kernel either.
+constexpr int kAttnTcHeads = 3;                          // up to 8 queries + key + value over 4 warps
+template <int HD> struct AttnPre { float gain[kAttnTcHeads][HD / 32], bias[kAttnTcHeads][HD / 32]; };
+template <int HD>
+__device__ __forceinline__ void attn_tc_pre(const AttnArgs& a, AttnPre<HD>& pre, int kvh, int split, int warp, int lane) {
+    const int G = a.n_q / a.n_kv;
+#pragma unroll
+    for (int k = 0; k < kAttnTcHeads; k++) {
+        const int h = warp + kAttnTcWarps * k;
+        const bool in = h < G || (h < G + 2 && split == a.n_splits - 1);
+        const void* gain = h < G ? a.q_gain : h == G ? a.k_gain : nullptr;
+        const void* bias = h < G ? a.q_bias : h == G ? a.k_bias : a.v_bias;
+        const int off = (h < G ? kvh * G + h : kvh) * HD;
+#pragma unroll
+        for (int i = 0; i < HD / 32; i++) {
+            pre.gain[k][i] = in && gain ? gain_at(gain, a.gain_kind, lane + 32 * i) : 0.0f;
+            pre.bias[k][i] = in && bias ? gain_at(bias, a.gain_kind, off + lane + 32 * i) : 0.0f;
+        }
+    }
+}
+__device__ __forceinline__ uint32_t attn_word(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+
+// Runs on exactly kAttnTcThreads threads (tid 0 ..) that synchronise on named barrier `bar_id`; `f` holds this warp's first tile (attn_tc_load_*),
+// `pre` its heads' gains and biases
+template <int HD, int MT, bool CL>
+__device__ __forceinline__ void attn_tc_body(const AttnArgs& a, unsigned char* smem, AttnTile<HD>& f, const AttnPre<HD>& pre, int kvh, int split, int p, int tid, int bar_id,
+                                             bool rope_ready) {
+    constexpr int NW = kAttnTcWarps, NP = NW + 1, T = kAttnTcThreads, KS = HD / 16, NT = HD / 8, N = HD / 32;
+    const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const bool second = g >= 4;
+    const int G = a.n_q / a.n_kv;
+    auto sync = [bar_id] { named_sync(bar_id, T); };
+    float (*s_q)[HD] = (float (*)[HD])smem;                 // [9][HD]: rotated q heads; row G = this step's k
+    float* s_v = (float*)smem + 9 * HD;                     // [HD]
+    float (*s_m)[8] = (float (*)[8])(s_v + HD);             // [NP][8]: one state per warp, and the own row's
+    float (*s_l)[8] = (float (*)[8])(s_v + HD + NP * 8);
+    int& s_last = *(int*)(s_v + HD + 2 * NP * 8);
+    float* s_rope = s_v + HD + 2 * NP * 8 + 4;              // [HD/2][2]: cos, sin
+    uint4* s_a = (uint4*)(s_rope + HD);                     // [MT][KS][32]: the queries as the tensor core's first operand
+    float* s_o = (float*)(s_a + MT * KS * 32);              // [NP][G][HD]
+    float4* s_t = (float4*)(s_o + NP * G * HD);             // [splits][chunk]: the cluster's (max, sum, out) of the outputs this CTA finishes
+    const size_t row_elems = (size_t)a.n_kv * HD;
+    if (CL) cluster_arrive_release();                       // (waited for before the first store into another CTA: it has started)
+    int r0, r1;
+    attn_tc_range(a, split, p, &r0, &r1);
+    const bool owns_new = split == a.n_splits - 1;
+    const float scale = 1.0f / sqrtf((float)HD);
+
+    // ---- this step's q heads of the group and, in the owner of the last split, its k and v: a warp per head, in registers (lane l holds the
+    // elements l, l + 32, ..: the rotation's partner is in the next lane or in the same one)
+    const int nheads = G + (owns_new ? 2 : 0);
+    if (!rope_ready) attn_fill_rope<HD>(a, s_rope, p, tid);
+    float x[kAttnTcHeads][N];
+#pragma unroll
+    for (int k = 0; k < kAttnTcHeads; k++) {
+        const int h = warp + NW * k;
+        if (h < nheads) {
+            const float* src = h < G ? a.q + ((size_t)kvh * G + h) * HD : h == G ? a.k_new + (size_t)kvh * HD : a.v_new + (size_t)kvh * HD;
+#pragma unroll
+            for (int i = 0; i < N; i++) x[k][i] = __ldcg(src + lane + 32 * i);
+        }
+    }
+    sync();                                                  // (the rotation table is there)
+#pragma unroll
+    for (int k = 0; k < kAttnTcHeads; k++) {
+        const int h = warp + NW * k;
+        if (h < nheads) {
+            if (h < G ? a.q_bias != nullptr : h == G ? a.k_bias != nullptr : a.v_bias != nullptr) {
+#pragma unroll
+                for (int i = 0; i < N; i++) x[k][i] = x[k][i] + pre.bias[k][i];
+            }
+            if (h > G) {
+#pragma unroll
+                for (int i = 0; i < N; i++) s_v[lane + 32 * i] = x[k][i];
+            } else {
+                if (h < G ? a.q_gain != nullptr : a.k_gain != nullptr) {
+                    float ss = 0.0f;
+#pragma unroll
+                    for (int i = 0; i < N; i++) ss = fmaf(x[k][i], x[k][i], ss);
+                    ss = warp_sum(ss);
+                    const float inv = 1.0f / sqrtf(ss * (1.0f / (float)HD) + a.qk_eps);
+#pragma unroll
+                    for (int i = 0; i < N; i++) x[k][i] = (inv * x[k][i]) * pre.gain[k][i];
+                }
+                // separately rounded products and sums, as the graph's Mul / Add nodes produce them
+                if (a.rope_style == 0) {
+#pragma unroll
+                    for (int i = 0; i < N; i++) {
+                        const float cs = s_rope[2 * ((lane + 32 * i) >> 1)], sn = s_rope[2 * ((lane + 32 * i) >> 1) + 1];
+                        const float other = __shfl_xor_sync(0xffffffffu, x[k][i], 1);
+                        x[k][i] = (lane & 1) ? __fadd_rn(__fmul_rn(other, sn), __fmul_rn(x[k][i], cs))
+                                             : __fadd_rn(__fmul_rn(x[k][i], cs), __fmul_rn(__fmul_rn(other, sn), -1.0f));
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < N / 2; i++) {
+                        const float cs = s_rope[2 * (lane + 32 * i)], sn = s_rope[2 * (lane + 32 * i) + 1];
+                        const float x0 = x[k][i], x1 = x[k][i + N / 2];
+                        x[k][i] = __fsub_rn(__fmul_rn(x0, cs), __fmul_rn(x1, sn));
+                        x[k][i + N / 2] = __fadd_rn(__fmul_rn(x1, cs), __fmul_rn(x0, sn));
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < N; i++) s_q[h][lane + 32 * i] = x[k][i];
+            }
+        }
+    }
+    sync();
+    // queries -> operand: step ks of thread column t covers dimensions 32 (ks / 2) + 8 t + 4 (ks % 2) .. + 3
+#pragma unroll 1
+    for (int idx = tid; idx < MT * KS * 32; idx += T) {
+        const int ln = idx & 31, ks = (idx >> 5) % KS, h = (idx >> 5) / KS * 4 + ((ln >> 2) & 3);
+        const float4 q = h < G ? *(const float4*)&s_q[h][(ks >> 1) * 32 + (ln & 3) * 8 + (ks & 1) * 4] : make_float4(0.f, 0.f, 0.f, 0.f);
+        uint4 w;
+        attn_terms(q.x, q.y, ln >= 16, &w.x, &w.y);
+        attn_terms(q.z, q.w, ln >= 16, &w.z, &w.w);
+        s_a[idx] = w;
+    }
+    if (owns_new && warp == NW - 1) {
+        // append this step's row to the cache; the rounded values are one more state: score, weight 1, value
+        const size_t off = kv_phys_row(a.pg, 0, 0, p) * row_elems + (size_t)kvh * HD;
+        float k[N], v[N];
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const __nv_bfloat16 kb = __float2bfloat16_rn(s_q[G][lane + 32 * i]), vb = __float2bfloat16_rn(s_v[lane + 32 * i]);
+            ((__nv_bfloat16*)a.k_cache)[off + lane + 32 * i] = kb;
+            ((__nv_bfloat16*)a.v_cache)[off + lane + 32 * i] = vb;
+            k[i] = __bfloat162float(kb); v[i] = __bfloat162float(vb);
+        }
+#pragma unroll 1
+        for (int h = 0; h < G; h++) {
+            float d = 0.0f;
+#pragma unroll
+            for (int i = 0; i < N; i++) d = fmaf(s_q[h][lane + 32 * i], k[i], d);
+            d = warp_sum(d);
+            if (lane == 0) { s_m[NW][h] = d * scale; s_l[NW][h] = 1.0f; }
+#pragma unroll
+            for (int i = 0; i < N; i++) s_o[((size_t)NW * G + h) * HD + lane + 32 * i] = v[i];
+        }
+    }
+    sync();
+
+    // ---- the cached rows
+    float o[MT][NT][4], mx[MT], l[MT];
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++) {
+        mx[mt] = -INFINITY; l[mt] = 0.0f;
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) o[mt][n][e] = 0.0f;
+    }
+#pragma unroll 1
+    for (int j0 = r0 + warp * kAttnTcTile; j0 < r1; j0 += NW * kAttnTcTile) {
+        float s[MT][2][4];
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) s[mt][0][e] = s[mt][1][e] = 0.0f;
+#pragma unroll
+        for (int ks = 0; ks < KS; ks++) {
+#pragma unroll
+            for (int mt = 0; mt < MT; mt++) {
+                const uint4 w = s_a[(mt * KS + ks) * 32 + lane];
+                const uint32_t qa[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int y = 0; y < 2; y++) attn_mma(s[mt][y], qa, attn_word(f.k[y][ks >> 1], 2 * (ks & 1)), attn_word(f.k[y][ks >> 1], 2 * (ks & 1) + 1));
+            }
+        }
+        const int jn = j0 + NW * kAttnTcTile;
+        if (jn < r1) attn_tc_load_k<HD>(a, f, kvh, jn, r1, lane);
+        const int j = j0 + 2 * t;                                     // this thread's keys: j, j + 1, j + 8, j + 9
+        uint32_t pa[MT][4];
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++) {
+            float v[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                float y = s[mt][e >> 1][e & 1] + s[mt][e >> 1][2 + (e & 1)];       // rows g and g + 8
+                y += __shfl_xor_sync(0xffffffffu, y, 16);                          // and the second terms' row
+                v[e] = j + (e >> 1) * 8 + (e & 1) < r1 ? y * scale : -INFINITY;
+            }
+            float tm = fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3]));
+            tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 1));
+            tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 2));
+            const float mn = fmaxf(mx[mt], tm);                       // a tile always holds at least one live key
+            const float corr = mx[mt] == -INFINITY ? 0.0f : expf(mx[mt] - mn);
+            mx[mt] = mn;
+            float ps = 0.0f;
+#pragma unroll
+            for (int e = 0; e < 4; e++) { v[e] = v[e] == -INFINITY ? 0.0f : expf(v[e] - mn); ps += v[e]; }
+            l[mt] = l[mt] * corr + ps;                                // per-lane partial sums, folded at the end
+            attn_terms(v[0], v[1], second, &pa[mt][0], &pa[mt][1]);
+            attn_terms(v[2], v[3], second, &pa[mt][2], &pa[mt][3]);
+            if (__any_sync(0xffffffffu, corr != 1.0f)) {
+#pragma unroll
+                for (int n = 0; n < NT; n++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) o[mt][n][e] *= corr;
+            }
+        }
+        // column g of tile 8 jj + i is dimension 64 jj + 8 g + i
+#pragma unroll
+        for (int jj = 0; jj < HD / 64; jj++)
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const uint32_t sel = (i & 1) ? 0x7632u : 0x5410u;
+                const uint32_t b0 = __byte_perm(attn_word(f.v[0][jj], i >> 1), attn_word(f.v[1][jj], i >> 1), sel);
+                const uint32_t b1 = __byte_perm(attn_word(f.v[2][jj], i >> 1), attn_word(f.v[3][jj], i >> 1), sel);
+#pragma unroll
+                for (int mt = 0; mt < MT; mt++) attn_mma(o[mt][jj * 8 + i], pa[mt], b0, b1);
+            }
+        if (jn < r1) attn_tc_load_v<HD>(a, f, kvh, jn, r1, lane);
+    }
+    // ---- add up the terms' rows and the lanes' sums, then the warps
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++) {
+        const int h = mt * 4 + (g & 3);
+        float lt = l[mt];
+        lt += __shfl_xor_sync(0xffffffffu, lt, 1);
+        lt += __shfl_xor_sync(0xffffffffu, lt, 2);
+        if (t == 0 && !second) { s_m[warp][h] = mx[mt]; s_l[warp][h] = lt; }
+#pragma unroll
+        for (int n = 0; n < NT; n++) {
+            float x0 = o[mt][n][0] + o[mt][n][2], x1 = o[mt][n][1] + o[mt][n][3];
+            x0 += __shfl_xor_sync(0xffffffffu, x0, 16);
+            x1 += __shfl_xor_sync(0xffffffffu, x1, 16);
+            float* dst = s_o + ((size_t)warp * G + h) * HD + (n >> 3) * 64 + 16 * t + (n & 7);
+            if (!second && h < G) { dst[0] = x0; dst[8] = x1; }
+        }
+    }
+    sync();
+    const int parts = owns_new ? NP : NW;
+    const int S = a.n_splits, total = G * HD, chunk = (total + S - 1) / S;      // outputs CTA r of the cluster finishes: [r * chunk, (r + 1) * chunk)
+    if (CL) cluster_wait_acquire();
+#pragma unroll 1
+    for (int idx = tid; idx < total; idx += T) {
+        const int h = idx / HD, e = idx - h * HD;
+        float M = -INFINITY, L = 0.0f, O = 0.0f;
+#pragma unroll
+        for (int w = 0; w < NP; w++) if (w < parts) M = fmaxf(M, s_m[w][h]);
+#pragma unroll
+        for (int w = 0; w < NP; w++)
+            if (w < parts) {
+                const float c = s_m[w][h] == -INFINITY ? 0.0f : expf(s_m[w][h] - M);
+                L = fmaf(s_l[w][h], c, L);
+                O = fmaf(s_o[(size_t)w * G * HD + idx], c, O);
+            }
+        if (CL) {
+            const int r = idx / chunk;
+            const uint32_t dst = cluster_map(smem_u32(s_t + split * chunk + (idx - r * chunk)), (uint32_t)r);
+            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "f"(M), "f"(L), "f"(O), "f"(0.0f) : "memory");
+        } else if (S == 1) {
+            a.out[(size_t)kvh * total + idx] = attn_finish(O, M, L, a.sinks, a.gain_kind, kvh * G + h);      // no other split to merge with
+        } else {
+            float* dst = a.part + (((size_t)kvh * S + split) * G + h) * (HD + 2);
+            dst[e] = O;
+            if (e == 0) { dst[HD] = M; dst[HD + 1] = L; }
+        }
+    }
+    if (CL) {
+        cluster_arrive_release();
+        cluster_wait_acquire();
+        for (int oi = tid; oi < chunk && split * chunk + oi < total; oi += T) {
+            // the ticket path's folding: batches of 8 splits into a running (max, sum, out)
+            float M = -INFINITY, L = 0.0f, O = 0.0f;
+#pragma unroll 1
+            for (int s0 = 0; s0 < S; s0 += 8) {
+                float4 v[8];
+                float Mb = M;
+#pragma unroll
+                for (int j = 0; j < 8; j++) v[j] = s0 + j < S ? s_t[(s0 + j) * chunk + oi] : make_float4(-INFINITY, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int j = 0; j < 8; j++) Mb = fmaxf(Mb, v[j].x);
+                const float c0 = (M == -INFINITY) ? 0.0f : expf(M - Mb);
+                L *= c0; O *= c0;
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const float c = (v[j].x == -INFINITY) ? 0.0f : expf(v[j].x - Mb);
+                    L = fmaf(v[j].y, c, L);
+                    O = fmaf(v[j].z, c, O);
+                }
+                M = Mb;
+            }
+            a.out[(size_t)kvh * total + split * chunk + oi] = attn_finish(O, M, L, a.sinks, a.gain_kind, kvh * G + (split * chunk + oi) / HD);
+        }
+    } else if (S > 1) {
+        attn_merge_ticket<HD>(a, &s_last, kvh, G, tid, T, bar_id);
+    }
 }
 
 }  // namespace lum

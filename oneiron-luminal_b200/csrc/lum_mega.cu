@@ -79,7 +79,20 @@ __device__ __noinline__ void attn_phase(const MegaArgs& a, const MegaLayer& L, u
     t.n_q = a.n_q; t.n_kv = a.n_kv; t.hd = a.hd; t.n_splits = a.n_splits; t.kv_bf16 = BF16; t.rope_style = a.rope_style;
     t.c_inv_d = a.c_inv_d; t.c_ln_theta = a.c_ln_theta; t.c_log2e = a.c_log2e; t.c_half_pi = a.c_half_pi; t.theta = a.theta;
     t.window = 0; t.max_seq = a.max_seq; t.status = a.status;
-    attn_decode_body<HD, GM, BF16>(t, scratch_smem, (int)blockIdx.x / a.n_splits, (int)blockIdx.x % a.n_splits, pos, tid, 1);
+    const int kvh = (int)blockIdx.x / a.n_splits, split = (int)blockIdx.x % a.n_splits;
+    if constexpr (BF16 && attn_tc_fits(HD, GM)) {
+        if (tid >= kAttnTcThreads) return;          // (all workers meet at the phase's grid barrier)
+        AttnTile<HD> f;
+        int r0, r1;
+        attn_tc_range(t, split, pos, &r0, &r1);
+        attn_tc_load_k<HD>(t, f, kvh, r0 + (tid >> 5) * kAttnTcTile, r1, tid & 31);
+        attn_tc_load_v<HD>(t, f, kvh, r0 + (tid >> 5) * kAttnTcTile, r1, tid & 31);
+        AttnPre<HD> pre;
+        attn_tc_pre<HD>(t, pre, kvh, split, tid >> 5, tid & 31);
+        attn_tc_body<HD, GM / 4, false>(t, scratch_smem, f, pre, kvh, split, pos, tid, 3, false);
+    } else {
+        attn_decode_body<HD, GM, BF16>(t, scratch_smem, kvh, split, pos, tid, 1);
+    }
 }
 
 // Phase p of layer l (p = 0..4), or the head phase (p = 5): fill in the projection's arguments.
