@@ -69,10 +69,10 @@ __device__ __forceinline__ void x_levels_to_smem(const float* x, int K, int8_t* 
 
 // ---- Rows of experts, streamed.  A warp works through a list of units, each two consecutive weight rows of one expert (contiguous int8 planes): it
 // keeps a ring of `stages` chunks (up to kMoeBlocks blocks of both rows) in shared memory, filled by bulk copies that one of its lanes issues, and
-// never waits for another warp.  What bounds the kernels is how many bytes are on their way: 8 warps x 4 stages x 5.8 KB = 184 KB per SM, against
-// the 12 KB that plain loads had in flight.  Two lanes share a block (16 bytes each: no bank conflicts), the activation levels of a block
+// never waits for another warp.  What bounds the kernels is how many bytes are on their way: 16 warps x 2 stages x 5.8 KB = 184 KB per SM, against
+// the 12 KB that plain loads had in flight (8 warps x 4 stages: 34.25 against 31.25 ms for 16 tokens of the gpt-oss-20B shape).  Two lanes share a block (16 bytes each: no bank conflicts), the activation levels of a block
 // serve both rows.  Scales and biases come with plain loads one unit ahead; nothing in the loop waits for a load made in the same turn.
-constexpr int kMoeWarps = 8, kMoeTrips = 6, kMoeBlocks = 16 * kMoeTrips, kMoeMaxStages = 4;
+constexpr int kMoeWarps = 16, kMoeTrips = 6, kMoeBlocks = 16 * kMoeTrips, kMoeMaxStages = 2;
 struct MoeRing { unsigned char* base; uint32_t bars; int stages, blocks; uint32_t issued, taken; };      // blocks: of one row, per stage
 __host__ __device__ inline size_t moe_ring_bytes(int stages, int blocks) { return (size_t)kMoeWarps * stages * blocks * 64; }
 
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_route(const MoeArgs a) {
 }
 
 // One CTA per SM: its warps take (selected expert, position) pairs in turn; gate and up are rows 2 i and 2 i + 1.
-// Measured (gpt-oss-20B shape, 4 experts, 70.5 MB, cold caches): 31.5 us with plain loads, 29.5 us.
+// Measured (gpt-oss-20B shape, 4 experts, 70.5 MB, cold caches): 31.5 us with plain loads, 29.5 us with 8 warps of four stages.
 __global__ void __launch_bounds__(kMoeWarps * 32, 1) moe_gate_up(const MoeArgs a, const int stages, const int blocks) {
     extern __shared__ __align__(128) unsigned char me_smem[];
     __shared__ __align__(8) unsigned long long bars[kMoeWarps * kMoeMaxStages];
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(kMoeWarps * 32, 1) moe_gate_up(const MoeArgs a
 // One CTA per SM takes pairs of output columns; a warp's unit is a pair's rows of one selected expert, and the experts' shares of a column meet in
 // shared memory, added in the order of the selection.  The routing was complete before this kernel could start (see moe_gate_up), so the
 // weights are on their way before the previous kernel is waited for.
-// Measured (gpt-oss-20B shape, 4 experts, 35.3 MB, cold caches): 37 us with plain loads and a warp per column, 22.2 us.
+// Measured (gpt-oss-20B shape, 4 experts, 35.3 MB, cold caches): 37 us with plain loads and a warp per column, 22.2 us with 8 warps of four stages.
 __global__ void __launch_bounds__(kMoeWarps * 32, 1) moe_down(const MoeArgs a, const int stages, const int blocks) {
     extern __shared__ __align__(128) unsigned char me_smem[];
     __shared__ __align__(8) unsigned long long bars[kMoeWarps * kMoeMaxStages];
@@ -435,13 +435,13 @@ cudaError_t launch_moe_experts(const MoeArgs& a_in, int sm_count, cudaStream_t s
     const size_t act_gu = 3 * (size_t)a.hidden + (size_t)(a.hidden / 32) * 4 + (size_t)a.top_k * sizeof(MoeSel);
     const size_t pairs = ((size_t)a.hidden / 2 + sm_count - 1) / sm_count;
     const size_t act_dn = (size_t)a.top_k * ((3 * (size_t)a.ffn + (size_t)(a.ffn / 32) * 4 + 15) & ~(size_t)15) + (size_t)a.top_k * sizeof(MoeSel) + pairs * a.top_k * 8;
-    // the ring: four stages of whole rows (up to 96 blocks) where they fit, down to two of 16 blocks
+    // the ring: two stages of whole rows (up to 96 blocks) where they fit, down to 16 blocks
     auto launch = [&](const void* fn, size_t act, int K) -> cudaError_t {
-        constexpr size_t kMost = 224 * 1024;
+        constexpr size_t kMost = 226 * 1024;
         int stages = kMoeMaxStages, blocks = K / 32 < kMoeBlocks ? K / 32 : kMoeBlocks;
-        while (act + moe_ring_bytes(stages, blocks) > kMost && (stages > 2 || blocks > 16)) {
-            if (stages > 2) stages--;
-            else blocks = blocks / 2 < 16 ? 16 : blocks / 2;
+        while (act + moe_ring_bytes(stages, blocks) > kMost && (stages > 1 || blocks > 16)) {
+            if (blocks > 16) blocks = blocks / 2 < 16 ? 16 : blocks / 2;
+            else stages--;
         }
         const size_t smem = act + moe_ring_bytes(stages, blocks);
         if (smem > kMost) return cudaErrorInvalidValue;
