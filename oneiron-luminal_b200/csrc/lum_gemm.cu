@@ -795,7 +795,7 @@ static SkinnyPlan gemm_plan(int groups, int nc, int K, int sms) {
     const int tpr = K / kTileK, most = nc == 64 ? kGsRG : 2 * kGsRG;       // two tiles share activation slices that are all resident
     SkinnyPlan best{1, (groups + most - 1) / most};
     double best_t = 1e30;
-    for (int ks = 1; ks <= 8 && ks <= tpr; ks++) {
+    for (int ks = 1; ks <= kMaxKsplit && ks <= tpr; ks++) {
         const double plane_us = (double)nc * groups * kTileRows * 8.0 / 6.5e6;
         for (int p = 1; p <= 64; p++) {                                     // items per SM
             int chunks = (int)((long long)sms * p / ks);
@@ -827,14 +827,13 @@ static GemmShape gemm_shape_wide(int n_rows_total, int M, int K, int sm_count) {
     const int tiles = (n_rows_total + kGmRows - 1) / kGmRows, tpr = K / kTileK;
     const double plane_us = (double)M * n_rows_total * 8.0 / 6.5e6;               // write + read of one plane of partial sums
     auto cost = [&](int nc, int ks, double t_tile) {
-        const long long items = (long long)tiles * ((M + nc - 1) / nc) * ks;
-        const long long rounds = (items + sm_count - 1) / sm_count;
+        const int rounds = (tiles * ((M + nc - 1) / nc) * ks + sm_count - 1) / sm_count;
         return (double)rounds * ((double)((tpr + ks - 1) / ks) * t_tile + 0.33 * t_tile) + (ks - 1) * plane_us;
     };
     int least = 1;
-    for (int ks = 2; ks <= 8 && ks <= tpr; ks++) {
+    for (int ks = 2; ks <= kMaxKsplit && ks <= tpr; ks++) {
         auto first = [&](int k) {
-            const long long rounds = ((long long)tiles * ((M + kGmMaxChunk - 1) / kGmMaxChunk) * k + sm_count - 1) / sm_count;
+            const int rounds = (tiles * ((M + kGmMaxChunk - 1) / kGmMaxChunk) * k + sm_count - 1) / sm_count;
             return (double)rounds * ((double)tpr / k + 0.33) * 14.4 + (k - 1) * plane_us;
         };
         if (first(ks) < first(least) * 0.97) least = ks;                          // a larger split has to pay for itself
@@ -843,7 +842,7 @@ static GemmShape gemm_shape_wide(int n_rows_total, int M, int K, int sm_count) {
     auto tile = [](int nc) { return 2.9 + 5.85 * nc / kGmMaxChunk; };
     double best_t = cost(kGmMaxChunk, least, tile(kGmMaxChunk));
     for (int nc = kGmMaxChunk; nc >= 80; nc -= 16)
-        for (int ks = least; ks <= 8 && ks <= tpr; ks++) {
+        for (int ks = least; ks <= kMaxKsplit && ks <= tpr; ks++) {
             const double t = cost(nc, ks, tile(nc));
             if (t < best_t * 0.98) { best_t = t; best = {nc, ks}; }
         }
