@@ -454,23 +454,53 @@ __device__ __forceinline__ void attn_decode_body(const AttnArgs& a, unsigned cha
     attn_merge_ticket<HD>(a, &s_last, kvh, G, tid, kAttnThreads, bar_id);
 }
 
-// ---- Products of attention on m16n8k16 tensor-core instructions (bf16 operands, f32 sums) without giving up f32 operands: K and V are bf16
+// ---- Products of attention on m16n8k16 tensor-core instructions (bf16 operands) without giving up f32 operands: K and V are bf16
 // already; an f32 query or softmax weight is the sum of THREE bf16 terms (24 bits: all of it), and the terms take the rows of the first
-// operand that a group of four query heads leaves free: row h holds head h's first term, row 4 + h its second, row 8 + h its third.
-// The three rows' results are added.
-__device__ __forceinline__ void attn_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+// operand that a group of four query heads leaves free: row h holds head h's first term, rows 4 + h and 12 + h its second and third, so that
+// the two small ones meet in one thread and the sum of the three is rounded once.
+//
+// The tensor core cuts every sum it hands back to 24 bits, always towards zero: carried from instruction to instruction, the loss grows with the
+// number of keys and does not cancel (30000 keys, one split: 2.1e-5 of the result, 2.5e-7 with f32 additions).  So a sum leaves the tensor
+// core after one instruction (16 products), and the rest is added up in f32, rounded to nearest: scores pairwise, values tile by tile.
+__device__ __forceinline__ void attn_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, float c2, float c3) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f), "f"(0.0f), "f"(c2), "f"(c3));
 }
-// Two neighbouring elements for this thread's two rows, g = lane / 4 and g + 8: the first and the third terms of head g (g < 4), or the second
-// terms of head g - 4 and nothing
+// Scores of eight keys, two of them this thread's: the sums of the KS instructions of 16 dimensions each; the third terms' row, 2^-16 of the rest,
+// is carried along inside
+template <int KS> struct AttnScore { float d[KS][2], c2, c3; };
+template <int KS>
+__device__ __forceinline__ void attn_mma_score(AttnScore<KS>& s, int ks, const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    float d[4];
+    attn_mma(d, a, b0, b1, ks ? s.c2 : 0.0f, ks ? s.c3 : 0.0f);
+    s.d[ks][0] = d[0]; s.d[ks][1] = d[1]; s.c2 = d[2]; s.c3 = d[3];
+}
+template <int KS>
+__device__ __forceinline__ float attn_score(AttnScore<KS>& s, int e) {
+#pragma unroll
+    for (int w = 1; w < KS; w *= 2)
+#pragma unroll
+        for (int i = 0; i + w < KS; i += 2 * w) s.d[i][e] += s.d[i + w][e];
+    const float x = s.d[0][e] + (e ? s.c3 : s.c2);                   // first term, or second and third
+    return x + __shfl_xor_sync(0xffffffffu, x, 16);
+}
+// values: 16 more keys, behind what the old ones are worth under the new maximum
+__device__ __forceinline__ void attn_mma_value(float (&o)[2], float corr, const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    float d[4];
+    attn_mma(d, a, b0, b1, 0.0f, 0.0f);
+    o[0] = fmaf(o[0], corr, d[0] + d[2]);
+    o[1] = fmaf(o[1], corr, d[1] + d[3]);
+}
+// Two neighbouring elements for this thread's two rows, g = lane / 4 and g + 8: the first terms of head g (g < 4) and nothing, or the second and
+// the third terms of head g - 4
 __device__ __forceinline__ void attn_terms(float x0, float x1, bool second, uint32_t* lo_row, uint32_t* hi_row) {
     const __nv_bfloat162 t1 = __floats2bfloat162_rn(x0, x1);
     const float r0 = x0 - __low2float(t1), r1 = x1 - __high2float(t1);
     const __nv_bfloat162 t2 = __floats2bfloat162_rn(r0, r1);
     const __nv_bfloat162 t3 = __floats2bfloat162_rn(r0 - __low2float(t2), r1 - __high2float(t2));
     *lo_row = second ? *(const uint32_t*)&t2 : *(const uint32_t*)&t1;
-    *hi_row = second ? 0u : *(const uint32_t*)&t3;
+    *hi_row = second ? *(const uint32_t*)&t3 : 0u;
 }
 
 // ---- Single-token attention over a bf16 cache on the tensor core: the form every decode step takes whose heads fit it (up to four query heads
@@ -669,22 +699,16 @@ __device__ __forceinline__ void attn_tc_body(const AttnArgs& a, unsigned char* s
     sync();
 
     // ---- the cached rows
-    float o[MT][NT][4], mx[MT], l[MT];
+    float o[MT][NT][2], mx[MT], l[MT];
 #pragma unroll
     for (int mt = 0; mt < MT; mt++) {
         mx[mt] = -INFINITY; l[mt] = 0.0f;
 #pragma unroll
-        for (int n = 0; n < NT; n++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) o[mt][n][e] = 0.0f;
+        for (int n = 0; n < NT; n++) o[mt][n][0] = o[mt][n][1] = 0.0f;
     }
 #pragma unroll 1
     for (int j0 = r0 + warp * kAttnTcTile; j0 < r1; j0 += NW * kAttnTcTile) {
-        float s[MT][2][4];
-#pragma unroll
-        for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) s[mt][0][e] = s[mt][1][e] = 0.0f;
+        AttnScore<KS> s[MT][2];
 #pragma unroll
         for (int ks = 0; ks < KS; ks++) {
 #pragma unroll
@@ -692,40 +716,34 @@ __device__ __forceinline__ void attn_tc_body(const AttnArgs& a, unsigned char* s
                 const uint4 w = s_a[(mt * KS + ks) * 32 + lane];
                 const uint32_t qa[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-                for (int y = 0; y < 2; y++) attn_mma(s[mt][y], qa, attn_word(f.k[y][ks >> 1], 2 * (ks & 1)), attn_word(f.k[y][ks >> 1], 2 * (ks & 1) + 1));
+                for (int y = 0; y < 2; y++) attn_mma_score(s[mt][y], ks, qa, attn_word(f.k[y][ks >> 1], 2 * (ks & 1)), attn_word(f.k[y][ks >> 1], 2 * (ks & 1) + 1));
             }
         }
         const int jn = j0 + NW * kAttnTcTile;
         if (jn < r1) attn_tc_load_k<HD>(a, f, kvh, jn, r1, lane);
         const int j = j0 + 2 * t;                                     // this thread's keys: j, j + 1, j + 8, j + 9
         uint32_t pa[MT][4];
+        float corr[MT];
 #pragma unroll
         for (int mt = 0; mt < MT; mt++) {
             float v[4];
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                float y = s[mt][e >> 1][e & 1] + s[mt][e >> 1][2 + (e & 1)];       // rows g and g + 8
-                y += __shfl_xor_sync(0xffffffffu, y, 16);                          // and the second terms' row
+                const float y = attn_score(s[mt][e >> 1], e & 1);
                 v[e] = j + (e >> 1) * 8 + (e & 1) < r1 ? y * scale : -INFINITY;
             }
             float tm = fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3]));
             tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 1));
             tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 2));
             const float mn = fmaxf(mx[mt], tm);                       // a tile always holds at least one live key
-            const float corr = mx[mt] == -INFINITY ? 0.0f : expf(mx[mt] - mn);
+            corr[mt] = mx[mt] == -INFINITY ? 0.0f : expf(mx[mt] - mn);
             mx[mt] = mn;
             float ps = 0.0f;
 #pragma unroll
             for (int e = 0; e < 4; e++) { v[e] = v[e] == -INFINITY ? 0.0f : expf(v[e] - mn); ps += v[e]; }
-            l[mt] = l[mt] * corr + ps;                                // per-lane partial sums, folded at the end
+            l[mt] = l[mt] * corr[mt] + ps;                            // per-lane partial sums, folded at the end
             attn_terms(v[0], v[1], second, &pa[mt][0], &pa[mt][1]);
             attn_terms(v[2], v[3], second, &pa[mt][2], &pa[mt][3]);
-            if (__any_sync(0xffffffffu, corr != 1.0f)) {
-#pragma unroll
-                for (int n = 0; n < NT; n++)
-#pragma unroll
-                    for (int e = 0; e < 4; e++) o[mt][n][e] *= corr;
-            }
         }
         // column g of tile 8 jj + i is dimension 64 jj + 8 g + i
 #pragma unroll
@@ -736,7 +754,7 @@ __device__ __forceinline__ void attn_tc_body(const AttnArgs& a, unsigned char* s
                 const uint32_t b0 = __byte_perm(attn_word(f.v[0][jj], i >> 1), attn_word(f.v[1][jj], i >> 1), sel);
                 const uint32_t b1 = __byte_perm(attn_word(f.v[2][jj], i >> 1), attn_word(f.v[3][jj], i >> 1), sel);
 #pragma unroll
-                for (int mt = 0; mt < MT; mt++) attn_mma(o[mt][jj * 8 + i], pa[mt], b0, b1);
+                for (int mt = 0; mt < MT; mt++) attn_mma_value(o[mt][jj * 8 + i], corr[mt], pa[mt], b0, b1);
             }
         if (jn < r1) attn_tc_load_v<HD>(a, f, kvh, jn, r1, lane);
     }
@@ -750,7 +768,7 @@ __device__ __forceinline__ void attn_tc_body(const AttnArgs& a, unsigned char* s
         if (t == 0 && !second) { s_m[warp][h] = mx[mt]; s_l[warp][h] = lt; }
 #pragma unroll
         for (int n = 0; n < NT; n++) {
-            float x0 = o[mt][n][0] + o[mt][n][2], x1 = o[mt][n][1] + o[mt][n][3];
+            float x0 = o[mt][n][0], x1 = o[mt][n][1];
             x0 += __shfl_xor_sync(0xffffffffu, x0, 16);
             x1 += __shfl_xor_sync(0xffffffffu, x1, 16);
             float* dst = s_o + ((size_t)warp * G + h) * HD + (n >> 3) * 64 + 16 * t + (n & 7);

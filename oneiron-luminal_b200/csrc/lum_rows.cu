@@ -213,11 +213,12 @@ __global__ void __launch_bounds__(256) attn_rows(const AttnRowsArgs a) {
 //   * a cluster of CTAs per (KV head, row), one CTA per split of the cached positions, four warps per CTA.  Warps do not wait for
 //     each other: each takes 16 keys at a time and fetches their K and V (cp.async, coalesced 16-byte pieces, rows swizzled so that
 //     ldmatrix reads them without bank conflicts) into its own ring in shared memory, ar_stages - 1 tiles ahead.
-//   * both products are tensor-core instructions over three bf16 terms of the f32 operand (attn_terms): nothing is rounded to fewer bits
-//     than the plain evaluation keeps.
+//   * both products are tensor-core instructions over three bf16 terms of the f32 operand (attn_terms), whose 24 bits they keep; what goes
+//     beyond one instruction is added up in f32 (attn_mma).
 //   * warps merge in shared memory, splits through the cluster's distributed shared memory: no partial results in global memory and no
 //     second kernel.
-// Measured (32 sequences x 2049 keys, 8 KV heads x 4 query heads, head dimension 128; 268 MB of cache): 53 us.  The form before it, with
+// Measured (32 sequences x 2049 keys, 8 KV heads x 4 query heads, head dimension 128; 268 MB of cache): 53 us with sums left in the tensor
+// core, a whole step of 32 Llama-3-8B rows 0.7 % slower this way (6.49 -> 6.53 ms).  The form before it, with
 // a lane per key and the products on CUDA cores (1700 instructions per warp and 32 keys, 16-byte loads 2 KiB apart), took 147 us and
 // 6 us more to merge.
 __device__ __forceinline__ void ar_ldsm4(uint32_t addr, uint32_t (&r)[4]) {
@@ -235,7 +236,7 @@ __host__ __device__ constexpr int ar_smem(int hd) { return 4 * ar_stages(hd) * 2
 
 // MT: groups of four query heads (G <= 4 MT)
 template <int HD, int MT>
-__global__ void __launch_bounds__(128) attn_rows_split(const AttnRowsArgs a, int n_splits) {
+__global__ void __launch_bounds__(128, 3) attn_rows_split(const AttnRowsArgs a, int n_splits) {
     constexpr int NW = 4, NT = HD / 8, KS = HD / 16, CH = HD / 8, GM = 4 * MT, NS = ar_stages(HD);
     constexpr int kSide = kArTile * HD * 2, kStage = 2 * kSide;     // bytes of one tile's K (or V); of both
     extern __shared__ __align__(128) unsigned char ar_sm[];
@@ -293,14 +294,12 @@ __global__ void __launch_bounds__(128) attn_rows_split(const AttnRowsArgs a, int
                 attn_terms(v.x, v.y, second, &qa[mt][ks][2 * e], &qa[mt][ks][2 * e + 1]);
             }
     }
-    float o[MT][NT][4], mx[MT], l[MT];
+    float o[MT][NT][2], mx[MT], l[MT];
 #pragma unroll
     for (int mt = 0; mt < MT; mt++) {
         mx[mt] = -INFINITY; l[mt] = 0.0f;
 #pragma unroll
-        for (int n = 0; n < NT; n++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) o[mt][n][e] = 0.0f;
+        for (int n = 0; n < NT; n++) o[mt][n][0] = o[mt][n][1] = 0.0f;
     }
     const int kkey = ((lane >> 4) << 3) + (lane & 7), kch = (lane >> 3) & 1;       // this lane's row and 16-byte group in a ldmatrix of K ...
     const int vkey = (((lane >> 3) & 1) << 3) + (lane & 7), vch = lane >> 4;        // ... and of V
@@ -310,54 +309,44 @@ __global__ void __launch_bounds__(128) attn_rows_split(const AttnRowsArgs a, int
         asm volatile("cp.async.wait_group %0;" ::"n"(NS - 1) : "memory");
         __syncwarp();
         const uint32_t kb = ring + (uint32_t)(i % NS) * kStage, vb = kb + kSide;
-        float s[MT][2][4];
-#pragma unroll
-        for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) s[mt][0][e] = s[mt][1][e] = 0.0f;
+        AttnScore<KS> s[MT][2];
 #pragma unroll
         for (int ks = 0; ks < KS; ks++) {
             uint32_t b[4];
             ar_ldsm4(kb + (uint32_t)(kkey * HD * 2 + (((ks * 2 + kch) ^ (kkey & 7)) << 4)), b);
 #pragma unroll
-            for (int mt = 0; mt < MT; mt++) { attn_mma(s[mt][0], qa[mt][ks], b[0], b[1]); attn_mma(s[mt][1], qa[mt][ks], b[2], b[3]); }
+            for (int mt = 0; mt < MT; mt++) { attn_mma_score(s[mt][0], ks, qa[mt][ks], b[0], b[1]); attn_mma_score(s[mt][1], ks, qa[mt][ks], b[2], b[3]); }
         }
         const int j = j_first + 64 * i + 2 * t;                       // this thread's keys: j, j + 1, j + 8, j + 9
         uint32_t pa[MT][4];
+        float corr[MT];
 #pragma unroll
         for (int mt = 0; mt < MT; mt++) {
             float v[4];
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                float x = s[mt][e >> 1][e & 1] + s[mt][e >> 1][2 + (e & 1)];       // rows g and g + 8
-                x += __shfl_xor_sync(0xffffffffu, x, 16);                          // and the second terms' row
+                const float x = attn_score(s[mt][e >> 1], e & 1);
                 v[e] = j + (e >> 1) * 8 + (e & 1) < k1 ? x * scale : -INFINITY;
             }
             float tm = fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3]));
             tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 1));
             tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 2));
             const float mn = fmaxf(mx[mt], tm);                       // a tile always holds at least one live key
-            const float corr = mx[mt] == -INFINITY ? 0.0f : expf(mx[mt] - mn);
+            corr[mt] = mx[mt] == -INFINITY ? 0.0f : expf(mx[mt] - mn);
             mx[mt] = mn;
             float ps = 0.0f;
 #pragma unroll
             for (int e = 0; e < 4; e++) { v[e] = v[e] == -INFINITY ? 0.0f : expf(v[e] - mn); ps += v[e]; }
-            l[mt] = l[mt] * corr + ps;                                // per-lane partial sums, folded at the end
+            l[mt] = l[mt] * corr[mt] + ps;                            // per-lane partial sums, folded at the end
             attn_terms(v[0], v[1], second, &pa[mt][0], &pa[mt][1]);
             attn_terms(v[2], v[3], second, &pa[mt][2], &pa[mt][3]);
-            if (__any_sync(0xffffffffu, corr != 1.0f)) {
-#pragma unroll
-                for (int n = 0; n < NT; n++)
-#pragma unroll
-                    for (int e = 0; e < 4; e++) o[mt][n][e] *= corr;
-            }
         }
 #pragma unroll
         for (int np = 0; np < NT / 2; np++) {
             uint32_t b[4];
             ar_ldsm4_t(vb + (uint32_t)(vkey * HD * 2 + (((np * 2 + vch) ^ (vkey & 7)) << 4)), b);
 #pragma unroll
-            for (int mt = 0; mt < MT; mt++) { attn_mma(o[mt][2 * np], pa[mt], b[0], b[1]); attn_mma(o[mt][2 * np + 1], pa[mt], b[2], b[3]); }
+            for (int mt = 0; mt < MT; mt++) { attn_mma_value(o[mt][2 * np], corr[mt], pa[mt], b[0], b[1]); attn_mma_value(o[mt][2 * np + 1], corr[mt], pa[mt], b[2], b[3]); }
         }
         __syncwarp();
     }
@@ -379,7 +368,7 @@ __global__ void __launch_bounds__(128) attn_rows_split(const AttnRowsArgs a, int
         if (t == 0 && !second) { s_m[warp * GM + h] = mx[mt]; s_l[warp * GM + h] = lt; }
 #pragma unroll
         for (int n = 0; n < NT; n++) {
-            float x0 = o[mt][n][0] + o[mt][n][2], x1 = o[mt][n][1] + o[mt][n][3];
+            float x0 = o[mt][n][0], x1 = o[mt][n][1];
             x0 += __shfl_xor_sync(0xffffffffu, x0, 16);
             x1 += __shfl_xor_sync(0xffffffffu, x1, 16);
             if (!second) *(float2*)(s_o + (warp * GM + h) * HD + n * 8 + 2 * t) = make_float2(x0, x1);

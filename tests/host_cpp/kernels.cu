@@ -1,0 +1,133 @@
+// Kernels called through the library's own launchers, without a model around them, against sums in 64 bits.  One check per command; prints a line
+// per case: name, largest or relative error, bound.
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <random>
+#include <string>
+#include <vector>
+
+#include "lum_rows.cuh"
+
+using namespace lum;
+
+#define CK(x) do { const cudaError_t e_ = (x); if (e_ != cudaSuccess) { std::printf("%s: %s\n", #x, cudaGetErrorString(e_)); std::exit(2); } } while (0)
+
+static int failures = 0;
+static void report(const std::string& what, double err, double bound) {
+    const bool ok = err <= bound;                       // (false for a NaN)
+    if (!ok) failures++;
+    std::printf("%s %s: %.3e, bound %.3e\n", ok ? "ok" : "FAILED", what.c_str(), err, bound);
+}
+
+template <typename T> struct Dev {                      // a device array, filled from or read into a vector
+    T* p = nullptr; size_t n;
+    explicit Dev(size_t n_) : n(n_) { CK(cudaMalloc(&p, n * sizeof(T))); CK(cudaMemset(p, 0, n * sizeof(T))); }
+    explicit Dev(const std::vector<T>& v) : Dev(v.size()) { put(v); }
+    ~Dev() { cudaFree(p); }
+    Dev(const Dev&) = delete;
+    void put(const std::vector<T>& v) { CK(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice)); }
+    std::vector<T> get() const { std::vector<T> v(n); CK(cudaDeviceSynchronize()); CK(cudaMemcpy(v.data(), p, n * sizeof(T), cudaMemcpyDeviceToHost)); return v; }
+};
+
+static std::vector<float> normal(std::mt19937& rng, size_t n, float std, float mean = 0.0f) {
+    std::normal_distribution<float> d(mean, std);
+    std::vector<float> v(n);
+    for (float& x : v) x = d(rng);
+    return v;
+}
+static uint16_t bf16_bits(float x) { uint32_t u; std::memcpy(&u, &x, 4); return (uint16_t)((u + 0x7fffu + ((u >> 16) & 1u)) >> 16); }
+static float bf16_value(uint16_t b) { const uint32_t u = (uint32_t)b << 16; float x; std::memcpy(&x, &u, 4); return x; }
+static std::vector<uint16_t> to_bf16(const std::vector<float>& v) { std::vector<uint16_t> b(v.size()); for (size_t i = 0; i < v.size(); i++) b[i] = bf16_bits(v[i]); return b; }
+static double rel(const std::vector<float>& got, const std::vector<double>& want) {
+    double a = 0, b = 0;
+    for (size_t i = 0; i < want.size(); i++) { a += (got[i] - want[i]) * (got[i] - want[i]); b += want[i] * want[i]; }
+    return std::sqrt(a / b);
+}
+
+// ---- attention of one token behind n cached rows of bf16 keys and values; queries as given (the rotation's angles are zero)
+struct Attention {
+    int nq, nkv, hd, n, max_seq;
+    std::vector<float> q;
+    std::vector<uint16_t> k, v;                         // n + 1 rows: the last is the token's own
+    Attention(int nq_, int nkv_, int hd_, int n_, float q_std, float v_mean) : nq(nq_), nkv(nkv_), hd(hd_), n(n_), max_seq((n_ + 64) / 64 * 64 + 64) {
+        std::mt19937 rng(n + nq);
+        q = normal(rng, (size_t)nq * hd, q_std);
+        k = to_bf16(normal(rng, (size_t)max_seq * nkv * hd, 1.0f));
+        v = to_bf16(normal(rng, (size_t)max_seq * nkv * hd, 1.0f, v_mean));
+    }
+    std::vector<double> exact() const {
+        std::vector<double> out((size_t)nq * hd), w(n + 1);
+        for (int h = 0; h < nq; h++) {
+            const size_t col = (size_t)(h / (nq / nkv)) * hd, ld = (size_t)nkv * hd;
+            double mx = -INFINITY, l = 0;
+            for (int j = 0; j <= n; j++) {
+                double d = 0;
+                for (int e = 0; e < hd; e++) d += (double)q[(size_t)h * hd + e] * bf16_value(k[j * ld + col + e]);
+                w[j] = d * (double)(1.0f / std::sqrt((float)hd));
+                mx = std::fmax(mx, w[j]);
+            }
+            for (int j = 0; j <= n; j++) l += w[j] = std::exp(w[j] - mx);
+            for (int j = 0; j <= n; j++)
+                for (int e = 0; e < hd; e++) out[(size_t)h * hd + e] += w[j] / l * bf16_value(v[j * ld + col + e]);
+        }
+        return out;
+    }
+    std::vector<float> own(const std::vector<uint16_t>& c) const {
+        std::vector<float> r((size_t)nkv * hd);
+        for (size_t i = 0; i < r.size(); i++) r[i] = bf16_value(c[(size_t)n * nkv * hd + i]);
+        return r;
+    }
+    // one decode step's kernel
+    std::vector<float> step(int splits, bool cluster) const {
+        DecodeState s{};
+        s.pos = n; s.max_seq = max_seq;
+        Dev<float> dq(q), dk(own(k)), dv(own(v)), out(q.size()), part((size_t)nq * splits * (hd + 2)), inv_freq((size_t)hd / 2);
+        Dev<uint16_t> kc(k), vc(v);
+        Dev<unsigned int> counters((size_t)nkv);
+        Dev<uint32_t> status(1);
+        Dev<DecodeState> state(std::vector<DecodeState>{s});
+        AttnArgs a{};
+        a.q = dq.p; a.k_new = dk.p; a.v_new = dv.p; a.k_cache = kc.p; a.v_cache = vc.p; a.out = out.p; a.part = part.p; a.counters = counters.p; a.state = state.p;
+        a.n_q = nq; a.n_kv = nkv; a.hd = hd; a.n_splits = splits; a.kv_bf16 = 1; a.rope_style = 2; a.inv_freq = inv_freq.p; a.attn_factor = 1.0f; a.max_seq = max_seq;
+        a.status = status.p; a.cluster = cluster;
+        CK(launch_attn_decode(a, nullptr));
+        return out.get();
+    }
+    // the same token as one of a step of several rows
+    std::vector<float> row() const {
+        Dev<float> dq(q), out(q.size());
+        Dev<uint16_t> kc(k), vc(v);
+        Dev<uint32_t> status(1);
+        Dev<int> pos(std::vector<int>{n});
+        AttnRowsArgs a{};
+        a.q_rot = dq.p; a.k_cache = kc.p; a.v_cache = vc.p; a.row_pos = pos.p; a.out = out.p; a.M = 1; a.n_q = nq; a.n_kv = nkv; a.hd = hd; a.kv_bf16 = 1;
+        a.max_seq = max_seq; a.max_batch = 1; a.status = status.p;
+        CK(launch_attn_rows(a, nullptr));
+        return out.get();
+    }
+};
+
+// Long sums stay sums of 32 bits.  A split's values are added up tile by tile, 64 keys of a CTA at a time: m additions of relative error 2^-24 at most
+// walk about sqrt(m) of them away, and scores, weights and each tile's own sum (cut, not rounded) are a few more.
+static void attention_sums() {
+    for (int hd : {64, 128})
+        for (float v_mean : {0.0f, 1.0f}) {
+            const Attention a(4, 1, hd, 30000, 1.0f, v_mean);
+            const std::vector<double> want = a.exact();
+            auto bound = [&](int splits) { return (4 + std::sqrt(a.n / 64.0 / splits)) * std::exp2(-24.0); };
+            const std::string what = std::to_string(hd) + (v_mean ? " same sign" : " both signs");
+            report("step, 1 split, " + what, rel(a.step(1, false), want), bound(1));
+            report("step, 8 splits, " + what, rel(a.step(8, false), want), bound(8));
+            report("step, cluster of 8, " + what, rel(a.step(8, true), want), bound(8));
+            report("row, " + what, rel(a.row(), want), bound(8));
+        }
+}
+
+int main(int argc, char** argv) {
+    const std::string what = argc > 1 ? argv[1] : "";
+    if (what == "attention-sums") attention_sums();
+    else { std::printf("unknown check\n"); return 2; }
+    return failures ? 1 : 0;
+}
