@@ -503,6 +503,40 @@ __device__ __forceinline__ void attn_terms(float x0, float x1, bool second, uint
     *hi_row = second ? *(const uint32_t*)&t3 : 0u;
 }
 
+// An infinity breaks the sum of terms (infinity times a zero term, or a first term rounded up to infinity): where a warp's state does not come out
+// finite, it takes its keys once more, element by element in f32.  Keys first + 64 i .. + 15 below `end`; q [G][HD].
+template <int HD>
+__device__ __noinline__ void attn_plain_keys(const __nv_bfloat16* k, const __nv_bfloat16* v, KvPages pg, int seq, int max_seq, size_t row_elems, int first, int end,
+                                             const float* q, int G, int lane, float* s_m, float* s_l, float* s_o) {
+    constexpr int N = HD / 32;
+    const float scale = 1.0f / sqrtf((float)HD);
+    __syncwarp();                                                    // (the state in place is overwritten)
+#pragma unroll 1
+    for (int h = 0; h < G; h++) {
+        float x[N], o[N], mx = -INFINITY, l = 0.0f;
+#pragma unroll
+        for (int i = 0; i < N; i++) { x[i] = q[h * HD + lane + 32 * i]; o[i] = 0.0f; }
+#pragma unroll 1
+        for (int j0 = first; j0 < end; j0 += 64)
+#pragma unroll 1
+            for (int j = j0; j < min(end, j0 + 16); j++) {
+                const size_t off = kv_phys_row(pg, seq, max_seq, j) * row_elems + lane;
+                float d = 0.0f;
+#pragma unroll
+                for (int i = 0; i < N; i++) d = fmaf(x[i], __bfloat162float(k[off + 32 * i]), d);
+                const float logit = warp_sum(d) * scale, mn = fmaxf(mx, logit);
+                const float corr = mx == -INFINITY ? 0.0f : expf(mx - mn), w = logit == -INFINITY ? 0.0f : expf(logit - mn);
+                l = l * corr + w;
+#pragma unroll
+                for (int i = 0; i < N; i++) o[i] = fmaf(w, __bfloat162float(v[off + 32 * i]), o[i] * corr);
+                mx = mn;
+            }
+        if (lane == 0) { s_m[h] = mx; s_l[h] = l; }
+#pragma unroll
+        for (int i = 0; i < N; i++) s_o[h * HD + lane + 32 * i] = o[i];
+    }
+}
+
 // ---- Single-token attention over a bf16 cache on the tensor core: the form every decode step takes whose heads fit it (up to four query heads
 // of 128 dimensions or eight of 64 per KV head; others, and f32 caches, take the form above).
 //
@@ -759,6 +793,7 @@ __device__ __forceinline__ void attn_tc_body(const AttnArgs& a, unsigned char* s
         if (jn < r1) attn_tc_load_v<HD>(a, f, kvh, jn, r1, lane);
     }
     // ---- add up the terms' rows and the lanes' sums, then the warps
+    float odd[2] = {0.0f, 0.0f};                            // sums of x * 0: 0, or NaN where something is not finite
 #pragma unroll
     for (int mt = 0; mt < MT; mt++) {
         const int h = mt * 4 + (g & 3);
@@ -766,15 +801,21 @@ __device__ __forceinline__ void attn_tc_body(const AttnArgs& a, unsigned char* s
         lt += __shfl_xor_sync(0xffffffffu, lt, 1);
         lt += __shfl_xor_sync(0xffffffffu, lt, 2);
         if (t == 0 && !second) { s_m[warp][h] = mx[mt]; s_l[warp][h] = lt; }
+        odd[0] = fmaf(mx[mt], 0.0f, odd[0]); odd[1] = fmaf(lt, 0.0f, odd[1]);
 #pragma unroll
         for (int n = 0; n < NT; n++) {
             float x0 = o[mt][n][0], x1 = o[mt][n][1];
             x0 += __shfl_xor_sync(0xffffffffu, x0, 16);
             x1 += __shfl_xor_sync(0xffffffffu, x1, 16);
+            odd[0] = fmaf(x0, 0.0f, odd[0]); odd[1] = fmaf(x1, 0.0f, odd[1]);
             float* dst = s_o + ((size_t)warp * G + h) * HD + (n >> 3) * 64 + 16 * t + (n & 7);
             if (!second && h < G) { dst[0] = x0; dst[8] = x1; }
         }
     }
+    const int j_first = r0 + warp * kAttnTcTile;
+    if (j_first < r1 && __any_sync(0xffffffffu, odd[0] + odd[1] != 0.0f))
+        attn_plain_keys<HD>((const __nv_bfloat16*)a.k_cache + (size_t)kvh * HD, (const __nv_bfloat16*)a.v_cache + (size_t)kvh * HD, a.pg, 0, 0, row_elems, j_first, r1,
+                            &s_q[0][0], G, lane, s_m[warp], s_l[warp], s_o + (size_t)warp * G * HD);
     sync();
     const int parts = owns_new ? NP : NW;
     const int S = a.n_splits, total = G * HD, chunk = (total + S - 1) / S;      // outputs CTA r of the cluster finishes: [r * chunk, (r + 1) * chunk)

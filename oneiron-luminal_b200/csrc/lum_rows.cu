@@ -359,6 +359,7 @@ __global__ void __launch_bounds__(128, 3) attn_rows_split(const AttnRowsArgs a, 
     float* s_l = s_m + NW * GM;                    // [NW][GM]
     float* s_fm = s_l + NW * GM;                   // [GM]
     float* s_fl = s_fm + GM;                       // [GM]
+    float odd[2] = {0.0f, 0.0f};                   // sums of x * 0: 0, or NaN where something is not finite
 #pragma unroll
     for (int mt = 0; mt < MT; mt++) {
         const int h = mt * 4 + (g & 3);
@@ -366,14 +367,19 @@ __global__ void __launch_bounds__(128, 3) attn_rows_split(const AttnRowsArgs a, 
         lt += __shfl_xor_sync(0xffffffffu, lt, 1);
         lt += __shfl_xor_sync(0xffffffffu, lt, 2);
         if (t == 0 && !second) { s_m[warp * GM + h] = mx[mt]; s_l[warp * GM + h] = lt; }
+        odd[0] = fmaf(mx[mt], 0.0f, odd[0]); odd[1] = fmaf(lt, 0.0f, odd[1]);
 #pragma unroll
         for (int n = 0; n < NT; n++) {
             float x0 = o[mt][n][0], x1 = o[mt][n][1];
             x0 += __shfl_xor_sync(0xffffffffu, x0, 16);
             x1 += __shfl_xor_sync(0xffffffffu, x1, 16);
+            odd[0] = fmaf(x0, 0.0f, odd[0]); odd[1] = fmaf(x1, 0.0f, odd[1]);
             if (!second) *(float2*)(s_o + (warp * GM + h) * HD + n * 8 + 2 * t) = make_float2(x0, x1);
         }
     }
+    if (n_it > 0 && __any_sync(0xffffffffu, odd[0] + odd[1] != 0.0f))
+        attn_plain_keys<HD>(kc, vc, a.pg, seq, a.max_seq, row_elems, j_first, k1, a.q_rot + ((size_t)m * a.n_q + (size_t)kvh * G) * HD, G, lane, s_m + warp * GM,
+                            s_l + warp * GM, s_o + warp * GM * HD);
     __syncthreads();
     float* out = a.out + ((size_t)m * a.n_q + (size_t)kvh * G) * HD;
     for (int idx = tid; idx < G * HD; idx += 128) {

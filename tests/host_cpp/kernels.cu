@@ -125,9 +125,47 @@ static void attention_sums() {
         }
 }
 
+// Infinite, undefined and huge elements go where the plain sums take them, and nowhere else.
+static void attention_specials() {
+    const float inf = INFINITY;
+    for (int hd : {64, 128})
+        for (int n : {40, 700})
+            for (int what = 0; what < 6; what++) {
+                Attention a(8, hd == 64 ? 1 : 2, hd, n, 1.0f, 0.0f);
+                const int key = n / 2 + 1, e = 5;
+                const size_t at = ((size_t)key * a.nkv) * hd + e;                    // element e of the first KV head's key
+                for (int h = 0; h < a.nq; h++) a.q[(size_t)h * hd + e] = 0.75f + 0.001f * h;
+                const char* name[] = {"a key of minus infinity", "a value of infinity", "an undefined value", "the lowest key", "the largest query", "two infinite values of one column"};
+                if (what == 0) a.k[at] = bf16_bits(-inf);
+                if (what == 1) a.v[at] = bf16_bits(inf);
+                if (what == 2) a.v[at] = 0x7fc0;
+                if (what == 3) a.k[at] = 0xff7f;
+                if (what == 4) {
+                    for (int h = 0; h < a.nq; h++) a.q[(size_t)h * hd + e] = 3.4e38f;
+                    for (int j = 0; j <= n; j++) for (int g = 0; g < a.nkv; g++) a.k[((size_t)j * a.nkv + g) * hd + e] = bf16_bits(j % 3 ? 2e-38f : -2e-38f);
+                }
+                if (what == 5) { a.v[at] = bf16_bits(-inf); a.v[at + (size_t)a.nkv * hd * 3] = bf16_bits(-inf); }
+                const std::vector<double> want = a.exact();
+                auto worst = [&](const std::vector<float>& got) {
+                    double m = 0;
+                    for (size_t i = 0; i < want.size(); i++) {
+                        if (std::isnan(want[i]) || std::isinf(want[i])) { if (!(std::isnan(want[i]) ? std::isnan(got[i]) : (double)got[i] == want[i])) return (double)INFINITY; }
+                        else if (!(std::fabs(got[i] - want[i]) <= m)) m = std::isnan(got[i]) ? INFINITY : std::fabs(got[i] - want[i]);
+                    }
+                    return m;
+                };
+                // values of size one, scores of up to ten: a hundred roundings
+                const std::string where = std::string(name[what]) + ", " + std::to_string(hd) + ", " + std::to_string(n);
+                report("step, 1 split, " + where, worst(a.step(1, false)), 100 * std::exp2(-24.0));
+                report("step, cluster of 4, " + where, worst(a.step(4, true)), 100 * std::exp2(-24.0));
+                report("row, " + where, worst(a.row()), 100 * std::exp2(-24.0));
+            }
+}
+
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "attention-sums") attention_sums();
+    else if (what == "attention-specials") attention_specials();
     else { std::printf("unknown check\n"); return 2; }
     return failures ? 1 : 0;
 }
