@@ -787,15 +787,31 @@ static int gemm_padded_rows(int M) { return M <= 64 ? 64 : M + kGmMaxChunk - 1; 
 size_t gemm_xq_bytes(int M, int K) { return (size_t)gemm_padded_rows(M) * K * 2 * kGmXTerms; }
 size_t gemm_sx_bytes(int M, int K) { (void)K; return (size_t)gemm_padded_rows(M) * 4; }
 
-// Up to 64 rows: K ranges and runs of row groups of a product.  An SM's time for one K-tile of n row groups is the largest of: its
+// The fewest K ranges a product may be cut into.  An accumulator's additions are cut to 24 bits, always towards zero: longer ranges cost accuracy,
+// and with operands of one sign the loss grows with the length.  So the split that a first, coarse estimate of the time gives (chunks of 32, 64
+// or 128 rows, items of 128 or 256 weight rows) is never undercut, whatever the finer estimates below would gain.
+// Measured, 28672 x 4096 at 2 to 64 rows, one range / three, error against 64 bits: normal operands 4.9e-6 / 1.7e-6, operands of one sign
+// 2.6e-5 / 8.0e-6; 16384 x 16384, one / eight: 1.07e-4 / 1.3e-5.
+static int gemm_least_split(int n_rows_total, int M, int K, int sm_count) {
+    const int nc = M <= 32 ? 32 : M <= 64 ? 64 : 128, tile_rows = M > 64 ? kGmRows : 128;
+    const int items = (n_rows_total + tile_rows - 1) / tile_rows * ((M + nc - 1) / nc), tpr = K / kTileK;
+    const double tile_us = M > 64 ? 14.4 : 16.0 * (0.16 + 0.43 * nc / 128.0), plane_us = (double)M * n_rows_total * 8.0 / 6.5e6;
+    auto cost = [&](int k) { return (double)(((long long)items * k + sm_count - 1) / sm_count) * ((double)tpr / k + 0.33) * tile_us + (k - 1) * plane_us; };
+    int best = 1;
+    for (int ks = 2; ks <= kMaxKsplit && ks <= tpr; ks++)
+        if (cost(ks) < cost(best) * 0.97) best = ks;                          // a larger split has to pay for itself
+    return best;
+}
+
+// Up to 64 rows: K ranges (at least `least`) and runs of row groups of a product.  An SM's time for one K-tile of n row groups is the largest of: its
 // share of HBM (4352 n bytes at 44 GB/s), the conversion (kGsCvtUs per tensor-core tile), and what comes
-// in from L2 and HBM together (90 GB/s); an item costs about 2.5 us beside that, a plane of partial sums its write and read at the copy rate.  Everything depends on the rows' class (nc) and not on their number, so that a plan holds for the class.
+// in from L2 and HBM together (90 GB/s); an item costs about 2.5 us beside that, a plane of partial sums its write and read at the copy rate.
 struct SkinnyPlan { int ks, chunks; };
-static SkinnyPlan gemm_plan(int groups, int nc, int K, int sms) {
+static SkinnyPlan gemm_plan(int groups, int nc, int K, int sms, int least) {
     const int tpr = K / kTileK, most = nc == 64 ? kGsRG : 2 * kGsRG;       // two tiles share activation slices that are all resident
-    SkinnyPlan best{1, (groups + most - 1) / most};
+    SkinnyPlan best{least, (groups + most - 1) / most};
     double best_t = 1e30;
-    for (int ks = 1; ks <= kMaxKsplit && ks <= tpr; ks++) {
+    for (int ks = least; ks <= kMaxKsplit && ks <= tpr; ks++) {
         const double plane_us = (double)nc * groups * kTileRows * 8.0 / 6.5e6;
         for (int p = 1; p <= 64; p++) {                                     // items per SM
             int chunks = (int)((long long)sms * p / ks);
@@ -814,30 +830,22 @@ static SkinnyPlan gemm_plan(int groups, int nc, int K, int sms) {
     return best;
 }
 
-// More rows: rows per chunk and K ranges per product.  Work items are equal, so a product takes ceil(items / SMs) rounds of one item each: with few
-// items per SM the last, partly filled round is a large share of the time (448 items over 148 SMs: 4 rounds for 3.03 rounds of work), and so are the
+// More rows: rows per chunk and K ranges (at least `least`) per product.  Work items are equal, so a product takes ceil(items / SMs) rounds of one item
+// each: with few items per SM the last, partly filled round is a large share of the time (448 items over 148 SMs: 4 rounds for 3.03 rounds of work), and so are the
 // rows that fill up the last chunk (387 rows in chunks of 128: a quarter).  Smaller chunks and more K ranges make both finer, but every item pays
 // its own pipeline fill and store, every extra range writes (and the consumer reads) another plane of partial sums, and the
 // converting warps set a floor.  Constants: measured, us per K-tile of one item (28672 x 4096 in chunks of 80 / 112 / 128 rows: 6.6 / 8.1 / 8.75),
-// an item's own cost a third of that, planes at the HBM copy rate.  An
-// accumulator's additions are cut to 24 bits, so longer ranges cost accuracy: the split that the first estimate gives (chunks of 128, items of 14 us
-// per K-tile) is never undercut.
+// an item's own cost a third of that, planes at the HBM copy rate.
 // Measured, alone, us (chunks of 128 / as chosen): 28672 x 4096 at 65 rows 74 / 58, 129 rows 143 / 109, 387 rows 264 / 231, 1000 rows 487 / 449.
-static GemmShape gemm_shape_wide(int n_rows_total, int M, int K, int sm_count) {
+// Other products, with their rows' preparation, against the kernel of chunks of 128 before it: 4096 x 14336 at 65 / 387 / 1000 rows 85 / 232 / 439 -> 52 / 159 /
+// 308, 19456 x 2560 82 / 235 / 347 -> 51 / 171 / 242, 2560 x 9728 63 / 124 / 234 -> 41 / 93 / 182.
+static GemmShape gemm_shape_wide(int n_rows_total, int M, int K, int sm_count, int least) {
     const int tiles = (n_rows_total + kGmRows - 1) / kGmRows, tpr = K / kTileK;
-    const double plane_us = (double)M * n_rows_total * 8.0 / 6.5e6;               // write + read of one plane of partial sums
+    const double plane_us = (double)M * n_rows_total * 8.0 / 6.5e6;   // write + read of one plane of partial sums
     auto cost = [&](int nc, int ks, double t_tile) {
         const int rounds = (tiles * ((M + nc - 1) / nc) * ks + sm_count - 1) / sm_count;
         return (double)rounds * ((double)((tpr + ks - 1) / ks) * t_tile + 0.33 * t_tile) + (ks - 1) * plane_us;
     };
-    int least = 1;
-    for (int ks = 2; ks <= kMaxKsplit && ks <= tpr; ks++) {
-        auto first = [&](int k) {
-            const int rounds = (tiles * ((M + kGmMaxChunk - 1) / kGmMaxChunk) * k + sm_count - 1) / sm_count;
-            return (double)rounds * ((double)tpr / k + 0.33) * 14.4 + (k - 1) * plane_us;
-        };
-        if (first(ks) < first(least) * 0.97) least = ks;                          // a larger split has to pay for itself
-    }
     GemmShape best{kGmMaxChunk, least};
     auto tile = [](int nc) { return 2.9 + 5.85 * nc / kGmMaxChunk; };
     double best_t = cost(kGmMaxChunk, least, tile(kGmMaxChunk));
@@ -849,9 +857,10 @@ static GemmShape gemm_shape_wide(int n_rows_total, int M, int K, int sm_count) {
     return best;
 }
 GemmShape gemm_shape(int n_rows_total, int M, int K, int sm_count) {
-    if (M > 64) return gemm_shape_wide(n_rows_total, M, K, sm_count);
+    const int least = gemm_least_split(n_rows_total, M, K, sm_count);
+    if (M > 64) return gemm_shape_wide(n_rows_total, M, K, sm_count, least);
     const int nc = M <= 16 ? 16 : M <= 32 ? 32 : 64;
-    return {nc, gemm_plan(n_rows_total / kTileRows, nc, K, sm_count).ks};
+    return {nc, gemm_plan(n_rows_total / kTileRows, nc, K, sm_count, least).ks};
 }
 
 cudaError_t launch_rows_quantize(const RowsArgs& a_in, cudaStream_t st) {
@@ -927,7 +936,7 @@ cudaError_t launch_gemm(const GemmArgs& a_in, int sm_count, cudaStream_t st) {
         // the row groups of one K range over the SMs it has, in as many rounds as the plan takes (the split itself was the caller's choice)
         int groups = 0;
         for (int s = 0; s < a.nseg; s++) groups += a.seg[s].rows / kTileRows;
-        const SkinnyPlan p = gemm_plan(groups, a.nc, a.K, sm_count);
+        const SkinnyPlan p = gemm_plan(groups, a.nc, a.K, sm_count, gemm_least_split(groups * kTileRows, a.M, a.K, sm_count));
         const int most = a.nc == 64 ? kGsRG : 2 * kGsRG;
         a.row_chunks = p.ks == a.ksplit ? p.chunks : (groups + most - 1) / most;
         items = (long long)a.row_chunks * a.ksplit;

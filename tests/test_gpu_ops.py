@@ -333,6 +333,32 @@ def test_gemm_q8_known_answers(torch_cuda, lib, n, k, m, mode):
     assert np.max(np.abs(ref1 - got[m - 1])) <= 16 * EPS * max(1.0, float(np.max(np.abs(ref1)))) * np.sqrt(k / 32)
 
 
+@pytest.mark.parametrize("n,k", [(28672, 4096), (19456, 2560), (28672, 14336), (16384, 16384)])
+@pytest.mark.parametrize("m", [2, 16, 33])
+def test_gemm_q8_sums_of_one_sign(torch_cuda, lib, n, k, m):
+    """Weights and activations of one sign: what the tensor core cuts off its sums (towards zero, up to 2^-23 of them at each of the additions, one per 16
+    columns, half as much while the sum grows evenly, and as much again inside an instruction) adds up, so a range must not be longer
+    than the coarse split allows."""
+    torch = torch_cuda
+    from test_product_shapes import coarse_split
+    g = torch.Generator(device="cuda").manual_seed(n + k + m)
+    q = torch.randint(1, 128, (n, k), dtype=torch.int8, device="cuda", generator=g)
+    s = (torch.rand((n, k // 32), device="cuda", generator=g) * 0.01 + 0.001).half()
+    x = torch.randn((m, k), device="cuda", generator=g).abs_()
+    torch.cuda.synchronize()
+    packed = torch.empty(lib.lum_q8_0_packed_bytes(n, k), dtype=torch.uint8, device="cuda")
+    ck(lib, lib.lum_op_q8_0_pack(q.data_ptr(), s.data_ptr(), n, k, packed.data_ptr(), None))
+    ws = torch.empty(lib.lum_op_gemm_q8_0_workspace(n, k, m), dtype=torch.uint8, device="cuda")
+    y = torch.empty((m, n), dtype=torch.float32, device="cuda")
+    ck(lib, lib.lum_op_gemm_q8_0_packed(packed.data_ptr(), n, k, x.data_ptr(), m, y.data_ptr(), ws.data_ptr(), ws.numel(), None))
+    torch.cuda.synchronize()
+    some = slice(0, n, 64)
+    want = x.double() @ (q[some].view(-1, k // 32, 32).double() * s[some].double()[..., None]).view(-1, k).T
+    err = float((y[:, some].double() - want).norm() / want.norm())
+    longest = -(-(k // 512) // coarse_split(n, m, k)) * 512
+    assert err <= longest / 16 * 2.0 ** -23, f"{err:.2e}"
+
+
 def test_gemm_q8_refuses_bad_arguments(torch_cuda, lib):
     assert lib.lum_op_gemm_q8_0_workspace(100, 512, 4) == 0 and lib.lum_op_gemm_q8_0_workspace(128, 500, 4) == 0
     assert lib.lum_op_gemm_q8_0_packed(None, 128, 512, None, 2, None, None, 0, None) != 0
