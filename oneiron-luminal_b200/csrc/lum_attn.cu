@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(kAttnTcThreads, 2) attn_decode_tc(const AttnAr
     const int p = a.state->pos;                 // settled several kernels back, like every cached row: see attn_decode
     const bool ok = p >= 0 && p < a.max_seq;
     AttnTile<HD> f;
-    AttnPre<HD> pre;
+    AttnPre<HD, kAttnTcThreads> pre;
     if (ok) {
         const int lane = threadIdx.x & 31, kvh = blockIdx.x;
         int r0, r1;
@@ -76,17 +76,8 @@ __global__ void __launch_bounds__(kAttnTcThreads, 2) attn_decode_tc(const AttnAr
         const int j0 = r0 + (threadIdx.x >> 5) * kAttnTcTile;
         attn_tc_load_k<HD>(a, f, kvh, j0, r1, lane);
         attn_tc_load_v<HD>(a, f, kvh, j0, r1, lane);
-        attn_tc_pre<HD>(a, pre, kvh, (int)blockIdx.y, (int)threadIdx.x >> 5, lane);
-        if (a.kv_prefetch) {
-            // one request per 128-byte line of the rows behind the first tiles
-            constexpr int kLines = HD * 2 / 128;
-            const int nc = r1 - r0 - kAttnTcWarps * kAttnTcTile;
-            for (int i = threadIdx.x; i < nc * 2 * kLines; i += kAttnTcThreads) {
-                const int r = r1 - nc + i / (2 * kLines), w = i % (2 * kLines);
-                const char* base = (const char*)(w < kLines ? a.k_cache : a.v_cache) + (kv_phys_row(a.pg, 0, 0, r) * a.n_kv + kvh) * (HD * 2) + (w % kLines) * 128;
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(base));
-            }
-        }
+        attn_tc_pre<HD, kAttnTcThreads>(a, pre, kvh, (int)blockIdx.y, (int)threadIdx.x >> 5, lane);
+        if (a.kv_prefetch) attn_tc_prefetch<HD>(a, kvh, r0 + kAttnTcWarps * kAttnTcTile, r1, (int)threadIdx.x, kAttnTcThreads);      // what the first tiles do not hold
         attn_fill_rope<HD, RS>(a, attn_rope_table(attn_smem, HD, kAttnTcWarps + 1), p, (int)threadIdx.x);
     }
     if (a.use_pdl) pdl_grid_wait();
@@ -94,7 +85,7 @@ __global__ void __launch_bounds__(kAttnTcThreads, 2) attn_decode_tc(const AttnAr
         if (threadIdx.x == 0) atomicOr(a.status, LUM_ST_BAD_POS);
         return;
     }
-    attn_tc_body<HD, MT, CL>(a, attn_smem, f, pre, (int)blockIdx.x, (int)blockIdx.y, p, (int)threadIdx.x, 2, true);
+    attn_tc_body<HD, MT, CL, kAttnTcThreads, true>(a, attn_smem, f, pre, (int)blockIdx.x, (int)blockIdx.y, p, (int)threadIdx.x, 2, true);
 }
 
 template <int HD, int GM, int RS>

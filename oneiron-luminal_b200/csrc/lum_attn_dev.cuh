@@ -566,6 +566,16 @@ __device__ __forceinline__ void attn_tc_range(const AttnArgs& a, int split, int 
     *r0 = min(p, lo + split * per);
     *r1 = min(p, *r0 + per);
 }
+// asks for rows [r0, r1) of a KV head to be brought into L2, one request per 128-byte line
+template <int HD>
+__device__ __forceinline__ void attn_tc_prefetch(const AttnArgs& a, int kvh, int r0, int r1, int tid, int threads) {
+    constexpr int kLines = HD * 2 / 128;
+    for (int i = tid; i < (r1 - r0) * 2 * kLines; i += threads) {
+        const int r = r0 + i / (2 * kLines), w = i % (2 * kLines);
+        const char* base = (const char*)(w < kLines ? a.k_cache : a.v_cache) + (kv_phys_row(a.pg, 0, 0, r) * a.n_kv + kvh) * (HD * 2) + (w % kLines) * 128;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(base));
+    }
+}
 template <int HD> struct AttnTile { uint4 k[2][HD / 32], v[4][HD / 64]; };
 template <int HD>
 __device__ __forceinline__ void attn_tc_load_k(const AttnArgs& a, AttnTile<HD>& f, int kvh, int j0, int r1, int lane) {
@@ -589,16 +599,16 @@ __device__ __forceinline__ void attn_tc_load_v(const AttnArgs& a, AttnTile<HD>& 
         for (int j = 0; j < HD / 64; j++) f.v[x][j] = in ? __ldcg(p + 8 * j) : make_uint4(0u, 0u, 0u, 0u);
     }
 }
-// Gains and biases of the heads this warp prepares (warp, warp + 4, ..: the group's queries, then the step's own key and value): they do not depend
+// Gains and biases of the heads this warp prepares (every T / 32nd: the group's queries, then the step's own key and value): they do not depend
 // on the previous kernel either.
-constexpr int kAttnTcHeads = 3;                          // up to 8 queries + key + value over 4 warps
-template <int HD> struct AttnPre { float gain[kAttnTcHeads][HD / 32], bias[kAttnTcHeads][HD / 32]; };
-template <int HD>
-__device__ __forceinline__ void attn_tc_pre(const AttnArgs& a, AttnPre<HD>& pre, int kvh, int split, int warp, int lane) {
+__host__ __device__ constexpr int attn_tc_heads(int T) { return (10 + T / 32 - 1) / (T / 32); }                  // up to 8 queries + key + value
+template <int HD, int T> struct AttnPre { float gain[attn_tc_heads(T)][HD / 32], bias[attn_tc_heads(T)][HD / 32]; };
+template <int HD, int T>
+__device__ __forceinline__ void attn_tc_pre(const AttnArgs& a, AttnPre<HD, T>& pre, int kvh, int split, int warp, int lane) {
     const int G = a.n_q / a.n_kv;
 #pragma unroll
-    for (int k = 0; k < kAttnTcHeads; k++) {
-        const int h = warp + kAttnTcWarps * k;
+    for (int k = 0; k < attn_tc_heads(T); k++) {
+        const int h = warp + T / 32 * k;
         const bool in = h < G || (h < G + 2 && split == a.n_splits - 1);
         const void* gain = h < G ? a.q_gain : h == G ? a.k_gain : nullptr;
         const void* bias = h < G ? a.q_bias : h == G ? a.k_bias : a.v_bias;
@@ -612,12 +622,12 @@ __device__ __forceinline__ void attn_tc_pre(const AttnArgs& a, AttnPre<HD>& pre,
 }
 __device__ __forceinline__ uint32_t attn_word(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 
-// Runs on exactly kAttnTcThreads threads (tid 0 ..) that synchronise on named barrier `bar_id`; `f` holds this warp's first tile (attn_tc_load_*),
-// `pre` its heads' gains and biases
-template <int HD, int MT, bool CL>
-__device__ __forceinline__ void attn_tc_body(const AttnArgs& a, unsigned char* smem, AttnTile<HD>& f, const AttnPre<HD>& pre, int kvh, int split, int p, int tid, int bar_id,
+// Runs on exactly T threads (tid 0 ..) that synchronise on named barrier `bar_id`; `pre` holds this warp's heads' gains and biases.  AHEAD: `f` holds
+// its first tile (attn_tc_load_*); otherwise it is loaded when the heads are ready.  Keys are taken by the first kAttnTcWarps warps.
+template <int HD, int MT, bool CL, int T, bool AHEAD>
+__device__ __forceinline__ void attn_tc_body(const AttnArgs& a, unsigned char* smem, AttnTile<HD>& f, const AttnPre<HD, T>& pre, int kvh, int split, int p, int tid, int bar_id,
                                              bool rope_ready) {
-    constexpr int NW = kAttnTcWarps, NP = NW + 1, T = kAttnTcThreads, KS = HD / 16, NT = HD / 8, N = HD / 32;
+    constexpr int NW = kAttnTcWarps, NP = NW + 1, TW = T / 32, NH = attn_tc_heads(T), KS = HD / 16, NT = HD / 8, N = HD / 32;
     const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const bool second = g >= 4;
     const int G = a.n_q / a.n_kv;
@@ -642,10 +652,10 @@ __device__ __forceinline__ void attn_tc_body(const AttnArgs& a, unsigned char* s
     // elements l, l + 32, ..: the rotation's partner is in the next lane or in the same one)
     const int nheads = G + (owns_new ? 2 : 0);
     if (!rope_ready) attn_fill_rope<HD>(a, s_rope, p, tid);
-    float x[kAttnTcHeads][N];
+    float x[NH][N];
 #pragma unroll
-    for (int k = 0; k < kAttnTcHeads; k++) {
-        const int h = warp + NW * k;
+    for (int k = 0; k < NH; k++) {
+        const int h = warp + TW * k;
         if (h < nheads) {
             const float* src = h < G ? a.q + ((size_t)kvh * G + h) * HD : h == G ? a.k_new + (size_t)kvh * HD : a.v_new + (size_t)kvh * HD;
 #pragma unroll
@@ -654,8 +664,8 @@ __device__ __forceinline__ void attn_tc_body(const AttnArgs& a, unsigned char* s
     }
     sync();                                                  // (the rotation table is there)
 #pragma unroll
-    for (int k = 0; k < kAttnTcHeads; k++) {
-        const int h = warp + NW * k;
+    for (int k = 0; k < NH; k++) {
+        const int h = warp + TW * k;
         if (h < nheads) {
             if (h < G ? a.q_bias != nullptr : h == G ? a.k_bias != nullptr : a.v_bias != nullptr) {
 #pragma unroll
@@ -708,7 +718,7 @@ __device__ __forceinline__ void attn_tc_body(const AttnArgs& a, unsigned char* s
         attn_terms(q.z, q.w, ln >= 16, &w.z, &w.w);
         s_a[idx] = w;
     }
-    if (owns_new && warp == NW - 1) {
+    if (owns_new && warp == TW - 1) {
         // append this step's row to the cache; the rounded values are one more state: score, weight 1, value
         const size_t off = kv_phys_row(a.pg, 0, 0, p) * row_elems + (size_t)kvh * HD;
         float k[N], v[N];
@@ -733,6 +743,11 @@ __device__ __forceinline__ void attn_tc_body(const AttnArgs& a, unsigned char* s
     sync();
 
     // ---- the cached rows
+    if (T == kAttnTcThreads || warp < NW) {
+    if (!AHEAD) {
+        attn_tc_load_k<HD>(a, f, kvh, r0 + warp * kAttnTcTile, r1, lane);
+        attn_tc_load_v<HD>(a, f, kvh, r0 + warp * kAttnTcTile, r1, lane);
+    }
     float o[MT][NT][2], mx[MT], l[MT];
 #pragma unroll
     for (int mt = 0; mt < MT; mt++) {
@@ -816,6 +831,7 @@ __device__ __forceinline__ void attn_tc_body(const AttnArgs& a, unsigned char* s
     if (j_first < r1 && __any_sync(0xffffffffu, odd[0] + odd[1] != 0.0f))
         attn_plain_keys<HD>((const __nv_bfloat16*)a.k_cache + (size_t)kvh * HD, (const __nv_bfloat16*)a.v_cache + (size_t)kvh * HD, a.pg, 0, 0, row_elems, j_first, r1,
                             &s_q[0][0], G, lane, s_m[warp], s_l[warp], s_o + (size_t)warp * G * HD);
+    }
     sync();
     const int parts = owns_new ? NP : NW;
     const int S = a.n_splits, total = G * HD, chunk = (total + S - 1) / S;      // outputs CTA r of the cluster finishes: [r * chunk, (r + 1) * chunk)
