@@ -787,6 +787,11 @@ static int gemm_padded_rows(int M) { return M <= 64 ? 64 : M + kGmMaxChunk - 1; 
 size_t gemm_xq_bytes(int M, int K) { return (size_t)gemm_padded_rows(M) * K * 2 * kGmXTerms; }
 size_t gemm_sx_bytes(int M, int K) { (void)K; return (size_t)gemm_padded_rows(M) * 4; }
 
+// Shapes hold for whole blocks of 16 rows: whoever sizes a buffer for every row count asks once per block (gemm_parts_rows).
+constexpr int kGmBlock = 16;
+static int block_first(int M) { return (M - 1) / kGmBlock * kGmBlock + 1; }
+static int block_last(int M) { return (M + kGmBlock - 1) / kGmBlock * kGmBlock; }
+
 // The fewest K ranges a product may be cut into.  An accumulator's additions are cut to 24 bits, always towards zero: longer ranges cost accuracy,
 // and with operands of one sign the loss grows with the length.  So the split that a first, coarse estimate of the time gives (chunks of 32, 64
 // or 128 rows, items of 128 or 256 weight rows) is never undercut, whatever the finer estimates below would gain.
@@ -795,7 +800,7 @@ size_t gemm_sx_bytes(int M, int K) { (void)K; return (size_t)gemm_padded_rows(M)
 static int gemm_least_split(int n_rows_total, int M, int K, int sm_count) {
     const int nc = M <= 32 ? 32 : M <= 64 ? 64 : 128, tile_rows = M > 64 ? kGmRows : 128;
     const int items = (n_rows_total + tile_rows - 1) / tile_rows * ((M + nc - 1) / nc), tpr = K / kTileK;
-    const double tile_us = M > 64 ? 14.4 : 16.0 * (0.16 + 0.43 * nc / 128.0), plane_us = (double)M * n_rows_total * 8.0 / 6.5e6;
+    const double tile_us = M > 64 ? 14.4 : 16.0 * (0.16 + 0.43 * nc / 128.0), plane_us = (double)block_first(M) * n_rows_total * 8.0 / 6.5e6;
     auto cost = [&](int k) { return (double)(((long long)items * k + sm_count - 1) / sm_count) * ((double)tpr / k + 0.33) * tile_us + (k - 1) * plane_us; };
     int best = 1;
     for (int ks = 2; ks <= kMaxKsplit && ks <= tpr; ks++)
@@ -841,7 +846,7 @@ static SkinnyPlan gemm_plan(int groups, int nc, int K, int sms, int least) {
 // 308, 19456 x 2560 82 / 235 / 347 -> 51 / 171 / 242, 2560 x 9728 63 / 124 / 234 -> 41 / 93 / 182.
 static GemmShape gemm_shape_wide(int n_rows_total, int M, int K, int sm_count, int least) {
     const int tiles = (n_rows_total + kGmRows - 1) / kGmRows, tpr = K / kTileK;
-    const double plane_us = (double)M * n_rows_total * 8.0 / 6.5e6;   // write + read of one plane of partial sums
+    const double plane_us = (double)block_last(M) * n_rows_total * 8.0 / 6.5e6;   // write + read of one plane of partial sums
     auto cost = [&](int nc, int ks, double t_tile) {
         const int rounds = (tiles * ((M + nc - 1) / nc) * ks + sm_count - 1) / sm_count;
         return (double)rounds * ((double)((tpr + ks - 1) / ks) * t_tile + 0.33 * t_tile) + (ks - 1) * plane_us;
@@ -861,6 +866,17 @@ GemmShape gemm_shape(int n_rows_total, int M, int K, int sm_count) {
     if (M > 64) return gemm_shape_wide(n_rows_total, M, K, sm_count, least);
     const int nc = M <= 16 ? 16 : M <= 32 ? 32 : 64;
     return {nc, gemm_plan(n_rows_total / kTileRows, nc, K, sm_count, least).ks};
+}
+// The most rows of partial sums (K ranges times rows) a product of up to `cap` rows needs.  Larger row counts come first, and those that even the
+// largest split could not bring above what was found are not looked at: a model's four products of up to 4096 rows take 0.25 ms (3.4 ms row by
+// row), once, when its buffers are made.
+size_t gemm_parts_rows(int n_rows_total, int K, int cap, int sm_count) {
+    size_t worst = 0;
+    for (int m = cap; m >= 1 && (size_t)kMaxKsplit * m > worst; m = block_first(m) - 1) {
+        const size_t need = (size_t)gemm_shape(n_rows_total, m, K, sm_count).ks * m;
+        if (need > worst) worst = need;
+    }
+    return worst;
 }
 
 cudaError_t launch_rows_quantize(const RowsArgs& a_in, cudaStream_t st) {

@@ -78,6 +78,7 @@ size_t gemm_sx_bytes(int M, int K);
 struct GemmShape { int nc, ks; };                // activation rows per chunk, K ranges (at most kMaxKsplit)
 constexpr int kMaxKsplit = 8;
 GemmShape gemm_shape(int n_rows_total, int M, int K, int sm_count);
+size_t gemm_parts_rows(int n_rows_total, int K, int cap, int sm_count);
 bool gemm_supported(const GemmArgs& a);
 cudaError_t launch_rows_quantize(const RowsArgs& a, cudaStream_t st);
 cudaError_t launch_gemm(const GemmArgs& a, int sm_count, cudaStream_t st);

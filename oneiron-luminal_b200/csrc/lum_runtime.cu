@@ -1120,14 +1120,7 @@ bool rows_supported(const lum_rt* rt) {
 }
 
 // floats the K-split partial planes of a product with n_out outputs per row can need, over every row count up to cap
-size_t rows_parts_floats(const lum_rt* rt, int n_out, int K, int cap) {
-    size_t worst = 0;
-    for (int m = cap; m >= 1 && (size_t)kMaxKsplit * m * n_out > worst; m--) {      // (fewer rows than that cannot need more)
-        const size_t need = (size_t)gemm_shape(n_out, m, K, rt->sm_count).ks * m * n_out;
-        if (need > worst) worst = need;
-    }
-    return worst;
-}
+size_t rows_parts_floats(const lum_rt* rt, int n_out, int K, int cap) { return gemm_parts_rows(n_out, K, cap, rt->sm_count) * n_out; }
 
 int ensure_rows(lum_rt* rt, int want_rows) {
     lum_rt::Rows& b = rt->rows;

@@ -44,3 +44,18 @@ def test_ranges_are_never_longer_than_the_coarse_split(shape, n, k):
         s = shape(n, m, k)
         assert s.nc % 16 == 0 and (s.nc in (16, 32, 64) and s.nc >= m if m <= 64 else 80 <= s.nc <= 128)
         assert coarse_split(n, m, k) <= s.ks <= min(8, k // 512), f"{m} rows"
+
+
+@pytest.mark.parametrize("n,k", PRODUCTS)
+def test_shapes_hold_for_blocks_of_sixteen_rows(shape, n, k):
+    for block in [0, 1, 2, 3, 4, 5, 7, 8, 15, 24, 31, 63, 127, 128, 200, 255]:
+        first = shape(n, 16 * block + 1, k)
+        assert all((s.nc, s.ks) == (first.nc, first.ks) for s in (shape(n, 16 * block + i, k) for i in range(2, 17))), f"rows from {16 * block + 1} on"
+
+
+@pytest.mark.parametrize("n,k", PRODUCTS)
+@pytest.mark.parametrize("cap", [1, 32, 33, 387, 1024, 4096])
+def test_room_for_partial_sums_covers_every_row_count(pkg, shape, n, k, cap):
+    f = pkg.load_library()["_ZN3lum15gemm_parts_rowsEiiii"]          # lum::gemm_parts_rows(outputs, inner, most rows, SMs)
+    f.restype, f.argtypes = C.c_size_t, [C.c_int] * 4
+    assert f(n, k, cap, SMS) == max(m * shape(n, m, k).ks for m in range(1, cap + 1))
