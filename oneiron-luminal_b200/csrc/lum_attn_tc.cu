@@ -272,12 +272,8 @@ bool attn_prompt_tc_supported(const AttnRowsArgs& a) {
 
 cudaError_t launch_attn_prompt_tc(const AttnRowsArgs& a, cudaStream_t st) {
     if (!attn_prompt_tc_supported(a)) return cudaErrorInvalidValue;
-    static bool attr_set = false;
-    if (!attr_set) {
-        const cudaError_t e = cudaFuncSetAttribute((const void*)attn_prompt_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kAtSmem);
-        if (e != cudaSuccess) return e;
-        attr_set = true;
-    }
+    static std::atomic<uint64_t> raised{0};
+    if (const cudaError_t e = allow_smem(raised, (const void*)attn_prompt_tc, kAtSmem)) return e;
     static const int swap = [] { const char* e = getenv("LUM_ATTN_TC_SWAP"); return e ? atoi(e) : 0; }();
     const int G = a.n_q / a.n_kv, QT = 128 / G;
     attn_prompt_tc<<<dim3(a.n_kv, (a.M + QT - 1) / QT), kAtThreads, kAtSmem, st>>>(a, G, swap);

@@ -7,7 +7,15 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "lum_device.hpp"
+
 namespace lum {
+
+// the dynamic shared memory that `fn` may be launched with, raised once per device
+inline cudaError_t allow_smem(std::atomic<uint64_t>& done, const void* fn, int bytes) {
+    return (cudaError_t)once_per_device(done, [](int* dev) { return (int)cudaGetDevice(dev); },
+                                        [&] { return (int)cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
+}
 
 // ---- status word -------------------------------------------------------------------------------
 // Kernels never trap.  A kernel that gives up (a wait that ran out of budget) ORs a code into a

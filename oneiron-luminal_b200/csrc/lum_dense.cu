@@ -621,12 +621,8 @@ cudaError_t launch_dense_gemm(const DenseArgs& a_in, int sm_count, cudaStream_t 
     int stages = (220 * 1024) / stage_bytes;
     if (stages > kDmMaxStages) stages = kDmMaxStages;
     const size_t smem = (size_t)stages * stage_bytes + 512;
-    static bool attr_set = false;
-    if (!attr_set) {
-        const cudaError_t e = cudaFuncSetAttribute((const void*)dense_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
-        if (e != cudaSuccess) return e;
-        attr_set = true;
-    }
+    static std::atomic<uint64_t> raised{0};
+    if (const cudaError_t e = allow_smem(raised, (const void*)dense_gemm_tc, 226 * 1024)) return e;
     const int n_tiles = mt * ((grp + TN - 1) / TN) * groups;
     dense_gemm_tc<<<n_tiles < sm_count ? n_tiles : sm_count, kDmThreads, smem, st>>>(a, TN, stages);
     return cudaGetLastError();

@@ -890,12 +890,8 @@ cudaError_t launch_rows_quantize(const RowsArgs& a_in, cudaStream_t st) {
     const size_t smem = (size_t)(((a.K >> 5) + C - 1) / C) * 128;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
     if (smem > 48 * 1024) {
-        static bool set = false;
-        if (!set) {
-            cudaError_t e = cudaFuncSetAttribute((const void*)rows_quantize, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            if (e != cudaSuccess) return e;
-            set = true;
-        }
+        static std::atomic<uint64_t> raised{0};
+        if (const cudaError_t e = allow_smem(raised, (const void*)rows_quantize, 200 * 1024)) return e;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows * C);
@@ -937,13 +933,8 @@ cudaError_t launch_gemm(const GemmArgs& a_in, int sm_count, cudaStream_t st) {
     const void* fn = wide ? (const void*)q8_gemm_tc : a.nc == 16 ? (const void*)q8_gemm_tc_skinny<16> : a.nc == 32 ? (const void*)q8_gemm_tc_skinny<32> : (const void*)q8_gemm_tc_skinny<64>;
     const size_t smem = wide ? kGmSmem : kGsSmem;
     const int threads = wide ? kGmThreads : kGsThreads;
-    static bool set[4] = {false, false, false, false};
-    const int which = wide ? 3 : a.nc / 32;
-    if (!set[which]) {
-        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        set[which] = true;
-    }
+    static std::atomic<uint64_t> raised[4] = {};
+    if (const cudaError_t e = allow_smem(raised[wide ? 3 : a.nc / 32], fn, (int)smem)) return e;
     long long items = 0;
     if (wide) {
         for (int s = 0; s < a.nseg; s++) items += (a.seg[s].rows + kGmRows - 1) / kGmRows;

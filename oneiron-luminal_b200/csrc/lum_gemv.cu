@@ -362,13 +362,8 @@ cudaError_t launch_gemv(const GemvArgs& a_in, int sm_count, cudaStream_t st) {
         const bool wide = env_narrow == 0 || a.K > 2 * kWorkers * 4;      // more than two float4 per worker thread
         const void* fn = peer ? (wide ? (const void*)q8_gemv_stream<true, true> : (const void*)q8_gemv_stream<true, false>)
                               : (wide ? (const void*)q8_gemv_stream<false, true> : (const void*)q8_gemv_stream<false, false>);
-        static bool attr_set[4] = {false, false, false, false};
-        const int which = (peer ? 2 : 0) + (wide ? 1 : 0);
-        if (!attr_set[which]) {
-            cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(226 * 1024));
-            if (e != cudaSuccess) return e;
-            attr_set[which] = true;
-        }
+        static std::atomic<uint64_t> raised[4] = {};
+        if (const cudaError_t e = allow_smem(raised[(peer ? 2 : 0) + (wide ? 1 : 0)], fn, 226 * 1024)) return e;
         if (smem > 226 * 1024) return cudaErrorInvalidValue;
         return launch_with_attrs(fn, dim3(grid), dim3(kGemvThreads), smem, st, a.use_pdl != 0, a);
     }

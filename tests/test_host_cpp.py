@@ -83,6 +83,23 @@ def test_cpp_serving_loop_on_a_stand_in_runtime(tmp_path):
     assert r.returncode == 0 and r.stdout.strip() == "ok 5", r.stdout + r.stderr
 
 
+def test_kernel_attributes_are_raised_per_device(tmp_path):
+    """Raising a kernel's shared memory counts for one device: what is kept in mind about it is kept per device (lum_device.hpp), by every launcher."""
+    csrc = os.path.join(ROOT, "oneiron-luminal_b200", "csrc")
+    out = str(tmp_path / "device_test")
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Wextra", "-Werror", "-pthread", "-I", csrc, os.path.join(ROOT, "tests", "host_cpp", "device_test.cpp"), "-o", out],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([out], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
+    for name in sorted(os.listdir(csrc)):
+        if name.endswith(".cu"):
+            text = open(os.path.join(csrc, name)).read()
+            if "cudaFuncSetAttribute" in text or "allow_smem" in text:
+                flags = [line.strip() for line in text.splitlines() if line.strip().startswith("static bool") and "(" not in line]
+                assert not flags, f"{name}: {flags}"
+
+
 @pytest.mark.gpu
 def test_cpp_serving_loop_equals_requests_alone(pkg, drive, tmp_path):
     """The C++ loop over the real runtime with a paged cache: five requests through three slots get the tokens they get alone."""
