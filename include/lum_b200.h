@@ -398,6 +398,9 @@ int32_t lum_get_stats(const lum_rt* rt, lum_stats* out);
  * for completion words that never come, gives up and returns.  Expected result: LUM_E_DEVICE (status 0x80), with the runtime
  * fully usable afterwards.  Nothing faults, traps or hangs; set wait_budget_ms to a few milliseconds first. */
 int32_t lum_debug_wait_timeout(lum_rt* rt);
+/* Test hook: the next n graph captures that ask for programmatic dependent launch fail, as on a driver that cannot capture its edges; the
+ * runtime then captures ordinary dependencies. */
+int32_t lum_debug_fail_pdl_captures(lum_rt* rt, int32_t n);
 
 /* ---------------------------------------------------------------------------------------------
  * Tensor parallelism over the GPUs of one node: one process and one runtime per GPU (the reference is single-GPU:

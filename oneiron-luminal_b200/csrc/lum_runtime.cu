@@ -205,6 +205,8 @@ struct lum_rt {
     cudaGraphExec_t g_full = nullptr, g_body = nullptr;   // whole step / step without the head
     int launches_full = 0;
     bool graph_pdl = false;
+    bool rows_pdl = false;                // steps of several rows: programmatic dependent launch (lum_batch_decode's capture may turn it off)
+    int fail_pdl_captures = 0;            // lum_debug_fail_pdl_captures
 
     uint64_t dim_s = 1, dim_p = 0;
     std::vector<int32_t> tokens_in;
@@ -996,13 +998,14 @@ int issue_step_sequential(lum_rt* rt, bool with_head, bool pdl, int* n_launch) {
     return 0;
 }
 
-int capture_graph(lum_rt* rt, bool with_head, bool pdl, cudaGraphExec_t* out, int* n_launch) {
+// What issue() launches on the runtime's stream, as a graph.  pdl: whether it asks for programmatic dependent launch.
+template <typename F>
+int capture_graph(lum_rt* rt, bool pdl, cudaGraphExec_t* out, F issue) {
     cudaGraph_t g = nullptr;
     CU(rt, cudaStreamBeginCapture(rt->stream, cudaStreamCaptureModeThreadLocal));
-    int r = rt->d.block_kind == 1   ? issue_step_blocks(rt, with_head, pdl, n_launch)
-            : rt->d.block_kind == 2 ? issue_step_sequential(rt, with_head, pdl, n_launch)
-                                    : issue_step(rt, with_head, pdl, n_launch);
+    int r = issue();
     cudaError_t e = cudaStreamEndCapture(rt->stream, &g);
+    if (!r && pdl && rt->fail_pdl_captures > 0) { rt->fail_pdl_captures--; r = fail(rt, LUM_E_CUDA, "capture: refused by lum_debug_fail_pdl_captures"); }
     if (r) { if (g) cudaGraphDestroy(g); return r; }
     if (e != cudaSuccess) return fail(rt, LUM_E_CUDA, "cudaStreamEndCapture: %s", cudaGetErrorString(e));
     e = cudaGraphInstantiate(out, g, 0);
@@ -1010,20 +1013,30 @@ int capture_graph(lum_rt* rt, bool with_head, bool pdl, cudaGraphExec_t* out, in
     if (e != cudaSuccess) { *out = nullptr; return fail(rt, LUM_E_CUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(e)); }
     return 0;
 }
+// issue(pdl) as a graph, with programmatic dependent launch if *pdl asks for it; where its edges cannot be captured, with ordinary dependencies
+// (*pdl then says so).
+template <typename F>
+int capture_graph_or_plain(lum_rt* rt, bool* pdl, cudaGraphExec_t* out, F issue) {
+    int r = capture_graph(rt, *pdl, out, [&] { return issue(*pdl); });
+    if (r && *pdl) {
+        cudaGetLastError();
+        *pdl = false;
+        r = capture_graph(rt, false, out, [&] { return issue(false); });
+    }
+    return r;
+}
 
 int ensure_graphs(lum_rt* rt) {
     if (!rt->cfg.use_graph || rt->g_full) return 0;
     bool pdl = rt->cfg.use_pdl != 0;
-    int r = capture_graph(rt, true, pdl, &rt->g_full, &rt->launches_full);
-    if (r && pdl) {
-        // Programmatic edges could not be captured: fall back to ordinary dependencies.
-        cudaGetLastError();
-        pdl = false;
-        r = capture_graph(rt, true, pdl, &rt->g_full, &rt->launches_full);
-    }
-    if (r) return r;
+    auto step = [&](bool with_head, bool p, int* n_launch) {
+        return rt->d.block_kind == 1   ? issue_step_blocks(rt, with_head, p, n_launch)
+               : rt->d.block_kind == 2 ? issue_step_sequential(rt, with_head, p, n_launch)
+                                       : issue_step(rt, with_head, p, n_launch);
+    };
+    if (int r = capture_graph_or_plain(rt, &pdl, &rt->g_full, [&](bool p) { return step(true, p, &rt->launches_full); })) return r;
     rt->graph_pdl = pdl;
-    return capture_graph(rt, false, pdl, &rt->g_body, nullptr);
+    return capture_graph(rt, pdl, &rt->g_body, [&] { return step(false, pdl, nullptr); });
 }
 
 int run_step(lum_rt* rt, bool with_head) {
@@ -1195,7 +1208,7 @@ int batch_sample(lum_rt* rt, int M, int* d_tok, int* d_pos, const int* d_seq, in
     lum_rt::Rows& b = rt->rows;
     const int V = rt->vocab_l;
     ArgmaxRowsArgs x{};
-    x.logits = b.logits; x.n_parts = n_parts; x.part_stride = (size_t)M * V; x.M = M; x.vocab = V; x.use_pdl = rt->cfg.use_pdl != 0;
+    x.logits = b.logits; x.n_parts = n_parts; x.part_stride = (size_t)M * V; x.M = M; x.vocab = V; x.use_pdl = rt->rows_pdl;
     if (!rt->sampling) { x.row_tok = d_tok; x.row_pos = d_pos; x.log = rt->b_log; x.step = rt->b_step; x.max_steps = rt->d.max_new_tokens; }
     CU(rt, launch_argmax_rows(x, rt->stream));          // with a sampler set it only adds up the partial planes
     if (rt->sampling) {
@@ -1381,7 +1394,7 @@ int run_rows(lum_rt* rt, int M, int* d_tok, int* d_pos, const int* d_seq, int se
     const lum_model_desc& d = rt->d;
     lum_rt::Rows& b = rt->rows;
     const int H = d.hidden, hd = d.head_dim, qd = rt->nq_l * hd, kvd = rt->nkv_l * hd, W = qd + 2 * kvd, F = rt->ffn_l;
-    const int gk = kind_of(d.embed_dtype), sms = rt->sm_count, pdl = rt->cfg.use_pdl != 0;
+    const int gk = kind_of(d.embed_dtype), sms = rt->sm_count, pdl = rt->rows_pdl;
     cudaStream_t st = rt->stream;
     const GemmShape g_qkv = gemm_shape(W, M, H, sms), g_o = gemm_shape(H, M, qd, sms), g_gu = gemm_shape(2 * F, M, H, sms), g_dn = gemm_shape(H, M, F, sms);
     const int ks_qkv = g_qkv.ks, ks_o = g_o.ks, ks_gu = g_gu.ks, ks_dn = g_dn.ks;
@@ -2069,7 +2082,7 @@ int32_t lum_create(const lum_config* cfg, lum_rt** out) {
     CU(nullptr, cudaGetDeviceProperties(&p, c.device));
     if (p.major < 10) return fail(nullptr, LUM_E_UNSUPPORTED, "device is sm_%d%d; this library is built for sm_100a only", p.major, p.minor);
     lum_rt* rt = new lum_rt();
-    rt->cfg = c; rt->sm_count = p.multiProcessorCount; rt->cc = p.major * 10 + p.minor; rt->mem_bytes = p.totalGlobalMem;
+    rt->cfg = c; rt->rows_pdl = c.use_pdl != 0; rt->sm_count = p.multiProcessorCount; rt->cc = p.major * 10 + p.minor; rt->mem_bytes = p.totalGlobalMem;
     {
         int khz = 0;
         cudaDeviceGetAttribute(&khz, cudaDevAttrClockRate, c.device);
@@ -2630,17 +2643,14 @@ int32_t lum_batch_decode(lum_rt* rt, int32_t n_steps) {
     const int M = rt->batch_n;
     if (rt->cfg.use_graph && (!rt->g_batch || rt->g_batch_n != M)) {
         if (rt->g_batch) { cudaGraphExecDestroy(rt->g_batch); rt->g_batch = nullptr; }
-        cudaGraph_t g = nullptr;
-        CU(rt, cudaStreamBeginCapture(rt->stream, cudaStreamCaptureModeThreadLocal));
         const uint64_t keep = rt->n_launches;
-        const int r = run_rows(rt, M, rt->rows.tok, rt->rows.pos, rt->rows.seq, 0, 2);
+        bool pdl = rt->cfg.use_pdl != 0;
+        const int r = capture_graph_or_plain(rt, &pdl, &rt->g_batch, [&](bool p) {
+            rt->rows_pdl = p;
+            return run_rows(rt, M, rt->rows.tok, rt->rows.pos, rt->rows.seq, 0, 2);
+        });
         rt->n_launches = keep;
-        cudaError_t e = cudaStreamEndCapture(rt->stream, &g);
-        if (r) { if (g) cudaGraphDestroy(g); return r; }
-        if (e != cudaSuccess) return fail(rt, LUM_E_CUDA, "batch_decode: cudaStreamEndCapture: %s", cudaGetErrorString(e));
-        e = cudaGraphInstantiate(&rt->g_batch, g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) { rt->g_batch = nullptr; return fail(rt, LUM_E_CUDA, "batch_decode: cudaGraphInstantiate: %s", cudaGetErrorString(e)); }
+        if (r) return r;
         rt->g_batch_n = M;
     }
     for (int s = 0; s < n_steps; s++) {
@@ -2697,6 +2707,13 @@ int32_t lum_debug_wait_timeout(lum_rt* rt) {
     cudaFree(seq);
     if (e != cudaSuccess) return fail(rt, LUM_E_CUDA, "debug_wait_timeout: %s", cudaGetErrorString(e));
     return check_status(rt);
+}
+
+// Test hook: the next n captures that ask for programmatic dependent launch fail.
+int32_t lum_debug_fail_pdl_captures(lum_rt* rt, int32_t n) {
+    if (!rt || n < 0) return fail(rt, LUM_E_INVALID, "debug_fail_pdl_captures: no runtime or a negative count");
+    rt->fail_pdl_captures = n;
+    return 0;
 }
 
 int32_t lum_tp_unique_id(uint8_t* out128) {

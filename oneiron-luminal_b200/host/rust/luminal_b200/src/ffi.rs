@@ -239,6 +239,7 @@ unsafe extern "C" {
     pub fn lum_stream(rt: *mut lum_rt) -> *mut c_void;
     pub fn lum_get_stats(rt: *const lum_rt, out: *mut lum_stats) -> i32;
     pub fn lum_debug_wait_timeout(rt: *mut lum_rt) -> i32;
+    pub fn lum_debug_fail_pdl_captures(rt: *mut lum_rt, n: i32) -> i32;
 
     pub fn lum_tp_unique_id(out128: *mut u8) -> i32;
     pub fn lum_tp_init(rt: *mut lum_rt, id128: *const u8, tp_size: i32, tp_rank: i32) -> i32;

@@ -250,6 +250,7 @@ def load_library() -> C.CDLL:
         "lum_op_sample_topk": (i32, [vp, i32, i32, P(Sampling), i32, vp, vp, vp]),
         "lum_get_stats": (i32, [vp, P(Stats)]),
         "lum_debug_wait_timeout": (i32, [vp]),
+        "lum_debug_fail_pdl_captures": (i32, [vp, i32]),
         "lum_op_status": (i32, [vp]),
         "lum_get_output": (i32, [vp, C.c_int64, P(C.c_float), sz]),
         "lum_get_output_raw": (i32, [vp, C.c_int64, vp, sz, P(u32), P(sz)]),
@@ -588,6 +589,10 @@ class B200Runtime:
     def debug_wait_timeout(self) -> None:
         """Test hook: one bounded wait runs out (raises LumError with code LUM_E_DEVICE); the runtime stays usable."""
         self._ck(self._lib.lum_debug_wait_timeout(self._h))
+
+    def debug_fail_pdl_captures(self, n: int) -> None:
+        """Test hook: the next `n` graph captures with programmatic dependent launch fail; ordinary dependencies take their place."""
+        self._ck(self._lib.lum_debug_fail_pdl_captures(self._h, n))
 
     def stats(self) -> Stats:
         st = Stats()

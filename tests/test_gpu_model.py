@@ -225,6 +225,27 @@ def test_launch_modes_agree(pkg, rt, graph, pdl, mega):
         other.close()
 
 
+def test_steps_are_captured_without_programmatic_launch_where_it_fails(pkg):
+    """One sequence's graph and a batch's: where programmatic dependent launch cannot be captured, ordinary dependencies give the same tokens and logits."""
+    desc = pkg.CONFIGS["small_q8"].copy(max_batch=3)
+    got = []
+    for refused in (0, 1):
+        rt = pkg.B200Runtime.initialize(device=0)
+        try:
+            rt.load_model(desc)
+            rt.synth(3)
+            rt.debug_fail_pdl_captures(refused)
+            tokens = rt.generate([5, 17, 1000], 4)
+            rt.debug_fail_pdl_captures(refused)
+            rt.batch_begin([7, 8, 9], [3, 3, 3])
+            rt.batch_decode(4)
+            got.append((tokens, rt.batch_get_decoded(4), [rt.batch_get_logits(b) for b in range(3)]))
+        finally:
+            rt.close()
+    assert got[0][0] == got[1][0] and (got[0][1] == got[1][1]).all()
+    assert all((a == b).all() for a, b in zip(got[0][2], got[1][2]))
+
+
 @pytest.mark.parametrize("splits", [2, 5, 8, 16])
 def test_attention_cluster_merge_equals_ticket_merge(pkg, rt, splits, monkeypatch):
     """The splits of a KV head merged through a thread-block cluster's shared memory (the default wherever a cluster of
