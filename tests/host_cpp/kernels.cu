@@ -8,6 +8,7 @@
 #include <string>
 #include <vector>
 
+#include "lum_moe.cuh"
 #include "lum_rows.cuh"
 
 using namespace lum;
@@ -162,10 +163,134 @@ static void attention_specials() {
             }
 }
 
+// Routed experts of several tokens, as an expert-parallel rank has them: some, all or none of a token's experts are this rank's.
+static void experts() {
+    struct Size { int hidden, ffn, n_experts, top_k; };
+    for (const Size z : {Size{256, 128, 8, 3}, Size{3200, 96, 6, 2}, Size{96, 3136, 5, 4}}) {
+        const int H = z.hidden, F = z.ffn, E = z.n_experts, K = z.top_k, T = 5, slot = (H + 2 * K + 3) / 4 * 4;
+        std::mt19937 rng(H + F);
+        auto ints = [&](size_t n, int lo, int hi) { std::vector<int> v(n); for (int& x : v) x = std::uniform_int_distribution<int>(lo, hi)(rng); return v; };
+        auto planes = [&](size_t rows, int k, std::vector<int8_t>& q, std::vector<__half>& d) {
+            q.resize(rows * k); d.resize(rows * k / 32);
+            const std::vector<int> i = ints(q.size(), -127, 127);
+            for (size_t j = 0; j < q.size(); j++) q[j] = (int8_t)i[j];
+            for (__half& x : d) x = __float2half(0.02f / std::sqrt((float)k) * (1 + std::uniform_real_distribution<float>(0, 1)(rng)));
+        };
+        std::vector<int8_t> gq, dq;
+        std::vector<__half> gs, ds;
+        planes((size_t)E * 2 * F, H, gq, gs);
+        planes((size_t)E * H, F, dq, ds);
+        const std::vector<float> gb = normal(rng, (size_t)E * 2 * F, 0.1f), db = normal(rng, (size_t)E * H, 0.1f);
+        std::vector<float> xf((size_t)T * slot);         // per token: activations, chosen experts, their weights
+        std::vector<int> chosen((size_t)T * K);
+        for (int t = 0; t < T; t++) {
+            const std::vector<float> x = normal(rng, H, 1.0f);
+            std::memcpy(&xf[(size_t)t * slot], x.data(), H * 4);
+            for (int k = 0; k < K; k++) {
+                // token 0: the first experts, 1: the last, then a mixture
+                const int e = t == 0 ? k : t == 1 ? E - 1 - k : (t * 3 + k * 2 + (2 * k >= E ? 1 : 0)) % E;
+                chosen[(size_t)t * K + k] = e;
+                std::memcpy(&xf[(size_t)t * slot + H + k], &e, 4);
+                xf[(size_t)t * slot + H + K + k] = 0.1f + 0.2f * k;
+            }
+        }
+        Dev<int8_t> dgq(gq), ddq(dq);
+        Dev<__half> dgs(gs), dds(ds);
+        Dev<float> dgb(gb), ddb(db), dxf(xf), sw((size_t)T * K * F);
+        Dev<uint32_t> status(1);
+        for (int first : {0, E / 2})
+            for (int n_local : {E - first, 2})
+                for (int tokens : {1, 2, T}) {
+                    Dev<float> out((size_t)T * H);
+                    MoeArgs a{};
+                    a.hidden = H; a.ffn = F; a.n_experts = E; a.top_k = K; a.slot = slot; a.xf_in = dxf.p; a.n_tokens = tokens; a.expert0 = first; a.n_local = n_local;
+                    a.gu_q = dgq.p + (size_t)first * 2 * F * H; a.gu_s = dgs.p + (size_t)first * 2 * F * H / 32; a.gu_bias = dgb.p + (size_t)first * 2 * F;
+                    a.dn_q = ddq.p + (size_t)first * H * F; a.dn_s = dds.p + (size_t)first * H * F / 32; a.dn_bias = ddb.p + (size_t)first * H;
+                    a.gain_kind = WK_F32; a.sw = sw.p; a.limit = 7.0f; a.status = status.p; a.out = out.p; a.out_ld = H;
+                    CK(launch_moe_experts(a, 148, nullptr));
+                    const std::vector<float> got = out.get();
+                    double num = 0, den = 0;
+                    for (int t = 0; t < tokens; t++) {
+                        std::vector<double> want(H);
+                        for (int k = 0; k < K; k++) {
+                            const int e = chosen[(size_t)t * K + k];
+                            if (e < first || e >= first + n_local) continue;
+                            std::vector<double> s(F);
+                            auto row = [&](const std::vector<int8_t>& q, const std::vector<__half>& d, size_t r, int n, auto x) {
+                                double v = 0;
+                                for (int i = 0; i < n; i++) v += (double)q[r * n + i] * (double)__half2float(d[(r * n + i) / 32]) * x(i);
+                                return v;
+                            };
+                            auto x = [&](int i) { return (double)xf[(size_t)t * slot + i]; };
+                            for (int i = 0; i < F; i++) {
+                                const size_t r = (size_t)e * 2 * F + 2 * i;
+                                const double g = std::fmin(row(gq, gs, r, H, x) + gb[r], 7.0), u = std::fmax(std::fmin(row(gq, gs, r + 1, H, x) + gb[r + 1], 7.0), -7.0);
+                                s[i] = (u + 1) * g / (1 + std::exp(-1.702 * g));
+                            }
+                            for (int c = 0; c < H; c++)
+                                want[c] += (double)xf[(size_t)t * slot + H + K + k] * (row(dq, ds, (size_t)e * H + c, F, [&](int i) { return s[i]; }) + db[(size_t)e * H + c]);
+                        }
+                        for (int c = 0; c < H; c++) { const double d = got[(size_t)t * H + c] - want[c]; num += d * d; den += want[c] * want[c]; }
+                    }
+                    for (size_t i = (size_t)tokens * H; i < got.size(); i++) num += (double)got[i] * got[i];          // nothing behind the last token
+                    // three levels keep 2^-24 of the largest magnitude, the rest are roundings of two sums in a row
+                    report(std::to_string(H) + " x " + std::to_string(F) + ", experts " + std::to_string(first) + " + " + std::to_string(n_local) + ", " + std::to_string(tokens) + " tokens",
+                           den > 0 ? std::sqrt(num / den) : num, 32 * std::exp2(-24.0));
+                }
+        uint32_t st = status.get()[0];
+        report("status", st, 0);
+    }
+}
+
+// bf16 matrices in the plain matrix-vector kernel, four rows per warp: rows per block that are no multiple of four or of 32, matrices that end inside a
+// group of four, columns that are no multiple of a warp's trip, the paired epilogue.
+static void matvec_bf16() {
+    struct Case { std::vector<int> rows; int k; bool pair; };
+    const std::vector<Case> cases = {{{1}, 8, false},      {{3}, 264, false},         {{37}, 2568, false},     {{9, 2, 5}, 512, false}, {{130, 33, 34}, 264, false},
+                                     {{5003}, 520, false}, {{6, 6}, 512, true},       {{45, 45}, 264, true},   {{2501, 2501}, 1032, true}, {{40003}, 512, false}, {{20000, 3, 1001}, 1024, false}};
+    for (const Case& c : cases) {
+        std::mt19937 rng(c.k + c.rows[0]);
+        const std::vector<float> x = normal(rng, c.k, 1.0f);
+        Dev<float> dx(x);
+        GemvArgs a{};
+        a.nseg = (int)c.rows.size(); a.K = c.k; a.wkind = WK_BF16; a.epi = c.pair ? EPI_SWIGLU : EPI_STORE; a.x = dx.p; a.gain_kind = WK_F32;
+        std::vector<std::vector<uint16_t>> w;
+        std::vector<Dev<uint16_t>*> dw;
+        std::vector<std::vector<double>> sums;
+        int total = 0;
+        for (int n : c.rows) {
+            w.push_back(to_bf16(normal(rng, (size_t)n * c.k, 1.0f / std::sqrt((float)c.k))));
+            dw.push_back(new Dev<uint16_t>(w.back()));
+            a.seg[sums.size()] = {dw.back()->p, nullptr, n, 0};
+            sums.emplace_back(n);
+            for (int r = 0; r < n; r++)
+                for (int i = 0; i < c.k; i++) sums.back()[r] += (double)bf16_value(w.back()[(size_t)r * c.k + i]) * x[i];
+            total += n;
+        }
+        std::vector<double> want;
+        if (c.pair) { total = c.rows[0]; for (int r = 0; r < total; r++) want.push_back(sums[0][r] / (1 + std::exp(-sums[0][r])) * sums[1][r]); }
+        else for (const auto& s : sums) want.insert(want.end(), s.begin(), s.end());
+        Dev<float> y((size_t)total + 8);                  // (eight behind the end: stay zero)
+        Dev<uint32_t> status(1);
+        a.y = y.p; a.status = status.p;
+        CK(launch_gemv(a, 148, nullptr));
+        std::vector<float> got = y.get();
+        for (int i = 0; i < 8; i++) if (got[total + i] != 0.0f) report("behind the end", 1, 0);
+        got.resize(total);
+        std::string what;
+        for (int n : c.rows) what += std::to_string(n) + " ";
+        // 32-bit sums of k products, folded over a warp
+        report(what + "x " + std::to_string(c.k) + (c.pair ? " paired" : ""), rel(got, want), (4 + std::sqrt(c.k / 32.0)) * std::exp2(-23.0));
+        for (auto* p : dw) delete p;
+    }
+}
+
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "attention-sums") attention_sums();
     else if (what == "attention-specials") attention_specials();
+    else if (what == "experts") experts();
+    else if (what == "matvec-bf16") matvec_bf16();
     else { std::printf("unknown check\n"); return 2; }
     return failures ? 1 : 0;
 }
