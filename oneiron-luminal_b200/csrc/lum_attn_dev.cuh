@@ -5,29 +5,6 @@
 
 namespace lum {
 
-
-
-template <bool BF16>
-__device__ __forceinline__ void load16(const void* base, size_t elem_off, float* out) {
-    if (BF16) {
-        const uint4* p = (const uint4*)((const uint16_t*)base + elem_off);
-        const uint4 a = p[0], b = p[1];
-        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            out[2 * i] = __uint_as_float(w[i] << 16);
-            out[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-        }
-    } else {
-        const float4* p = (const float4*)((const float*)base + elem_off);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const float4 v = p[i];
-            out[4 * i] = v.x; out[4 * i + 1] = v.y; out[4 * i + 2] = v.z; out[4 * i + 3] = v.w;
-        }
-    }
-}
-
 __device__ __forceinline__ float gain_at(const void* g, int kind, int i) {
     return kind == WK_BF16 ? bf16_bits_to_f32(((const uint16_t*)g)[i]) : ((const float*)g)[i];
 }
@@ -122,28 +99,6 @@ __device__ __forceinline__ void raw_to_float_impl(float4 r, float* out) { out[0]
 __device__ __forceinline__ void raw_to_float_impl(float2 r, float* out) { out[0] = r.x; out[1] = r.y; }
 template <bool BF16, int DPL>
 __device__ __forceinline__ void raw_to_float(typename RawRow<BF16, DPL>::type r, float* out) { raw_to_float_impl(r, out); }
-
-template <bool BF16, int DPL>
-__device__ __forceinline__ void load_dpl(const void* base, size_t elem_off, float* out) {
-    if (BF16) {
-        if (DPL == 4) {
-            const uint2 r = *(const uint2*)((const uint16_t*)base + elem_off);
-            out[0] = __uint_as_float(r.x << 16); out[1] = __uint_as_float(r.x & 0xffff0000u);
-            out[2] = __uint_as_float(r.y << 16); out[3] = __uint_as_float(r.y & 0xffff0000u);
-        } else {
-            const uint32_t r = *(const uint32_t*)((const uint16_t*)base + elem_off);
-            out[0] = __uint_as_float(r << 16); out[1] = __uint_as_float(r & 0xffff0000u);
-        }
-    } else {
-        if (DPL == 4) {
-            const float4 r = *(const float4*)((const float*)base + elem_off);
-            out[0] = r.x; out[1] = r.y; out[2] = r.z; out[3] = r.w;
-        } else {
-            const float2 r = *(const float2*)((const float*)base + elem_off);
-            out[0] = r.x; out[1] = r.y;
-        }
-    }
-}
 
 // The cached rows a CTA will walk do not depend on the projections of the current step (rows [.., p) were written by earlier
 // steps), so a kernel that still waits for those projections can already ask for them to be brought into L2: one request

@@ -218,23 +218,8 @@ __device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
 
 // kind::f16 with binary16 operands, f32 accumulators, both operands K-major, shape M x N (K = 16)
 __host__ __device__ constexpr uint32_t umma_idesc_f16(int M, int N) { return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24); }
-__device__ __forceinline__ void umma_f16_ss(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-// the same with the A operand in tensor memory: lane = row, 32-bit column j = elements 2j, 2j + 1 of the row
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// the B descriptor given as its two halves (the high half is the same for every operand of a kernel)
+// The A operand lies in tensor memory: lane = row, 32-bit column j = elements 2j, 2j + 1 of the row.  The B descriptor is given as its two halves
+// (the high half is the same for every operand of a kernel).
 __device__ __forceinline__ void umma_f16_ts2(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 db, {%2, %3};\n\t"
@@ -879,14 +864,14 @@ size_t gemm_parts_rows(int n_rows_total, int K, int cap, int sm_count) {
     return worst;
 }
 
-cudaError_t launch_rows_quantize(const RowsArgs& a_in, cudaStream_t st) {
+cudaError_t launch_rows_quantize(const RowsArgs& a_in, int sm_count, cudaStream_t st) {
     RowsArgs a = a_in;
     if (a.M <= 0 || a.K <= 0 || (a.K % 32) || a.n_parts < 1 || a.nc < 16 || a.nc > kGmMaxChunk || a.nc % 16) return cudaErrorInvalidValue;
     const int nc = a.nc;
     const int rows = (a.M + nc - 1) / nc * nc;            // padding rows of the last chunk are zeroed by their own CTAs
     // CTAs per row: up to eight while the rows alone leave SMs idle, of at least eight slices each
     int C = 1;
-    while (C < kRqMaxCluster && rows * C * 2 <= 4 * 148 && (a.K >> 5) / (C * 2) >= 8) C *= 2;
+    while (C < kRqMaxCluster && rows * C * 2 <= 4 * sm_count && (a.K >> 5) / (C * 2) >= 8) C *= 2;
     const size_t smem = (size_t)(((a.K >> 5) + C - 1) / C) * 128;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
     if (smem > 48 * 1024) {
@@ -1008,7 +993,7 @@ extern "C" int32_t lum_op_gemm_q8_0_packed(const void* packed, int32_t n, int32_
     const GemmShape shape = gemm_shape(n, m, k, 148);
     RowsArgs r{};
     r.nc = shape.nc; r.a = x; r.n_parts = 1; r.part_stride = 0; r.ld = k; r.M = m; r.K = k; r.xq = xq; r.sx = sx;
-    cudaError_t e = launch_rows_quantize(r, st);
+    cudaError_t e = launch_rows_quantize(r, sms, st);
     GemmArgs g{};
     g.nseg = 1; g.seg[0] = {(const unsigned char*)packed, n, 0}; g.K = k; g.xq = xq; g.sx = sx; g.M = m;
     g.nc = shape.nc; g.ksplit = shape.ks;

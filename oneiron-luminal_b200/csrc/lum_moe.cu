@@ -15,7 +15,7 @@
 // Expert weights are Q8_0 planes (int8 [rows, K] and one binary16 scale per 32): a row is one contiguous run.  Converting every int8
 // weight to f32 (a quarter-rate instruction each) binds such a kernel at about 1 TB/s, so — as in the streaming GEMV — the ACTIVATIONS
 // go to the integer side instead: a CTA writes the token's activation vector as three int8 levels per 32-block, x ~= s (a1 + a2/254 +
-// a3/254^2) (error <= max|x| 2^-24), into shared memory once, and a weight block then costs 24 integer dot-product instructions (dp4a)
+// a3/254^2) (error <= 1.03 max|x| 2^-24), into shared memory once, and a weight block then costs 24 integer dot-product instructions (dp4a)
 // and a few conversions.
 #include "lum_gemv_dev.cuh"
 #include "lum_moe.cuh"

@@ -506,7 +506,7 @@ cudaError_t launch_rope_append_rows(const RopeRowsArgs& a, cudaStream_t st) {
     return launch_rows_pdl(fn, dim3((unsigned)(a.M * ((a.n_q + 2 * a.n_kv + 7) / 8))), dim3(256), params, a.use_pdl, st);
 }
 
-cudaError_t launch_attn_rows(const AttnRowsArgs& a, cudaStream_t st) {
+cudaError_t launch_attn_rows(const AttnRowsArgs& a, int sm_count, cudaStream_t st) {
     const int G = a.n_kv > 0 ? a.n_q / a.n_kv : 0;
     static const int env_split = [] { const char* e = getenv("LUM_ATTN_ROWS_SPLIT"); return e ? atoi(e) : 1; }();
     if (env_split && a.kv_bf16 && a.window == 0 && (a.hd == 128 || a.hd == 64) && G >= 1 && G <= (a.hd == 128 ? 4 : 8) && (((uintptr_t)a.k_cache | (uintptr_t)a.v_cache) & 15) == 0 &&
@@ -517,9 +517,10 @@ cudaError_t launch_attn_rows(const AttnRowsArgs& a, cudaStream_t st) {
             cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) return e;
         }
-        // Splits per (KV head, row): rounds of resident CTAs (three per SM) times the keys of one, plus what a CTA costs beside its keys —
-        // about the time of 100 of them.  The positions are on the device, so a context of middling length (1024 keys) stands for all.
-        const long long pairs = (long long)a.n_kv * a.M, slots = 3 * 148;
+        // Splits per (KV head, row): rounds of resident CTAs (three per SM: what the ring of a 128-dimension head and the registers allow; counted for
+        // the others too) times the keys of one, plus what a CTA costs beside its keys — about the time of 100 of them.  The positions are on
+        // the device, so a context of middling length (1024 keys) stands for all.
+        const long long pairs = (long long)a.n_kv * a.M, slots = 3ll * sm_count;
         int splits = 1;
         for (int s = 2; s <= kAttnRowsMaxSplits; s++) {
             auto cost = [&](int n) { return (double)((pairs * n + slots - 1) / slots) * (1024.0 / n + 100.0); };

@@ -11,7 +11,7 @@ struct GemmArgs {
     GemmSeg seg[3];
     int nseg;
     int K;
-    const int8_t* xq;        // activation operand as rows_quantize writes it: three binary16 terms per element, tensor-core order
+    const int8_t* xq;        // activation operand as rows_quantize writes it: two binary16 terms per element, tensor-core order
     const float* sx;         // [rows]: the power-of-two factor that turns a row's accumulators into its outputs
     int M, nc, m_chunks;     // nc: activation rows per chunk, as the rows were written (gemm_shape); m_chunks is set by the launcher
     int row_chunks;          // up to 64 rows: runs of row groups (set by the launcher)
@@ -56,7 +56,7 @@ struct RopeRowsArgs {
 struct AttnRowsArgs {
     const float* q_rot;        // [M][n_q * hd]
     const void* k_cache; const void* v_cache;
-    KvPages pg;                // pages of at least 64 rows: a tile of 32 or 64 keys that starts on a multiple of its size lies in one page
+    KvPages pg;                // pages of at least 64 rows: a tile of 16 or 64 keys that starts on a multiple of its size lies in one page
     const int* row_pos; const int* row_seq; int seq0;
     float* out;                // [M][n_q * hd]
     int M, n_q, n_kv, hd, kv_bf16, window, max_seq, max_batch;
@@ -80,14 +80,14 @@ constexpr int kMaxKsplit = 8;
 GemmShape gemm_shape(int n_rows_total, int M, int K, int sm_count);
 size_t gemm_parts_rows(int n_rows_total, int K, int cap, int sm_count);
 bool gemm_supported(const GemmArgs& a);
-cudaError_t launch_rows_quantize(const RowsArgs& a, cudaStream_t st);
+cudaError_t launch_rows_quantize(const RowsArgs& a, int sm_count, cudaStream_t st);
 cudaError_t launch_gemm(const GemmArgs& a, int sm_count, cudaStream_t st);
 cudaError_t launch_embed_rows(const void* table, int kind, int H, int vocab, const int* row_tok, float* x, int M, uint32_t* status, cudaStream_t st);
 // the same plus the sinusoidal position vector (see EmbedArgs::pos_freq; null: none), rows ldx floats apart
 cudaError_t launch_embed_rows_sinusoid(const void* table, int kind, int H, int vocab, const int* row_tok, const int* row_pos, const double* pos_freq, float* x, int ldx,
                                        int M, uint32_t* status, cudaStream_t st);
 cudaError_t launch_rope_append_rows(const RopeRowsArgs& a, cudaStream_t st);
-cudaError_t launch_attn_rows(const AttnRowsArgs& a, cudaStream_t st);
+cudaError_t launch_attn_rows(const AttnRowsArgs& a, int sm_count, cudaStream_t st);
 constexpr int kAttnRowsMaxSplits = 8;                            // CTAs of a portable cluster
 bool attn_prompt_tc_supported(const AttnRowsArgs& a);            // lum_attn_tc.cu: rows of one sequence, bf16 cache, head dimension 128
 cudaError_t launch_attn_prompt_tc(const AttnRowsArgs& a, cudaStream_t st);

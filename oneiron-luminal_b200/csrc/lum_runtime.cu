@@ -1400,7 +1400,7 @@ int run_rows(lum_rt* rt, int M, int* d_tok, int* d_pos, const int* d_seq, int se
     const int ks_qkv = g_qkv.ks, ks_o = g_o.ks, ks_gu = g_gu.ks, ks_dn = g_dn.ks;
     CU(rt, launch_embed_rows(rt->embed.w, rt->embed.kind, H, d.vocab, d_tok, b.xr, M, rt->status, st));
     uint64_t launches = 1;
-    auto quant = [&](RowsArgs& r, int K, GemmShape gs) -> cudaError_t { r.M = M; r.K = K; r.nc = gs.nc; r.xq = b.xq; r.sx = b.sx; r.use_pdl = pdl; launches++; return launch_rows_quantize(r, st); };
+    auto quant = [&](RowsArgs& r, int K, GemmShape gs) -> cudaError_t { r.M = M; r.K = K; r.nc = gs.nc; r.xq = b.xq; r.sx = b.sx; r.use_pdl = pdl; launches++; return launch_rows_quantize(r, sms, st); };
     auto gemm = [&](GemmArgs& g, int K, GemmShape gs, float* y, int ldy) -> cudaError_t {
         g.K = K; g.xq = b.xq; g.sx = b.sx; g.M = M; g.nc = gs.nc; g.ksplit = gs.ks; g.y = y; g.ldy = ldy; g.part_stride = (size_t)M * ldy; g.status = rt->status; g.use_pdl = pdl;
         launches++;
@@ -1438,7 +1438,7 @@ int run_rows(lum_rt* rt, int M, int* d_tok, int* d_pos, const int* d_seq, int se
             // many rows of one sequence (a prompt): the tensor-core kernel; few rows, or rows of different sequences: one CTA per row
             static const int env_tc = [] { const char* e = getenv("LUM_ATTN_TC"); return e ? atoi(e) : 1; }();
             if (env_tc && M >= 16 && attn_prompt_tc_supported(a)) CU(rt, launch_attn_prompt_tc(a, st));
-            else CU(rt, launch_attn_rows(a, st));
+            else CU(rt, launch_attn_rows(a, sms, st));
             launches += 2;
         }
         {   // attention output -> operand of the o projection

@@ -105,7 +105,7 @@ struct Attention {
         AttnRowsArgs a{};
         a.q_rot = dq.p; a.k_cache = kc.p; a.v_cache = vc.p; a.row_pos = pos.p; a.out = out.p; a.M = 1; a.n_q = nq; a.n_kv = nkv; a.hd = hd; a.kv_bf16 = 1;
         a.max_seq = max_seq; a.max_batch = 1; a.status = status.p;
-        CK(launch_attn_rows(a, nullptr));
+        CK(launch_attn_rows(a, 148, nullptr));
         return out.get();
     }
 };
