@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
 // Same arithmetic, but the regime is the other one: the weights are the stream that matters (HBM-bound), and everything else has to
 // keep up with 23 bytes of them per SM and clock, which is 187 clocks per 32-column slice of 128 weight rows.
 //   * Work items are runs of up to 32 row groups of 8 weight rows, over the concatenated matrices, times a range of K-tiles: the row groups
-//     are dealt out evenly (gemm_plan), so that all SMs finish together and few K ranges (planes of partial sums) are needed.  An item of
+//     are dealt out evenly (gemm_plan), so that all SMs finish together whatever the K ranges (planes of partial sums).  An item of
 //     more than 16 row groups is two tensor-core tiles that take turns on each K-tile and share its activation slices in shared memory.
 //   * Weights are staged by bulk copies of whole 4352-byte tiles, half an item's row groups of one K-tile per stage, two stages.
 //   * 16 warps convert: four per quarter of the tensor-memory lanes, each one slice of the four of a hand-over (two loads, 32 weights in
@@ -470,8 +470,10 @@ __global__ void __launch_bounds__(kGmThreads, 1) q8_gemm_tc(const GemmArgs a) {
 //   * Activations: a chunk is 16, 32 or 64 rows, whichever holds the step; a slice is 128 bytes per row, and with 32 rows a CTA reads as many
 //     bytes of them from L2 as of weights from HBM if it has one tensor-core tile, half as many if it has two.
 // Measured, alone, back to back over weights that L2 does not hold (us at 32 rows / 5 rows; before: q8_gemm_tc_layer_shapes of the profiles, a chunk
-// of 32 rows for both): qkv 6144 x 4096 39.5 -> 16.6 / 15.5, gate|up 28672 x 4096 111.3 -> 43.3 / 41.1, down 4096 x 14336 68.8 -> 26.8 / 22.7,
-// vocabulary 128256 x 4096 323.1 -> 152.7 / 139.5 (3.7 and 4.0 TB/s of weights).  What is left is latency: set-up and first copies, about 5 us
+// of 32 rows for both): qkv 6144 x 4096 39.5 -> 16.5 / 14.8, gate|up 28672 x 4096 111.3 -> 52.1 / 45.2 (three K ranges, which gemm_least_split asks for;
+// one range: 43.3 / 41.1), down 4096 x 14336 68.8 -> 26.7 / 22.7, vocabulary 128256 x 4096 323.1 -> 152.8 / 141.0 (3.7 and 4.0 TB/s of weights).
+// 33 to 64 rows, with their rows' preparation: gate|up 135 -> 76 at 33 rows, 140 -> 85 at 64; down 79 -> 51, 80 -> 52; vocabulary 431 -> 221, 435 ->
+// 219.  What is left is latency: set-up and first copies, about 5 us
 // that a dependent launch hides, and hand-overs of about 800 clocks per four slices where the conversion's issue slots are 440.
 constexpr int kGsRG = 16;                           // row groups per tensor-core tile
 constexpr int kGsWRow = kTileBytes;                 // 4352: one tile, quants then scales, as streamed

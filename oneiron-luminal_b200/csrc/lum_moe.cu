@@ -186,7 +186,7 @@ __device__ __forceinline__ int moe_selected(const MoeArgs& a, const float* xf, M
 
 // A cluster of eight CTAs per token: each normalises the row for itself and takes every eighth expert, a warp per expert; the first CTA gathers the logits
 // and selects.  Gains and router rows do not depend on the previous kernel: a warp has its own on the way before it waits for that.
-// Measured (gpt-oss-20B shape, cold caches): 16.3 us with one CTA of 512 threads, 8.0 us this way.
+// Measured (gpt-oss-20B shape, cold caches): 16.3 us with one CTA of 512 threads, 8.5 us this way.
 constexpr int kRouteCtas = 8, kRouteWarps = 4, kRouteAhead = 12, kRouteTrips = 8;
 __global__ void __launch_bounds__(kRouteWarps * 32) moe_route(const MoeArgs a) {
     extern __shared__ __align__(16) float mr_smem[];          // xf [H], logits [E]
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_route(const MoeArgs a) {
 }
 
 // One CTA per SM: its warps take (selected expert, position) pairs in turn; gate and up are rows 2 i and 2 i + 1.
-// Measured (gpt-oss-20B shape, 4 experts, 70.5 MB, cold caches): 31.5 us with plain loads, 29.5 us with 8 warps of four stages.
+// Measured (gpt-oss-20B shape, 4 experts, 70.5 MB, cold caches): 31.5 us with plain loads, 29.5 us with 8 warps of four stages, 24.4 us with 16 of two.
 __global__ void __launch_bounds__(kMoeWarps * 32, 1) moe_gate_up(const MoeArgs a, const int stages, const int blocks) {
     extern __shared__ __align__(128) unsigned char me_smem[];
     __shared__ __align__(8) unsigned long long bars[kMoeWarps * kMoeMaxStages];
@@ -337,7 +337,8 @@ __global__ void __launch_bounds__(kMoeWarps * 32, 1) moe_gate_up(const MoeArgs a
 // One CTA per SM takes pairs of output columns; a warp's unit is a pair's rows of one selected expert, and the experts' shares of a column meet in
 // shared memory, added in the order of the selection.  The routing was complete before this kernel could start (see moe_gate_up), so the
 // weights are on their way before the previous kernel is waited for.
-// Measured (gpt-oss-20B shape, 4 experts, 35.3 MB, cold caches): 37 us with plain loads and a warp per column, 22.2 us with 8 warps of four stages.
+// Measured (gpt-oss-20B shape, 4 experts, 35.3 MB, cold caches): 37 us with plain loads and a warp per column, 22.2 us with 8 warps of four stages,
+// 21.3 us with 16 of two.
 __global__ void __launch_bounds__(kMoeWarps * 32, 1) moe_down(const MoeArgs a, const int stages, const int blocks) {
     extern __shared__ __align__(128) unsigned char me_smem[];
     __shared__ __align__(8) unsigned long long bars[kMoeWarps * kMoeMaxStages];

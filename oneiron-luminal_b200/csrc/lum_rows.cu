@@ -217,8 +217,8 @@ __global__ void __launch_bounds__(256) attn_rows(const AttnRowsArgs a) {
 //     beyond one instruction is added up in f32 (attn_mma).
 //   * warps merge in shared memory, splits through the cluster's distributed shared memory: no partial results in global memory and no
 //     second kernel.
-// Measured (32 sequences x 2049 keys, 8 KV heads x 4 query heads, head dimension 128; 268 MB of cache): 53 us with sums left in the tensor
-// core, a whole step of 32 Llama-3-8B rows 0.7 % slower this way (6.49 -> 6.53 ms).  The form before it, with
+// Measured (32 sequences x 2049 keys, 8 KV heads x 4 query heads, head dimension 128; 268 MB of cache): 53.4 us with sums left in the
+// tensor core, 55.4 us this way.  The form before it, with
 // a lane per key and the products on CUDA cores (1700 instructions per warp and 32 keys, 16-byte loads 2 KiB apart), took 147 us and
 // 6 us more to merge.
 __device__ __forceinline__ void ar_ldsm4(uint32_t addr, uint32_t (&r)[4]) {
