@@ -430,28 +430,37 @@ cudaError_t launch_moe_route(const MoeArgs& a_in, int n_tokens, cudaStream_t st)
     void* params[] = {&a};
     return launch1((const void*)moe_route, dim3(n_tokens * kRouteCtas), dim3(kRouteWarps * 32), ((size_t)a.hidden + a.n_experts) * 4, params, kRouteCtas, a.use_pdl, st);
 }
+// Shared memory of an expert kernel beside its ring: activation levels and block scales, the selection, and (down) a CTA's results
+size_t moe_gate_up_bytes(int H, int top_k) { return 3 * (size_t)H + (size_t)(H / 32) * 4 + (size_t)top_k * sizeof(MoeSel); }
+size_t moe_down_bytes(int H, int F, int top_k, int sm_count) {
+    const size_t pairs = ((size_t)H / 2 + sm_count - 1) / sm_count;
+    return (size_t)top_k * ((3 * (size_t)F + (size_t)(F / 32) * 4 + 15) & ~(size_t)15) + (size_t)top_k * sizeof(MoeSel) + pairs * top_k * 8;
+}
+// The ring beside `act` bytes: two stages of whole rows (up to 96 blocks) where they fit, then shorter ones, then one stage; 0 where not even
+// a block per warp fits.  Whatever 200 KB of levels and scales hold is taken (hidden up to 65536, eight experts of ffn up to 8192).
+int moe_ring_fit(size_t act, int K, int* stages, int* blocks) {
+    constexpr size_t kMost = 226 * 1024;
+    int s = kMoeMaxStages, b = K / 32 < kMoeBlocks ? K / 32 : kMoeBlocks;
+    while (act + moe_ring_bytes(s, b) > kMost && (s > 1 || b > 1)) {
+        if (b > 16) b = b / 2 < 16 ? 16 : b / 2;
+        else if (s > 1) s--;
+        else b = b / 2;
+    }
+    *stages = s; *blocks = b;
+    return act + moe_ring_bytes(s, b) <= kMost;
+}
 cudaError_t launch_moe_experts(const MoeArgs& a_in, int sm_count, cudaStream_t st) {
     MoeArgs a = a_in;
     if ((a.hidden % 32) || (a.ffn % 32) || a.top_k < 1) return cudaErrorInvalidValue;
-    const size_t act_gu = 3 * (size_t)a.hidden + (size_t)(a.hidden / 32) * 4 + (size_t)a.top_k * sizeof(MoeSel);
-    const size_t pairs = ((size_t)a.hidden / 2 + sm_count - 1) / sm_count;
-    const size_t act_dn = (size_t)a.top_k * ((3 * (size_t)a.ffn + (size_t)(a.ffn / 32) * 4 + 15) & ~(size_t)15) + (size_t)a.top_k * sizeof(MoeSel) + pairs * a.top_k * 8;
-    // the ring: two stages of whole rows (up to 96 blocks) where they fit, down to 16 blocks
     auto launch = [&](const void* fn, size_t act, int K) -> cudaError_t {
-        constexpr size_t kMost = 226 * 1024;
-        int stages = kMoeMaxStages, blocks = K / 32 < kMoeBlocks ? K / 32 : kMoeBlocks;
-        while (act + moe_ring_bytes(stages, blocks) > kMost && (stages > 1 || blocks > 16)) {
-            if (blocks > 16) blocks = blocks / 2 < 16 ? 16 : blocks / 2;
-            else stages--;
-        }
-        const size_t smem = act + moe_ring_bytes(stages, blocks);
-        if (smem > kMost) return cudaErrorInvalidValue;
+        int stages, blocks;
+        if (!moe_ring_fit(act, K, &stages, &blocks)) return cudaErrorInvalidValue;
         void* params[] = {&a, &stages, &blocks};
-        return launch1(fn, dim3(sm_count), dim3(kMoeWarps * 32), smem, params, 1, a.use_pdl, st);
+        return launch1(fn, dim3(sm_count), dim3(kMoeWarps * 32), act + moe_ring_bytes(stages, blocks), params, 1, a.use_pdl, st);
     };
-    cudaError_t e = launch((const void*)moe_gate_up, act_gu, a.hidden);
+    cudaError_t e = launch((const void*)moe_gate_up, moe_gate_up_bytes(a.hidden, a.top_k), a.hidden);
     if (e != cudaSuccess) return e;
-    return launch((const void*)moe_down, act_dn, a.ffn);
+    return launch((const void*)moe_down, moe_down_bytes(a.hidden, a.ffn, a.top_k, sm_count), a.ffn);
 }
 cudaError_t launch_moe_combine(float* x, const float* parts, int n_parts, int part_ld, int H, cudaStream_t st) {
     moe_combine<<<(H + 255) / 256, 256, 0, st>>>(x, parts, n_parts, part_ld, H);

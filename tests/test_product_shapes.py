@@ -1,4 +1,5 @@
-"""How the products of several rows are cut up (host side of lum_gemm.cu, no GPU): rows per chunk and ranges of the inner dimension."""
+"""How kernels are cut up (host side of lum_gemm.cu and lum_moe.cu, no GPU): rows per chunk and ranges of the inner dimension of products of several
+rows, rings of the expert kernels."""
 import ctypes as C
 import math
 
@@ -59,3 +60,29 @@ def test_room_for_partial_sums_covers_every_row_count(pkg, shape, n, k, cap):
     f = pkg.load_library()["_ZN3lum15gemm_parts_rowsEiiii"]          # lum::gemm_parts_rows(outputs, inner, most rows, SMs)
     f.restype, f.argtypes = C.c_size_t, [C.c_int] * 4
     assert f(n, k, cap, SMS) == max(m * shape(n, m, k).ks for m in range(1, cap + 1))
+
+
+def test_expert_kernels_take_every_size_whose_activations_fit(pkg):
+    """200 KB of activation levels and block scales have always been taken, whatever else lies beside them."""
+    lib = pkg.load_library()
+    fit = lib["_ZN3lum12moe_ring_fitEmiPiS0_"]
+    fit.restype, fit.argtypes = C.c_int, [C.c_size_t, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int)]
+    gate_up, down = lib["_ZN3lum17moe_gate_up_bytesEii"], lib["_ZN3lum14moe_down_bytesEiiii"]
+    gate_up.restype, gate_up.argtypes, down.restype, down.argtypes = C.c_size_t, [C.c_int] * 2, C.c_size_t, [C.c_int] * 4
+    stages, blocks = C.c_int(), C.c_int()
+
+    def ring(act, k):
+        ok = fit(act, k, C.byref(stages), C.byref(blocks))
+        assert not ok or (1 <= stages.value <= 2 and 1 <= blocks.value <= min(96, k // 32) and act + 16 * 64 * stages.value * blocks.value <= 226 * 1024)
+        return (stages.value, blocks.value) if ok else None
+
+    for hidden in (32, 96, 2880, 4096, 16384, 47104, 50016, 65536):
+        assert 3 * hidden + hidden // 8 <= 200 * 1024 and ring(gate_up(hidden, 8), hidden)
+        for top_k in range(1, 9):
+            most = max(f for f in range(32, 70000, 32) if top_k * ((3 * f + f // 8 + 15) // 16 * 16) <= 200 * 1024)
+            for ffn in (32, 96, 2880, most):
+                if ffn <= most:
+                    assert ring(down(hidden, ffn, top_k, SMS), ffn), f"{hidden} x {ffn}, {top_k} experts"
+    # the configured shape keeps whole rows in two stages
+    assert ring(gate_up(2880, 4), 2880) == (2, 90) and ring(down(2880, 2880, 4, SMS), 2880) == (2, 90)
+    assert ring(230 * 1024, 2880) is None
