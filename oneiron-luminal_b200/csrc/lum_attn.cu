@@ -167,6 +167,7 @@ cudaError_t launch_attn_decode(const AttnArgs& a_in, cudaStream_t st) {
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
     }
+    if (const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) return e;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[2];
     attn_fill_config(a, G, cl, st, &cfg, at);
@@ -178,6 +179,7 @@ cudaError_t launch_attn_decode(const AttnArgs& a_in, cudaStream_t st) {
 // `RowEmbed` (crates/luminal_cuda/src/block/ops.rs:1921-1944): x = table[token, :], widened to f32.
 __global__ void __launch_bounds__(256) embed_row(const EmbedArgs a) {
     if (a.use_pdl) { pdl_launch_dependents(); pdl_grid_wait(); }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n_zero; i += gridDim.x * blockDim.x) a.zero_ctr[i] = 0u;
     if (a.seq_inc && blockIdx.x == 0 && threadIdx.x == 0) *a.seq_inc += 1u;     // every kernel after this one sees the new value
     const int tok = a.state->tok;
     if (tok < 0 || tok >= a.state->vocab) {

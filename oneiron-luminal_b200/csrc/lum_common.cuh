@@ -11,10 +11,13 @@
 
 namespace lum {
 
-// the dynamic shared memory that `fn` may be launched with, raised once per device
-inline cudaError_t allow_smem(std::atomic<uint64_t>& done, const void* fn, int bytes) {
-    return (cudaError_t)once_per_device(done, [](int* dev) { return (int)cudaGetDevice(dev); },
-                                        [&] { return (int)cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
+// the dynamic shared memory that `fn` may be launched with, raised once per device.  `whole`: the SM keeps all of it as shared memory while `fn` runs, so that
+// a CTA of the next kernel finds room beside it (the split is otherwise made for the kernel that comes to an empty SM).
+inline cudaError_t allow_smem(std::atomic<uint64_t>& done, const void* fn, int bytes, bool whole = false) {
+    return (cudaError_t)once_per_device(done, [](int* dev) { return (int)cudaGetDevice(dev); }, [&] {
+        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        return (int)(e == cudaSuccess && whole ? cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) : e);
+    });
 }
 
 // ---- status word -------------------------------------------------------------------------------
@@ -127,7 +130,7 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* p, uint32_t bytes) 
 // guarded by this and not by a comparison of the lane: behind `lane == 0` the compiler does not know that a single thread is left, and the
 // code it then makes of an instruction with operands in uniform registers takes 60 clocks to issue whatever the instruction's size.
 // Measured, clocks per tcgen05.mma of M 128, K 32 bytes, back to back (branch on the lane / elected): kind::f16 with A in tensor memory
-// 62 / 17 at N 32, 62 / 33 at N 64, 65 / 65 at N 128; kind::i8 from shared memory 52 / 45 at N 48.
+// 62 / 17 at N 32, 62 / 33 at N 64, 65 / 65 at N 128.
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
@@ -140,32 +143,10 @@ __device__ __forceinline__ uint64_t umma_smem_desc(uint32_t smem_addr, uint32_t 
     return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)((lbo >> 4) & 0x3fffu) << 16) | ((uint64_t)((sbo >> 4) & 0x3fffu) << 32) |
            (1ull << 46);   // bits 46-47: descriptor version of sm_100
 }
-// Instruction descriptor of kind::i8: s32 accumulators, s8 x s8, both operands K-major, shape M x N (K = 32).
-__host__ __device__ constexpr uint32_t umma_idesc_s8(int M, int N) {
-    return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
 // The two halves of such a descriptor, for callers that step through many operands: `lo` carries the start address and
 // lbo (advance it by bytes / 16 to move the operand), `hi` carries sbo and the version and stays fixed.
 __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr, uint32_t lbo) { return ((smem_addr >> 4) & 0x3fffu) | (((lbo >> 4) & 0x3fffu) << 16); }
 __host__ __device__ constexpr uint32_t umma_desc_hi(uint32_t sbo) { return ((sbo >> 4) & 0x3fffu) | (1u << 14); }
-// D[tmem] = A[smem] * B[smem]^T (accumulators overwritten).  Issued by ONE thread.
-__device__ __forceinline__ void umma_s8_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(0u)
-        : "memory");
-}
-// Same with the descriptors given as halves (both operands share `hi`).
-__device__ __forceinline__ void umma_s8_ss_split(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-        "setp.ne.b32 p, %4, %4;\n\t"
-        "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %4, p;\n\t}"
-        ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc)
-        : "memory");
-}
 // `bar` receives one arrival when every tcgen05.mma this thread issued before has completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -228,6 +209,12 @@ __device__ __forceinline__ float bf16_bits_to_f32(uint16_t h) { return __uint_as
 
 // named barrier over `n` threads (n a multiple of 32); id 0 is __syncthreads' own
 __device__ __forceinline__ void named_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+// named_sync that tells every thread whether any of them had `v` set
+__device__ __forceinline__ bool named_or(int id, int n, bool v) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r) : "r"((uint32_t)v), "r"(id), "r"(n) : "memory");
+    return r != 0;
+}
 // arrive without waiting (the waiting side calls named_sync with the same id and total count)
 __device__ __forceinline__ void named_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 

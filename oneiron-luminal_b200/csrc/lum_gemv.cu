@@ -6,15 +6,11 @@
 // Decode is bound by HBM bandwidth: every weight byte is read exactly once per token and nothing
 // else is large.  Two kernels:
 //
-//  * q8_gemv_stream — the hot path.  One CTA per SM, three kinds of warps (lum_gemv_dev.cuh).  A producer warp
-//    walks the CTA's share of the weight matrix in tiles of 8 rows x 512 columns (4096 int8 in tensor-core
-//    operand order plus their 128 binary16 scales) and fetches up to 8 of them per ring stage with one bulk
-//    asynchronous copy (cp.async.bulk, completion counted on an mbarrier).  A tensor-core warp issues one
-//    tcgen05.mma (kind::i8, M128 N48 K32) per tile straight from the stage; the exact int32 dot products land in
-//    tensor memory, from where 8 draining warps read them back, apply the block scales and reduce the rows.
-//    The weight stream does not depend on the activations, so under programmatic dependent launch the producer
-//    starts filling the ring while the previous kernel is still running; only the other warps wait for the
-//    grid dependency.
+//  * q8_gemv_stream — the hot path (lum_gemv_dev.cuh).  A producer warp walks the CTA's share of the weight matrix in
+//    tiles of 8 rows x 512 columns (4096 int8 plus their 128 binary16 scales) and fetches up to 4 of them per ring stage with
+//    one bulk asynchronous copy (cp.async.bulk, completion counted on an mbarrier); eight consumer warps take a tile each.
+//    A CTA is half an SM, so that under programmatic dependent launch the next projection's CTAs are resident, set up and
+//    have filled their rings (the weight stream does not depend on the activations) while this one still works.
 //  * gemv_direct — any K, f32 / bf16 / Q8_0 weights, plain vector loads, one warp per row (bf16: per four rows).
 //    Used for the small all-f32 model and for shapes the streaming kernel does not take.
 //
@@ -23,18 +19,10 @@
 // ops.rs:135-146), SwiGLU (`RowSwishMul`, ops.rs:303-325) or the greedy sampler
 // (examples/llama/src/main.rs:137-148) into their epilogue.
 //
-// Q8_0 arithmetic in the streaming kernel.  Converting int8 -> f32 costs a quarter-rate instruction
-// per weight, which caps an SM near 29 weights/clock — barely above the 23 weights/clock one SM must
-// sustain at full HBM speed.  So the activations are moved to the integer side instead, without
-// giving up their f32 precision: each 32-block of x is written as
-//     x ~= s * (a1 + a2/254 + a3/254^2),   a1, a2, a3 int8 vectors, s = max|x| / 127
-// (three successive int8 roundings of the residual; |error| <= max|x| * 2^-24 per element, the
-// same order as f32 rounding).  A weight block then contributes
-//     d * s * (q.a1 + (q.a2)/254 + (q.a3)/254^2),   d = the block's binary16 scale
-// with the three integer dot products exact: they are three of the 48 accumulator columns one tensor-core
-// instruction produces for each of the tile's 128 (block, row) pairs.  The direct kernel keeps the plain
+// The streaming kernel works on integer levels of the activations (lum_gemv_dev.cuh); the direct kernel keeps the plain
 // f32 form sum_i float(q_i) * x_i.  (The CPU restatement multiplies each weight by its scale first and sums
 // sequentially; all three differ by f32 rounding only.)
+#include <algorithm>
 #include <cstdlib>
 
 #include "lum_gemv_dev.cuh"
@@ -84,48 +72,34 @@ __device__ __forceinline__ float dot4_s8(uint32_t w, float4 x, float acc) {
 // ------------------------------------------------------------------------------ streaming kernel (one op)
 
 
-// WIDE: K above 4096 (up to 16384): the prologue then holds up to eight float4 per thread instead of two.
-template <bool PEER, bool WIDE>
-__global__ void __launch_bounds__(kGemvThreads, 1) q8_gemv_stream(const GemvArgs a) {
-    constexpr int TRIPS = WIDE ? kXTrips : 2;
+template <bool PEER, bool ONE>
+__global__ void __launch_bounds__(kGemvThreads, PEER ? 1 : 2) q8_gemv_stream(const GemvArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_abort;
     const int tid = threadIdx.x;
-    const int warp = tid >> 5, lane = tid & 31;
     GemvSmem g;
-    gemv_carve(smem, a.K, a.stages, &s_abort, &g);
-    if (tid == 0 && blockIdx.x == 0 && a.job_ctr_zero) *a.job_ctr_zero = 0u;
-    const uint32_t tmem = gemv_cta_begin(g, tid, &s_abort);
+    const GemvPlan plan = gemv_plan(a, (int)blockIdx.x, (int)gridDim.x, -1);
+    gemv_carve(smem, a.k_smem, GemvRings{a.ring_n[0], a.ring_n[1], a.ring_t[0], a.ring_t[1]}, &s_abort, &g);
+    gemv_cta_begin(g, tid, &s_abort);
     if (a.use_pdl) pdl_launch_dependents();
-    const GemvPlan plan = gemv_plan(a, (int)gridDim.x, a.job_ctr != nullptr);
 
-    if (warp == kProducerWarp) {
+    if (tid >= kConsumers) {
         // producer: the weight stream does not depend on the previous kernel, so it starts at once
         if (elect_one()) {
-            ProducerRing pr{0, 0u, 0};
-            if (!gemv_produce(a, plan, g, pr, (int)blockIdx.x, (int)gridDim.x, a.job_ctr, a.status)) gemv_producer_drain(g, pr, a.status);
+            ProducerRing pr{};
+            if (!gemv_produce(a, plan, g, pr, a.job_ctr ? a.job_ctr + plan.range : nullptr, a.status)) gemv_producer_drain(g, pr, a.status);
         }
-        return;
-    }
-    if (warp == kMmaWarp) {
-        if (elect_one()) {
-            MmaRing mr{0, 0u, 0u, 0u, 0u};
-            gemv_mma_issue(a, plan, g, mr, tmem, a.status);
-        }
-        gemv_mma_end(g, tmem, lane, a.status);
         return;
     }
     GainRegs gr;
-    gemv_gain_preload<TRIPS>(a, tid, gr);      // independent of the previous kernel: fetched while waiting for it
+    gemv_gain_preload(a, tid, gr);             // independent of the previous kernel: fetched while waiting for it
     if (a.use_pdl) pdl_grid_wait();
     XSource xs{};
     xs.x = a.x; xs.x_add = a.x_add; xs.x_out = a.x_out;
     xs.parts = a.parts; xs.part_flags = a.part_flags; xs.n_parts = a.n_parts; xs.part_stride = a.part_stride; xs.parts_tag = a.parts_tag; xs.seq = a.seq; xs.parts_ll = a.parts_ll;
     ArgBest best{-INFINITY, -1};
-    ConsumerRing cr{0, 0u, 0u, 0u};
-    gemv_consume<PEER, TRIPS>(a, xs, blockIdx.x == 0, plan, g, cr, tid, tmem, a.status, &best, gr);
-    if (tid >= kConsumers) return;
-    gemv_consumers_done();
+    ConsumerRing cr{0, 0u};
+    gemv_consume<PEER, ONE>(a, xs, blockIdx.x == 0, plan, g, cr, tid, a.status, &best, gr);
     if (PEER && a.epi == EPI_PEER && !a.peer_ll) peer_publish(a, tid, kConsumers, 2);
     if (a.epi == EPI_ARGMAX) argmax_finish(a, best, tid, kConsumers, 2);
 }
@@ -238,7 +212,6 @@ __global__ void __launch_bounds__(256, WK == WK_BF16 ? kDirectBf16Ctas : 0) gemv
     float* xs = scratch + 64;                  // K floats (K rounded up to 4)
     float* vals = xs + ((a.K + 3) & ~3);       // 2 * max rows per CTA
 
-    if (tid == 0 && blockIdx.x == 0 && a.job_ctr_zero) *a.job_ctr_zero = 0u;   // this kernel claims nothing, but keeps the rotation going
     if (a.use_pdl) { pdl_launch_dependents(); pdl_grid_wait(); }
     gemv_load_x(a, xs, tid, 256, scratch, 1);
 
@@ -331,46 +304,55 @@ cudaError_t launch_gemv(const GemvArgs& a_in, int sm_count, cudaStream_t st) {
     if (rows_total <= 0 || a.K <= 0) return cudaErrorInvalidValue;
 
     if (gemv_stream_supported(a)) {
-        // Share of the jobs every CTA owns without claiming.  One kernel per operation: none (measured best: a CTA that starts
-        // late, because its SM was still busy with the previous kernel, then simply finds less left to claim).
-        static const int env_static = [] { const char* e = getenv("LUM_STATIC_PERMILLE"); return e ? atoi(e) + 1 : 1; }();
-        if (a.debug == 0) a.debug = env_static;
         static const int env_slack = [] { const char* e = getenv("LUM_CLAIM_SLACK"); return e ? atoi(e) + 1 : 0; }();
         if (a.max_units == 0) a.max_units = env_slack;
         a.KC = kTileK;
-        const int tpr = a.K / kTileK, gpf = tpr >= 5 ? 1 : kFillTiles / tpr;
-        int jobs = (rows_total / kTileRows + gpf - 1) / gpf;
-        if (a.ksplit == 2 && a.epi == EPI_STORE && a.nseg == 1 && gemv_can_ksplit(a.K, a.seg[0].kc)) jobs *= 2; else a.ksplit = 0;
-        int grid = sm_count < jobs ? sm_count : jobs;
-        const size_t fixed = gemv_fixed_smem(a.K);
-        // One CTA per SM (576 threads).  Three stages (102 KiB in flight per SM) are enough to keep HBM busy; a deeper ring
-        // was measured slower (6 stages: -2.5 % tokens/s on the decode step, +8 % time on the kernel alone) — more claimed
-        // ahead by the CTAs that start first, more requests queued in the memory system.  LUM_GEMV_STAGES overrides.
-        int stages = 3;
-        static const int env_stages = [] { const char* e = getenv("LUM_GEMV_STAGES"); return e ? atoi(e) : 0; }();
-        if (env_stages > 0) stages = env_stages;
-        const int fit = (int)((226 * 1024 - (long)fixed) / kFillBytes);
-        if (stages > fit) stages = fit;
-        if (stages > kMaxStages) stages = kMaxStages;
-        if (stages < 2) stages = 2;
-        a.stages = stages;
-        const size_t smem = fixed + (size_t)stages * kFillBytes;
-        // two instantiations: with and without the tensor-parallel paths (partial vectors of other ranks in, peer stores out)
+        const bool ranges = a.ksplit > 1 && a.epi == EPI_STORE && a.nseg == 1 && a.ksplit <= gemv_k_ranges(a.K, a.seg[0].kc) && sm_count >= a.K / kTileK && !a.gain && !a.x_add && !a.n_parts && !a.x_out;
+        if (a.ksplit > 1 && !ranges) return cudaErrorInvalidValue;      // the caller's consumer expects that many partial vectors
+        const int tpr = a.K / kTileK;
+        a.k_smem = a.K;
+        int grid = sm_count;
+        if (ranges) {
+            int most = 0;
+            for (int r = 0; r < a.ksplit; r++) most = std::max(most, gemv_range_tile(tpr, a.ksplit, r + 1) - gemv_range_tile(tpr, a.ksplit, r));
+            a.k_smem = most * kTileK;
+        } else {
+            const int gpf = tpr > kFillTiles ? 1 : kJobTiles / tpr, jobs = (rows_total / kTileRows + gpf - 1) / gpf;
+            if (jobs < grid) grid = jobs;
+        }
+        const size_t fixed = gemv_fixed_smem(a.k_smem);
+        // Up to 4096 elements a CTA takes half an SM: rings of 75 to 91 KB.  So that the next projection's CTAs can only spread one to an SM, whatever
+        // order this one's leave in, every other projection asks for a little more than half (`wide_smem`): two of these don't fit an SM, nor
+        // do one and two of the others.  Longer vectors take an SM to themselves.
+        constexpr size_t kHalf = 109 * 1024 - 256, kWide = 114 * 1024, kAll = 226 * 1024;
+        const int tiles = a.k_smem / kTileK;
+        GemvRings rings{1, 1, kFillTiles, kFillTiles};
+        if (tiles > kFillTiles && tiles < kJobTiles) rings.t1 = tiles - kFillTiles;
+        const size_t room = fixed + 4 * kFillBytes <= kHalf ? kHalf : kAll;
+        for (int i = 0; i < 2 * 3 - 2; i++) {                // in turn, up to three stages each
+            GemvRings more = rings;
+            (more.n0 > more.n1 ? more.n1 : more.n0)++;
+            if (fixed + more.bytes() > room) break;
+            rings = more;
+        }
+        if (const size_t need = fixed + rings.bytes(); need > kAll) return cudaErrorInvalidValue;
+        a.ring_n[0] = rings.n0; a.ring_n[1] = rings.n1; a.ring_t[0] = rings.t0; a.ring_t[1] = rings.t1;
+        const int fills = (a.epi == EPI_SWIGLU ? 2 : 1) * ((tiles + kJobTiles - 1) / kJobTiles);          // of a job, in the first ring
+        a.own_jobs = a.job_ctr ? rings.n1 / fills : 0;
+        size_t smem = fixed + rings.bytes();
+        if (a.wide_smem && smem < kWide) smem = kWide;
+        // instantiations: with and without the tensor-parallel paths (partial vectors of other ranks in, peer stores out); a tile of the row group per warp, or any K
         const bool peer = a.n_peers > 0 || a.parts_ll || a.part_flags != nullptr || a.epi == EPI_PEER;
-        // One instantiation serves every K: alternating between a narrow and a wide kernel costs more in instruction-cache
-        // misses than the narrow one saves (measured: 415 against 439 tokens/s); the narrow one stays for models whose
-        // every projection is short.
-        static const int env_narrow = [] { const char* e = getenv("LUM_GEMV_NARROW"); return e ? atoi(e) : 0; }();
-        const bool wide = env_narrow == 0 || a.K > 2 * kWorkers * 4;      // more than two float4 per worker thread
-        const void* fn = peer ? (wide ? (const void*)q8_gemv_stream<true, true> : (const void*)q8_gemv_stream<true, false>)
-                              : (wide ? (const void*)q8_gemv_stream<false, true> : (const void*)q8_gemv_stream<false, false>);
+        const int fewest = ranges ? tpr / a.ksplit : tpr;
+        const bool one = fewest > kFillTiles && tiles <= kJobTiles;
+        const void* fn = peer ? (one ? (const void*)q8_gemv_stream<true, true> : (const void*)q8_gemv_stream<true, false>)
+                              : (one ? (const void*)q8_gemv_stream<false, true> : (const void*)q8_gemv_stream<false, false>);
         static std::atomic<uint64_t> raised[4] = {};
-        if (const cudaError_t e = allow_smem(raised[(peer ? 2 : 0) + (wide ? 1 : 0)], fn, 226 * 1024)) return e;
-        if (smem > 226 * 1024) return cudaErrorInvalidValue;
+        if (const cudaError_t e = allow_smem(raised[(peer ? 2 : 0) + one], fn, (int)kAll, true)) return e;
         return launch_with_attrs(fn, dim3(grid), dim3(kGemvThreads), smem, st, a.use_pdl != 0, a);
     }
 
-    if (a.ksplit == 2) return cudaErrorInvalidValue;     // the caller's consumer expects two partial vectors: only the streaming kernel makes them
+    if (a.ksplit > 1) return cudaErrorInvalidValue;      // the caller's consumer expects several partial vectors: only the streaming kernel makes them
     // direct kernel: a few CTAs per SM's worth of rows, at least 8 rows per CTA; a large bf16 / f32 matrix gets as many CTAs as
     // an SM can hold, so that enough loads are in flight to keep HBM busy
     int grid = sm_count * (a.wkind != WK_Q8 && (long long)rows_total * a.K >= (1ll << 24) ? (a.wkind == WK_BF16 ? kDirectBf16Ctas : 8) : 2);

@@ -1,26 +1,27 @@
 // Device-side building blocks of the streaming Q8_0 matrix-vector product, shared by the one-op
 // kernel (lum_gemv.cu) and the whole-token persistent kernel (lum_mega.cu).  A "phase" is one
-// y = W x over one CTA's share of the weight stream.  Three kinds of warps cooperate through
-// mbarriers:
+// y = W x over one CTA's share of the weight stream.  Two kinds of warps cooperate through mbarriers:
 //
-//   producer warp      gemv_produce()    one lane arms ring stages and issues one bulk copy (up to 8
-//                                        tiles, 34 KiB) per stage.
-//   tensor-core warp   gemv_mma_issue()  one lane waits for a stage to land and issues one tcgen05.mma
-//                                        (kind::i8, M = 128, N = 48, K = 32) per tile: the weights go from
-//                                        shared memory into the tensor core without passing through
-//                                        registers, the exact int32 dot products land in tensor memory.
-//   draining warps     gemv_consume()    all 16 worker warps quantise x into three int8 levels (the B
-//                                        operand); then 8 of them read the accumulators back (tcgen05.ld),
-//                                        apply the block scales in f32, reduce row sums in a fixed order
-//                                        and run the epilogue (store / residual add / SwiGLU / greedy sample).
+//   producer warp    gemv_produce()   one lane arms ring stages and issues one bulk copy (up to 4 tiles, 17 KiB) per stage.
+//   consumer warps   gemv_consume()   eight warps quantise x into three int8 levels, then take a tile each off the ring: the
+//                                     int8 weights go from shared memory through mma.sync.m16n8k32 against the levels as they
+//                                     are, exact int32 sums land in registers; the block scales are applied in f32, rows are
+//                                     reduced in a fixed order and the epilogue (store / residual add / SwiGLU / greedy
+//                                     sample) runs on the finished rows.
 //
-// Why the tensor core for a matrix-vector product: Q8_0 has one scale per 32 weights, so the arithmetic
-// per weight outside the integer multiply-add is small, but the multiply-adds themselves (three per weight,
-// one per activation level) cost the CUDA cores about 0.75 half-rate dp4a issue slots per weight — roughly
-// the time HBM needs to deliver the weight.  One M128 N48 K32 instruction does the 12288 useful (and 184320
-// ignored) multiply-adds of a tile in a few dozen cycles; per weight the draining threads are left with
-// 1/32 of an int->float conversion and a handful of FMAs, so they catch up quickly after every stall (grid
-// barrier, attention, prologue) and the weight stream from HBM is the only thing that takes time.
+// What bounds it: HBM while weights stream, and between two phases the time from the previous one's last row to this one's
+// first: hand-over, activations, first tiles.  A CTA therefore takes half an SM (288 threads, 112 registers, 110 KB), so that
+// under programmatic dependent launch the next phase's CTA is set up and has its ring full of weights while this one still
+// works.  The form before it, tcgen05 kind::i8 over 576 threads and 512 columns of tensor memory, had an SM to itself: the next
+// phase could not ask for a byte before it was gone.  The legacy tensor path is the right one here: a tile is 8 rows, one
+// vector fills 2 of an instruction's 8 columns, and accumulators in registers need no hand-over to a draining warp.
+//
+// Arithmetic.  Q8_0 has one scale per 32 weights.  Converting int8 -> f32 costs a quarter-rate instruction per weight, which caps an SM near
+// 29 weights a clock, barely above the 23 it must sustain at full HBM speed.  So the activations move to the integer side without
+// giving up their f32 precision: each 32-block of x is written as
+//     x ~= s * (a1 + a2/254 + a3/254^2),   a1, a2, a3 int8 vectors, s = max|x| / 127
+// (three successive int8 roundings of the residual; |error| <= max|x| * 2^-24 per element, the order of f32 rounding).  A block
+// then contributes d * s * (q.a1 + (q.a2)/254 + (q.a3)/254^2), d = the block's binary16 scale, with the three dot products exact.
 //
 // The ring keeps running across phases, so in the persistent kernel the producer streams the next
 // operation's weights while the other warps are still finishing (or waiting for the grid-wide
@@ -37,52 +38,51 @@
 namespace lum {
 
 
-constexpr int kWorkers = 512;            // 16 worker warps: activation prologue, attention (persistent kernel); warps 0-7 also drain the accumulators
-constexpr int kConsumers = 256;          // the first 8 worker warps = two warpgroups, each owning one tensor-memory slot
-constexpr int kProducerWarp = 16;        // issues the bulk copies
-constexpr int kMmaWarp = 17;             // owns tensor memory and issues the tensor-core instructions
-constexpr int kGemvThreads = 576;
+constexpr int kConsumers = 256;          // eight consumer warps: activation prologue, tiles, epilogue
+constexpr int kGemvThreads = kConsumers + 32;   // and the producer warp
 constexpr int kTileK = 512;              // columns of one tile = 16 blocks of 32
 constexpr int kTileRows = 8;             // weight rows of one tile (a "row group")
-constexpr int kTileQ = 4096;             // int8 bytes of one tile: 128 (block, row) pairs x 32 quants, in tensor-core operand order
-constexpr int kTileBytes = kTileQ + 256; // + the 128 binary16 scales of those pairs
-constexpr int kFillTiles = 8;            // tiles per ring stage
+constexpr int kTileQ = 4096;             // int8 bytes of one tile: block b, row r at b * 256 + (byte / 16) * 128 + r * 16 + byte % 16
+constexpr int kTileBytes = kTileQ + 256; // + the 128 binary16 scales, entry b * 8 + r
+constexpr int kFillTiles = 4;            // tiles per ring stage, at most: one for each of the four warps that share a ring
+constexpr int kJobTiles = 2 * kFillTiles;   // tiles one turn of both rings holds
 constexpr int kFillBytes = kFillTiles * kTileBytes;
-constexpr int kBarBytes = 640;           // mbarriers (320 B), then 64 words of reduction scratch
+constexpr int kBarBytes = 640;           // mbarriers, 64 words of reduction scratch at 384
 constexpr int kMaxStages = 16;
 constexpr int kChunkRG = 16;             // row groups whose sums are held before an epilogue pass (>= 2 x 8: one SwiGLU job of one-tile rows)
 constexpr int kRedFloats = kChunkRG * 64;   // [slot][consumer warp][row]
-constexpr int kValsFloats = kChunkRG * 8;
 constexpr int kMetaEnd = -1;
-constexpr int kTmemCols = 512;           // all of an SM's tensor memory: 2 slots x 4 tiles x 64 columns (48 used per tile)
-constexpr int kMmaN = 48;                // accumulator columns per tile: 16 blocks x 3 activation levels
-constexpr int kXqTileBytes = 1536;       // activation bytes per tile: 48 operand rows x 32
+constexpr int kXqTileBytes = 1536;       // operand bytes of x per tile: 512 columns x 3 levels
 
-// fields of meta2[stage]
-constexpr uint32_t kM2JobEnd = 1u << 16, kM2Up = 1u << 17, kM2First = 1u << 18, kM2Half = 1u << 19;
-constexpr int kUnitHalf = 1 << 30;        // unit_of[]: the slot holds the second K half of its row group
-__device__ __forceinline__ uint32_t m2_pack(int ntiles, int c0, int n_rg, bool job_end, int part, bool first, int half) {
-    return (uint32_t)ntiles | ((uint32_t)c0 << 4) | ((uint32_t)n_rg << 12) | (job_end ? kM2JobEnd : 0u) | (part ? kM2Up : 0u) |
-           (first ? kM2First : 0u) | (half ? kM2Half : 0u);
+// fields of meta[stage].y: tiles of the fill, its first tile, row groups of the job part, flags
+constexpr uint32_t kM2JobEnd = 1u << 16, kM2Up = 1u << 17, kM2First = 1u << 18;
+__device__ __forceinline__ uint32_t m2_pack(int ntiles, int c0, int n_rg, bool job_end, int part, bool first) {
+    return (uint32_t)ntiles | ((uint32_t)c0 << 4) | ((uint32_t)n_rg << 12) | (job_end ? kM2JobEnd : 0u) | (part ? kM2Up : 0u) | (first ? kM2First : 0u);
 }
+// The two rings of a CTA: stages [0, n0) belong to consumer warps 0-3, [n0, n0 + n1) to warps 4-7; a stage of ring w holds t_w tiles.
+struct GemvRings {
+    int n0, n1, t0, t1;
+    __host__ __device__ int stages() const { return n0 + n1; }
+    __host__ __device__ size_t bytes() const { return (size_t)(n0 * t0 + n1 * t1) * kTileBytes; }
+};
 
 // Shared-memory carve-up used by a streaming phase.
 struct GemvSmem {
     uint32_t full0, empty0;      // per-stage mbarriers (shared-space addresses): bytes landed / stage released
-    uint32_t tfull0, tempty0;    // accumulators of a fill written (tcgen05.commit) / read back by all 8 draining warps
-    uint32_t xready, mdone, fin; // activations quantised (per phase) / (unused) / last instruction retired
-    uint32_t tmem_slot;          // where tcgen05.alloc leaves the base address
     float* scratch;              // 64 words
-    int8_t* xq;                  // activations as a tensor-core operand: rows (block, level), 32 bytes each, core-matrix order
+    unsigned char* xq;           // activations as the B operand: per tile [4][24 lanes][16 B], see gemv_load_xfrag
     float* xsc;                  // K / 32 block scales of x
     float* red;                  // kRedFloats
-    float* vals;                 // kValsFloats
     int* unit_of;                // kChunkRG: global row-group id held in each local slot of the current chunk
     int* pair_of;                // kChunkRG: SwiGLU: slot of the matching up rows (gate slots) or -1 (up slots)
+    int* span_of;                // kChunkRG: the consumer warps that hold sums of the slot: first | number << 8
     int2* meta;                  // kMaxStages: x = first row-group id of the fill in each ring stage, or kMetaEnd;
                                  //             y = tiles / first tile / row groups / flags of the fill (m2_pack)
-    unsigned char* stage0;       // ring of `stages` x kFillBytes, 128-byte aligned
-    int stages;
+    unsigned char* stage0;       // the rings, 128-byte aligned
+    GemvRings rings;
+    __device__ int first(int w) const { return w ? rings.n0 : 0; }
+    __device__ int count(int w) const { return w ? rings.n1 : rings.n0; }
+    __device__ unsigned char* at(int w, int st) const { return stage0 + (size_t)(w ? rings.n0 * rings.t0 + st * rings.t1 : st * rings.t0) * kTileBytes; }
     volatile int* abort;         // CTA-wide: a wait ran out of budget; stop waiting, finish fast
 };
 
@@ -90,44 +90,25 @@ struct GemvSmem {
 // barriers (activation operand, scales, reduction scratch) is at least this large, for a caller that borrows it between
 // phases (the persistent kernel's attention).
 __host__ __device__ inline size_t gemv_fixed_smem(int K, size_t scratch_bytes = 0) {
-    const size_t area = (size_t)K * 3 + (size_t)(K / 32) * 4 + (size_t)kRedFloats * 4 + (size_t)kValsFloats * 4;
-    return (size_t)kBarBytes + (area > scratch_bytes ? area : scratch_bytes) + (size_t)(2 * kChunkRG + 2 * kMaxStages) * 4 + 256;
+    const size_t area = (size_t)K * 3 + (size_t)(K / 32) * 4 + (size_t)kRedFloats * 4;
+    return (size_t)kBarBytes + (area > scratch_bytes ? area : scratch_bytes) + (size_t)(3 * kChunkRG + 2 * kMaxStages) * 4 + 256;
 }
 
-__device__ __forceinline__ void gemv_carve(unsigned char* smem, int K, int stages, volatile int* abort, GemvSmem* g, size_t scratch_bytes = 0) {
+__device__ __forceinline__ void gemv_carve(unsigned char* smem, int K, const GemvRings& rings, volatile int* abort, GemvSmem* g, size_t scratch_bytes = 0) {
     g->full0 = smem_u32(smem);
     g->empty0 = g->full0 + 8u * kMaxStages;
-    g->tfull0 = g->empty0 + 8u * kMaxStages;
-    g->tempty0 = g->tfull0 + 16u;
-    g->xready = g->tempty0 + 16u;
-    g->mdone = g->xready + 8u;
-    g->fin = g->mdone + 8u;
-    g->tmem_slot = g->fin + 8u;
     g->scratch = (float*)(smem + 384);
-    g->xq = (int8_t*)(smem + kBarBytes);
+    g->xq = smem + kBarBytes;
     g->xsc = (float*)(g->xq + 3 * (size_t)K);
     g->red = g->xsc + (K >> 5);
-    g->vals = g->red + kRedFloats;
-    g->unit_of = (int*)(g->vals + kValsFloats);
-    if ((size_t)((unsigned char*)g->unit_of - (unsigned char*)g->xq) < scratch_bytes) g->unit_of = (int*)((unsigned char*)g->xq + ((scratch_bytes + 15) & ~(size_t)15));
+    g->unit_of = (int*)(g->red + kRedFloats);
+    if ((size_t)((unsigned char*)g->unit_of - g->xq) < scratch_bytes) g->unit_of = (int*)(g->xq + ((scratch_bytes + 15) & ~(size_t)15));
     g->pair_of = g->unit_of + kChunkRG;
-    g->meta = (int2*)(g->pair_of + kChunkRG);
+    g->span_of = g->pair_of + kChunkRG;
+    g->meta = (int2*)(g->span_of + kChunkRG);
     g->stage0 = (unsigned char*)(((uintptr_t)(g->meta + kMaxStages) + 127) & ~(uintptr_t)127);
-    g->stages = stages;
+    g->rings = rings;
     g->abort = abort;
-}
-
-__device__ __forceinline__ void gemv_init_barriers(const GemvSmem& g) {
-    for (int s = 0; s < g.stages; s++) {
-        mbar_init(g.full0 + 8u * s, 1);
-        mbar_init(g.empty0 + 8u * s, kConsumers / 32);       // the 8 draining warps (they arrive after the tensor core has retired the stage's instructions)
-    }
-    mbar_init(g.tfull0, 1);
-    mbar_init(g.tempty0, kConsumers / 32);
-    mbar_init(g.xready, kWorkers / 32);
-    mbar_init(g.mdone, 1);
-    mbar_init(g.fin, 1);
-    mbar_fence_init();
 }
 
 __device__ __forceinline__ float load_gain(const void* g, int kind, int i) {
@@ -160,37 +141,35 @@ __device__ __forceinline__ void argbest_take(ArgBest& b, float ov, int oi) {
 }
 
 // Epilogue over the finished row groups of a chunk: slot s holds row group unit_of[s] (rows unit_of[s] * 8 ..), its 8 row
-// sums at vals[s*8 ..].  Plain phases: row group ids count over the concatenated segments.  SwiGLU phases: gate slots carry
-// the slot of the matching up rows in pair_of[s] (up slots carry -1) and only they produce output.
+// sums vals(s*8 ..).  Plain phases: row group ids count over the concatenated segments.  SwiGLU phases: gate slots carry
+// the slot of the matching up rows, pair_of(s) (up slots carry -1) and only they produce output.
 // For EPI_ARGMAX the rows are stored and thread 0 folds the chunk's best into *best.
 // PEER = false compiles the tensor-parallel paths out: the kernel's code size is latency (it has to stay well inside the
-// instruction cache: measured, 100 KB -> 135 KB of code cost 12 % tokens/s on one GPU).
-template <bool PEER = false>
-__device__ __forceinline__ void gemv_epilogue_units(const GemvArgs& a, const float* vals, const int* unit_of, const int* pair_of, int n_slots,
-                                                    int tid, int nthreads, float* scratch, int bar_id, ArgBest* best) {
+// instruction cache: measured, 100 KB -> 135 KB of code cost 12 % tokens/s on one GPU).  `range`: the K range of the sums (GemvArgs::ksplit).
+template <bool PEER = false, typename Vals, typename Pair>
+__device__ __forceinline__ void gemv_epilogue_units(const GemvArgs& a, Vals vals, const int* unit_of, Pair pair_of, int n_slots,
+                                                    int tid, int nthreads, float* scratch, int bar_id, ArgBest* best, size_t range) {
     const int n = n_slots * kTileRows;
     if (a.epi == EPI_SWIGLU) {
         for (int i = tid; i < n; i += nthreads) {
-            const int sl = i >> 3, r = i & 7, pr = pair_of[sl];
-            if (pr >= 0) a.y[unit_of[sl] * kTileRows + r] = swiglu(vals[i], vals[pr * kTileRows + r]);
+            const int sl = i >> 3, r = i & 7, pr = pair_of(sl);
+            if (pr >= 0) a.y[unit_of[sl] * kTileRows + r] = swiglu(vals(i), vals(pr * kTileRows + r));
         }
     } else if (a.epi == EPI_STORE) {
         for (int i = tid; i < n; i += nthreads) {
-            const int u = unit_of[i >> 3];
-            float* y = (u & kUnitHalf) ? a.y + a.y_half_stride : a.y;
-            const int row = (u & (kUnitHalf - 1)) * kTileRows + (i & 7);
-            y[row] = (a.bias && !(u & kUnitHalf)) ? vals[i] + load_gain(a.bias, a.gain_kind, row) : vals[i];
+            const int row = unit_of[i >> 3] * kTileRows + (i & 7);
+            a.y[range * a.y_range_stride + row] = (a.bias && range == 0) ? vals(i) + load_gain(a.bias, a.gain_kind, row) : vals(i);
         }
     } else if (a.epi == EPI_RESID) {
         for (int i = tid; i < n; i += nthreads) {
             const int row = unit_of[i >> 3] * kTileRows + (i & 7);
-            const float v = a.bias ? vals[i] + load_gain(a.bias, a.gain_kind, row) : vals[i];
+            const float v = a.bias ? vals(i) + load_gain(a.bias, a.gain_kind, row) : vals(i);
             a.y[row] = a.resid[row] + v;
         }
     } else if (PEER && a.epi == EPI_PEER) {
         for (int i = tid; i < n; i += nthreads) {
             const int row = unit_of[i >> 3] * kTileRows + (i & 7);
-            const float v = vals[i];
+            const float v = vals(i);
             if (a.peer_ll) {
                 const uint32_t word = peer_word(__ldcg(a.seq), a.peer_tag);
 #pragma unroll
@@ -206,7 +185,7 @@ __device__ __forceinline__ void gemv_epilogue_units(const GemvArgs& a, const flo
         ArgBest b{-INFINITY, -1};
         for (int i = tid; i < n; i += nthreads) {
             const int row = unit_of[i >> 3] * kTileRows + (i & 7);
-            const float v = vals[i];
+            const float v = vals(i);
             a.y[row] = v;
             argbest_take(b, v, row);
         }
@@ -394,205 +373,206 @@ static __device__ __noinline__ float4 ll_load4(const uint2* p, uint32_t word, ui
 }
 
 // The RMSNorm gains do not depend on the previous operation, so a kernel can fetch them while it still waits for its
-// grid dependency: thread tid keeps the gains of the elements it will quantise (trip it: float4 number it * kWorkers + tid).
-constexpr int kXTrips = 8;                  // K <= 16384: at most 8 float4 per worker thread
+// grid dependency: thread tid keeps the gains of the first elements it will quantise (gemv_f4 of turn 0).
+constexpr int kXTrips = 4;                  // float4 of x a consumer thread holds at a time: 4096 elements per CTA, a tile per warp
+// number of the it-th float4 that a thread takes in turn b
+__device__ __forceinline__ int gemv_f4(int tid, int b, int it) { return b * (kXTrips * kConsumers) + (tid >> 5) * (kTileK / 4) + it * 32 + (tid & 31); }
 struct GainRegs { uint2 b[kXTrips]; bool loaded; };
-template <int TRIPS = kXTrips>
 __device__ __forceinline__ void gemv_gain_preload(const GemvArgs& a, int tid, GainRegs& gr) {
     gr.loaded = a.gain != nullptr && a.gain_kind == WK_BF16;
     if (!gr.loaded) return;
     const int n4 = a.K >> 2;
 #pragma unroll
-    for (int it = 0; it < TRIPS; it++) {
-        const int f4 = it * kWorkers + tid;
+    for (int it = 0; it < kXTrips; it++) {
+        const int f4 = gemv_f4(tid, 0, it);
         gr.b[it] = f4 < n4 ? ((const uint2*)a.gain)[f4] : make_uint2(0u, 0u);
     }
 }
 
-// Prologue: activations (optionally RMS-normalised, times the gains) -> three int8 levels + one f32 scale per 32-block
-// (x ~= s * (a1 + a2/254 + a3/254^2)), written as the B operand of the tensor-core instruction: operand row 3 * block + level
-// holds that level's 32 bytes, rows grouped by 8 into core matrices (two per group: bytes 0-15 and 16-31 of each row).
-// Runs on all kWorkers threads; 8 consecutive threads own one block.  Every thread first issues all of its loads (the
-// vector sits in L2, a microsecond away: one round trip, not one per trip), keeps them in registers for both passes, and
-// ends with the writes published to the tensor core (xready) and to the other workers (named barrier 1).
-// TRIPS: float4 loads per worker thread the code is built for (K <= 2048 * TRIPS): a kernel for short vectors carries a
-// quarter of the prologue's code.
-template <bool PEER = false, int TRIPS = kXTrips>
-__device__ __forceinline__ void gemv_quantize_x(const GemvArgs& a, const XSource& xs, bool is_writer, const GemvSmem& g, int tid, const GainRegs& gr) {
-    const int K = a.K, n4 = K >> 2;
-    auto load4 = [&](int f4) -> float4 {
-        float4 t;
-        if (xs.x) {
-            t = ((const float4*)xs.x)[f4];
-        } else if (xs.table_kind == WK_BF16) {
-            const uint2 r = ((const uint2*)((const uint16_t*)xs.table + (size_t)xs.token * K))[f4];
-            t.x = __uint_as_float(r.x << 16); t.y = __uint_as_float(r.x & 0xffff0000u);
-            t.z = __uint_as_float(r.y << 16); t.w = __uint_as_float(r.y & 0xffff0000u);
-        } else {
-            t = ((const float4*)((const float*)xs.table + (size_t)xs.token * K))[f4];
+// How a phase's matrices are cut into jobs.
+//   A matrix [N, K] (K a multiple of 512, N of 8) is a stream of tiles: row group rg = rows [8 rg, 8 rg + 8), tile t of it =
+//   columns [512 t, 512 t + 512); tiles of a row group are consecutive, row groups follow each other.  tpr = K / 512.
+//   A CTA works on the tiles [t0, t0 + nt) of every row group it takes: all of them, or (ksplit) one of the K ranges, which the
+//   CTAs share out in proportion to their tiles.  A job is what one CTA must do as a whole: one row group, with nt <= 4 as many (gpf) as make up to
+//   8 tiles; for SwiGLU the same of the gate matrix followed by the same of the up matrix.  A job part is cut into fills of up to 4
+//   tiles, which go to the two rings in turn (a part of one fill sends the second ring an empty one: both see every job).
+struct GemvPlan {
+    int tpr, t0, nt, gpf, sub;
+    int range;        // which K range this CTA works on, cta / n_cta: its number among that range's CTAs
+    int cta, n_cta;
+    int J;            // jobs in the phase (of this range)
+    int js;           // jobs every CTA owns without claiming: c, c + n_cta, ..; the others, from js * n_cta on, are claimed
+    int seg_job0[4];  // first job of each segment (plain phases)
+    int seg_rg0[4];   // first global row-group id of each segment
+    int nrg[3];       // row groups per segment
+};
+__device__ __forceinline__ GemvPlan gemv_plan(const GemvArgs& a, int cta, int n_cta, int own_permille) {
+    GemvPlan p;
+    p.tpr = a.K / kTileK;
+    p.range = 0; p.cta = cta; p.n_cta = n_cta; p.t0 = 0; p.nt = p.tpr;
+    if (a.ksplit > 1) {
+        for (int r = 0; r < a.ksplit; r++) {
+            const int b0 = gemv_range_tile(p.tpr, a.ksplit, r), b1 = gemv_range_tile(p.tpr, a.ksplit, r + 1);
+            const int c0 = b0 * n_cta / p.tpr, c1 = b1 * n_cta / p.tpr;
+            if (cta >= c0 && cta < c1) { p.range = r; p.cta = cta - c0; p.n_cta = c1 - c0; p.t0 = b0; p.nt = b1 - b0; }
         }
-        return t;
-    };
-    float4 xv[TRIPS];
-    constexpr int kSmallTrips = 2, kPartBatch = 4;
-    if (n4 <= kSmallTrips * kWorkers && (xs.n_parts > 0 || xs.x_add)) {
-        // A short vector made of several terms (residual stream + partial vectors of the ranks or of the K halves + a plain
-        // addend): few registers per term, so every term's loads are in flight together — one trip to L2 instead of one per
-        // term.  What does not depend on the other ranks is requested before their words are waited for.  The sums are formed
-        // in the same order as below: x, the parts in rank order, the addend.
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 ua[kSmallTrips];
+    }
+    p.gpf = p.nt > kFillTiles ? 1 : kJobTiles / p.nt;
+    p.sub = a.epi == EPI_SWIGLU ? 2 : 1;
+    int jobs = 0, rgs = 0;
+    for (int i = 0; i < 3; i++) {
+        const int n = i < a.nseg ? a.seg[i].rows / kTileRows : 0;
+        p.nrg[i] = n;
+        p.seg_job0[i] = jobs;
+        p.seg_rg0[i] = rgs;
+        if (a.epi != EPI_SWIGLU || i == 0) { jobs += (n + p.gpf - 1) / p.gpf; rgs += n; }
+    }
+    p.seg_job0[3] = jobs;
+    p.seg_rg0[3] = rgs;
+    p.J = jobs;
+    // (a launch of one operation says how many it owns: those its rings hold)
+    p.js = own_permille >= 0 ? (int)((long long)p.J * own_permille / 1000 / p.n_cta) : min(a.own_jobs, p.J / p.n_cta);
+    return p;
+}
+
+// Prologue: activations (optionally RMS-normalised, times the gains) -> three int8 levels + one f32 scale per 32-block, laid out as
+// the B operand of the tensor-core instruction (gemv_load_xfrag).  Runs on the kConsumers threads; 8 consecutive threads own one
+// block, a warp a tile of every turn.  A thread issues the loads of up to four float4 (of every term) at once: the vector sits in L2, most of a microsecond away, and up
+// to 4096 elements take one trip and stay in registers for both passes.  Longer vectors go around again, twice when they are normalised.
+// x_out (if asked for) is the raw sum of the terms.  ONE: see gemv_consume.
+template <bool PEER, bool ONE>
+__device__ __forceinline__ void gemv_quantize_x(const GemvArgs& a, const XSource& xs, bool is_writer, const GemvPlan& p, const GemvSmem& g, int tid, const GainRegs& gr) {
+    const int f40 = p.t0 * (kTileK / 4), n4 = p.nt * (kTileK / 4);          // this CTA's columns
+    const int nb = ONE ? 1 : (n4 + kXTrips * kConsumers - 1) / (kXTrips * kConsumers);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (PEER && xs.n_parts > 0 && xs.part_flags) peer_wait_parts(xs.part_flags, xs.n_parts, xs.seq, xs.parts_tag, a.status, tid, kConsumers, 2);
+    float4 xv[kXTrips];
+    float ss = 0.0f, inv = 1.0f;
+    // with a norm: one turn over the vector for its squares, then one to quantise (the same registers when it fits them)
+#pragma unroll 1
+    for (int step = a.gain ? 0 : nb; step < 2 * nb; step++) {
+        const bool quant = step >= nb;
+        const int b = quant ? step - nb : step;
+        if (!(quant && a.gain && nb == 1)) {
+            constexpr int kPartBatch = 2;
 #pragma unroll
-        for (int it = 0; it < TRIPS; it++) xv[it] = zero;
-#pragma unroll
-        for (int it = 0; it < kSmallTrips; it++) {
-            const int f4 = it * kWorkers + tid;
-            xv[it] = f4 < n4 ? load4(f4) : zero;
-            ua[it] = (xs.x_add && f4 < n4) ? ((const float4*)xs.x_add)[f4] : zero;
-        }
-        if (PEER && xs.n_parts > 0 && xs.part_flags) peer_wait_parts(xs.part_flags, xs.n_parts, xs.seq, xs.parts_tag, a.status, tid, kWorkers, 1);
-        if (PEER && xs.parts_ll) {
-            // every element carries its own completion word: all loads of two ranks' vectors go out together, stragglers are
-            // waited for one by one
-            const uint32_t word = peer_word(__ldcg(xs.seq), xs.parts_tag);
+            for (int it = 0; it < kXTrips; it++) {
+                const int f4 = gemv_f4(tid, b, it);
+                xv[it] = zero;
+                if (f4 < n4) {
+                    if (xs.x) {
+                        xv[it] = ((const float4*)xs.x)[f40 + f4];
+                    } else if (xs.table_kind == WK_BF16) {
+                        const uint2 r = ((const uint2*)((const uint16_t*)xs.table + (size_t)xs.token * a.K))[f4];
+                        xv[it] = make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xffff0000u));
+                    } else {
+                        xv[it] = ((const float4*)((const float*)xs.table + (size_t)xs.token * a.K))[f4];
+                    }
+                }
+            }
+            // the sums are formed in this order: x, the parts (ranks or K ranges) in theirs, the addend
+            if (PEER && xs.parts_ll) {
+                // every element carries its own completion word: the loads of two ranks' vectors go out together, stragglers are waited for one by one
+                const uint32_t word = peer_word(__ldcg(xs.seq), xs.parts_tag);
 #ifndef LUM_LL_BATCH
 #define LUM_LL_BATCH 2
 #endif
-            // ranks whose vectors are requested together.  Measured on 2 GPUs, same call: 1 -> 558.7, 2 -> 553.6, 4 -> 495.2 tokens/s
-            // (four ranks' loads in flight cost registers: the kernel spills); 2 is what the 4- and 8-GPU numbers were measured with
-            constexpr int kLLBatch = LUM_LL_BATCH;
+                // ranks whose vectors are requested together.  Measured on 2 GPUs, same call: 1 -> 558.7, 2 -> 553.6, 4 -> 495.2 tokens/s
+                // (four ranks' loads in flight cost registers: the kernel spills); 2 is what the 4- and 8-GPU numbers were measured with
+                constexpr int kLLBatch = LUM_LL_BATCH;
 #pragma unroll 1
-            for (int r0 = 0; r0 < xs.n_parts; r0 += kLLBatch) {
-                uint4 raw[kLLBatch][kSmallTrips][2];
+                for (int r0 = 0; r0 < xs.n_parts; r0 += kLLBatch) {
+                    uint4 raw[kLLBatch][kXTrips][2];
 #pragma unroll
-                for (int j = 0; j < kLLBatch; j++) {
-                    const uint2* pr = (const uint2*)xs.parts + (size_t)min(r0 + j, xs.n_parts - 1) * xs.part_stride;
+                    for (int j = 0; j < kLLBatch; j++) {
+                        const uint2* pr = (const uint2*)xs.parts + (size_t)min(r0 + j, xs.n_parts - 1) * xs.part_stride;
 #pragma unroll
-                    for (int it = 0; it < kSmallTrips; it++) {
-                        const int f4 = min(it * kWorkers + tid, n4 - 1);
-                        raw[j][it][0] = ld_ll2(pr + 4 * f4);
-                        raw[j][it][1] = ld_ll2(pr + 4 * f4 + 2);
+                        for (int it = 0; it < kXTrips; it++) {
+                            const int f4 = min(gemv_f4(tid, b, it), n4 - 1);
+                            raw[j][it][0] = ld_ll2(pr + 4 * f4);
+                            raw[j][it][1] = ld_ll2(pr + 4 * f4 + 2);
+                        }
                     }
-                }
 #pragma unroll
-                for (int j = 0; j < kLLBatch; j++) {
-                    if (r0 + j < xs.n_parts) {
-                        const uint2* pr = (const uint2*)xs.parts + (size_t)(r0 + j) * xs.part_stride;
+                    for (int j = 0; j < kLLBatch; j++) {
+                        if (r0 + j < xs.n_parts) {
+                            const uint2* pr = (const uint2*)xs.parts + (size_t)(r0 + j) * xs.part_stride;
 #pragma unroll
-                        for (int it = 0; it < kSmallTrips; it++) {
-                            const int f4 = it * kWorkers + tid;
-                            if (f4 < n4) {
-                                const uint4 a4 = raw[j][it][0], b4 = raw[j][it][1];
-                                float4 v = make_float4(__uint_as_float(a4.x), __uint_as_float(a4.z), __uint_as_float(b4.x), __uint_as_float(b4.z));
-                                if (a4.y != word || a4.w != word || b4.y != word || b4.w != word) v = ll_load4(pr + 4 * f4, word, a.status, a.wait_cycles);
-                                xv[it].x += v.x; xv[it].y += v.y; xv[it].z += v.z; xv[it].w += v.w;
+                            for (int it = 0; it < kXTrips; it++) {
+                                const int f4 = gemv_f4(tid, b, it);
+                                if (f4 < n4) {
+                                    const uint4 a4 = raw[j][it][0], b4 = raw[j][it][1];
+                                    float4 v = make_float4(__uint_as_float(a4.x), __uint_as_float(a4.z), __uint_as_float(b4.x), __uint_as_float(b4.z));
+                                    if (a4.y != word || a4.w != word || b4.y != word || b4.w != word) v = ll_load4(pr + 4 * f4, word, a.status, a.wait_cycles);
+                                    xv[it].x += v.x; xv[it].y += v.y; xv[it].z += v.z; xv[it].w += v.w;
+                                }
                             }
                         }
                     }
                 }
-            }
-        } else {
+            } else {
 #pragma unroll 1
-        for (int r0 = 0; r0 < xs.n_parts; r0 += kPartBatch) {
-            float4 u[kPartBatch][kSmallTrips];
+                for (int r0 = 0; r0 < xs.n_parts; r0 += kPartBatch) {
+                    float4 u[kPartBatch][kXTrips];
 #pragma unroll
-            for (int j = 0; j < kPartBatch; j++) {
-                const float4* pr = (const float4*)(xs.parts + (size_t)(r0 + j) * xs.part_stride);
+                    for (int j = 0; j < kPartBatch; j++) {
+                        const float4* pr = (const float4*)(xs.parts + (size_t)(r0 + j) * xs.part_stride);
 #pragma unroll
-                for (int it = 0; it < kSmallTrips; it++) {
-                    const int f4 = it * kWorkers + tid;
-                    u[j][it] = (r0 + j < xs.n_parts && f4 < n4) ? __ldcg(pr + f4) : zero;     // written by other GPUs / CTAs: read around L1
-                }
-            }
+                        for (int it = 0; it < kXTrips; it++) {
+                            const int f4 = gemv_f4(tid, b, it);
+                            u[j][it] = (r0 + j < xs.n_parts && f4 < n4) ? __ldcg(pr + f4) : zero;     // written by other GPUs / CTAs: read around L1
+                        }
+                    }
 #pragma unroll
-            for (int j = 0; j < kPartBatch; j++) {
-                if (r0 + j < xs.n_parts) {
+                    for (int j = 0; j < kPartBatch; j++) {
+                        if (r0 + j < xs.n_parts) {
 #pragma unroll
-                    for (int it = 0; it < kSmallTrips; it++) { xv[it].x += u[j][it].x; xv[it].y += u[j][it].y; xv[it].z += u[j][it].z; xv[it].w += u[j][it].w; }
-                }
-            }
-        }
-        }
-        if (xs.x_add) {
-#pragma unroll
-            for (int it = 0; it < kSmallTrips; it++) { xv[it].x += ua[it].x; xv[it].y += ua[it].y; xv[it].z += ua[it].z; xv[it].w += ua[it].w; }
-        }
-    } else {
-        if (PEER && xs.n_parts > 0 && xs.part_flags) peer_wait_parts(xs.part_flags, xs.n_parts, xs.seq, xs.parts_tag, a.status, tid, kWorkers, 1);
-#pragma unroll
-        for (int it = 0; it < TRIPS; it++) {
-            const int f4 = it * kWorkers + tid;
-            xv[it] = f4 < n4 ? load4(f4) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        if (xs.n_parts > 0) {
-            // written by other GPUs into this GPU's memory: read around L1; rank order, so every rank forms the same sums
-#pragma unroll 1
-            for (int r = 0; r < xs.n_parts; r++) {
-                const float4* pr = (const float4*)(xs.parts + (size_t)r * xs.part_stride);
-#pragma unroll
-                for (int it = 0; it < TRIPS; it++) {
-                    const int f4 = it * kWorkers + tid;
-                    if (f4 < n4) {
-                        const float4 u = (PEER && xs.parts_ll) ? ll_load4((const uint2*)xs.parts + (size_t)r * xs.part_stride + 4 * f4, peer_word(__ldcg(xs.seq), xs.parts_tag), a.status, a.wait_cycles)
-                                                     : __ldcg(pr + f4);
-                        xv[it].x += u.x; xv[it].y += u.y; xv[it].z += u.z; xv[it].w += u.w;
+                            for (int it = 0; it < kXTrips; it++) { xv[it].x += u[j][it].x; xv[it].y += u[j][it].y; xv[it].z += u[j][it].z; xv[it].w += u[j][it].w; }
+                        }
                     }
                 }
             }
-        }
-        if (xs.x_add) {
+            if (xs.x_add) {
 #pragma unroll
-            for (int it = 0; it < TRIPS; it++) {
-                const int f4 = it * kWorkers + tid;
-                if (f4 < n4) { const float4 u = ((const float4*)xs.x_add)[f4]; xv[it].x += u.x; xv[it].y += u.y; xv[it].z += u.z; xv[it].w += u.w; }
+                for (int it = 0; it < kXTrips; it++) {
+                    const int f4 = gemv_f4(tid, b, it);
+                    if (f4 < n4) { const float4 u = ((const float4*)xs.x_add)[f4]; xv[it].x += u.x; xv[it].y += u.y; xv[it].z += u.z; xv[it].w += u.w; }
+                }
+            }
+            if (xs.x_out && is_writer && (!quant || !a.gain)) {
+#pragma unroll
+                for (int it = 0; it < kXTrips; it++) {
+                    const int f4 = gemv_f4(tid, b, it);
+                    if (f4 < n4) ((float4*)xs.x_out)[f4] = xv[it];
+                }
             }
         }
-    }
-    if (xs.x_out && is_writer) {
+        if (!quant) {
 #pragma unroll
-        for (int it = 0; it < TRIPS; it++) {
-            const int f4 = it * kWorkers + tid;
-            if (f4 < n4) ((float4*)xs.x_out)[f4] = xv[it];
-        }
-    }
-    float inv = 1.0f;
-    if (a.gain) {
-        float ss = 0.0f;
-#pragma unroll
-        for (int it = 0; it < TRIPS; it++) {      // absent trips hold zeros
-            const float4 t = xv[it];
-            ss = fmaf(t.x, t.x, ss); ss = fmaf(t.y, t.y, ss); ss = fmaf(t.z, t.z, ss); ss = fmaf(t.w, t.w, ss);
-        }
-        ss = block_sum(ss, g.scratch, tid, kWorkers, 1, false);   // the prologue ends in a barrier before anything touches the scratch again
-        const float mean = ss * (1.0f / (float)(a.k_norm > 0 ? a.k_norm : K));
-        inv = 1.0f / sqrtf(mean + a.eps);
-    }
-    // all threads run every trip so the 8-lane shuffles always have their partners (K is a multiple of 32: a block never
-    // straddles the end); trips past the end of the vector are skipped as a whole warp
-    // The loop is unrolled by two only — the kernel's code size is latency (measured: the decode step of a model with tiny
-    // projections takes 961 us with this loop rolled against 1226 us with all eight trips unrolled; on the Llama-3-8B shape
-    // rolled 437.6, by two 442.2, by eight 439 tokens/s) — and picks its trip's registers with selects, so the loaded values
-    // never leave the register file.
-    const int trips = (n4 + kWorkers - 1) / kWorkers;
-#pragma unroll 2
-    for (int it = 0; it < TRIPS; it++) {
-        if (it < trips) {
-            const int f4 = it * kWorkers + tid;
-            const bool in = f4 < n4;
-            float4 cur = xv[0];
-            uint2 gb = gr.b[0];
-#pragma unroll
-            for (int k = 1; k < TRIPS; k++) {
-                if (it == k) { cur = xv[k]; gb = gr.b[k]; }
+            for (int it = 0; it < kXTrips; it++) {      // absent elements hold zeros
+                const float4 t = xv[it];
+                ss = fmaf(t.x, t.x, ss); ss = fmaf(t.y, t.y, ss); ss = fmaf(t.z, t.z, ss); ss = fmaf(t.w, t.w, ss);
             }
-            float e[4] = {cur.x, cur.y, cur.z, cur.w};
-            if (a.gain && in) {
+            if (b == nb - 1) {
+                ss = block_sum(ss, g.scratch, tid, kConsumers, 2, false);   // the prologue ends in a barrier before anything touches the scratch again
+                const float mean = ss * (1.0f / (float)(a.k_norm > 0 ? a.k_norm : a.K));
+                inv = 1.0f / sqrtf(mean + a.eps);
+            }
+            continue;
+        }
+#pragma unroll
+        for (int it = 0; it < kXTrips; it++) {
+            const int f4 = gemv_f4(tid, b, it);
+            if (f4 >= n4) continue;                      // n4 is a multiple of 128: a warp is in or out as a whole
+            float e[4] = {xv[it].x, xv[it].y, xv[it].z, xv[it].w};
+            if (a.gain) {
                 if (gr.loaded) {
+                    const uint2 gb = b == 0 ? gr.b[it] : ((const uint2*)a.gain)[f40 + f4];
                     e[0] = (inv * e[0]) * __uint_as_float(gb.x << 16); e[1] = (inv * e[1]) * __uint_as_float(gb.x & 0xffff0000u);
                     e[2] = (inv * e[2]) * __uint_as_float(gb.y << 16); e[3] = (inv * e[3]) * __uint_as_float(gb.y & 0xffff0000u);
                 } else {
-#pragma unroll
-                    for (int j = 0; j < 4; j++) e[j] = (inv * e[j]) * load_gain(a.gain, a.gain_kind, f4 * 4 + j);
+                    const float4 gf = ((const float4*)a.gain)[f40 + f4];
+                    e[0] = (inv * e[0]) * gf.x; e[1] = (inv * e[1]) * gf.y; e[2] = (inv * e[2]) * gf.z; e[3] = (inv * e[3]) * gf.w;
                 }
             }
             float amax = fmaxf(fmaxf(fabsf(e[0]), fabsf(e[1])), fmaxf(fabsf(e[2]), fabsf(e[3])));
@@ -619,259 +599,153 @@ __device__ __forceinline__ void gemv_quantize_x(const GemvArgs& a, const XSource
                 p2 |= (__float_as_uint(t2) & 0xffu) << (8 * j);
                 p3 |= (__float_as_uint(t3) & 0xffu) << (8 * j);
             }
-            if (in) {
-                const int blk = f4 >> 3, j0 = (f4 & 7) << 2;                 // this thread's 4 bytes: columns j0..j0+3 of block blk
-                const int inner = ((j0 >> 4) << 7) + (j0 & 15);
-                const int n1 = 3 * blk, n2 = n1 + 1, n3 = n1 + 2;              // operand rows of the three levels
-                *(uint32_t*)(g.xq + ((n1 >> 3) << 8) + ((n1 & 7) << 4) + inner) = p1;
-                *(uint32_t*)(g.xq + ((n2 >> 3) << 8) + ((n2 & 7) << 4) + inner) = p2;
-                *(uint32_t*)(g.xq + ((n3 >> 3) << 8) + ((n3 & 7) << 4) + inner) = p3;
-                if ((tid & 7) == 0) g.xsc[blk] = s1;
-            }
+            // block -> (tile, half of the tile, number in it): columns of the operand are (half, level); see gemv_load_xfrag
+            const int blk = f4 >> 3, j = f4 & 7, i = blk & 7;
+            uint32_t* dst = (uint32_t*)(g.xq + (size_t)(blk >> 4) * kXqTileBytes + (i >> 1) * 384 + (((blk >> 3) & 1) * 12 + (j & 3)) * 16 + (i & 1) * 8 + (j >> 2) * 4);
+            dst[0] = p1; dst[16] = p2; dst[32] = p3;
+            if ((tid & 7) == 0) g.xsc[blk] = s1;
         }
     }
-    fence_proxy_async_smem();
-    __syncwarp();
-    if ((tid & 31) == 0) mbar_arrive(g.xready);
-    named_sync(1, kWorkers);
-}
-
-// How a phase's matrices are cut into jobs.
-//   A matrix [N, K] (K a multiple of 512, N of 8) is a stream of tiles: row group rg = rows [8 rg, 8 rg + 8), tile t of it =
-//   columns [512 t, 512 t + 512); tiles of a row group are consecutive, row groups follow each other.  tpr = K / 512.
-//   A fill (one ring stage, one bulk copy) is up to 8 consecutive tiles: with tpr >= 5 a slice of one row group, otherwise
-//   gpf = 8 / tpr whole row groups.  A job is what one CTA must do as a whole: the fills of one row group (gpf == 1) or one
-//   fill of gpf row groups; for SwiGLU the same for the gate matrix followed by the same for the up matrix.
-struct GemvPlan {
-    int tpr, gpf, sub;
-    int ks;           // 2: every row group is two jobs, one per K half (long single matrices only)
-    int J;            // jobs in the phase
-    int js;           // jobs statically owned by every CTA: CTA c has [c*js, (c+1)*js)
-    int pool0;        // first pooled job: [pool0, J) are claimed dynamically (or, without a counter, split statically)
-    int seg_job0[4];  // first job of each segment (plain phases)
-    int seg_rg0[4];   // first global row-group id of each segment
-    int nrg[3];       // row groups per segment
-};
-__device__ __forceinline__ GemvPlan gemv_plan(const GemvArgs& a, int n_cta, bool dynamic) {
-    GemvPlan p;
-    p.tpr = a.K / kTileK;
-    p.gpf = p.tpr >= 5 ? 1 : kFillTiles / p.tpr;
-    p.sub = a.epi == EPI_SWIGLU ? 2 : 1;
-    p.ks = (a.ksplit == 2 && a.epi == EPI_STORE && a.nseg == 1 && gemv_can_ksplit(a.K, a.seg[0].kc)) ? 2 : 1;
-    int jobs = 0, rgs = 0;
-    for (int i = 0; i < 3; i++) {
-        const int n = i < a.nseg ? a.seg[i].rows / kTileRows : 0;
-        p.nrg[i] = n;
-        p.seg_job0[i] = jobs;
-        p.seg_rg0[i] = rgs;
-        if (a.epi != EPI_SWIGLU || i == 0) { jobs += (n + p.gpf - 1) / p.gpf * p.ks; rgs += n; }
-    }
-    p.seg_job0[3] = jobs;
-    p.seg_rg0[3] = rgs;
-    p.J = jobs;
-    if (dynamic) {
-        const int permille = a.debug > 0 ? a.debug - 1 : 750;   // statically owned share (a.debug carries a tuning override)
-        p.js = (int)((long long)p.J * permille / 1000 / n_cta);
-        p.pool0 = p.js * n_cta;
-    } else {
-        p.js = 0;                                            // everything in the "pool", split evenly by CTA index
-        p.pool0 = 0;
-    }
-    return p;
+    if (ONE) __syncwarp();                               // a warp multiplies by what it wrote itself
+    else named_sync(2, kConsumers);
 }
 
 // Ring positions, carried across phases.
-struct ProducerRing { int stage; uint32_t par; long long armed; };
-struct ConsumerRing { int stage; uint32_t par; uint32_t tpar; uint32_t ppar; };          // tpar: accumulator hand-over parity; ppar: phase parity
-struct MmaRing { int stage; uint32_t par; uint32_t tpar; uint32_t busy; uint32_t xpar; };   // busy: accumulators issued and not yet known drained
+struct ProducerRing { int stage[2]; uint32_t par[2]; long long armed[2]; };
+struct ConsumerRing { int stage; uint32_t par; };
 
-// Producer side of one phase: ONE lane (lane 0 of the producer warp) walks this CTA's static jobs, then claims pooled
-// jobs with atomicAdd on *job_ctr (the next claim is always in flight while the current job is being issued), and
-// closes the phase with an END marker stage.  With job_ctr == null the pool is split evenly by CTA index instead.
+// Producer side of one phase: ONE lane of the producer warp walks this CTA's own jobs, then claims others
+// with atomicAdd on *job_ctr (two claims are in flight while a job is being issued: one takes about as long as a job), and
+// closes the phase with an END marker in each ring.  With job_ctr == null the jobs are split evenly by CTA index instead.
 // Returns false if a wait ran out of budget (or the CTA is already aborting).
-__device__ __forceinline__ bool gemv_produce(const GemvArgs& a, const GemvPlan& p, const GemvSmem& g, ProducerRing& r, int cta, int n_cta,
+__device__ __forceinline__ bool gemv_produce(const GemvArgs& a, const GemvPlan& p, const GemvSmem& g, ProducerRing& r,
                                              unsigned int* job_ctr, uint32_t* status) {
-    const int S = g.stages;
-    auto next_stage = [&]() -> bool {        // wait until the ring position is free
+    // tiles > 0: a copy of them; 0: nothing to copy (an empty fill, the END marker)
+    auto emit = [&](int w, const unsigned char* src, int tiles, int unit, uint32_t m2) -> bool {
+        const int slot = g.first(w) + r.stage[w];
         if (*g.abort) return false;
-        if (!mbar_wait_abortable(g.empty0 + 8u * r.stage, r.par ^ 1u, g.abort)) {
+        if (!mbar_wait_abortable(g.empty0 + 8u * slot, r.par[w] ^ 1u, g.abort)) {        // until the ring position is free
             if (!*g.abort) { atomicOr(status, LUM_ST_WAIT_EMPTY); *g.abort = 1; }
             return false;
         }
-        return true;
-    };
-    auto advance = [&]() { r.armed++; if (++r.stage == S) { r.stage = 0; r.par ^= 1u; } };
-    auto emit = [&](const unsigned char* src, int ntiles, int c0, int n_rg, int rg_global, bool job_end, int part, bool first, int half) -> bool {
-        if (!next_stage()) return false;
-        const uint32_t fb = g.full0 + 8u * r.stage;
-        const uint32_t bytes = (uint32_t)ntiles * kTileBytes;
-        g.meta[r.stage] = make_int2(rg_global, (int)m2_pack(ntiles, c0, n_rg, job_end, part, first, half));
-        mbar_arrive_expect_tx(fb, bytes);
-        bulk_g2s(smem_u32(g.stage0 + (size_t)r.stage * kFillBytes), src, bytes, fb);
-        advance();
+        const uint32_t fb = g.full0 + 8u * slot;
+        g.meta[slot] = make_int2(unit, (int)m2);
+        if (tiles > 0) {
+            mbar_arrive_expect_tx(fb, (uint32_t)tiles * kTileBytes);
+            bulk_g2s(smem_u32(g.at(w, r.stage[w])), src, (uint32_t)tiles * kTileBytes, fb);
+        } else {
+            mbar_arrive(fb);
+        }
+        r.armed[w]++;
+        if (++r.stage[w] == g.count(w)) { r.stage[w] = 0; r.par[w] ^= 1u; }
         return true;
     };
     auto issue_job = [&](int j) -> bool {
-        if (p.ks == 2) {
-            // one K half of one row group: tiles [t0, t1)
-            const int rg = j >> 1, half = j & 1, t0 = half * (p.tpr >> 1), t1 = t0 + (p.tpr >> 1);
-            const unsigned char* base = (const unsigned char*)a.seg[0].w + (size_t)rg * p.tpr * kTileBytes;
-            for (int c = t0; c < t1; c += kFillTiles) {
-                const int nt = min(kFillTiles, t1 - c);
-                if (!emit(base + (size_t)c * kTileBytes, nt, c, 1, rg, c + kFillTiles >= t1, 0, c == t0, half)) return false;
-            }
-            return true;
-        }
         int sg = 0;
         if (a.epi != EPI_SWIGLU) while (sg < a.nseg - 1 && j >= p.seg_job0[sg + 1]) sg++;
         const int rg = (j - p.seg_job0[sg]) * p.gpf;                      // first row group of the job, inside its segment
-        const int n_rg = min(p.gpf, p.nrg[sg] - rg);
+        const int n_rg = min(p.gpf, p.nrg[sg] - rg), T = n_rg * p.nt;
+#pragma unroll 1
         for (int part = 0; part < p.sub; part++) {
-            const unsigned char* base = (const unsigned char*)a.seg[sg + part].w + (size_t)rg * p.tpr * kTileBytes;
+            const unsigned char* base = (const unsigned char*)a.seg[sg + part].w + ((size_t)rg * p.tpr + p.t0) * kTileBytes;
             const bool last_part = part == p.sub - 1;
-            if (p.tpr <= kFillTiles) {
-                if (!emit(base, n_rg * p.tpr, 0, n_rg, p.seg_rg0[sg] + rg, last_part, part, true, 0)) return false;
-            } else {
-                for (int c = 0; c < p.tpr; c += kFillTiles) {
-                    const int nt = min(kFillTiles, p.tpr - c);
-                    if (!emit(base + (size_t)c * kTileBytes, nt, c, 1, p.seg_rg0[sg] + rg, last_part && c + kFillTiles >= p.tpr, part, c == 0, 0)) return false;
-                }
+#pragma unroll 1
+            for (int c = 0; c < T; c += kJobTiles) {
+                const int c1 = c + kFillTiles;
+                if (!emit(0, base + (size_t)c * kTileBytes, min(kFillTiles, T - c), p.seg_rg0[sg] + rg, m2_pack(min(kFillTiles, T - c), c, n_rg, last_part && c + kJobTiles >= T, part, c == 0))) return false;
+                if (c > 0 && c1 >= T) break;
+                const int n1 = max(0, min(kFillTiles, T - c1));
+                if (!emit(1, base + (size_t)c1 * kTileBytes, n1, p.seg_rg0[sg] + rg, m2_pack(n1, c1, n_rg, last_part && c1 + kJobTiles >= T, part, c == 0))) return false;
             }
         }
         return true;
     };
 
-    const int npool = p.J - p.pool0;
-    unsigned int claim = 0;
-    if (job_ctr && npool > 0) claim = atomicAdd(job_ctr, 1u);               // first claim travels while the static part is issued
-    for (int j = cta * p.js; j < (cta + 1) * p.js; j++)
-        if (!issue_job(j)) return false;
     if (job_ctr) {
         // A CTA that starts early (its SM was free while the previous kernel still ran elsewhere) could fill its whole ring
         // with claims before the others have started, and then has to drain it alone after the grid dependency resolves:
         // measured on the o projection, the last CTA finished 3-5 us after the median.  So a CTA takes at most its even
         // share plus one; a claim is only made when it will be used.
-        const int cap = (p.J + n_cta - 1) / n_cta + (a.max_units > 0 ? a.max_units - 1 : 1) - p.js;   // a.max_units: tuning override of the slack
-        int taken = 0;
-        while ((int)claim < npool) {
-            const unsigned int nxt = taken + 1 < cap ? atomicAdd(job_ctr, 1u) : (unsigned int)npool;
-            if (!issue_job(p.pool0 + (int)claim)) return false;
-            taken++;
-            claim = nxt;
+        const unsigned int base = (unsigned int)(p.js * p.n_cta), none = (unsigned int)p.J;
+        const int cap = (p.J + p.n_cta - 1) / p.n_cta + (a.max_units > 0 ? a.max_units - 1 : 1) - p.js;   // a.max_units: tuning override of the slack
+        unsigned int c0 = none, c1 = none;
+        if (base < none && cap > 0) c0 = base + atomicAdd(job_ctr, 1u);     // these travel while the own jobs are issued
+        if (base < none && cap > 1) c1 = base + atomicAdd(job_ctr, 1u);
+        for (int i = 0; i < p.js; i++)
+            if (!issue_job(p.cta + i * p.n_cta)) return false;
+#pragma unroll 1
+        for (int taken = 2; c0 < none; taken++) {
+            const unsigned int nxt = taken < cap && c1 < none ? base + atomicAdd(job_ctr, 1u) : none;
+            if (!issue_job((int)c0)) return false;
+            c0 = c1; c1 = nxt;
         }
     } else {
-        const int j0 = p.pool0 + (int)((long long)cta * npool / n_cta), j1 = p.pool0 + (int)((long long)(cta + 1) * npool / n_cta);
-        for (int j = j0; j < j1; j++)
+#pragma unroll 1
+        for (int j = p.cta; j < p.J; j += p.n_cta)
             if (!issue_job(j)) return false;
     }
-    // END marker: a stage with no bytes
-    if (!next_stage()) return false;
-    g.meta[r.stage] = make_int2(kMetaEnd, 0);
-    mbar_arrive(g.full0 + 8u * r.stage);
-    advance();
-    return true;
+    return emit(0, nullptr, 0, kMetaEnd, 0u) && emit(1, nullptr, 0, kMetaEnd, 0u);
 }
 
 // After an aborted run: never leave the CTA while a copy into its shared memory may still be in flight.
 // Wait (bounded) for every fill armed in the last ring revolution to land.
 __device__ __forceinline__ void gemv_producer_drain(const GemvSmem& g, const ProducerRing& r, uint32_t* status) {
-    const int S = g.stages;
-    int st = r.stage;
-    uint32_t par = r.par;
-    const long long back = r.armed < S ? r.armed : S;
-    for (long long i = 0; i < back; i++) {
-        if (st == 0) { st = S; par ^= 1u; }
-        st--;
-        if (!mbar_wait(g.full0 + 8u * st, par)) { atomicOr(status, LUM_ST_WAIT_DRAIN); return; }
+    for (int w = 0; w < 2; w++) {
+        const int S = g.count(w);
+        int st = r.stage[w];
+        uint32_t par = r.par[w];
+        const long long back = r.armed[w] < S ? r.armed[w] : S;
+        for (long long i = 0; i < back; i++) {
+            if (st == 0) { st = S; par ^= 1u; }
+            st--;
+            if (!mbar_wait(g.full0 + 8u * (g.first(w) + st), par)) { atomicOr(status, LUM_ST_WAIT_DRAIN); return; }
+        }
     }
 }
 
-// Tensor-core side of one phase, run by ONE thread (lane 0 of the tensor-core warp).  For every fill that lands it issues
-// one tcgen05.mma per tile — A = the tile's 128 (block, row) vectors of 32 int8 weights straight from the ring stage,
-// B = the 48 activation rows (16 blocks x 3 levels) of the tile's K range, D = 128 lanes x 48 int32 columns of tensor
-// memory (tile i of the fill at column 64 i), overwritten — and has "accumulators written" signalled when they retire.
-// Lane (8 b + r) of tile t, column 3 b + l is the exact integer dot product of row r's block b with level l of the
-// matching activation block; the other 45 columns of a lane pair the weights with other blocks' activations and are
-// never read.  Measured on B200: an instruction of this shape occupies the tensor pipe for 40 (N 16) to 45 (N 48)
-// cycles, and tcgen05.ld issued while instructions are in flight completes only after they retire — so the fill's
-// instructions are issued back to back and the read-back follows as one burst, the two strictly alternating.
-__device__ __forceinline__ bool gemv_mma_issue(const GemvArgs& a, const GemvPlan& p, const GemvSmem& g, MmaRing& r, uint32_t tmem, uint32_t* status) {
-    const int S = g.stages;
-    auto fail = [&](uint32_t code) { if (!*g.abort) { atomicOr(status, code); *g.abort = 1; } return false; };
-    if (*g.abort) return false;
-    if (!mbar_wait_abortable(g.xready, r.xpar, g.abort)) return fail(LUM_ST_WAIT_TMEM);
-    r.xpar ^= 1u;
-    tc_fence_after_sync();
-    // operand descriptors: start address and lbo (128 B) in the low word, sbo (256 B) and the version in the high word
-    const uint32_t xq_lo = umma_desc_lo(smem_u32(g.xq), 128u);
-    const uint32_t st_lo = umma_desc_lo(smem_u32(g.stage0), 128u);
-    constexpr uint32_t hi = umma_desc_hi(256u);
-    constexpr uint32_t idesc = umma_idesc_s8(128, kMmaN);
-    const int tpr = p.tpr;
-    const bool wrap = p.gpf > 1;
-    for (;;) {
-        // the previous fill's accumulators must have been read back before they are overwritten; waiting for that first
-        // costs nothing while the next fill is still in flight
-        if (r.busy) {
-            if (!mbar_wait_abortable(g.tempty0, r.tpar, g.abort)) return fail(LUM_ST_WAIT_TMEM);
-            r.tpar ^= 1u;
-            r.busy = 0u;
-        }
-        if (!mbar_wait_abortable(g.full0 + 8u * r.stage, r.par, g.abort)) return fail(LUM_ST_WAIT_FULL);
-        const int2 mm = g.meta[r.stage];
-        const int u = mm.x;
-        if (u != kMetaEnd) {
-            const uint32_t m2 = (uint32_t)mm.y;
-            const int nt = (int)(m2 & 15u), c0 = (int)((m2 >> 4) & 255u);
-            uint32_t a_lo = st_lo + (uint32_t)r.stage * (kFillBytes >> 4);
-            uint32_t b_lo = xq_lo + (uint32_t)c0 * (kXqTileBytes >> 4);
-            tc_fence_after_sync();
-            if (nt == kFillTiles && !wrap) {
-                // the common case, straight-line: eight instructions, 45 cycles of the tensor pipe each
+// The operands of one tile.  A warp multiplies by m16n8k32 with the weights as A: rows 0-7 are the tile's 8 rows in block i, rows 8-15 the same
+// 8 rows in block 8 + i; ldmatrix brings a row's weights 4 t .. 4 t + 3 of each half of a block to lane (row, t) as the instruction wants them.
+// Column n = (half of the tile, level) of B holds that level of that half's block i (a half's fourth column repeats the third); the products of one half's rows with the
+// other half's columns, and of the fourth columns, are not read.  Lane (g, t) ends up with row g of block (t / 2) * 8 + i: levels 1 and 2 (t even) or level 3 (t odd).
+__device__ __forceinline__ void gemv_load_xfrag(const GemvSmem& g, int tile, int lane, uint32_t (&b)[4][4], float4& sx) {
+    const int n = lane >> 2;
+    const unsigned char* p = g.xq + (size_t)tile * kXqTileBytes + (((n >> 2) * 3 + min(n & 3, 2)) * 4 + (lane & 3)) * 16;
 #pragma unroll
-                for (int i = 0; i < kFillTiles; i++)
-                    umma_s8_ss_split(tmem + (uint32_t)(64 * i), a_lo + (uint32_t)i * (kTileBytes >> 4), b_lo + (uint32_t)i * (kXqTileBytes >> 4), hi, idesc);
-            } else {
-                uint32_t d = tmem;
-                int t = c0;                                  // the tile's position along K
-#pragma unroll 1
-                for (int i = 0; i < nt; i++) {
-                    umma_s8_ss_split(d, a_lo, b_lo, hi, idesc);
-                    d += 64u;
-                    a_lo += kTileBytes >> 4;
-                    b_lo += kXqTileBytes >> 4;
-                    if (wrap && ++t == tpr) { t = 0; b_lo = xq_lo; }
-                }
-            }
-            umma_commit(g.tfull0);
-        } else {
-            mbar_arrive(g.tfull0);                           // the END marker travels the same way, with nothing to read back
-        }
-        r.busy = 1u;                                         // every hand-over, END included, is answered on tempty
-        if (++r.stage == S) { r.stage = 0; r.par ^= 1u; }
-        if (u == kMetaEnd) break;
+    for (int s = 0; s < 4; s++) {
+        const uint4 v = *(const uint4*)(p + s * 384);
+        b[s][0] = v.x; b[s][1] = v.y; b[s][2] = v.z; b[s][3] = v.w;
     }
-    return true;
+    sx = *(const float4*)(g.xsc + tile * 16 + ((lane & 2) << 2) + ((lane & 1) << 2));
+}
+__device__ __forceinline__ void gemv_ldmatrix(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void gemv_mma(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
 
-// Consumer side of one phase, called by all kWorkers threads: quantise x (everyone), then the first kConsumers threads
-// take fills off the ring until the END marker.  Warpgroup w (4 warps = the 128 lanes of tensor memory) drains slot w:
-// thread (warp q, lane) owns lane 32 q + lane of every tile = block 4 q + lane / 8, row lane % 8, reads its three int32 dot
-// products, turns them into the block's f32 contribution and adds up its tiles; per fill and row group the 4 block-lanes
-// of a warp that share a row are folded with two shuffles and the 8 warps' partials are summed in a fixed order at the
-// end of a chunk, followed by the epilogue.  For EPI_ARGMAX, *best (thread 0) receives this CTA's best row.
-template <bool PEER = false, int TRIPS = kXTrips>
+// Consumer side of one phase, called by the kConsumers threads: quantise x, then take fills off this warp's ring until the END marker, a tile
+// of each fill.  A lane's share of a tile is one row in half of its blocks (even lanes: levels 1 and 2, odd ones: level 3), four lanes are folded with two
+// shuffles, the warps' sums wait in shared memory and are added in a fixed order at the end of a
+// chunk, followed by the epilogue.  For EPI_ARGMAX, *best (thread 0) receives this CTA's best row.
+// ONE: five to eight tiles per row group (K of 2049 to 4096, or a K range): a job part is one fill of each ring, a warp has the same tile of every
+// row group, whose columns it has quantised itself.  Most of what the loop does besides the tile falls away (270 -> 150 instructions a tile), and so does a barrier.
+template <bool PEER, bool ONE>
 __device__ __forceinline__ void gemv_consume(const GemvArgs& a, const XSource& xs, bool is_writer, const GemvPlan& p, const GemvSmem& g,
-                                             ConsumerRing& cr, int tid, uint32_t tmem, uint32_t* status, ArgBest* best, const GainRegs& gr) {
-    gemv_quantize_x<PEER, TRIPS>(a, xs, is_writer, g, tid, gr);
-    if (tid >= kConsumers) return;
-    const int lane = tid & 31, warp = tid >> 5, wg = warp >> 2, q = warp & 3;
-    const int S = g.stages, tpr = p.tpr;
-    const int kbl = (q << 2) + (lane >> 3);              // this thread's block inside a tile
-    const int m = (q << 5) + lane;                       // its tensor-memory lane = (block, row) index inside a tile
-    const uint32_t tlane = tmem + ((uint32_t)(q << 5) << 16) + (uint32_t)(256 * wg + 12 * q);
-    const int sel = lane >> 3;
-
+                                             ConsumerRing& cr, int tid, uint32_t* status, ArgBest* best, const GainRegs& gr) {
+    gemv_quantize_x<PEER, ONE>(a, xs, is_writer, p, g, tid, gr);
+    const int lane = tid & 31, warp = tid >> 5, wg = warp >> 2, wj = warp & 3;
+    const int S = g.count(wg), first = g.first(wg);
+    const uint32_t ring = smem_u32(g.at(wg, 0)) + (uint32_t)wj * kTileBytes + lane * 16, stride = (uint32_t)(wg ? g.rings.t1 : g.rings.t0) * kTileBytes;
+    const uint32_t sc0 = kTileQ - lane * 16 + ((lane & 2) << 6) + ((lane & 1) << 6) + ((lane >> 2) << 1);           // this lane's first block scale in a tile
+    float* const red = g.red + warp * 8 + (lane >> 2);
+    uint32_t b[4][4];
+    float4 sx;
+    const bool odd = lane & 1, low = lane & 2;
+    const int m1 = odd ? 1 : 254, m2c = odd ? 0 : 1;
+    int cur = -1;                                        // the tile position whose activations b holds
+    if (ONE && warp < p.nt) gemv_load_xfrag(g, warp, lane, b, sx);
     auto fail = [&](uint32_t code) { if (!*g.abort) { atomicOr(status, code); *g.abort = 1; } };
     int slot = 0, slot_base = 0;
     bool ended = false;
@@ -880,144 +754,104 @@ __device__ __forceinline__ void gemv_consume(const GemvArgs& a, const XSource& x
         slot = 0;
 #pragma unroll 1
         for (;;) {
-            // "accumulators written" is the wait that blocks.  The accumulators are read back first and the slot handed back at
-            // once — that hand-over paces the tensor core; everything else happens off that path.  All four tiles of the slot
-            // are read whether or not the fill has them (absent tiles leave stale integers that are never used; an END marker
-            // has nothing new at all), in four loads and one wait (65-100 cycles).
-            if (!mbar_wait_abortable(g.tfull0, cr.tpar, g.abort)) { fail(LUM_ST_WAIT_TMEM); ended = true; break; }
-            cr.tpar ^= 1u;
-            tc_fence_after_sync();
-            uint32_t va[16], vb[16], vc[16], vd[16];
-            tmem_ld16(tlane, va);
-            tmem_ld16(tlane + 64u, vb);
-            tmem_ld16(tlane + 128u, vc);
-            tmem_ld16(tlane + 192u, vd);
-            tmem_ld_wait();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(g.tempty0);
-            // The stage has landed (the tensor-core warp waited for it); observing its barrier here, complete at the first
-            // attempt, makes the bulk copy's bytes and the producer's meta word visible to this thread by the book.
-            if (!mbar_wait_abortable(g.full0 + 8u * cr.stage, cr.par, g.abort)) { fail(LUM_ST_WAIT_FULL); ended = true; break; }
-            const int2 mm = g.meta[cr.stage];
-            const int u = mm.x;
-            if (u == kMetaEnd) {
-                __syncwarp();
-                if (lane == 0) mbar_arrive(g.empty0 + 8u * cr.stage);
-                if (++cr.stage == S) { cr.stage = 0; cr.par ^= 1u; }
-                ended = true;
-                break;
-            }
+            const int st = first + cr.stage;
+            if (!mbar_wait_abortable(g.full0 + 8u * st, cr.par, g.abort)) { fail(LUM_ST_WAIT_FULL); ended = true; break; }
+            const int2 mm = g.meta[st];
             const uint32_t m2 = (uint32_t)mm.y;
-            const int nt = (int)(m2 & 15u), c0 = (int)((m2 >> 4) & 255u), n_rg = (int)((m2 >> 12) & 15u);
-            const unsigned char* st = g.stage0 + (size_t)cr.stage * kFillBytes;
-            const bool first = (m2 & kM2First) != 0;       // first fill of a job part: its row groups take new slots
-            if (first) {
+            const bool mine = ONE ? warp < p.nt && mm.x != kMetaEnd : wj < (int)(m2 & 15u);
+            const uint32_t wp = ring + (uint32_t)cr.stage * stride;
+            uint32_t wx[4][4], wy[4][4];
+            uint16_t dw[4];
+            if (mine) {
+#pragma unroll
+                for (int s = 0; s < 4; s++) {            // in the order they are multiplied
+                    gemv_ldmatrix(wp + ((s & 1) * 2 + (s >> 1)) * 512, wx[(s & 1) * 2 + (s >> 1)]);
+                    gemv_ldmatrix(wp + 2048 + ((s & 1) * 2 + (s >> 1)) * 512, wy[(s & 1) * 2 + (s >> 1)]);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) asm volatile("ld.shared.u16 %0, [%1];" : "=h"(dw[i]) : "r"(wp + sc0 + i * 16) : "memory");
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(g.empty0 + 8u * st);            // everything this warp needs of the stage is in its registers
+            if (++cr.stage == S) { cr.stage = 0; cr.par ^= 1u; }
+            if (mm.x == kMetaEnd) { ended = true; break; }
+            if (ONE) {
+                if (warp == 7 && lane == 0) g.unit_of[slot] = mm.x;
+                slot_base = slot++;
+            } else if (m2 & kM2First) {                  // first fill of a job part: its row groups take new slots
+                const int n_rg = (int)((m2 >> 12) & 15u);
                 slot_base = slot;
                 slot += n_rg;
-                if (tid < n_rg) {
-                    g.unit_of[slot_base + tid] = (u + tid) | ((m2 & kM2Half) ? kUnitHalf : 0);
-                    g.pair_of[slot_base + tid] = (m2 & kM2Up) ? -1 : slot_base + n_rg + tid;
+                if (warp == 7 && lane < n_rg) {          // (a warp with less to do wherever a row group has fewer than eight tiles)
+                    g.unit_of[slot_base + lane] = mm.x + lane;
+                    g.pair_of[slot_base + lane] = (m2 & kM2Up) ? -1 : slot_base + n_rg + lane;
+                    g.span_of[slot_base + lane] = (p.gpf > 1 ? lane * p.nt : 0) | min(p.nt, kJobTiles) << 8;
                 }
             }
-            // The only thing the draining warps need from the stage are their block scales: fetch them and release the stage
-            // (its quants were consumed by the tensor core before "accumulators written" was signalled).
-            float dw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            {
-                const __half* wsc = (const __half*)(st + (size_t)(4 * wg) * kTileBytes + kTileQ) + m;
+            if (mine) {
+                int sl = slot_base;
+                if (!ONE) {
+                    int t = (int)((m2 >> 4) & 255u) + wj;
+                    if (p.gpf > 1) { sl += t / p.nt; t %= p.nt; }
+                    if (t != cur) { gemv_load_xfrag(g, t, lane, b, sx); cur = t; }
+                }
+                float v = 0.0f;
+                // Lanes t and t ^ 1 hold levels 1, 2 and level 3 of the same row and blocks: of blocks i and i + 4 the even lane completes the first, the odd
+                // one the second.  Four instructions are issued before the first result is used.
 #pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (4 * wg + j < nt) dw[j] = __half2float(wsc[j * (kTileBytes / 2)]);
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(g.empty0 + 8u * cr.stage);
-            if (++cr.stage == S) { cr.stage = 0; cr.par ^= 1u; }
-            float val[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            if (4 * wg < nt) {
-#define LUM_SEL(v, o) (int)(sel == 0 ? v[o] : sel == 1 ? v[3 + o] : sel == 2 ? v[6 + o] : v[9 + o])
-                const int i1[4] = {LUM_SEL(va, 0), LUM_SEL(vb, 0), LUM_SEL(vc, 0), LUM_SEL(vd, 0)};
-                const int i2[4] = {LUM_SEL(va, 1), LUM_SEL(vb, 1), LUM_SEL(vc, 1), LUM_SEL(vd, 1)};
-                const int i3[4] = {LUM_SEL(va, 2), LUM_SEL(vb, 2), LUM_SEL(vc, 2), LUM_SEL(vd, 2)};
-#undef LUM_SEL
-                // the K position of this warpgroup's first tile (narrow matrices: tile index modulo tiles per row group)
-                int t = c0 + 4 * wg;
-                if (p.gpf > 1) t = t % tpr;
+                for (int h = 0; h < 2; h++) {
+                    int c[4][4];
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    if (4 * wg + j < nt) {
-                        const float sx = g.xsc[(t << 4) + kbl];
-                        t++;
-                        if (p.gpf > 1 && t == tpr) t = 0;
-                        // i1 * 254 + i2 fits an int32 (|i1| <= 32 * 127 * 127): one conversion fewer
-                        const float tt = fmaf((float)i3[j], 1.0f / 64516.0f, (float)(i1[j] * 254 + i2[j]) * (1.0f / 254.0f));
-                        val[j] = tt * (sx * dw[j]);
+                    for (int k = 0; k < 4; k++) {
+                        const int s = h + (k & 1) * 2, o = k & 2;                     // blocks 2 h, 2 h + 4, 2 h + 1, 2 h + 5
+                        gemv_mma(c[k], wx[s][o], wy[s][o], wx[s][o + 1], wy[s][o + 1], b[s][o], b[s][o + 1]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; k += 2) {
+                        // i1 * 254 + i2 fits an int32 (|i1| <= 32 * 128 * 127): one conversion for both
+                        const int qa = (low ? c[k][2] : c[k][0]) * m1 + (low ? c[k][3] : c[k][1]) * m2c;
+                        const int qb = (low ? c[k + 1][2] : c[k + 1][0]) * m1 + (low ? c[k + 1][3] : c[k + 1][1]) * m2c;
+                        const int got = __shfl_xor_sync(0xffffffffu, odd ? qa : qb, 1);
+                        const int i12 = odd ? got : qa, i3 = odd ? qb : got;
+                        const int i = 2 * h + (k >> 1);
+                        const float x = i == 0 ? sx.x : i == 1 ? sx.y : i == 2 ? sx.z : sx.w;
+                        const float tt = fmaf((float)i3, 1.0f / 64516.0f, (float)i12 * (1.0f / 254.0f));
+                        v = fmaf(tt, x * __half2float(__ushort_as_half(dw[i])), v);
                     }
                 }
+                v += __shfl_xor_sync(0xffffffffu, v, 1);
+                v += __shfl_xor_sync(0xffffffffu, v, 2);
+                if ((lane & 3) == 0) red[sl * 64] = ONE || (m2 & kM2First) ? v : red[sl * 64] + v;
             }
-            // fold this warp's tiles into the fill's row groups: lanes with equal (lane & 7) hold the same row
-            if (p.gpf == 1) {
-                float v = (val[0] + val[1]) + (val[2] + val[3]);
-                v += __shfl_xor_sync(0xffffffffu, v, 8);
-                v += __shfl_xor_sync(0xffffffffu, v, 16);
-                if (lane < 8) {
-                    float* dst = g.red + (size_t)slot_base * 64 + warp * 8 + lane;
-                    *dst = first ? v : *dst + v;
-                }
-            } else {
-#pragma unroll 1
-                for (int rgl = 0; rgl < n_rg; rgl++) {
-                    float v = 0.0f;
-#pragma unroll
-                    for (int j = 0; j < 4; j++) v += ((4 * wg + j) / tpr == rgl) ? val[j] : 0.0f;
-                    v += __shfl_xor_sync(0xffffffffu, v, 8);
-                    v += __shfl_xor_sync(0xffffffffu, v, 16);
-                    if (lane < 8) g.red[(size_t)(slot_base + rgl) * 64 + warp * 8 + lane] = v;
-                }
-            }
-            if ((m2 & kM2JobEnd) && slot + p.sub * p.gpf > kChunkRG) break;
+            if (ONE ? slot == kChunkRG : (m2 & kM2JobEnd) && slot + p.sub * p.gpf > kChunkRG) break;
         }
-        named_sync(2, kConsumers);
-        // fixed-order sum of the 8 warps' partials -> vals, then the epilogue for this chunk's row groups
-        for (int i = tid; i < slot * kTileRows; i += kConsumers) {
-            const float* rp = g.red + (size_t)(i >> 3) * 64 + (i & 7);
+        ended = named_or(2, kConsumers, ended);          // (a warp that gave up takes the others along: every barrier below stays attended)
+        // the warps' sums of a row, added in a fixed order, straight into the epilogue
+        auto sum = [&](int i) {
+            const int span = ONE ? p.nt << 8 : g.span_of[i >> 3];
+            const float* rp = g.red + (size_t)(i >> 3) * 64 + (span & 255) * 8 + (i & 7);
             float t = 0.0f;
 #pragma unroll
-            for (int w = 0; w < 8; w++) t += rp[w * 8];
-            g.vals[i] = t;
-        }
-        named_sync(2, kConsumers);
-        if (slot > 0) gemv_epilogue_units<PEER>(a, g.vals, g.unit_of, g.pair_of, slot, tid, kConsumers, g.scratch, 2, best);
-        named_sync(2, kConsumers);
+            for (int w = 0; w < 8; w++) if (w < (span >> 8)) t += rp[w * 8];
+            return t;
+        };
+        auto pair = [&](int sl) { return ONE ? (sl & 1 ? -1 : sl + 1) : g.pair_of[sl]; };
+        if (slot > 0) gemv_epilogue_units<PEER>(a, sum, g.unit_of, pair, slot, tid, kConsumers, g.scratch, 2, best, (size_t)p.range);
+        if (!ended) named_sync(2, kConsumers);
     }
-    // (The END marker reaches the draining warps through the tensor-core warp, so they cannot finish a phase before it has:
-    // the "activations quantised" barrier of the next phase never runs more than one phase ahead of its waiter.)
 }
 
-// Kernel start (all threads of the CTA): barriers, tensor memory.  Returns the tensor-memory base address.
-__device__ __forceinline__ uint32_t gemv_cta_begin(const GemvSmem& g, int tid, volatile int* abort_word) {
+// Kernel start (all threads of the CTA): barriers.
+__device__ __forceinline__ void gemv_cta_begin(const GemvSmem& g, int tid, volatile int* abort_word) {
     if (tid == 0) {
         *abort_word = 0;
-        gemv_init_barriers(g);
+        for (int s = 0; s < g.rings.stages(); s++) {
+            mbar_init(g.full0 + 8u * s, 1);
+            mbar_init(g.empty0 + 8u * s, kConsumers / 64);
+        }
+        mbar_fence_init();
     }
-    if ((tid >> 5) == kMmaWarp) tmem_alloc(g.tmem_slot, kTmemCols);
-    tc_fence_before_sync();
     __syncthreads();
-    tc_fence_after_sync();
-    uint32_t base;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(base) : "r"(g.tmem_slot));
-    return base;
-}
-// Kernel end.  The draining warps call gemv_consumers_done() after their last phase; the tensor-core warp calls
-// gemv_mma_end(), which waits (bounded) for the last instruction it issued, then for the draining warps, and frees tensor memory.
-__device__ __forceinline__ void gemv_consumers_done() { tc_fence_before_sync(); named_arrive(4, kConsumers + 32); }
-__device__ __forceinline__ void gemv_mma_end(const GemvSmem& g, uint32_t tmem, int lane, uint32_t* status) {
-    if (elect_one()) {
-        umma_commit(g.fin);
-        if (!mbar_wait(g.fin, 0u)) atomicOr(status, LUM_ST_WAIT_TMEM);
-    }
-    __syncwarp();
-    named_sync(4, kConsumers + 32);
-    tc_fence_after_sync();
-    tmem_dealloc(tmem, kTmemCols);
 }
 
 }  // namespace lum

@@ -69,16 +69,17 @@ struct GemvArgs {
     uint32_t* status;
     // geometry of the streaming kernel
     int KC;                // tile width of the packed layout (set by the launcher)
-    int stages;
+    int ring_n[2], ring_t[2];   // stages of the two rings and tiles per stage (set by the launcher)
+    int own_jobs;          // with job_ctr: jobs a CTA takes without claiming (set by the launcher)
+    int wide_smem;         // 1: ask for a little more than half an SM's shared memory (two such CTAs never share an SM)
+    int k_smem;            // activations a CTA holds: K, or the longest K range (set by the launcher)
     int max_units;         // tuning override: 1 + extra jobs a CTA may claim beyond its even share (0 = default)
     int use_pdl;
     int force_direct;      // 1: never take the streaming kernel (operator tests compare the two)
-    int debug;             // tuning override: 1 + permille of the jobs owned statically (0 = default)
-    unsigned int* job_ctr; // streaming kernel: zeroed counter the producers claim pooled jobs from (null: static split)
-    unsigned int* job_ctr_zero;   // optional: a counter of a launch far enough away in stream order, zeroed by CTA 0 for its next use
-    int ksplit;            // 2: EPI_STORE over one long-K matrix cut into two K halves per row group (twice the jobs, half the size);
-                           // half h's partial sums go to y + h * y_half_stride and the consumer of y adds the two vectors up
-    int y_half_stride;
+    unsigned int* job_ctr; // streaming kernel: zeroed counters the producers claim pooled jobs from, one per K range (null: static split)
+    int ksplit;            // > 1: EPI_STORE over one long-K matrix cut into that many K ranges, each worked on by its own CTAs (which then hold
+                           // that range's activations only); range r's partial sums go to y + r * y_range_stride, the consumer of y adds the vectors up
+    int y_range_stride;
     // Tensor parallel without a collective kernel.  Producing side (EPI_PEER): peer_out[r] is rank r's buffer for THIS rank's
     // partial vector (r == own rank included), peer_flag[r] the word in rank r's memory that says it is complete.
     float* peer_out[kMaxPeers];
@@ -157,6 +158,8 @@ struct EmbedArgs {
     const DecodeState* state;
     uint32_t* status;
     int use_pdl;
+    unsigned int* zero_ctr;// optional: n_zero words zeroed by this kernel (the step's job-claim counters: nothing of the previous step still runs, nothing of
+    int n_zero;            // this one starts before it is over)
     const double* pos_freq;// optional [ceil(H / 2)]: sin (entry 2i) and cos (2i + 1) of position * pos_freq[i] are added
 };
 // entries 2 i and 2 i + 1 of the sinusoidal position vector (angles in f64: exact to f32 rounding at any position)
@@ -178,8 +181,12 @@ __device__ __forceinline__ void embed_row_into(const void* table, int kind, int 
 // message of the last failed stand-alone operator on this thread (read back through lum_last_error(NULL))
 void set_op_error(const char* msg);
 
-// whether a [N, K] Q8_0 matrix (kc: its layout, see GemvSeg) can be run as two K halves per row group (GemvArgs::ksplit)
-__host__ __device__ inline bool gemv_can_ksplit(int K, int kc) { const int tpr = K / 512; return kc == 512 && K % 512 == 0 && tpr > 8 && (tpr & 1) == 0; }
+// How many K ranges a long-K Q8_0 matrix (kc: its layout, see GemvSeg) runs as (GemvArgs::ksplit; 1: not cut), and the first tile of range r.
+// Ranges of at most 4096 columns: a consumer thread then holds its share of the vector in registers, and a range's activations leave room
+// for two CTAs on an SM.
+constexpr int kMaxKRanges = 4;
+__host__ __device__ inline int gemv_k_ranges(int K, int kc) { const int tpr = K / 512, r = (tpr + 7) / 8; return kc == 512 && K % 512 == 0 && r <= kMaxKRanges ? (r > 1 ? r : 1) : 1; }
+__host__ __device__ inline int gemv_range_tile(int tpr, int ranges, int r) { return r * tpr / ranges; }
 
 // launchers (each returns the CUDA error of the launch)
 cudaError_t launch_gemv(const GemvArgs& a, int sm_count, cudaStream_t st);

@@ -16,9 +16,8 @@
 // stages full with bulk copies, regardless of where the consumer warps are.  While the consumers sit
 // in a grid barrier, run attention, or quantise the next activation vector, the producer is already
 // fetching the next operation's weights, so HBM never waits for a kernel boundary.  The multiply-adds
-// run on the tensor core (a third warp role, see lum_gemv_dev.cuh), which leaves the draining warps so
-// little to do per weight that they empty a full ring in a fraction of the time HBM took to fill it:
-// a stall is paid for only to the extent that it outlasts the ring.
+// run on the tensor core (lum_gemv_dev.cuh), so that the consumers empty a full ring in a fraction of the
+// time HBM took to fill it: a stall is paid for only to the extent that it outlasts the ring.
 #include <cstdlib>
 
 #include "lum_attn_dev.cuh"
@@ -34,8 +33,10 @@ namespace lum {
 // consumer threads; thread 0 arrives and waits, the rest wait on the named barrier.  The wait is bounded
 // (LUM_WAIT_BUDGET_CYCLES); once it runs out the kernel-wide abort flag is raised and every later wait
 // in every CTA returns at once.
+constexpr int kMegaWorkers = 512;        // attention, grid barriers; the first kConsumers of them are the consumers of the weight stream
+constexpr int kMegaThreads = kMegaWorkers + 32;
 __device__ __forceinline__ void grid_barrier(const MegaArgs& a, unsigned long long& seq, volatile int* cta_abort, int tid) {
-    named_sync(1, kWorkers);                        // all of this CTA's writes of the phase are issued
+    named_sync(1, kMegaWorkers);                        // all of this CTA's writes of the phase are issued
     if (tid == 0) {
         __threadfence();
         // gbar[0] counts arrivals; gbar[16] (its own 128-byte line, so polls do not queue behind the atomics) holds the
@@ -65,7 +66,7 @@ __device__ __forceinline__ void grid_barrier(const MegaArgs& a, unsigned long lo
         __threadfence();
     }
     seq++;
-    named_sync(1, kWorkers);
+    named_sync(1, kMegaWorkers);
 }
 
 __device__ __forceinline__ AttnArgs attn_phase_args(const MegaArgs& a, const MegaLayer& L, bool bf16) {
@@ -86,7 +87,7 @@ __device__ __forceinline__ void attn_phase_prefetch(const MegaArgs& a, const Meg
         const AttnArgs t = attn_phase_args(a, L, BF16);
         int r0, r1;
         attn_tc_range(t, (int)blockIdx.x % a.n_splits, pos, &r0, &r1);
-        attn_tc_prefetch<HD>(t, (int)blockIdx.x / a.n_splits, r0, r1, tid, kWorkers);
+        attn_tc_prefetch<HD>(t, (int)blockIdx.x / a.n_splits, r0, r1, tid, kMegaWorkers);
     }
 }
 template <int HD, int GM, bool BF16>
@@ -100,9 +101,9 @@ __device__ __noinline__ void attn_phase(const MegaArgs& a, const MegaLayer& L, u
         // token (32 layers of 32 / 8 heads of 128) behind 512 / 3000 rows: 5.13 / 5.68 with 128 workers and nothing asked for ahead, 4.89 / 5.28 this
         // way, 4.95 / 5.28 with a warp per key
         AttnTile<HD> f;
-        AttnPre<HD, kWorkers> pre;
-        attn_tc_pre<HD, kWorkers>(t, pre, kvh, split, tid >> 5, tid & 31);
-        attn_tc_body<HD, GM / 4, false, kWorkers, false>(t, scratch_smem, f, pre, kvh, split, pos, tid, 1, false);
+        AttnPre<HD, kMegaWorkers> pre;
+        attn_tc_pre<HD, kMegaWorkers>(t, pre, kvh, split, tid >> 5, tid & 31);
+        attn_tc_body<HD, GM / 4, false, kMegaWorkers, false>(t, scratch_smem, f, pre, kvh, split, pos, tid, 1, false);
     } else {
         attn_decode_body<HD, GM, BF16>(t, scratch_smem, kvh, split, pos, tid, 1);
     }
@@ -113,7 +114,7 @@ __device__ __noinline__ void attn_phase(const MegaArgs& a, const MegaLayer& L, u
 __device__ __forceinline__ bool phase_gemv(const MegaArgs& a, const MegaLayer& L, int p, GemvArgs* out) {
     const int H = a.hidden, qd = a.n_q * a.hd, kvd = a.n_kv * a.hd;
     GemvArgs g{};
-    g.wkind = WK_Q8; g.gain_kind = a.gain_kind; g.eps = a.eps; g.status = a.status; g.stages = a.stages;
+    g.wkind = WK_Q8; g.gain_kind = a.gain_kind; g.eps = a.eps; g.status = a.status;
     switch (p) {
         case 0:   // q, k, v projections (RMSNorm in the prologue)
             g.K = H; g.KC = a.kc_h; g.epi = EPI_STORE; g.nseg = 3;
@@ -145,22 +146,19 @@ __device__ __forceinline__ bool phase_gemv(const MegaArgs& a, const MegaLayer& L
 }
 
 template <int HD, int GM, bool BF16>
-__global__ void __launch_bounds__(kGemvThreads, 1) decode_mega(const MegaArgs a) {
+__global__ void __launch_bounds__(kMegaThreads, 1) decode_mega(const MegaArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_abort;
     __shared__ int s_tok;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int cta = (int)blockIdx.x, ncta = (int)gridDim.x;
     GemvSmem g;
-    gemv_carve(smem, a.k_max, a.stages, &s_abort, &g, attn_smem_bytes(HD, GM));
-    const uint32_t tmem = gemv_cta_begin(g, tid, &s_abort);
+    gemv_carve(smem, a.k_max, GemvRings{(a.stages + 1) / 2, a.stages / 2, kFillTiles, kFillTiles}, &s_abort, &g, attn_smem_bytes(HD, GM));
+    gemv_cta_begin(g, tid, &s_abort);
 
-    const bool is_producer = warp == kProducerWarp, is_mma = warp == kMmaWarp;
-    const bool is_worker = warp < kWorkers / 32;
-    ProducerRing pring{0, 0u, 0};
-    ConsumerRing cring{0, 0u, 0u, 0u};
-    MmaRing mring{0, 0u, 0u, 0u, 0u};
-    bool issuing = true;
+    const bool is_worker = warp < kMegaWorkers / 32, is_producer = !is_worker;
+    ProducerRing pring{};
+    ConsumerRing cring{0, 0u};
     unsigned long long seq = a.gbar_base;             // grid barriers passed so far
     unsigned long long pseq = a.gbar_base;            // running phase number: picks the job-claim counter of each phase
     bool producing = true;
@@ -172,7 +170,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) decode_mega(const MegaArgs a)
             // Refuse the whole launch the same way in every CTA (all read the same state): nothing was written yet.
             if (cta == 0 && tid == 0) atomicOr(a.status, pos < 0 || pos + a.n_tokens > a.max_seq ? LUM_ST_BAD_POS : LUM_ST_BAD_TOKEN);
             if (tid == 0) s_abort = 1;
-            named_sync(1, kWorkers);
+            named_sync(1, kMegaWorkers);
         }
     }
 
@@ -189,7 +187,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) decode_mega(const MegaArgs a)
             GemvArgs ga;
             const bool streams = phase_gemv(a, L, p, &ga);
             GemvPlan plan{};
-            if (streams) plan = gemv_plan(ga, ncta, true);
+            if (streams) plan = gemv_plan(ga, cta, ncta, 750);
             unsigned int* ctr = a.job_ctr + (pseq % kJobCtrRing);
             // Re-zero the claim counter that phase pseq + 32 will use: its last user was phase pseq - 32, and no CTA can
             // be that far behind or ahead (a producer leads its consumers by at most one ring of stages, each phase
@@ -198,10 +196,8 @@ __global__ void __launch_bounds__(kGemvThreads, 1) decode_mega(const MegaArgs a)
             pseq++;
             if (is_producer) {
                 if (streams && elect_one() && producing) {
-                    producing = gemv_produce(ga, plan, g, pring, cta, ncta, ctr, a.status);
+                    producing = gemv_produce(ga, plan, g, pring, ctr, a.status);
                 }
-            } else if (is_mma) {
-                if (streams && elect_one() && issuing) issuing = gemv_mma_issue(ga, plan, g, mring, tmem, a.status);
             } else if (!streams) {
                 // RoPE + cache append + attention
                 if (!s_abort) attn_phase<HD, GM, BF16>(a, L, (unsigned char*)g.xq, pos, tid);
@@ -212,10 +208,12 @@ __global__ void __launch_bounds__(kGemvThreads, 1) decode_mega(const MegaArgs a)
                 else xs.x = p == 2 ? a.attn : p == 4 ? a.h : a.x;
                 ArgBest best{-INFINITY, -1};
                 if (!s_abort) {
-                    GainRegs gr;
-                    gemv_gain_preload(ga, tid, gr);
                     if (p == 0) attn_phase_prefetch<HD, GM, BF16>(a, L, pos, tid);
-                    gemv_consume(ga, xs, cta == 0, plan, g, cring, tid, tmem, a.status, &best, gr);
+                    if (tid < kConsumers) {
+                        GainRegs gr;
+                        gemv_gain_preload(ga, tid, gr);
+                        gemv_consume<false, false>(ga, xs, cta == 0, plan, g, cring, tid, a.status, &best, gr);
+                    }
                 }
                 if (p == 5 && tid == 0) { a.part_val[cta] = best.v; a.part_idx[cta] = best.i; }
                 grid_barrier(a, seq, &s_abort, tid);
@@ -225,7 +223,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) decode_mega(const MegaArgs a)
                         const int fi = argmax_final(a.part_val, a.part_idx, ncta, lane).i;
                         if (lane == 0) s_tok = fi;
                     }
-                    named_sync(1, kWorkers);
+                    named_sync(1, kMegaWorkers);
                     const int sampled = s_abort ? 0 : max(0, s_tok);
                     if (cta == 0 && tid == 0 && !s_abort) {
                         DecodeState* st = a.state;
@@ -247,11 +245,6 @@ __global__ void __launch_bounds__(kGemvThreads, 1) decode_mega(const MegaArgs a)
         if (elect_one() && (s_abort || !producing)) gemv_producer_drain(g, pring, a.status);
         return;
     }
-    if (is_mma) {
-        gemv_mma_end(g, tmem, lane, a.status);
-        return;
-    }
-    if (tid < kConsumers) gemv_consumers_done();
     if (cta == 0 && tid == 0 && !s_abort) {
         a.state->pos = pos;
         a.state->tok = tok;
@@ -296,12 +289,12 @@ cudaError_t launch_mega(const MegaArgs& a_in, int sm_count, cudaStream_t st) {
     if (smem > 226 * 1024) return cudaErrorInvalidValue;
     // every CTA must be resident at once: the grid barrier relies on it
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kGemvThreads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kMegaThreads, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorLaunchOutOfResources;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sm_count);
-    cfg.blockDim = dim3(kGemvThreads);
+    cfg.blockDim = dim3(kMegaThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];

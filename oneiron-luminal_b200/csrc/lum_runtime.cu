@@ -192,6 +192,7 @@ struct lum_rt {
     SampleParams* d_sample = nullptr;   // device copy of `samp` (read by sample_rows: captured graphs stay valid when values change)
     SampleParams samp{1.0f, 1.0f, 1, 0, 0ull};
     bool sampling = false;              // false: the greedy sample of the head kernel / argmax_rows stands
+    int part_ld = 0;                  // floats between the K ranges of `part`
     bool down_ksplit = true;          // LUM_DOWN_KSPLIT=0: the down projection as one job per row group
     bool attn_cluster = false;        // the splits of a KV head merge through a thread-block cluster (LUM_ATTN_CLUSTER=0: global partials + arrival ticket)
     bool kv_prefetch = true;          // LUM_KV_PREFETCH=0: attention does not warm L2 with its cached rows before the projections finish
@@ -509,7 +510,7 @@ int check_status(lum_rt* rt) {
     if (st) {
         cudaMemsetAsync(rt->status, 0, sizeof st, rt->stream);
         // kernels that gave up may have left their arrival tickets and job-claim counters mid-count: start them over
-        if (rt->step_ctr) cudaMemsetAsync(rt->step_ctr, 0, ((size_t)4 * rt->d.n_layers + 1) * sizeof(unsigned int), rt->stream);
+        if (rt->step_ctr) cudaMemsetAsync(rt->step_ctr, 0, ((size_t)4 * rt->d.n_layers + 1) * kMaxKRanges * sizeof(unsigned int), rt->stream);
         if (rt->attn_cnt) cudaMemsetAsync(rt->attn_cnt, 0, (size_t)rt->nkv_l * 4, rt->stream);
         if (rt->am_cnt) cudaMemsetAsync(rt->am_cnt, 0, 4, rt->stream);
         if (rt->peer_ticket) cudaMemsetAsync(rt->peer_ticket, 0, 4, rt->stream);
@@ -579,14 +580,15 @@ int issue_step(lum_rt* rt, bool with_head, bool pdl, int* n_launch) {
         n++;
         return 0;
     };
-    // Dynamic job claiming: projection number gi of the step claims from its own counter, and re-zeroes the counter of the
-    // projection half a step away in stream order — used (and quiescent) long before, next used long after — so that every
-    // counter is zero again when its projection comes round in the next step.  The two maps (with and without the
-    // vocabulary projection) are both bijections that zero a counter either before its use in the same step or after it.
+    // Dynamic job claiming: projection number gi of the step claims from counters of its own, zeroed by the step's first kernel.
     const int n_proj = (d.n_experts > 0 ? 2 : 4) * d.n_layers + (with_head ? 1 : 0);     // streaming projections per step (routed experts have kernels of their own)
     int gi = 0;
+    bool prev_wide = false;             // the kernel before is a projection with the wide size
     auto claim_ctr = [&](GemvArgs& g) {
-        if (n_proj >= 8 && rt->step_ctr) { g.job_ctr = rt->step_ctr + gi; g.job_ctr_zero = rt->step_ctr + (gi + n_proj / 2) % n_proj; }
+        if (rt->step_ctr) g.job_ctr = rt->step_ctr + (size_t)gi * kMaxKRanges;
+        // Consecutive projections alternate between the two sizes of shared memory; behind a kernel of another kind the wide one
+        g.wide_smem = !prev_wide;
+        prev_wide = g.wide_smem != 0;
         gi++;
     };
     // Fused exchange (after lum_tp_peer_import): a K-sharded projection stores each finished row into every rank's buffer
@@ -596,7 +598,7 @@ int issue_step(lum_rt* rt, bool with_head, bool pdl, int* n_launch) {
     const bool fused = tp && rt->peers_open;
     uint32_t pending_tag = 0;
     int pending_buf = 0;
-    bool pending_halves = false;
+    int pending_ranges = 0;             // K ranges of the last down projection that have not joined the stream yet
     auto sym_flag = [&](unsigned char* base, int buf, int rank) { return (uint32_t*)(base + ((size_t)buf * kMaxPeers + rank) * 128); };
     // partial vectors as {value bits, completion word} pairs: 8 bytes per element
     auto sym_part = [&](unsigned char* base, int buf, int rank) { return (float*)(base + 4096) + ((size_t)buf * rt->tp_size + rank) * H * 2; };
@@ -613,9 +615,9 @@ int issue_step(lum_rt* rt, bool with_head, bool pdl, int* n_launch) {
         if (fused) {
             g.parts = sym_part(rt->sym, pending_buf, 0); g.part_flags = nullptr; g.parts_ll = 1;    // each element carries its own completion word
             g.n_parts = rt->tp_size; g.part_stride = H; g.parts_tag = pending_tag; g.seq = rt->tp_seq;
-        } else if (pending_halves) {
-            g.parts = rt->part; g.n_parts = 2; g.part_stride = H;      // the two K halves of the down projection (same GPU: no words to wait for)
-            pending_halves = false;
+        } else if (pending_ranges) {
+            g.parts = rt->part; g.n_parts = pending_ranges; g.part_stride = rt->part_ld;      // the K ranges of the down projection (same GPU: no words to wait for)
+            pending_ranges = 0;
         } else {
             g.x_add = rt->part;
         }
@@ -626,6 +628,7 @@ int issue_step(lum_rt* rt, bool with_head, bool pdl, int* n_launch) {
     e.table = rt->embed.w; e.kind = rt->embed.kind; e.H = H; e.x = rt->x; e.state = rt->state; e.status = rt->status;
     e.use_pdl = 0;   // first kernel of the step: ordinary stream order behind the previous step
     e.seq_inc = rt->tp_seq;
+    if (rt->step_ctr) { e.zero_ctr = rt->step_ctr; e.n_zero = n_proj * kMaxKRanges; }
     CU(rt, launch_embed(e, st)); n++;
 
     for (int l = 0; l < d.n_layers; l++) {
@@ -671,6 +674,7 @@ int issue_step(lum_rt* rt, bool with_head, bool pdl, int* n_launch) {
             t.l2_pf_ptr[1] = w.up.w; t.l2_pf_bytes[1] = want < ub ? want : ub;
         }
         CU(rt, launch_attn_decode(t, st)); n++;
+        prev_wide = false;
 
         // o projection (+ residual)
         GemvArgs o{};
@@ -699,6 +703,7 @@ int issue_step(lum_rt* rt, bool with_head, bool pdl, int* n_launch) {
             m.dn_q = (const int8_t*)w.exp_dn.w; m.dn_s = w.exp_dn.s; m.dn_bias = w.exp_dn_b.w;
             m.sw = rt->moe_sw; m.limit = d.swiglu_limit; m.status = rt->status; m.use_pdl = pdl; m.out_ld = H;
             CU(rt, launch_moe_route(m, 1, st)); n++;
+            prev_wide = false;
             if (rt->ep_size > 1) {
                 const int T = rt->ep_size;
                 if (int r2 = ep_all_to_all(rt, rt->moe_xf, rt->moe_recv, (size_t)rt->moe_slot)) return r2;      // dispatch
@@ -729,11 +734,10 @@ int issue_step(lum_rt* rt, bool with_head, bool pdl, int* n_launch) {
         dn.K = (int)w.down.kdev; dn.x = rt->h;
         if (fused) publish_to_peers(dn, 1, (uint32_t)(2 * l + 2));
         else if (tp) { dn.epi = EPI_STORE; dn.y = rt->part; }
-        else if (rt->down_ksplit && gemv_can_ksplit(dn.K, w.down.kc)) {
-            // One GPU: the long-K projection as two jobs per row group (a job is then 61 KB instead of 122 KB: the kernel's
-            // tail, one job long, halves); the two partial vectors join the residual stream in the next prologue.
-            dn.epi = EPI_STORE; dn.y = rt->part; dn.ksplit = 2; dn.y_half_stride = H;
-            pending = true; pending_halves = true;
+        else if (rt->down_ksplit && gemv_stream_supported(dn) && gemv_k_ranges(dn.K, w.down.kc) > 1 && rt->sm_count >= dn.K / 512) {
+            // One GPU: the long-K projection as K ranges of at most 4096 columns; their partial vectors join the residual stream in the next prologue.
+            dn.epi = EPI_STORE; dn.y = rt->part; dn.ksplit = gemv_k_ranges(dn.K, w.down.kc); dn.y_range_stride = rt->part_ld;
+            pending = true; pending_ranges = dn.ksplit;
         }
         else { dn.epi = EPI_RESID; dn.y = cur; dn.resid = cur; }
         claim_ctr(dn);
@@ -2307,7 +2311,7 @@ int32_t lum_clear_intermediates(lum_rt* rt) {
     const lum_model_desc& d = rt->d;
     CU(rt, cudaMemsetAsync(rt->x, 0, (size_t)d.hidden * 4, rt->stream));
     if (rt->x2) CU(rt, cudaMemsetAsync(rt->x2, 0, (size_t)d.hidden * 4, rt->stream));
-    if (rt->part) CU(rt, cudaMemsetAsync(rt->part, 0, (size_t)2 * d.hidden * 4, rt->stream));
+    if (rt->part) CU(rt, cudaMemsetAsync(rt->part, 0, (size_t)kMaxKRanges * rt->part_ld * 4, rt->stream));
     CU(rt, cudaMemsetAsync(rt->qkv, 0, rt->qkv_floats * 4, rt->stream));
     CU(rt, cudaMemsetAsync(rt->attn, 0, rt->attn_floats * 4, rt->stream));
     CU(rt, cudaMemsetAsync(rt->h, 0, rt->h_floats * 4, rt->stream));
@@ -2891,10 +2895,11 @@ int32_t lum_model_init(lum_rt* rt, const lum_model_desc* dp) {
     const int G = d.n_q_heads / d.n_kv_heads;
     TRY(dev_alloc(rt, (void**)&rt->x, Hpad * 4));
     TRY(dev_alloc(rt, (void**)&rt->x2, Hpad * 4));
-    TRY(dev_alloc(rt, (void**)&rt->part, (size_t)2 * Hpad * 4));   // a reduced partial vector, or the two K halves of the down projection
+    rt->part_ld = (int)Hpad;          // columns behind the last real one stay zero
+    TRY(dev_alloc(rt, (void**)&rt->part, (size_t)kMaxKRanges * Hpad * 4));   // a reduced partial vector, or the K ranges of the down projection
     cudaMemsetAsync(rt->x, 0, Hpad * 4, rt->stream);
     cudaMemsetAsync(rt->x2, 0, Hpad * 4, rt->stream);
-    cudaMemsetAsync(rt->part, 0, (size_t)2 * Hpad * 4, rt->stream);
+    cudaMemsetAsync(rt->part, 0, (size_t)kMaxKRanges * Hpad * 4, rt->stream);
     if (d.rope_style == 2) {
         // YaRN inverse frequencies (examples/gpt_oss/src/model.rs:47-81): binary64 on the host, stored as f32
         std::vector<float> inv((size_t)hd / 2);
@@ -2950,8 +2955,8 @@ int32_t lum_model_init(lum_rt* rt, const lum_model_desc* dp) {
     TRY(dev_alloc(rt, (void**)&rt->attn_part, (size_t)rt->nkv_l * splits * G * (hd + 2) * 4));
     TRY(dev_alloc(rt, (void**)&rt->attn_cnt, (size_t)rt->nkv_l * 4));
     TRY(alloc_decode_state(rt));
-    TRY(dev_alloc(rt, (void**)&rt->step_ctr, ((size_t)4 * d.n_layers + 1) * sizeof(unsigned int)));
-    cudaMemsetAsync(rt->step_ctr, 0, ((size_t)4 * d.n_layers + 1) * sizeof(unsigned int), rt->stream);
+    TRY(dev_alloc(rt, (void**)&rt->step_ctr, ((size_t)4 * d.n_layers + 1) * kMaxKRanges * sizeof(unsigned int)));
+    cudaMemsetAsync(rt->step_ctr, 0, ((size_t)4 * d.n_layers + 1) * kMaxKRanges * sizeof(unsigned int), rt->stream);
 #undef TRY
     cudaMemsetAsync(rt->attn_cnt, 0, (size_t)rt->nkv_l * 4, rt->stream);
 

@@ -287,12 +287,94 @@ static void matvec_bf16() {
     }
 }
 
+// Q8_0 matrices in the streaming matrix-vector kernel: every number of tiles a row group can have (a tile per warp, several row groups per job, several turns
+// of the rings), K ranges, jobs claimed or dealt out, all epilogues but the sampler's, vectors made of several terms.
+static void matvec_q8() {
+    struct Case { std::vector<int> rows; int k, ranges, parts; bool pair, resid, claims, norm; };
+    const std::vector<Case> cases = {
+        {{8}, 512, 1, 0, false, false, false, false},          {{264, 16, 8}, 512, 1, 0, false, false, true, false}, {{40, 40}, 512, 1, 0, true, false, true, true},
+        {{72, 8}, 1024, 1, 2, false, false, true, true},       {{1208}, 1536, 1, 0, false, true, true, false},       {{24, 24}, 1536, 1, 0, true, false, false, true},
+        {{136, 8, 8}, 2048, 1, 4, false, false, true, true},   {{2560}, 2560, 1, 3, false, true, true, true},        {{1240, 1240}, 2560, 1, 0, true, false, true, true},
+        {{648}, 3072, 1, 0, false, true, false, false},        {{512, 40, 40}, 3584, 1, 0, false, false, true, true}, {{4096}, 4096, 1, 1, false, false, true, true},
+        {{2008, 2008}, 4096, 1, 4, true, false, true, true},   {{96}, 4608, 1, 0, false, false, true, true},         {{64, 64}, 6144, 1, 2, true, false, true, true},
+        {{264}, 4608, 2, 0, false, false, true, false},        {{1208}, 9728, 3, 0, false, false, true, false},      {{1200}, 14336, 4, 0, false, false, true, false},
+        {{40}, 14336, 4, 0, false, false, false, false},       {{328}, 14336, 1, 0, false, true, true, false},       {{80}, 16384, 4, 0, false, false, true, false}};
+    for (const Case& c : cases) {
+        std::mt19937 rng(c.k + c.rows[0] + c.parts);
+        const int K = c.k, nb = K / 32;
+        std::vector<std::vector<float>> terms;
+        for (int i = 0; i <= c.parts; i++) terms.push_back(normal(rng, K, 1.0f));
+        std::vector<float> x = terms[0], parts;
+        for (int i = 1; i <= c.parts; i++) { for (int j = 0; j < K; j++) x[j] += terms[i][j]; parts.insert(parts.end(), terms[i].begin(), terms[i].end()); }
+        const std::vector<uint16_t> gain = to_bf16(normal(rng, K, 0.1f, 1.0f));
+        std::vector<double> xe(x.begin(), x.end());
+        if (c.norm) {
+            double ss = 0;
+            for (double v : xe) ss += v * v;
+            for (int j = 0; j < K; j++) xe[j] *= bf16_value(gain[j]) / std::sqrt(ss / K + 1e-5);
+        }
+        Dev<float> dx(terms[0]), dparts(parts.empty() ? std::vector<float>(1) : parts), dxo(K);
+        Dev<uint16_t> dgain(gain);
+        Dev<unsigned int> ctr(kMaxKRanges);
+        Dev<uint32_t> status(1);
+        GemvArgs a{};
+        a.nseg = (int)c.rows.size(); a.K = K; a.wkind = WK_Q8; a.epi = c.pair ? EPI_SWIGLU : c.resid ? EPI_RESID : EPI_STORE; a.x = dx.p; a.gain_kind = WK_BF16; a.status = status.p;
+        if (c.norm) { a.gain = dgain.p; a.eps = 1e-5f; }
+        if (c.parts) { a.parts = dparts.p; a.n_parts = c.parts; a.part_stride = K; a.x_out = dxo.p; }
+        if (c.claims) a.job_ctr = ctr.p;
+        std::vector<Dev<unsigned char>*> packed;
+        std::vector<std::vector<double>> sums;
+        int total = 0;
+        for (int n : c.rows) {
+            std::vector<int8_t> q((size_t)n * K);
+            std::vector<__half> s((size_t)n * nb);
+            for (auto& v : q) v = (int8_t)((int)(rng() % 256) - 128);
+            for (auto& v : s) v = __float2half(0.0005f + 0.001f * (rng() % 1000) / 1000.0f);
+            Dev<int8_t> dq(q);
+            Dev<__half> ds(s);
+            packed.push_back(new Dev<unsigned char>(q8_packed_bytes(n, K)));
+            CK(launch_q8_pack_units(dq.p, ds.p, n, K, q8_pack_kc(n, K), packed.back()->p, nullptr));
+            CK(cudaDeviceSynchronize());
+            a.seg[sums.size()] = {packed.back()->p, nullptr, n, q8_pack_kc(n, K)};
+            sums.emplace_back(n);
+            for (int r = 0; r < n; r++)
+                for (int b = 0; b < nb; b++) {
+                    double t = 0;
+                    for (int i = 0; i < 32; i++) t += (double)q[(size_t)r * K + b * 32 + i] * xe[b * 32 + i];
+                    sums.back()[r] += t * (double)__half2float(s[(size_t)r * nb + b]);
+                }
+            total += n;
+        }
+        std::vector<float> res = normal(rng, total, 1.0f);
+        std::vector<double> want;
+        if (c.pair) { total = c.rows[0]; for (int r = 0; r < total; r++) want.push_back(sums[0][r] / (1 + std::exp(-sums[0][r])) * sums[1][r]); }
+        else for (const auto& s : sums) want.insert(want.end(), s.begin(), s.end());
+        if (c.resid) for (int r = 0; r < total; r++) want[r] += res[r];
+        Dev<float> y((size_t)total * c.ranges + 8), dres(res);
+        a.y = y.p; a.resid = dres.p;
+        if (c.ranges > 1) { a.ksplit = c.ranges; a.y_range_stride = total; }
+        CK(launch_gemv(a, 148, nullptr));
+        std::vector<float> raw = y.get(), got(total);
+        for (int i = 0; i < 8; i++) if (raw[(size_t)total * c.ranges + i] != 0.0f) report("behind the end", 1, 0);
+        for (int r = 0; r < c.ranges; r++) for (int i = 0; i < total; i++) got[i] += raw[(size_t)r * total + i];
+        std::string what;
+        for (int n : c.rows) what += std::to_string(n) + " ";
+        // three levels keep 2^-24 of a block's largest magnitude (about two to three standard deviations), every sum of the vector's terms and of the blocks rounds once more
+        report(what + "x " + std::to_string(K) + " in " + std::to_string(c.ranges) + " ranges, epilogue " + std::to_string(a.epi) + ", " + std::to_string(c.parts) + " terms more" + (c.claims ? ", claimed" : ""),
+               rel(got, want), 16 * std::exp2(-24.0));
+        if (c.parts) { const std::vector<float> xo = dxo.get(); report("the vector itself", rel(xo, std::vector<double>(x.begin(), x.end())), std::exp2(-24.0)); }
+        report("status", status.get()[0], 0);
+        for (auto* p : packed) delete p;
+    }
+}
+
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "attention-sums") attention_sums();
     else if (what == "attention-specials") attention_specials();
     else if (what == "experts") experts();
     else if (what == "matvec-bf16") matvec_bf16();
+    else if (what == "matvec-q8") matvec_q8();
     else { std::printf("unknown check\n"); return 2; }
     return failures ? 1 : 0;
 }
