@@ -393,7 +393,7 @@ __device__ __forceinline__ void gemv_gain_preload(const GemvArgs& a, int tid, Ga
 //   A matrix [N, K] (K a multiple of 512, N of 8) is a stream of tiles: row group rg = rows [8 rg, 8 rg + 8), tile t of it =
 //   columns [512 t, 512 t + 512); tiles of a row group are consecutive, row groups follow each other.  tpr = K / 512.
 //   A CTA works on the tiles [t0, t0 + nt) of every row group it takes: all of them, or (ksplit) one of the K ranges, which the
-//   CTAs share out in proportion to their tiles.  A job is what one CTA must do as a whole: one row group, with nt <= 4 as many (gpf) as make up to
+//   CTAs share out in proportion to their tiles.  A job is what one CTA must do as a whole: one row group, where it is whole and has up to 4 tiles as many (gpf) as make up to
 //   8 tiles; for SwiGLU the same of the gate matrix followed by the same of the up matrix.  A job part is cut into fills of up to 4
 //   tiles, which go to the two rings in turn (a part of one fill sends the second ring an empty one: both see every job).
 struct GemvPlan {
@@ -417,7 +417,7 @@ __device__ __forceinline__ GemvPlan gemv_plan(const GemvArgs& a, int cta, int n_
             if (cta >= c0 && cta < c1) { p.range = r; p.cta = cta - c0; p.n_cta = c1 - c0; p.t0 = b0; p.nt = b1 - b0; }
         }
     }
-    p.gpf = p.nt > kFillTiles ? 1 : kJobTiles / p.nt;
+    p.gpf = p.nt > kFillTiles || p.nt < p.tpr ? 1 : kJobTiles / p.nt;      // (only whole row groups follow each other in memory)
     p.sub = a.epi == EPI_SWIGLU ? 2 : 1;
     int jobs = 0, rgs = 0;
     for (int i = 0; i < 3; i++) {
