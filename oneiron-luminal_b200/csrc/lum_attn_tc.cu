@@ -3,12 +3,17 @@
 // kernel walks the cache once per (KV head, query group, row); here 128 / G query rows times the G query heads of a KV head
 // form the 128 rows of one tensor-core tile and share every K/V tile they read).
 //
-// One CTA = one KV head x one tile of QT = 128 / G query rows.  Per tile of 64 cached positions:
-//     S = Q K^T          tcgen05.mma kind::f16, M = 128, N = 64, K = 128: 8 instructions per Q operand
-//     online softmax     8 warps read S from tensor memory (thread = row, half of the keys), scale, mask, exponentiate
-//     O_t = P V          M = 128, N = 128, K = 64: 4 instructions per P operand; V is read as stored (MN-major operand)
-//     O = O * alpha + O_t   in registers (thread = row, half of the head dimension)
-// K/V tiles arrive through cp.async, the next tile's copies in flight while the current one is computed.
+// One CTA = one KV head x one tile of QT = 128 / G query rows; 16 warps, four threads per row of the tile.  Per tile of 128 cached positions:
+//     S = Q K^T          tcgen05.mma kind::f16, M = 128, N = 128, K = 128: 8 instructions per Q operand
+//     online softmax     a thread reads 32 scores of its row from tensor memory, scales, masks, exponentiates, and stores the weights'
+//                        two terms back over them
+//     O_t = P V          M = 128, N = 128, K = 128, P from tensor memory: 8 instructions per P operand; V is read as stored (MN-major operand)
+//     O = O * alpha + O_t   in registers (a thread has 32 of the row's dimensions)
+// What bounds it: per tile 32 instructions of 64 clocks on the tensor core, 1024 clocks of exponentials, about 1300 issue slots per scheduler.  So the
+// three run side by side: S(t + 1) is computed while tile t's scores are exponentiated (two score buffers, both terms of P fit the scores'
+// own columns), O_t is added up after P(t + 1) has been handed over (two output buffers).  A tile's sum is taken out of the tensor core after 16 instructions,
+// the low terms first: its accumulator cuts every addition to 24 bits.  K/V tiles arrive through cp.async, two tiles ahead.
+// The CTAs with the most keys start first.
 //
 // Accuracy.  The oracle computes this in f32 from f32 queries and bf16 cache values.  The cache values are bf16 already, so
 // they enter the tensor core exactly.  The f32 operands — the queries and the softmax weights — are split into two bf16
@@ -26,17 +31,18 @@ namespace lum {
 namespace {
 
 constexpr int kAtHD = 128;           // head dimension
-constexpr int kAtKT = 64;            // cached positions per tile
-constexpr int kAtThreads = 256;
+constexpr int kAtKT = 64;            // cached positions per tile of the band kernel
+constexpr int kAtThreads = 256;      // of the band kernel
 // shared memory (bytes): operands in the tensor core's no-swizzle core-matrix order, [16-byte column group][row][16 bytes]
-constexpr int kAtQBytes = 128 * kAtHD * 2;          // 32 KiB per Q term
-constexpr int kAtKVBytes = kAtKT * kAtHD * 2;       // 16 KiB per K or V tile
-constexpr int kAtPBytes = 128 * kAtKT * 2;          // 16 KiB per P term
-constexpr int kAtOffQhi = 0, kAtOffQlo = kAtQBytes, kAtOffK = 2 * kAtQBytes, kAtOffV = kAtOffK + 2 * kAtKVBytes,
-              kAtOffPhi = kAtOffV + 2 * kAtKVBytes, kAtOffPlo = kAtOffPhi + kAtPBytes, kAtOffMisc = kAtOffPlo + kAtPBytes;
-constexpr int kAtMiscBytes = 2048;                  // 2 mbarriers, the tensor-memory slot, per-row exchange of maxima / sums
-constexpr int kAtSmem = kAtOffMisc + kAtMiscBytes;
-constexpr uint32_t kAtTmemCols = 256;               // S: columns 0..63, O_t: columns 64..191
+constexpr int kAtPBytes = 128 * kAtKT * 2;          // 16 KiB per P term of the band kernel
+constexpr int kApKT = 128, kApWarps = 16, kApLoaders = 3, kApThreads = (kApWarps + 1 + kApLoaders) * 32;      // prompt kernel: cached positions per tile, softmax warps; one more issues the tensor core's work, three load
+constexpr int kApGroup = 128 * 16 + 16;             // Q: a 16-byte column group of 128 rows; the next one starts 16 bytes further on, so that a row's groups lie in different banks
+constexpr int kApQBytes = kAtHD / 8 * kApGroup;     // per Q term
+// K and V tiles: two halves of 64 dimensions, 128 rows of 128 bytes each, a row's 16-byte pieces in the order piece ^ (row % 8) (the tensor core's 128-byte
+// swizzle).  So a copy's 32-byte sectors stay together on their way into shared memory: as single 16-byte pieces (no swizzle) a warp's copy of 512 bytes took 30 clocks.
+constexpr int kApHalf = 128 * 128, kApOperand = 2 * kApHalf;
+constexpr int kApOffK = 0, kApOffV = 2 * kApOperand, kApOffQ = 4 * kApOperand, kApOffMisc = kApOffQ + 2 * kApQBytes;
+constexpr int kApSmem = kApOffMisc + 128 + 2 * 4 * 128 * 4;       // barriers, slot, flags; per-row exchange of maxima (two tiles in turn) / sums
 
 // kind::f16, bf16 x bf16 -> f32; b_mn: the B operand is MN-major (V as stored: the head dimension contiguous)
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, bool b_mn) {
@@ -49,6 +55,34 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t da, uint64_t
         ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// the same with the A operand in tensor memory
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// whole warp: 32 consecutive columns of this thread's lane
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
+                   "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+                   "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+                 : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
+                   "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
+                   "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+// Operand with the 128-byte swizzle.  K-major: rows of 128 bytes (K advances by bytes inside them), sbo between groups of 8 rows.  MN-major: rows of 64
+// elements of MN, K down the rows, sbo between groups of 8, lbo to the next 64 elements of MN.
+__device__ __forceinline__ uint64_t umma_smem_desc_sw128(uint32_t addr, uint32_t lbo, uint32_t sbo) { return umma_smem_desc(addr, lbo, sbo) | (2ull << 61); }
+constexpr float kLog2e = 1.4426950408889634f;
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t src_bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
@@ -64,41 +98,68 @@ __device__ __forceinline__ void split2(float x0, float x1, uint32_t* hi, uint32_
     *lo = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
 }
 
+// the same, two conversions at a time
+__device__ __forceinline__ void split2_rn(float x0, float x1, uint32_t* hi, uint32_t* lo) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
+    const uint32_t b = *(const uint32_t*)&h;
+    const __nv_bfloat162 l = __floats2bfloat162_rn(x0 - __uint_as_float(b << 16), x1 - __uint_as_float(b & 0xffff0000u));
+    *hi = b;
+    *lo = *(const uint32_t*)&l;
+}
+
 }  // namespace
 
 // G = query heads per KV head (1, 2, 4 or 8): MMA row r = g * QT + qi is query row q0 + qi of head kvh * G + g.
-__global__ void __launch_bounds__(kAtThreads, 1) attn_prompt_tc(const AttnRowsArgs a, int G, int lbo_sbo_swap) {
-    extern __shared__ __align__(128) unsigned char smem[];
+// Measured, 32 / 8 heads of 128: 4096 rows from position 0 1278 -> 326 us (422 issued TFLOP/s), 387 rows behind 1021 positions 119 -> 36 us.  What a tile waits for now
+// is its K and V: LDGSTS of 512 bytes per 24 clocks.
+__global__ void __launch_bounds__(kApThreads, 1) attn_prompt_tc(const AttnRowsArgs a, int G) {
+    extern __shared__ __align__(1024) unsigned char smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int kvh = blockIdx.x, QT = 128 / G, q0 = blockIdx.y * QT;
-    const uint32_t s_base = smem_u32(smem);
-    const uint32_t bar_s = s_base + kAtOffMisc, bar_o = bar_s + 8, tmem_slot = bar_s + 16;
-    float* x_max = (float*)(smem + kAtOffMisc + 64);          // [2 halves][128 rows]
-    int* s_flag = (int*)(smem + kAtOffMisc + 64 + 1024);      // [0]: largest position of the CTA's rows, [1]: a wait ran out
+    const int kvh = blockIdx.x, QT = 128 / G, q0 = (int)(gridDim.y - 1 - blockIdx.y) * QT;
+    const uint32_t s_base = smem_u32(smem), misc = s_base + kApOffMisc;
+    const uint32_t bar_k = misc, bar_s = misc + 16, bar_p = misc + 32, bar_o = misc + 48, bar_f = misc + 64, bar_v = misc + 80;       // two of each: tile t uses number t % 2
+    int* s_flag = (int*)(smem + kApOffMisc + 104);              // [0], [1]: largest position of the CTA's rows, minus the smallest; [2]: a wait ran out
+    float* x_max = (float*)(smem + kApOffMisc + 128);          // [tile % 2][4 threads of a row][128 rows]
 
-    if (tid == 0) { mbar_init(bar_s, 1); mbar_init(bar_o, 1); mbar_fence_init(); s_flag[0] = -1; s_flag[1] = 0; }
-    if (warp == 0) tmem_alloc(tmem_slot, kAtTmemCols);
+    if (tid == 0) {
+        for (int i = 0; i < 2; i++) {
+            mbar_init(bar_k + 8 * i, kApLoaders);              // K(t) has landed
+            mbar_init(bar_v + 8 * i, kApLoaders);              // V(t)
+            mbar_init(bar_s + 8 * i, 1);                       // S(t) is there (and K(t) no longer read)
+            mbar_init(bar_p + 8 * i, kApWarps);                // P(t) is stored
+            mbar_init(bar_o + 8 * i, 1);                       // O_t is there (and V(t) no longer read)
+            mbar_init(bar_f + 8 * i, kApWarps);                // O_t has been added up
+        }
+        mbar_fence_init();
+        s_flag[0] = -1; s_flag[1] = -0x7fffffff; s_flag[2] = 0;
+    }
+    if (warp == kApWarps) tmem_alloc(misc + 96, 512);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = *(volatile uint32_t*)(smem + kAtOffMisc + 16);
+    const uint32_t tmem = *(volatile uint32_t*)(smem + kApOffMisc + 96);
 
-    // this thread's row of the tile, for the softmax and the output
-    const int row = (warp & 3) * 32 + lane, half = warp >> 2;
-    const int g_row = row / QT, qi_row = row - g_row * QT, m_row = q0 + qi_row;
-    const bool row_ok = m_row < a.M;
+    // this thread's row of the tile, its quarter of a tile's keys and of the head's dimensions
+    const bool softmax = warp < kApWarps;
+    const int row = (warp & 3) * 32 + lane, qr = warp >> 2;
+    const int g_row = row / QT, m_row = q0 + row - g_row * QT;
+    const bool row_ok = softmax && m_row < a.M;
     int pos_row = row_ok ? a.row_pos[m_row] : -1;
     if (pos_row >= a.max_seq) pos_row = -1;                    // flagged by the kernel that appended the row
     {
-        int pm = pos_row;
+        int hi = pos_row, lo = row_ok ? -pos_row : -0x7fffffff;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) pm = max(pm, __shfl_xor_sync(0xffffffffu, pm, o));
-        if (lane == 0 && pm >= 0) atomicMax(&s_flag[0], pm);
+        for (int o = 16; o > 0; o >>= 1) { hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o)); lo = max(lo, __shfl_xor_sync(0xffffffffu, lo, o)); }
+        if (lane == 0 && qr == 0) { atomicMax(&s_flag[0], hi); atomicMax(&s_flag[1], lo); }
     }
+    __syncthreads();
+    const int pos_max = s_flag[0], pos_min = -s_flag[1];
+    const int n_tiles = pos_max >= 0 ? pos_max / kApKT + 1 : 0;
 
+    const size_t row_elems = (size_t)a.n_kv * kAtHD;
     // ---- Q tile -> two bf16 operands in shared memory
     const size_t qd = (size_t)a.n_q * kAtHD;
-    for (int ch = tid; ch < 128 * 16; ch += kAtThreads) {
+    for (int ch = tid; ch < 128 * 16; ch += kApThreads) {
         const int r = ch >> 4, c = ch & 15;                    // 16 threads read one row's 512 bytes
         const int g = r / QT, qi = r - g * QT, m = q0 + qi;
         uint4 hi = make_uint4(0u, 0u, 0u, 0u), lo = hi;
@@ -108,160 +169,172 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_prompt_tc(const AttnRowsAr
             split2(v0.x, v0.y, &hi.x, &lo.x); split2(v0.z, v0.w, &hi.y, &lo.y);
             split2(v1.x, v1.y, &hi.z, &lo.z); split2(v1.z, v1.w, &hi.w, &lo.w);
         }
-        *(uint4*)(smem + kAtOffQhi + c * 2048 + r * 16) = hi;
-        *(uint4*)(smem + kAtOffQlo + c * 2048 + r * 16) = lo;
+        *(uint4*)(smem + kApOffQ + c * kApGroup + r * 16) = hi;
+        *(uint4*)(smem + kApOffQ + kApQBytes + c * kApGroup + r * 16) = lo;
     }
+    fence_proxy_async_smem();
     __syncthreads();
-    const int pos_max = s_flag[0];
-    const int n_tiles = pos_max >= 0 ? pos_max / kAtKT + 1 : 0;
 
-    const size_t row_elems = (size_t)a.n_kv * kAtHD;
-    const __nv_bfloat16* kc = (const __nv_bfloat16*)a.k_cache + (size_t)kvh * kAtHD;
-    const __nv_bfloat16* vc = (const __nv_bfloat16*)a.v_cache + (size_t)kvh * kAtHD;
-    // one K and one V tile: 64 positions x 16 column groups = 1024 16-byte chunks each; a warp takes 8 positions x 4 groups
-    auto load_tile = [&](int t, int buf) {
-        const uint32_t kdst = s_base + kAtOffK + buf * kAtKVBytes, vdst = s_base + kAtOffV + buf * kAtKVBytes;
-        // the tile's 64 positions start on a multiple of 64: one sequence slot or one page (of at least 64 rows) holds them all;
-        // its first position is at most pos_max, so it is mapped
-        const size_t tile_row = kv_phys_row(a.pg, a.seq0, a.max_seq, t * kAtKT);
+    // A wait that runs out of its budget is remembered; what follows neither waits nor multiplies any more, but meets every barrier.
+    auto wait = [&](uint32_t bar, int t) {
+        if (*(volatile int*)&s_flag[2]) return;
+        if (!mbar_wait(bar + 8u * (t & 1), (uint32_t)(t >> 1) & 1u)) *(volatile int*)&s_flag[2] = 1;
+    };
+    auto arrive = [&](uint32_t bar, int t) { __syncwarp(); if (lane == 0) mbar_arrive(bar + 8u * (t & 1)); };
+    constexpr uint32_t idesc_s = idesc_bf16(128, kApKT, false), idesc_o = idesc_bf16(128, kAtHD, true);
+    if (warp == kApWarps) {
+        // S(t + 1) goes out before P(t) is waited for: the tensor core works through both while tile t's, then tile t + 1's scores are exponentiated
+        if (elect_one()) {
+#pragma unroll 1
+            for (int t = 0; t <= n_tiles; t++) {
+                if (t < n_tiles) {
+                    wait(bar_k, t);
+                    if (*(volatile int*)&s_flag[2]) break;
+                    tc_fence_after_sync();
+                    const uint32_t kb = s_base + kApOffK + (t & 1) * kApOperand, d = tmem + (uint32_t)(t & 1) * 128u;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int ch = tid + i * kAtThreads;
-            const int w = ch >> 5, l = ch & 31;                // 32 "warp slots" of 32 chunks
-            const int key = (w >> 2) * 8 + (l >> 2), c = (w & 3) * 4 + (l & 3);
-            const int j = t * kAtKT + key;
-            const bool in = j <= pos_max;                      // rows never written (or beyond the capacity) read as zeros
-            const size_t off = (tile_row + (size_t)(in ? key : 0)) * row_elems + c * 8;
-            cp_async16(kdst + c * 1024 + key * 16, kc + off, in ? 16u : 0u);
-            cp_async16(vdst + c * 1024 + key * 16, vc + off, in ? 16u : 0u);
+                    for (int term = 1; term >= 0; term--)
+#pragma unroll
+                        for (int ks = 0; ks < kAtHD / 16; ks++)            // K = 16 elements = two 16-byte column groups per instruction
+                            umma_bf16(d, umma_smem_desc(s_base + kApOffQ + term * kApQBytes + ks * 2 * kApGroup, kApGroup, 128), umma_smem_desc_sw128(kb + (ks >> 2) * kApHalf + (ks & 3) * 32, 16, 1024), idesc_s, (term == 0 || ks) ? 1u : 0u);
+                    umma_commit(bar_s + 8u * (t & 1));
+                }
+                if (t > 0) {
+                    const int u = t - 1;
+                    wait(bar_v, u);
+                    wait(bar_p, u);
+                    if (u > 1) wait(bar_f, u - 2);
+                    if (*(volatile int*)&s_flag[2]) break;
+                    tc_fence_after_sync();
+                    const uint32_t vb = s_base + kApOffV + (u & 1) * kApOperand, p = tmem + (uint32_t)(u & 1) * 128u, d = tmem + 256u + (uint32_t)(u & 1) * 128u;
+                    // V as stored: 64 head dimensions of 8 positions are 1024 bytes, the other 64 dimensions half a tile further on
+#pragma unroll
+                    for (int term = 1; term >= 0; term--)
+#pragma unroll
+                        for (int ks = 0; ks < kApKT / 16; ks++)            // 16 positions per instruction: eight columns of a term
+                            umma_bf16_ts(d, p + (uint32_t)((ks >> 1) * 32 + term * 16 + (ks & 1) * 8), umma_smem_desc_sw128(vb + ks * 2048, kApHalf, 1024), idesc_o, (term == 0 || ks) ? 1u : 0u);
+                    umma_commit(bar_o + 8u * (u & 1));
+                }
+            }
         }
-        cp_async_commit();
+        __syncwarp();
+    } else if (!softmax) {
+        // K(0), K(1), V(0), K(2), V(1), ..: a tile's copies go out as soon as its buffer is no longer read, the one before is handed over when it has landed.
+        // A warp's instruction takes two positions' 256 bytes.  Half a tile's positions start on a multiple of 64: one sequence slot or one page (of at least
+        // 64 rows) holds them all; rows never written (or beyond the capacity) read as zeros.
+        uint32_t last = 0u;                                    // the barrier of the tile still on its way
+        auto load = [&](const void* cache, int t, uint32_t dst, uint32_t full, uint32_t unread) {
+            if (t >= n_tiles) return;
+            if (t > 1) wait(unread, t - 2);
+            const int k0 = (warp - kApWarps - 1) * 2 + (lane >> 4);                       // this lane's first position of a half
+            dst += (uint32_t)(t & 1) * kApOperand + ((lane >> 3) & 1) * kApHalf + k0 * 128;
+#pragma unroll 1
+            for (int h = 0; h < 2; h++, dst += 64 * 128) {
+                const int j0 = t * kApKT + h * 64, live = min(64, pos_max + 1 - j0);
+                const __nv_bfloat16* src = (const __nv_bfloat16*)cache + (size_t)kvh * kAtHD + (lane & 15) * 8;
+                if (live > 0) src += kv_phys_row(a.pg, a.seq0, a.max_seq, j0) * row_elems;
+#pragma unroll
+                for (int i = 0; i < (32 + kApLoaders - 1) / kApLoaders; i++) {
+                    const int key = k0 + i * 2 * kApLoaders;
+                    if (key < 64) cp_async16(dst + i * 256 * kApLoaders + (((lane & 7) ^ (key & 7)) << 4), src + (key < live ? (size_t)key * row_elems : 0), key < live ? 16u : 0u);
+                }
+            }
+            cp_async_commit();
+            if (last) {
+                cp_async_wait<1>();
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(last);
+            }
+            last = full + 8u * (t & 1);
+        };
+        load(a.k_cache, 0, s_base + kApOffK, bar_k, bar_s);
+#pragma unroll 1
+        for (int t = 0; t < n_tiles; t++) {
+            load(a.k_cache, t + 1, s_base + kApOffK, bar_k, bar_s);
+            load(a.v_cache, t, s_base + kApOffV, bar_v, bar_o);
+        }
+        if (last) {
+            cp_async_wait<0>();
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(last);
+        }
+    }
+
+    float o[32];
+#pragma unroll
+    for (int i = 0; i < 32; i++) o[i] = 0.0f;
+    float m_run = -INFINITY, l_run = 0.0f, alpha = 1.0f;
+    const float scale = kLog2e / sqrtf((float)kAtHD);          // weights are powers of two
+    const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(qr * 32);
+    auto add_output = [&](int t) {                             // O = O alpha(t) + O_t
+        wait(bar_o, t);
+        tc_fence_after_sync();
+        uint32_t v[32];
+        tmem_ld32(mine + 256u + (uint32_t)(t & 1) * 128u, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; i++) o[i] = fmaf(o[i], alpha, __uint_as_float(v[i]));
+        tc_fence_before_sync();
+        arrive(bar_f, t);
     };
 
-    float o_acc[64];
-#pragma unroll
-    for (int i = 0; i < 64; i++) o_acc[i] = 0.0f;
-    float m_run = -INFINITY, l_run = 0.0f;
-    const float scale = 1.0f / sqrtf((float)kAtHD);
-    constexpr uint32_t idesc_s = idesc_bf16(128, kAtKT, false), idesc_o = idesc_bf16(128, kAtHD, true);
-    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-
-    if (n_tiles > 0) load_tile(0, 0);
-    uint32_t phase = 0;
-    bool failed = false;
 #pragma unroll 1
-    for (int t = 0; t < n_tiles; t++) {
-        const int buf = t & 1;
-        if (t + 1 < n_tiles) { load_tile(t + 1, buf ^ 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
-        fence_proxy_async_smem();
-        __syncthreads();
-        if (warp == 0 && elect_one()) {
-            tc_fence_after_sync();
-            const uint32_t kb = s_base + kAtOffK + buf * kAtKVBytes;
-#pragma unroll
-            for (int term = 0; term < 2; term++) {
-                const uint32_t qb = s_base + (term ? kAtOffQlo : kAtOffQhi);
-#pragma unroll
-                for (int ks = 0; ks < kAtHD / 16; ks++)       // K = 16 elements = two 16-byte column groups per instruction
-                    umma_bf16(tmem, umma_smem_desc(qb + ks * 2 * 2048, 2048, 128), umma_smem_desc(kb + ks * 2 * 1024, 1024, 128), idesc_s,
-                              (term | ks) ? 1u : 0u);
-            }
-            umma_commit(bar_s);
-        }
-        if (!mbar_wait(bar_s, phase)) failed = true;
+    for (int t = softmax ? 0 : n_tiles; t < n_tiles; t++) {
+        wait(bar_s, t);
         tc_fence_after_sync();
-
-        // ---- softmax of this thread's row over its 32 keys of the tile
-        float s[32];
-        {
-            uint32_t v[16];
-            tmem_ld16(lane_base + half * 32, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; i++) s[i] = __uint_as_float(v[i]);
-            tmem_ld16(lane_base + half * 32 + 16, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; i++) s[16 + i] = __uint_as_float(v[i]);
-        }
-        const int j0 = t * kAtKT + half * 32;
+        uint32_t v[32];
+        tmem_ld32(mine + (uint32_t)(t & 1) * 128u, v);
+        tmem_ld_wait();
         float mx = -INFINITY;
+        const int j0 = t * kApKT + qr * 32;
+        if (t * kApKT + kApKT - 1 > pos_min) {                 // some row does not see all of the tile
 #pragma unroll
-        for (int i = 0; i < 32; i++) {
-            s[i] = (j0 + i <= pos_row) ? s[i] * scale : -INFINITY;
-            mx = fmaxf(mx, s[i]);
+            for (int i = 0; i < 32; i++) if (j0 + i > pos_row) v[i] = 0xff800000u;
         }
-        x_max[half * 128 + row] = mx;
-        named_sync(1, kAtThreads);
-        const float m_new = fmaxf(m_run, fmaxf(mx, x_max[(half ^ 1) * 128 + row]));
-        const float alpha = (m_new == -INFINITY) ? 1.0f : expf(m_run - m_new);      // m_run = -inf: exp(-inf) = 0
+#pragma unroll
+        for (int i = 0; i < 32; i++) mx = fmaxf(mx, __uint_as_float(v[i]));
+        float* xm = x_max + (t & 1) * 512 + row;
+        xm[qr * 128] = mx;
+        named_sync(1 + (warp & 3), 128);                       // the four warps that share these rows
+        const float m_new = fmaxf(m_run, fmaxf(fmaxf(xm[0], xm[128]), fmaxf(xm[256], xm[384])));
+        const float alpha_t = m_new == m_run ? 1.0f : ex2((m_run - m_new) * scale);      // m_run = -inf: 0
+        const float off = m_new == -INFINITY ? 0.0f : -m_new * scale;
         float psum = 0.0f;
-        uint32_t ph[16], pl[16];
+        uint32_t pk[32];                                       // high terms, low terms
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-            const float p0 = (s[i] == -INFINITY) ? 0.0f : expf(s[i] - m_new);
-            const float p1 = (s[i + 1] == -INFINITY) ? 0.0f : expf(s[i + 1] - m_new);
+            const float p0 = ex2(fmaf(__uint_as_float(v[i]), scale, off)), p1 = ex2(fmaf(__uint_as_float(v[i + 1]), scale, off));
             psum += p0 + p1;
-            split2(p0, p1, &ph[i >> 1], &pl[i >> 1]);
+            split2_rn(p0, p1, &pk[i >> 1], &pk[16 + (i >> 1)]);
         }
-        l_run = l_run * alpha + psum;
+        l_run = l_run * alpha_t + psum;
         m_run = m_new;
-#pragma unroll
-        for (int c = 0; c < 4; c++) {                          // 4 column groups of 8 keys
-            const int off = (half * 4 + c) * 2048 + row * 16;
-            *(uint4*)(smem + kAtOffPhi + off) = make_uint4(ph[c * 4], ph[c * 4 + 1], ph[c * 4 + 2], ph[c * 4 + 3]);
-            *(uint4*)(smem + kAtOffPlo + off) = make_uint4(pl[c * 4], pl[c * 4 + 1], pl[c * 4 + 2], pl[c * 4 + 3]);
-        }
-        fence_proxy_async_smem();
+        tmem_st32(mine + (uint32_t)(t & 1) * 128u, pk);        // over this thread's own scores
+        tmem_st_wait();
         tc_fence_before_sync();
-        __syncthreads();
-        if (warp == 0 && elect_one()) {
-            tc_fence_after_sync();
-            const uint32_t vb = s_base + kAtOffV + buf * kAtKVBytes;
-            // V as stored: 16-byte groups of 8 head dimensions, 1024 bytes apart along the head dimension (MN), 8 positions = 128
-            // contiguous bytes along K
-            const uint32_t v_lbo = lbo_sbo_swap ? 1024u : 128u, v_sbo = lbo_sbo_swap ? 128u : 1024u;
-#pragma unroll
-            for (int term = 0; term < 2; term++) {
-                const uint32_t pb = s_base + (term ? kAtOffPlo : kAtOffPhi);
-#pragma unroll
-                for (int ks = 0; ks < kAtKT / 16; ks++)       // 16 positions per instruction
-                    umma_bf16(tmem + 64, umma_smem_desc(pb + ks * 2 * 2048, 2048, 128), umma_smem_desc(vb + ks * 256, v_lbo, v_sbo), idesc_o,
-                              (term | ks) ? 1u : 0u);
-            }
-            umma_commit(bar_o);
-        }
-        if (!mbar_wait(bar_o, phase)) failed = true;
-        tc_fence_after_sync();
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            uint32_t v[16];
-            tmem_ld16(lane_base + 64 + half * 64 + c * 16, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; i++) o_acc[c * 16 + i] = fmaf(o_acc[c * 16 + i], alpha, __uint_as_float(v[i]));
-        }
-        tc_fence_before_sync();
-        phase ^= 1u;
-        if (__syncthreads_or(failed ? 1 : 0)) { if (tid == 0) s_flag[1] = 1; break; }       // the tensor core never answered: give up, together
+        arrive(bar_p, t);
+        if (t > 0) add_output(t - 1);
+        alpha = alpha_t;
     }
-    cp_async_wait<0>();
+    if (softmax && n_tiles > 0) add_output(n_tiles - 1);
     __syncthreads();
-    if (s_flag[1] && tid == 0 && a.status) atomicOr(a.status, LUM_ST_WAIT_TMEM);
+    if (s_flag[2] && tid == 0 && a.status) atomicOr(a.status, LUM_ST_WAIT_TMEM);
 
-    // ---- out = O / l, l = the two halves' sums
-    x_max[half * 128 + row] = l_run;
+    // ---- out = O / l, l = the four quarters' sums
+    if (softmax) x_max[qr * 128 + row] = l_run;
     __syncthreads();
-    const float l_tot = l_run + x_max[(half ^ 1) * 128 + row];
+    const float l_tot = (x_max[row] + x_max[128 + row]) + (x_max[256 + row] + x_max[384 + row]);
     if (row_ok) {
         const float inv = l_tot > 0.0f ? 1.0f / l_tot : 0.0f;
-        float4* dst = (float4*)(a.out + (size_t)m_row * qd + ((size_t)kvh * G + g_row) * kAtHD + half * 64);
+        float4* dst = (float4*)(a.out + (size_t)m_row * qd + ((size_t)kvh * G + g_row) * kAtHD + qr * 32);
 #pragma unroll
-        for (int i = 0; i < 16; i++) dst[i] = make_float4(o_acc[4 * i] * inv, o_acc[4 * i + 1] * inv, o_acc[4 * i + 2] * inv, o_acc[4 * i + 3] * inv);
+        for (int i = 0; i < 8; i++) dst[i] = make_float4(o[4 * i] * inv, o[4 * i + 1] * inv, o[4 * i + 2] * inv, o[4 * i + 3] * inv);
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, kAtTmemCols);
+    if (warp == kApWarps) tmem_dealloc(tmem, 512);
 }
 
 bool attn_prompt_tc_supported(const AttnRowsArgs& a) {
@@ -273,10 +346,9 @@ bool attn_prompt_tc_supported(const AttnRowsArgs& a) {
 cudaError_t launch_attn_prompt_tc(const AttnRowsArgs& a, cudaStream_t st) {
     if (!attn_prompt_tc_supported(a)) return cudaErrorInvalidValue;
     static std::atomic<uint64_t> raised{0};
-    if (const cudaError_t e = allow_smem(raised, (const void*)attn_prompt_tc, kAtSmem)) return e;
-    static const int swap = [] { const char* e = getenv("LUM_ATTN_TC_SWAP"); return e ? atoi(e) : 0; }();
+    if (const cudaError_t e = allow_smem(raised, (const void*)attn_prompt_tc, kApSmem)) return e;
     const int G = a.n_q / a.n_kv, QT = 128 / G;
-    attn_prompt_tc<<<dim3(a.n_kv, (a.M + QT - 1) / QT), kAtThreads, kAtSmem, st>>>(a, G, swap);
+    attn_prompt_tc<<<dim3(a.n_kv, (a.M + QT - 1) / QT), kApThreads, kApSmem, st>>>(a, G);
     return cudaGetLastError();
 }
 
@@ -301,8 +373,6 @@ namespace {
 __device__ __forceinline__ void cluster_st_f32x4(uint32_t addr, float4 v) {
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
-constexpr float kLog2e = 1.4426950408889634f;
-__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 // x = hi + lo in bf16 with the high term cut off instead of rounded (no conversion instruction for it; |x - hi - lo| <= 2^-17 |x| all the same)
 __device__ __forceinline__ void split2_cut(float x0, float x1, uint32_t* hi, uint32_t* lo) {
     const uint32_t b0 = __float_as_uint(x0), b1 = __float_as_uint(x1);
@@ -330,7 +400,7 @@ __host__ __device__ inline BandSmem band_smem(int dkp, int dvp, int maps) {
 
 template <int DVH>
 __global__ void __launch_bounds__(kAtThreads, 1) attn_band_tc(const BandArgs a) {
-    extern __shared__ __align__(128) unsigned char smem[];
+    extern __shared__ __align__(1024) unsigned char smem[];
     const QkvArgs& p = a.p;
     const int dkp = p.dkp, dvp = p.dvp, kgr = dkp / 8, vgr = dvp / 8;
     const BandSmem L = band_smem(dkp, dvp, p.maps);

@@ -110,6 +110,57 @@ struct Attention {
     }
 };
 
+// Rows of a prompt behind `first` cached ones: tiles of 128 keys and of 128 / (heads per K/V head) rows, on and off their edges; a cache of pages.
+static void attention_prompt() {
+    struct Case { int nq, nkv, rows, first; bool pages; };
+    const std::vector<Case> cases = {{8, 2, 16, 0, false},   {4, 4, 128, 0, false},  {4, 4, 129, 127, false}, {8, 2, 33, 95, false},  {16, 2, 17, 111, true},
+                                     {8, 2, 96, 1000, true}, {8, 4, 65, 191, true},  {4, 1, 31, 383, false},  {8, 1, 200, 56, false}, {2, 2, 300, 1, true}};
+    for (const Case& c : cases) {
+        const int hd = 128, n = c.first + c.rows, max_seq = (n + 63) / 64 * 64, G = c.nq / c.nkv;
+        std::mt19937 rng(n * 7 + c.nq);
+        const size_t ld = (size_t)c.nkv * hd, qd = (size_t)c.nq * hd;
+        const std::vector<float> q = normal(rng, (size_t)c.rows * qd, 1.0f);
+        std::vector<uint16_t> k = to_bf16(normal(rng, max_seq * ld, 1.0f)), v = to_bf16(normal(rng, max_seq * ld, 1.0f, 0.5f));
+        std::vector<int> pos(c.rows), table(max_seq / 64);
+        for (int i = 0; i < c.rows; i++) pos[i] = c.first + i;
+        std::vector<uint16_t> kp = k, vp = v;               // with pages: in another order, and what no row may see is not a number
+        for (int i = 0; i < max_seq / 64; i++) table[i] = c.pages ? max_seq / 64 - 1 - i : i;
+        for (int j = 0; j < max_seq; j++)
+            for (size_t e = 0; e < ld; e++) {
+                const size_t to = ((size_t)table[j / 64] * 64 + j % 64) * ld + e;
+                kp[to] = j < n ? k[j * ld + e] : 0x7fc0; vp[to] = j < n ? v[j * ld + e] : 0x7fc0;
+            }
+        Dev<float> dq(q), out(q.size());
+        Dev<uint16_t> kc(kp), vc(vp);
+        Dev<int> dpos(pos), dtable(table);
+        Dev<uint32_t> status(1);
+        AttnRowsArgs a{};
+        a.q_rot = dq.p; a.k_cache = kc.p; a.v_cache = vc.p; a.row_pos = dpos.p; a.out = out.p; a.M = c.rows; a.n_q = c.nq; a.n_kv = c.nkv; a.hd = hd; a.kv_bf16 = 1;
+        a.max_seq = max_seq; a.max_batch = 1; a.status = status.p;
+        if (c.pages) { a.pg.table = dtable.p; a.pg.lg = 6; a.pg.pages_per_seq = max_seq / 64; }
+        CK(launch_attn_prompt_tc(a, nullptr));
+        std::vector<double> want(q.size()), w(n);
+        for (int m = 0; m < c.rows; m++)
+            for (int h = 0; h < c.nq; h++) {
+                const size_t col = (size_t)(h / G) * hd, row = (size_t)m * qd + (size_t)h * hd;
+                double mx = -INFINITY, l = 0;
+                for (int j = 0; j <= pos[m]; j++) {
+                    double d = 0;
+                    for (int e = 0; e < hd; e++) d += (double)q[row + e] * bf16_value(k[j * ld + col + e]);
+                    w[j] = d / std::sqrt((double)hd);
+                    mx = std::fmax(mx, w[j]);
+                }
+                for (int j = 0; j <= pos[m]; j++) l += w[j] = std::exp(w[j] - mx);
+                for (int j = 0; j <= pos[m]; j++)
+                    for (int e = 0; e < hd; e++) want[row + e] += w[j] / l * bf16_value(v[j * ld + col + e]);
+            }
+        // queries and weights keep 2^-17 of themselves in two bf16 terms; a score of 128 products then moves by less than 2^-17 on average, and a sum of
+        // 16 instructions is cut to 24 bits that many times
+        report(std::to_string(c.nq) + " / " + std::to_string(c.nkv) + " heads, rows " + std::to_string(c.first) + " + " + std::to_string(c.rows) + (c.pages ? ", pages" : ""), rel(out.get(), want), std::exp2(-16.0));
+        report("status", status.get()[0], 0);
+    }
+}
+
 // Long sums stay sums of 32 bits.  A split's values are added up tile by tile, 64 keys of a CTA at a time: m additions of relative error 2^-24 at most
 // walk about sqrt(m) of them away, and scores, weights and each tile's own sum (cut, not rounded) are a few more.
 static void attention_sums() {
@@ -372,6 +423,7 @@ int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "attention-sums") attention_sums();
     else if (what == "attention-specials") attention_specials();
+    else if (what == "attention-prompt") attention_prompt();
     else if (what == "experts") experts();
     else if (what == "matvec-bf16") matvec_bf16();
     else if (what == "matvec-q8") matvec_q8();
