@@ -435,6 +435,37 @@ __device__ __forceinline__ GemvPlan gemv_plan(const GemvArgs& a, int cta, int n_
     return p;
 }
 
+// Four elements of a block whose largest magnitude is amax -> four bytes of each level; returns the block's scale.
+__device__ __forceinline__ float gemv_levels(const float (&e)[4], float amax, uint32_t (&p)[3]) {
+    const float s1 = amax * (1.0f / 127.0f);
+    const float i1 = amax > 0.0f ? 127.0f / amax : 0.0f;
+    const float s2 = s1 * (1.0f / 254.0f), i2 = i1 * 254.0f;
+    const float i3 = i1 * 64516.0f;
+    // Round to nearest by adding 1.5 * 2^23: the sum's low mantissa bits are the integer in two's complement,
+    // so its low byte is the int8 value — no float->int conversion or rint (both quarter-rate instructions).
+    // |e * i1| <= 127 and every residual is at most half a step of the level before, so no clamping is needed.
+    constexpr float kMagic = 12582912.0f;
+    p[0] = p[1] = p[2] = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const float t1 = fmaf(e[j], i1, kMagic);
+        const float r1 = fmaf(-s1, t1 - kMagic, e[j]);
+        const float t2 = fmaf(r1, i2, kMagic);
+        const float r2 = fmaf(-s2, t2 - kMagic, r1);
+        const float t3 = fmaf(r2, i3, kMagic);
+        p[0] |= (__float_as_uint(t1) & 0xffu) << (8 * j);
+        p[1] |= (__float_as_uint(t2) & 0xffu) << (8 * j);
+        p[2] |= (__float_as_uint(t3) & 0xffu) << (8 * j);
+    }
+    return s1;
+}
+// Where the first level's word j (columns 4 j .. 4 j + 3) of block blk goes in the operand (gemv_load_xfrag); the other levels 16 words further on each.
+// Columns of the operand are (half of the tile, level); a block is number blk % 8 of its half.
+__device__ __forceinline__ int gemv_level_word(int blk, int j) {
+    const int i = blk & 7;
+    return ((blk >> 4) * kXqTileBytes + (i >> 1) * 384 + (((blk >> 3) & 1) * 12 + (j & 3)) * 16 + (i & 1) * 8 + (j >> 2) * 4) >> 2;
+}
+
 // Prologue: activations (optionally RMS-normalised, times the gains) -> three int8 levels + one f32 scale per 32-block, laid out as
 // the B operand of the tensor-core instruction (gemv_load_xfrag).  Runs on the kConsumers threads; 8 consecutive threads own one
 // block, a warp a tile of every turn.  A thread issues the loads of up to four float4 (of every term) at once: the vector sits in L2, most of a microsecond away, and up
@@ -579,30 +610,11 @@ __device__ __forceinline__ void gemv_quantize_x(const GemvArgs& a, const XSource
             amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
             amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
             amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-            const float s1 = amax * (1.0f / 127.0f);
-            const float i1 = amax > 0.0f ? 127.0f / amax : 0.0f;
-            const float s2 = s1 * (1.0f / 254.0f), i2 = i1 * 254.0f;
-            const float i3 = i1 * 64516.0f;
-            // Round to nearest by adding 1.5 * 2^23: the sum's low mantissa bits are the integer in two's complement,
-            // so its low byte is the int8 value — no float->int conversion or rint (both quarter-rate instructions).
-            // |e * i1| <= 127 and every residual is at most half a step of the level before, so no clamping is needed.
-            constexpr float kMagic = 12582912.0f;
-            uint32_t p1 = 0, p2 = 0, p3 = 0;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const float t1 = fmaf(e[j], i1, kMagic);
-                const float r1 = fmaf(-s1, t1 - kMagic, e[j]);
-                const float t2 = fmaf(r1, i2, kMagic);
-                const float r2 = fmaf(-s2, t2 - kMagic, r1);
-                const float t3 = fmaf(r2, i3, kMagic);
-                p1 |= (__float_as_uint(t1) & 0xffu) << (8 * j);
-                p2 |= (__float_as_uint(t2) & 0xffu) << (8 * j);
-                p3 |= (__float_as_uint(t3) & 0xffu) << (8 * j);
-            }
-            // block -> (tile, half of the tile, number in it): columns of the operand are (half, level); see gemv_load_xfrag
-            const int blk = f4 >> 3, j = f4 & 7, i = blk & 7;
-            uint32_t* dst = (uint32_t*)(g.xq + (size_t)(blk >> 4) * kXqTileBytes + (i >> 1) * 384 + (((blk >> 3) & 1) * 12 + (j & 3)) * 16 + (i & 1) * 8 + (j >> 2) * 4);
-            dst[0] = p1; dst[16] = p2; dst[32] = p3;
+            uint32_t lv[3];
+            const float s1 = gemv_levels(e, amax, lv);
+            const int blk = f4 >> 3;
+            uint32_t* dst = (uint32_t*)g.xq + gemv_level_word(blk, f4 & 7);
+            dst[0] = lv[0]; dst[16] = lv[1]; dst[32] = lv[2];
             if ((tid & 7) == 0) g.xsc[blk] = s1;
         }
     }

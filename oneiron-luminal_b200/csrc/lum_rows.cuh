@@ -73,6 +73,22 @@ struct ArgmaxRowsArgs {
     int use_pdl;
 };
 
+// Products of two to five rows (lum_few.cu): y[range][m][n] over the concatenated matrices, operand from launch_rows_levels
+constexpr int kFewMax = 5;
+struct FewArgs {
+    const void* w[3]; int rows[3]; int nseg;         // packed Q8_0 matrices [rows, K]
+    int K, M;
+    const int8_t* xq; const float* sx;               // levels in operand order and block scales (few_xq_bytes, few_sx_floats)
+    float* y; int ldy; size_t part_stride;           // planes of the K ranges
+    uint32_t* status;
+    int use_pdl;
+};
+int few_ranges(int K, int sm_count);                 // K ranges of such a product; 0: not taken
+size_t few_xq_bytes(int M, int K);
+size_t few_sx_floats(int M, int K);
+cudaError_t launch_rows_levels(const RowsArgs& a, int sm_count, cudaStream_t st);
+cudaError_t launch_few(const FewArgs& f, int sm_count, cudaStream_t st);
+
 size_t gemm_xq_bytes(int M, int K);
 size_t gemm_sx_bytes(int M, int K);
 struct GemmShape { int nc, ks; };                // activation rows per chunk, K ranges (at most kMaxKsplit)

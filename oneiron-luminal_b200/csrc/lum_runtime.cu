@@ -214,6 +214,7 @@ struct lum_rt {
 
     // ---- steps that carry several rows (prompt processing, batched decode): buffers of the tensor-core path, made on first use
     struct Rows {
+        int down_parts = 1;               // planes of the last pass's down projection
         int cap = 0;                      // rows a pass can take
         int *tok = nullptr, *pos = nullptr, *seq = nullptr;          // [cap] per-row token / position / sequence
         float *xr = nullptr, *q_rot = nullptr, *attn = nullptr;      // residual rows [cap][H]; rotated queries and attention output [cap][qd]
@@ -1401,11 +1402,28 @@ int run_rows(lum_rt* rt, int M, int* d_tok, int* d_pos, const int* d_seq, int se
     const int gk = kind_of(d.embed_dtype), sms = rt->sm_count, pdl = rt->rows_pdl;
     cudaStream_t st = rt->stream;
     const GemmShape g_qkv = gemm_shape(W, M, H, sms), g_o = gemm_shape(H, M, qd, sms), g_gu = gemm_shape(2 * F, M, H, sms), g_dn = gemm_shape(H, M, F, sms);
-    const int ks_qkv = g_qkv.ks, ks_o = g_o.ks, ks_gu = g_gu.ks, ks_dn = g_dn.ks;
+    // Up to five rows: the products on integer levels (lum_few.cu), where every K is one they take and the planes' buffers (of at least 32 rows) hold their K ranges
+    const int r_h = few_ranges(H, sms), r_q = few_ranges(qd, sms), r_f = few_ranges(F, sms);
+    const bool few = M <= kFewMax && r_h && r_q && r_f && W % 8 == 0 && (head != 2 || (r_h == 1 && rt->lm_head.kc));
+    const int ks_qkv = few ? r_h : g_qkv.ks, ks_o = few ? r_q : g_o.ks, ks_gu = few ? r_h : g_gu.ks, ks_dn = few ? r_f : g_dn.ks;
+    b.down_parts = ks_dn;
     CU(rt, launch_embed_rows(rt->embed.w, rt->embed.kind, H, d.vocab, d_tok, b.xr, M, rt->status, st));
     uint64_t launches = 1;
-    auto quant = [&](RowsArgs& r, int K, GemmShape gs) -> cudaError_t { r.M = M; r.K = K; r.nc = gs.nc; r.xq = b.xq; r.sx = b.sx; r.use_pdl = pdl; launches++; return launch_rows_quantize(r, sms, st); };
+    auto quant = [&](RowsArgs& r, int K, GemmShape gs) -> cudaError_t {
+        r.M = M; r.K = K; r.nc = gs.nc; r.xq = b.xq; r.sx = b.sx; r.use_pdl = pdl;
+        launches++;
+        if (few) { r.sx = (float*)(b.xq + few_xq_bytes(M, K)); return launch_rows_levels(r, sms, st); }
+        return launch_rows_quantize(r, sms, st);
+    };
     auto gemm = [&](GemmArgs& g, int K, GemmShape gs, float* y, int ldy) -> cudaError_t {
+        if (few) {
+            FewArgs f{};
+            f.nseg = g.nseg; f.K = K; f.M = M; f.xq = b.xq; f.sx = (const float*)(b.xq + few_xq_bytes(M, K)); f.y = y; f.ldy = ldy; f.part_stride = (size_t)M * ldy;
+            f.status = rt->status; f.use_pdl = pdl;
+            for (int s = 0; s < g.nseg; s++) { f.w[s] = g.seg[s].w; f.rows[s] = g.seg[s].rows; }      // (their columns follow each other in y)
+            launches++;
+            return launch_few(f, sms, st);
+        }
         g.K = K; g.xq = b.xq; g.sx = b.sx; g.M = M; g.nc = gs.nc; g.ksplit = gs.ks; g.y = y; g.ldy = ldy; g.part_stride = (size_t)M * ldy; g.status = rt->status; g.use_pdl = pdl;
         launches++;
         return launch_gemm(g, sms, st);
@@ -1504,7 +1522,7 @@ int run_rows(lum_rt* rt, int M, int* d_tok, int* d_pos, const int* d_seq, int se
         GemmArgs g{};
         g.nseg = 1; g.seg[0] = {(const unsigned char*)rt->lm_head.w, V, 0};
         CU(rt, gemm(g, H, g_v, b.logits, V));
-        if (int r2 = batch_sample(rt, M, d_tok, d_pos, d_seq, g_v.ks, &launches)) return r2;
+        if (int r2 = batch_sample(rt, M, d_tok, d_pos, d_seq, few ? r_h : g_v.ks, &launches)) return r2;
     }
     rt->n_launches += launches;
     return 0;
@@ -1522,7 +1540,7 @@ int want_row(lum_rt* rt, int m, int M, size_t slot) {
     a.nseg = 1; a.seg[0] = {hw.w, hw.s, (int)hw.rows, hw.kc};
     a.K = H; a.epi = EPI_STORE; a.gain = rt->final_norm.w; a.y = rt->want_logits + slot * rt->vocab_l;
     a.x = b.xr + (size_t)m * H;
-    a.parts = b.down + (size_t)m * H; a.n_parts = gemm_shape(H, M, rt->ffn_l, rt->sm_count).ks; a.part_stride = M * H;
+    a.parts = b.down + (size_t)m * H; a.n_parts = b.down_parts; a.part_stride = M * H;
     CU(rt, launch_gemv(a, rt->sm_count, rt->stream));
     rt->n_launches++;
     return 0;

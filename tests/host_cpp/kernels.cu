@@ -419,6 +419,81 @@ static void matvec_q8() {
     }
 }
 
+// Two to five rows: rows formed and quantised (plain, behind a norm, SwiGLU of two sums; planes, residual), then multiplied; every number of tiles, K ranges.
+static void few_rows() {
+    struct Case { std::vector<int> rows; int k, m, planes; bool norm, pair; };
+    const std::vector<Case> cases = {{{8}, 2560, 2, 1, false, false},        {{1200, 40, 8}, 4096, 5, 4, true, false}, {{9600}, 4096, 5, 1, false, false}, {{264}, 3072, 3, 2, true, false},
+                                     {{640}, 14336, 5, 1, false, true},      {{72, 72}, 3584, 5, 3, true, false},      {{1192}, 9728, 4, 2, false, true},   {{96}, 8192, 3, 1, false, false},
+                                     {{16, 7184}, 2560, 5, 1, true, false},  {{88}, 5120, 2, 1, false, true},          {{4096}, 3584, 1, 1, false, false}};
+    for (const Case& c : cases) {
+        const int K = c.k, M = c.m, nb = K / 32, ld = c.pair ? 2 * K : K, R = few_ranges(K, 148);
+        std::mt19937 rng(K + M);
+        const std::vector<float> in = normal(rng, (size_t)c.planes * M * ld, 1.0f), resid = normal(rng, (size_t)M * K, 1.0f);
+        const std::vector<uint16_t> gain = to_bf16(normal(rng, K, 0.1f, 1.0f));
+        std::vector<double> x((size_t)M * K);
+        for (int m = 0; m < M; m++) {
+            double ss = 0;
+            for (int i = 0; i < K; i++) {
+                double v = 0, u = 0;
+                for (int p = 0; p < c.planes; p++) { v += in[((size_t)p * M + m) * ld + i]; if (c.pair) u += in[((size_t)p * M + m) * ld + K + i]; }
+                if (c.pair) v = v / (1 + std::exp(-v)) * u;
+                if (c.norm) v += resid[(size_t)m * K + i];
+                x[(size_t)m * K + i] = v;
+                ss += v * v;
+            }
+            if (c.norm) for (int i = 0; i < K; i++) x[(size_t)m * K + i] *= bf16_value(gain[i]) / std::sqrt(ss / K + 1e-5);
+        }
+        Dev<float> din(in), dres(resid), out((size_t)M * K), sx(few_sx_floats(M, K));
+        Dev<uint16_t> dgain(gain);
+        Dev<int8_t> xq(few_xq_bytes(M, K));
+        Dev<uint32_t> status(1);
+        RowsArgs r{};
+        r.a = din.p; r.n_parts = c.planes; r.part_stride = (size_t)M * ld; r.ld = ld; r.M = M; r.K = K; r.xq = xq.p; r.sx = sx.p; r.gain_kind = WK_BF16;
+        if (c.pair) r.b = din.p + K;
+        if (c.norm) { r.gain = dgain.p; r.eps = 1e-5f; r.resid = dres.p; r.resid_ld = K; r.out = out.p; r.out_ld = K; }
+        CK(launch_rows_levels(r, 148, nullptr));
+        FewArgs f{};
+        f.nseg = (int)c.rows.size(); f.K = K; f.M = M; f.xq = xq.p; f.sx = sx.p; f.status = status.p;
+        std::vector<Dev<unsigned char>*> packed;
+        int total = 0;
+        for (int n : c.rows) total += n;
+        std::vector<double> want((size_t)M * total);
+        int col = 0;
+        for (size_t sg = 0; sg < c.rows.size(); sg++) {
+            const int n = c.rows[sg];
+            std::vector<int8_t> q((size_t)n * K);
+            std::vector<__half> s((size_t)n * nb);
+            for (auto& v : q) v = (int8_t)((int)(rng() % 256) - 128);
+            for (auto& v : s) v = __float2half(0.0005f + 0.001f * (rng() % 1000) / 1000.0f);
+            Dev<int8_t> dq(q);
+            Dev<__half> ds(s);
+            packed.push_back(new Dev<unsigned char>(q8_packed_bytes(n, K)));
+            CK(launch_q8_pack_units(dq.p, ds.p, n, K, q8_pack_kc(n, K), packed.back()->p, nullptr));
+            CK(cudaDeviceSynchronize());
+            f.w[sg] = packed.back()->p; f.rows[sg] = n;
+            for (int m = 0; m < M; m++)
+                for (int i = 0; i < n; i++)
+                    for (int b = 0; b < nb; b++) {
+                        double t = 0;
+                        for (int e = 0; e < 32; e++) t += (double)q[(size_t)i * K + b * 32 + e] * x[(size_t)m * K + b * 32 + e];
+                        want[(size_t)m * total + col + i] += t * (double)__half2float(s[(size_t)i * nb + b]);
+                    }
+            col += n;
+        }
+        Dev<float> y((size_t)R * M * total + 8);
+        f.y = y.p; f.ldy = total; f.part_stride = (size_t)M * total;
+        CK(launch_few(f, 148, nullptr));
+        const std::vector<float> raw = y.get();
+        std::vector<float> got((size_t)M * total);
+        for (int i = 0; i < 8; i++) if (raw[(size_t)R * M * total + i] != 0.0f) report("behind the end", 1, 0);
+        for (int k = 0; k < R; k++) for (size_t i = 0; i < got.size(); i++) got[i] += raw[(size_t)k * M * total + i];
+        // as for one vector: three levels, a norm's factor and the sums of blocks and of planes round
+        report(std::to_string(total) + " x " + std::to_string(K) + ", " + std::to_string(M) + " rows, " + std::to_string(R) + " ranges", rel(got, want), 16 * std::exp2(-24.0));
+        report("status", status.get()[0], 0);
+        for (auto* p : packed) delete p;
+    }
+}
+
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "attention-sums") attention_sums();
@@ -427,6 +502,7 @@ int main(int argc, char** argv) {
     else if (what == "experts") experts();
     else if (what == "matvec-bf16") matvec_bf16();
     else if (what == "matvec-q8") matvec_q8();
+    else if (what == "few-rows") few_rows();
     else { std::printf("unknown check\n"); return 2; }
     return failures ? 1 : 0;
 }
