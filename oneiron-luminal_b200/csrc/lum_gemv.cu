@@ -30,8 +30,8 @@
 namespace lum {
 
 // Prologue of the plain-load kernel: bring x into shared memory as f32 (optionally RMS-normalised and
-// scaled by the gains).
-__device__ __forceinline__ void gemv_load_x(const GemvArgs& a, float* xs, int tid, int nthreads, float* scratch, int bar_id) {
+// scaled by the gains).  gain0: element tid's, asked for before the grid dependency was waited for.
+__device__ __forceinline__ void gemv_load_x(const GemvArgs& a, float* xs, int tid, int nthreads, float* scratch, int bar_id, float gain0) {
     const int K = a.K;
     if (a.n_parts > 0 && a.part_flags) peer_wait_parts(a.part_flags, a.n_parts, a.seq, a.parts_tag, a.status, tid, nthreads, bar_id);
     // the raw activations first (x, plus a reduced partial or the ranks' partials in rank order), then the norm over them
@@ -53,10 +53,10 @@ __device__ __forceinline__ void gemv_load_x(const GemvArgs& a, float* xs, int ti
         ss = fmaf(v, v, ss);
     }
     if (a.gain) {
-        ss = block_sum(ss, scratch, tid, nthreads, bar_id);
+        ss = block_sum(ss, scratch, tid, nthreads, bar_id, false);      // (a barrier follows before the scratch is written again)
         const float mean = ss * (1.0f / (float)(a.k_norm > 0 ? a.k_norm : K));
         const float inv = 1.0f / sqrtf(mean + a.eps);
-        for (int k = tid; k < K; k += nthreads) xs[k] = (inv * xs[k]) * load_gain(a.gain, a.gain_kind, k);
+        for (int k = tid; k < K; k += nthreads) xs[k] = (inv * xs[k]) * (k == tid ? gain0 : load_gain(a.gain, a.gain_kind, k));
     }
     named_sync(bar_id, nthreads);
 }
@@ -137,8 +137,10 @@ __device__ __forceinline__ void bf16_rows_dot(const uint4* const (&w)[N], int n8
     }
 }
 
+// pre: f32 rows: the first kRowAhead float4 of this lane, when they are there already
+constexpr int kRowAhead = 4;
 template <int WK>
-__device__ __forceinline__ float row_dot(const GemvSeg& sg, int row, int K, const float* xs, int lane) {
+__device__ __forceinline__ float row_dot(const GemvSeg& sg, int row, int K, const float* xs, int lane, const float4* pre = nullptr) {
     float acc = 0.0f;
     if (WK == WK_Q8) {
         // planes: quants [N,K] + scales [N,K/32].  packed (kc > 0): the streaming kernel's tile stream — per row group of
@@ -174,7 +176,16 @@ __device__ __forceinline__ float row_dot(const GemvSeg& sg, int row, int K, cons
         if ((K & 3) == 0) {
             const float4* w4 = (const float4*)w;
             const float4* x4 = (const float4*)xs;
-            for (int i = lane; i < (K >> 2); i += 32) {
+            int i = lane;
+            if (pre) {
+#pragma unroll
+                for (int t = 0; t < kRowAhead; t++, i += 32)
+                    if (i < (K >> 2)) {
+                        const float4 a = pre[t], b = x4[i];
+                        acc = fmaf(a.x, b.x, acc); acc = fmaf(a.y, b.y, acc); acc = fmaf(a.z, b.z, acc); acc = fmaf(a.w, b.w, acc);
+                    }
+            }
+            for (; i < (K >> 2); i += 32) {
                 const float4 a = w4[i], b = x4[i];
                 acc = fmaf(a.x, b.x, acc); acc = fmaf(a.y, b.y, acc); acc = fmaf(a.z, b.z, acc); acc = fmaf(a.w, b.w, acc);
             }
@@ -212,9 +223,6 @@ __global__ void __launch_bounds__(256, WK == WK_BF16 ? kDirectBf16Ctas : 0) gemv
     float* xs = scratch + 64;                  // K floats (K rounded up to 4)
     float* vals = xs + ((a.K + 3) & ~3);       // 2 * max rows per CTA
 
-    if (a.use_pdl) { pdl_launch_dependents(); pdl_grid_wait(); }
-    gemv_load_x(a, xs, tid, 256, scratch, 1);
-
     const int sub = paired ? 2 : 1;
     auto row_of = [&](int i, int* sg) {
         const int h = i / n;
@@ -224,6 +232,23 @@ __global__ void __launch_bounds__(256, WK == WK_BF16 ? kDirectBf16Ctas : 0) gemv
         else while (*sg < a.nseg - 1 && row >= a.seg[*sg].rows) { row -= a.seg[*sg].rows; (*sg)++; }
         return row;
     };
+    if (a.use_pdl) pdl_launch_dependents();
+    // What does not depend on the previous kernel is on its way before that is waited for: the gain of element tid, the start of each warp's first f32 row.  A small
+    // model's step is a chain of trips to L2 (tiny_f32 of the configurations, 31 steps of 12 kernels: 1490 -> 1337 us).
+    const float gain0 = a.gain && tid < a.K ? load_gain(a.gain, a.gain_kind, tid) : 0.0f;
+    float4 pre[WK == WK_F32 ? kRowAhead : 1];
+    const bool ahead = WK == WK_F32 && (a.K & 3) == 0 && warp < n * sub;
+    if (ahead) {
+        int sg;
+        const int row = row_of(warp, &sg);
+        const float4* w = (const float4*)((const float*)a.seg[sg].w + (size_t)row * a.K);
+#pragma unroll
+        for (int t = 0; t < kRowAhead; t++) pre[WK == WK_F32 ? t : 0] = lane + 32 * t < (a.K >> 2) ? __ldg(w + lane + 32 * t) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (a.use_pdl) pdl_grid_wait();
+    const float resid0 = a.epi == EPI_RESID && tid < n ? a.resid[row0 + tid] : 0.0f;
+    gemv_load_x(a, xs, tid, 256, scratch, 1, gain0);
+
     if (WK == WK_BF16 && (a.K & 7) == 0) {
         // Four rows at a time: vocabulary projection of 151936 x 2560 (778 MB) 222 us with one, 125 us = 6.2 TB/s with four.  At every size: where a CTA
         // has eight rows two of its warps work, and that is still no slower than eight with a row each (back to back, us with one / four:
@@ -249,13 +274,13 @@ __global__ void __launch_bounds__(256, WK == WK_BF16 ? kDirectBf16Ctas : 0) gemv
         for (int i = warp; i < n * sub; i += 8) {
             int sg;
             const int row = row_of(i, &sg);
-            const float v = row_dot<WK>(a.seg[sg], row, a.K, xs, lane);
+            const float v = row_dot<WK>(a.seg[sg], row, a.K, xs, lane, ahead && i == warp ? pre : nullptr);
             if (lane == 0) vals[i] = v;
         }
     }
     named_sync(1, 256);
     ArgBest best{-INFINITY, -1};
-    gemv_epilogue_rows(a, vals, row0, n, tid, 256, scratch, 1, &best);
+    gemv_epilogue_rows(a, vals, row0, n, tid, 256, scratch, 1, &best, resid0);
     if (a.epi == EPI_ARGMAX) argmax_finish(a, best, tid, 256, 1);
     if (a.epi == EPI_PEER && !a.peer_ll) peer_publish(a, tid, 256, 1);
 }

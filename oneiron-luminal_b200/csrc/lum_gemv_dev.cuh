@@ -207,15 +207,15 @@ __device__ __forceinline__ void gemv_epilogue_units(const GemvArgs& a, Vals vals
 }
 
 // Same for a contiguous run of rows (the plain-load kernel): vals[i] is logical row row0 + i (SwiGLU: gate sums in
-// vals[0..n), up sums in vals[n..2n)).
+// vals[0..n), up sums in vals[n..2n)).  resid0: element tid of the residual.
 __device__ __forceinline__ void gemv_epilogue_rows(const GemvArgs& a, const float* vals, int row0, int n, int tid, int nthreads,
-                                                   float* scratch, int bar_id, ArgBest* best) {
+                                                   float* scratch, int bar_id, ArgBest* best, float resid0) {
     if (a.epi == EPI_STORE) {
         for (int i = tid; i < n; i += nthreads) a.y[row0 + i] = a.bias ? vals[i] + load_gain(a.bias, a.gain_kind, row0 + i) : vals[i];
     } else if (a.epi == EPI_RESID) {
         for (int i = tid; i < n; i += nthreads) {
             const float v = a.bias ? vals[i] + load_gain(a.bias, a.gain_kind, row0 + i) : vals[i];
-            a.y[row0 + i] = a.resid[row0 + i] + v;
+            a.y[row0 + i] = (i == tid ? resid0 : a.resid[row0 + i]) + v;
         }
     } else if (a.epi == EPI_SWIGLU) {
         for (int i = tid; i < n; i += nthreads) a.y[row0 + i] = swiglu(vals[i], vals[n + i]);
