@@ -42,7 +42,8 @@ constexpr int kApQBytes = kAtHD / 8 * kApGroup;     // per Q term
 // swizzle).  So a copy's 32-byte sectors stay together on their way into shared memory: as single 16-byte pieces (no swizzle) a warp's copy of 512 bytes took 30 clocks.
 constexpr int kApHalf = 128 * 128, kApOperand = 2 * kApHalf;
 constexpr int kApOffK = 0, kApOffV = 2 * kApOperand, kApOffQ = 4 * kApOperand, kApOffMisc = kApOffQ + 2 * kApQBytes;
-constexpr int kApSmem = kApOffMisc + 128 + 2 * 4 * 128 * 4;       // barriers, slot, flags; per-row exchange of maxima (two tiles in turn) / sums
+constexpr int kApTab = 288;                        // floats of a quarter's bias table: two heads of 16 + 127 distances at most
+constexpr int kApSmem = kApOffMisc + 128 + 2 * 4 * 128 * 4 + 4 * kApTab * 4;       // barriers, slot, flags; per-row exchange of maxima (two tiles in turn) / sums; biases
 
 // kind::f16, bf16 x bf16 -> f32; b_mn: the B operand is MN-major (V as stored: the head dimension contiguous)
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, bool b_mn) {
@@ -112,7 +113,23 @@ __device__ __forceinline__ void split2_rn(float x0, float x1, uint32_t* hi, uint
 // G = query heads per KV head (1, 2, 4 or 8): MMA row r = g * QT + qi is query row q0 + qi of head kvh * G + g.
 // Measured, 32 / 8 heads of 128: 4096 rows from position 0 1278 -> 326 us (422 issued TFLOP/s), 387 rows behind 1021 positions 119 -> 36 us.  What a tile waits for now
 // is its K and V: LDGSTS of 512 bytes per 24 clocks.
-__global__ void __launch_bounds__(kApThreads, 1) attn_prompt_tc(const AttnRowsArgs a, int G) {
+//
+// BAND: the layers described one by one whose heads have this size (band_is_prompt): a window or chunks of keys, queries that carry the score's factor, a distance bias
+// r1 ln(1 + r2 d), output as bf16 in the operand of the next product.  The bias is evaluated once per (head, distance) of a tile, by the four warps that share
+// the head's rows, for the tile after this one.  Measured, 4096 rows of 32 / 8 heads, window 4096, biased: 936 us as tiles of attn_band_tc, 407 us.
+struct PromptArgs {
+    const float* q;                                            // [M][n_kv * G * 128]
+    const void *k_cache, *v_cache;
+    KvPages pg;
+    const int* row_pos; int seq0;
+    int M, n_kv, max_seq;
+    float scale;                                               // of the scores, log2 e included
+    float* out;                                                // [M][n_kv * G * 128]
+    int window, chunk; const float *r1, *r2; RowOperand op;    // BAND
+    uint32_t* status;
+};
+template <bool BAND>
+__global__ void __launch_bounds__(kApThreads, 1) attn_prompt_tc(const PromptArgs a, int G) {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kvh = blockIdx.x, QT = 128 / G, q0 = (int)(gridDim.y - 1 - blockIdx.y) * QT;
@@ -120,6 +137,7 @@ __global__ void __launch_bounds__(kApThreads, 1) attn_prompt_tc(const AttnRowsAr
     const uint32_t bar_k = misc, bar_s = misc + 16, bar_p = misc + 32, bar_o = misc + 48, bar_f = misc + 64, bar_v = misc + 80;       // two of each: tile t uses number t % 2
     int* s_flag = (int*)(smem + kApOffMisc + 104);              // [0], [1]: largest position of the CTA's rows, minus the smallest; [2]: a wait ran out
     float* x_max = (float*)(smem + kApOffMisc + 128);          // [tile % 2][4 threads of a row][128 rows]
+    float* const tab = x_max + 2 * 4 * 128 + ((threadIdx.x >> 5) & 3) * kApTab;       // BAND: this quarter's heads' biases by distance
 
     if (tid == 0) {
         for (int i = 0; i < 2; i++) {
@@ -147,24 +165,27 @@ __global__ void __launch_bounds__(kApThreads, 1) attn_prompt_tc(const AttnRowsAr
     int pos_row = row_ok ? a.row_pos[m_row] : -1;
     if (pos_row >= a.max_seq) pos_row = -1;                    // flagged by the kernel that appended the row
     {
-        int hi = pos_row, lo = row_ok ? -pos_row : -0x7fffffff;
+        int hi = pos_row, lo = pos_row >= 0 ? -pos_row : -0x7fffffff;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) { hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o)); lo = max(lo, __shfl_xor_sync(0xffffffffu, lo, o)); }
         if (lane == 0 && qr == 0) { atomicMax(&s_flag[0], hi); atomicMax(&s_flag[1], lo); }
     }
     __syncthreads();
     const int pos_max = s_flag[0], pos_min = -s_flag[1];
-    const int n_tiles = pos_max >= 0 ? pos_max / kApKT + 1 : 0;
+    // no row sees a key before `low`; this row sees distances 0 .. reach - 1
+    const int low = !BAND || pos_max < 0 ? 0 : a.chunk > 0 ? pos_min / a.chunk * a.chunk : a.window > 0 && pos_min + 1 > a.window ? pos_min + 1 - a.window : 0;
+    const int reach = !BAND ? 0x7fffffff : a.chunk > 0 ? max(pos_row, 0) % a.chunk + 1 : a.window > 0 ? a.window : 0x7fffffff;
+    const int t_lo = low / kApKT, n_tiles = pos_max >= 0 ? pos_max / kApKT + 1 - t_lo : 0;
 
     const size_t row_elems = (size_t)a.n_kv * kAtHD;
     // ---- Q tile -> two bf16 operands in shared memory
-    const size_t qd = (size_t)a.n_q * kAtHD;
+    const size_t qd = (size_t)a.n_kv * G * kAtHD;
     for (int ch = tid; ch < 128 * 16; ch += kApThreads) {
         const int r = ch >> 4, c = ch & 15;                    // 16 threads read one row's 512 bytes
         const int g = r / QT, qi = r - g * QT, m = q0 + qi;
         uint4 hi = make_uint4(0u, 0u, 0u, 0u), lo = hi;
         if (m < a.M) {
-            const float4* src = (const float4*)(a.q_rot + (size_t)m * qd + ((size_t)kvh * G + g) * kAtHD + c * 8);
+            const float4* src = (const float4*)(a.q + (size_t)m * qd + ((size_t)kvh * G + g) * kAtHD + c * 8);
             const float4 v0 = src[0], v1 = src[1];
             split2(v0.x, v0.y, &hi.x, &lo.x); split2(v0.z, v0.w, &hi.y, &lo.y);
             split2(v1.x, v1.y, &hi.z, &lo.z); split2(v1.z, v1.w, &hi.w, &lo.w);
@@ -230,7 +251,7 @@ __global__ void __launch_bounds__(kApThreads, 1) attn_prompt_tc(const AttnRowsAr
             dst += (uint32_t)(t & 1) * kApOperand + ((lane >> 3) & 1) * kApHalf + k0 * 128;
 #pragma unroll 1
             for (int h = 0; h < 2; h++, dst += 64 * 128) {
-                const int j0 = t * kApKT + h * 64, live = min(64, pos_max + 1 - j0);
+                const int j0 = (t_lo + t) * kApKT + h * 64, live = min(64, pos_max + 1 - j0);
                 const __nv_bfloat16* src = (const __nv_bfloat16*)cache + (size_t)kvh * kAtHD + (lane & 15) * 8;
                 if (live > 0) src += kv_phys_row(a.pg, a.seq0, a.max_seq, j0) * row_elems;
 #pragma unroll
@@ -266,7 +287,7 @@ __global__ void __launch_bounds__(kApThreads, 1) attn_prompt_tc(const AttnRowsAr
 #pragma unroll
     for (int i = 0; i < 32; i++) o[i] = 0.0f;
     float m_run = -INFINITY, l_run = 0.0f, alpha = 1.0f;
-    const float scale = kLog2e / sqrtf((float)kAtHD);          // weights are powers of two
+    const float scale = a.scale;                               // weights are powers of two
     const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(qr * 32);
     auto add_output = [&](int t) {                             // O = O alpha(t) + O_t
         wait(bar_o, t);
@@ -280,6 +301,17 @@ __global__ void __launch_bounds__(kApThreads, 1) attn_prompt_tc(const AttnRowsAr
         arrive(bar_f, t);
     };
 
+    // BAND: the 32 rows of a quarter belong to one head or to 32 / QT of them, QT rows (at most 32 here) each; entry x of a head is distance d0 + x
+    const int tq = min(QT, 32), tw = tq + kApKT - 1, in_head = (row & 31) % tq;
+    auto fill_tab = [&](int t) {
+        const int d0 = a.row_pos[min(q0 + ((warp & 3) * 32) % QT, a.M - 1)] - (t_lo + t) * kApKT - (kApKT - 1);      // first row, last key (rows are consecutive positions)
+        for (int x = qr * 32 + lane; x < (32 / tq) * tw; x += 128) {
+            const int g = x / tw, h = kvh * G + ((warp & 3) * 32) / QT + g;
+            tab[x] = a.r1[h] * logf(fmaf(a.r2[h], (float)max(d0 + x - g * tw, 0), 1.0f));
+        }
+    };
+    const bool biased = BAND && a.r1 != nullptr;
+    if (biased && softmax && n_tiles > 0) fill_tab(0);
 #pragma unroll 1
     for (int t = softmax ? 0 : n_tiles; t < n_tiles; t++) {
         wait(bar_s, t);
@@ -288,10 +320,16 @@ __global__ void __launch_bounds__(kApThreads, 1) attn_prompt_tc(const AttnRowsAr
         tmem_ld32(mine + (uint32_t)(t & 1) * 128u, v);
         tmem_ld_wait();
         float mx = -INFINITY;
-        const int j0 = t * kApKT + qr * 32;
-        if (t * kApKT + kApKT - 1 > pos_min) {                 // some row does not see all of the tile
+        const int dist0 = pos_row - ((t_lo + t) * kApKT + qr * 32);          // distance of this thread's first key
+        if (biased) {
+            named_sync(1 + (warp & 3), 128);                   // the table is there
+            const float* my = tab + ((row & 31) / tq) * tw + in_head + kApKT - 1 - qr * 32;
 #pragma unroll
-            for (int i = 0; i < 32; i++) if (j0 + i > pos_row) v[i] = 0xff800000u;
+            for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) - my[-i]);
+        }
+        if (__any_sync(0xffffffffu, dist0 < 31 || dist0 >= reach)) {         // some key of some row of the warp is out of sight
+#pragma unroll
+            for (int i = 0; i < 32; i++) if (dist0 - i < 0 || dist0 - i >= reach) v[i] = 0xff800000u;
         }
 #pragma unroll
         for (int i = 0; i < 32; i++) mx = fmaxf(mx, __uint_as_float(v[i]));
@@ -315,6 +353,7 @@ __global__ void __launch_bounds__(kApThreads, 1) attn_prompt_tc(const AttnRowsAr
         tmem_st_wait();
         tc_fence_before_sync();
         arrive(bar_p, t);
+        if (biased && t + 1 < n_tiles) fill_tab(t + 1);        // (this tile's has been read: the maxima were exchanged since)
         if (t > 0) add_output(t - 1);
         alpha = alpha_t;
     }
@@ -328,9 +367,23 @@ __global__ void __launch_bounds__(kApThreads, 1) attn_prompt_tc(const AttnRowsAr
     const float l_tot = (x_max[row] + x_max[128 + row]) + (x_max[256 + row] + x_max[384 + row]);
     if (row_ok) {
         const float inv = l_tot > 0.0f ? 1.0f / l_tot : 0.0f;
-        float4* dst = (float4*)(a.out + (size_t)m_row * qd + ((size_t)kvh * G + g_row) * kAtHD + qr * 32);
+        const int col = (kvh * G + g_row) * kAtHD + qr * 32;
+        if (BAND) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) dst[i] = make_float4(o[4 * i] * inv, o[4 * i + 1] * inv, o[4 * i + 2] * inv, o[4 * i + 3] * inv);
+            for (int c = 0; c < 4; c++) {
+                uint32_t w[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const __nv_bfloat162 b = __floats2bfloat162_rn(o[c * 8 + 2 * i] * inv, o[c * 8 + 2 * i + 1] * inv);
+                    w[i] = *(const uint32_t*)&b;
+                }
+                *(uint4*)((unsigned char*)a.op.p + row_operand_off(WK_BF16, a.op.chunks, m_row, col + c * 8)) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+        } else {
+            float4* dst = (float4*)(a.out + (size_t)m_row * qd + col);
+#pragma unroll
+            for (int i = 0; i < 8; i++) dst[i] = make_float4(o[4 * i] * inv, o[4 * i + 1] * inv, o[4 * i + 2] * inv, o[4 * i + 3] * inv);
+        }
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -346,9 +399,29 @@ bool attn_prompt_tc_supported(const AttnRowsArgs& a) {
 cudaError_t launch_attn_prompt_tc(const AttnRowsArgs& a, cudaStream_t st) {
     if (!attn_prompt_tc_supported(a)) return cudaErrorInvalidValue;
     static std::atomic<uint64_t> raised{0};
-    if (const cudaError_t e = allow_smem(raised, (const void*)attn_prompt_tc, kApSmem)) return e;
+    if (const cudaError_t e = allow_smem(raised, (const void*)attn_prompt_tc<false>, kApSmem)) return e;
     const int G = a.n_q / a.n_kv, QT = 128 / G;
-    attn_prompt_tc<<<dim3(a.n_kv, (a.M + QT - 1) / QT), kApThreads, kApSmem, st>>>(a, G);
+    PromptArgs b{};
+    b.q = a.q_rot; b.k_cache = a.k_cache; b.v_cache = a.v_cache; b.pg = a.pg; b.row_pos = a.row_pos; b.seq0 = a.seq0; b.M = a.M; b.n_kv = a.n_kv; b.max_seq = a.max_seq;
+    b.scale = kLog2e / sqrtf((float)kAtHD); b.out = a.out; b.status = a.status;
+    attn_prompt_tc<false><<<dim3(a.n_kv, (a.M + QT - 1) / QT), kApThreads, kApSmem, st>>>(b, G);
+    return cudaGetLastError();
+}
+
+// Whether a band layer runs as attn_prompt_tc<true>: one map, heads of 128, 1, 2, 4 or 8 query heads per K/V head.  (Everything else: attn_band_tc.)
+static bool band_is_prompt(const BandArgs& a) {
+    const QkvArgs& p = a.p;
+    const int R = p.n_kv > 0 ? p.n_q / p.n_kv : 0;
+    return p.maps <= 1 && p.dk == kAtHD && p.dv == kAtHD && p.dkp == kAtHD && p.dvp == kAtHD && (R == 1 || R == 2 || R == 4 || R == 8) && ((uintptr_t)a.q & 15) == 0;
+}
+static cudaError_t launch_band_as_prompt(const BandArgs& a, cudaStream_t st) {
+    static std::atomic<uint64_t> raised{0};
+    if (const cudaError_t e = allow_smem(raised, (const void*)attn_prompt_tc<true>, kApSmem)) return e;
+    const int G = a.p.n_q / a.p.n_kv, QT = 128 / G;
+    PromptArgs b{};
+    b.q = a.q; b.k_cache = a.k_cache; b.v_cache = a.v_cache; b.pg = a.pg; b.row_pos = a.row_pos; b.seq0 = a.seq0; b.M = a.M; b.n_kv = a.p.n_kv; b.max_seq = a.max_seq;
+    b.scale = kLog2e; b.window = a.window; b.chunk = a.chunk; b.r1 = a.r1; b.r2 = a.r2; b.op = a.out; b.status = a.status;
+    attn_prompt_tc<true><<<dim3(a.p.n_kv, (a.M + QT - 1) / QT), kApThreads, kApSmem, st>>>(b, G);
     return cudaGetLastError();
 }
 
@@ -696,6 +769,7 @@ bool band_prompt_tc_supported(const BandArgs& a) {
 
 cudaError_t launch_band_prompt_tc(const BandArgs& a, cudaStream_t st) {
     if (!band_prompt_tc_supported(a)) return cudaErrorInvalidValue;
+    if (band_is_prompt(a)) return launch_band_as_prompt(a, st);
     const int dvh = (a.p.dvp / 2 + 15) / 16 * 16;
     const void* fn = dvh <= 16 ? (const void*)attn_band_tc<16> : dvh <= 32 ? (const void*)attn_band_tc<32> : dvh <= 64 ? (const void*)attn_band_tc<64>
                      : dvh <= 96 ? (const void*)attn_band_tc<96> : (const void*)attn_band_tc<128>;

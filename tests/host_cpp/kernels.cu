@@ -1,5 +1,6 @@
 // Kernels called through the library's own launchers, without a model around them, against sums in 64 bits.  One check per command; prints a line
 // per case: name, largest or relative error, bound.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -8,6 +9,7 @@
 #include <string>
 #include <vector>
 
+#include "lum_dense.cuh"
 #include "lum_moe.cuh"
 #include "lum_rows.cuh"
 
@@ -157,6 +159,62 @@ static void attention_prompt() {
         // queries and weights keep 2^-17 of themselves in two bf16 terms; a score of 128 products then moves by less than 2^-17 on average, and a sum of
         // 16 instructions is cut to 24 bits that many times
         report(std::to_string(c.nq) + " / " + std::to_string(c.nkv) + " heads, rows " + std::to_string(c.first) + " + " + std::to_string(c.rows) + (c.pages ? ", pages" : ""), rel(out.get(), want), std::exp2(-16.0));
+        report("status", status.get()[0], 0);
+    }
+}
+
+// The same kernel for layers described one by one: windows, chunks, a bias by distance, one to eight query heads per K/V head.
+static void attention_band() {
+    struct Case { int nq, nkv, rows, first, window, chunk; bool bias; };
+    const std::vector<Case> cases = {{4, 4, 130, 0, 0, 0, true},      {8, 4, 65, 300, 128, 0, true},  {8, 2, 97, 1000, 300, 0, true}, {8, 1, 50, 255, 1, 0, true},
+                                     {8, 2, 129, 511, 512, 0, false}, {8, 1, 33, 127, 0, 100, true},  {4, 2, 200, 64, 0, 256, false}, {4, 1, 40, 900, 129, 0, true}};
+    for (const Case& c : cases) {
+        const int hd = 128, n = c.first + c.rows, max_seq = (n + 63) / 64 * 64, G = c.nq / c.nkv, chunks = c.nq * hd / 64;
+        std::mt19937 rng(n * 5 + c.nq + c.window);
+        const size_t ld = (size_t)c.nkv * hd, qd = (size_t)c.nq * hd;
+        const std::vector<float> q = normal(rng, (size_t)c.rows * qd, 0.09f);
+        const std::vector<uint16_t> k = to_bf16(normal(rng, max_seq * ld, 1.0f)), v = to_bf16(normal(rng, max_seq * ld, 1.0f, 0.5f));
+        std::vector<float> r1(c.nq), r2(c.nq);
+        for (int h = 0; h < c.nq; h++) { r1[h] = 0.1f + 0.2f * h; r2[h] = 0.05f + 0.07f * h; }
+        std::vector<int> pos(c.rows);
+        for (int i = 0; i < c.rows; i++) pos[i] = c.first + i;
+        const int rows_up = (c.rows + 127) / 128 * 128;
+        Dev<float> dq(q), d1(r1), d2(r2);
+        Dev<uint16_t> kc(k), vc(v), out((size_t)rows_up * qd);
+        Dev<int> dpos(pos);
+        Dev<uint32_t> status(1);
+        BandArgs a{};
+        a.p.n_q = c.nq; a.p.n_kv = c.nkv; a.p.dk = a.p.dv = a.p.dkp = a.p.dvp = hd; a.p.maps = 1;
+        a.q = dq.p; a.k_cache = kc.p; a.v_cache = vc.p; a.kv_bf16 = 1; a.row_pos = dpos.p; a.M = c.rows; a.window = c.window; a.chunk = c.chunk; a.max_seq = max_seq; a.max_batch = 1;
+        if (c.bias) { a.r1 = d1.p; a.r2 = d2.p; }
+        a.out_kind = WK_BF16; a.out.p = out.p; a.out.chunks = chunks; a.status = status.p;
+        CK(launch_band_prompt_tc(a, nullptr));
+        const std::vector<uint16_t> raw = out.get();
+        std::vector<float> got(q.size());
+        std::vector<double> want(q.size()), w(n);
+        for (int m = 0; m < c.rows; m++)
+            for (size_t e = 0; e < qd; e++)
+                got[m * qd + e] = bf16_value(raw[((((size_t)(m >> 7) * chunks + (e >> 6)) * 16 + ((m & 127) >> 3)) * 1024 + ((e >> 3) & 7) * 128 + (m & 7) * 16 + (e & 7) * 2) / 2]);
+        for (int m = 0; m < c.rows; m++)
+            for (int h = 0; h < c.nq; h++) {
+                const size_t col = (size_t)(h / G) * hd, row = (size_t)m * qd + (size_t)h * hd;
+                int j0 = 0;
+                if (c.window) j0 = std::max(0, pos[m] + 1 - c.window);
+                if (c.chunk) j0 = pos[m] / c.chunk * c.chunk;
+                double mx = -INFINITY, l = 0;
+                for (int j = j0; j <= pos[m]; j++) {
+                    double d = 0;
+                    for (int e = 0; e < hd; e++) d += (double)q[row + e] * bf16_value(k[j * ld + col + e]);
+                    w[j] = d - (c.bias ? r1[h] * std::log1p((double)r2[h] * (pos[m] - j)) : 0.0);
+                    mx = std::fmax(mx, w[j]);
+                }
+                for (int j = j0; j <= pos[m]; j++) l += w[j] = std::exp(w[j] - mx);
+                for (int j = j0; j <= pos[m]; j++)
+                    for (int e = 0; e < hd; e++) want[row + e] += w[j] / l * bf16_value(v[j * ld + col + e]);
+            }
+        // outputs are rounded to bf16: at most 2^-9 of each
+        report(std::to_string(c.nq) + " / " + std::to_string(c.nkv) + " heads, rows " + std::to_string(c.first) + " + " + std::to_string(c.rows) + ", window " + std::to_string(c.window) + ", chunk " +
+               std::to_string(c.chunk) + (c.bias ? ", bias" : ""), rel(got, want), std::exp2(-9.0));
         report("status", status.get()[0], 0);
     }
 }
@@ -499,6 +557,7 @@ int main(int argc, char** argv) {
     if (what == "attention-sums") attention_sums();
     else if (what == "attention-specials") attention_specials();
     else if (what == "attention-prompt") attention_prompt();
+    else if (what == "attention-band") attention_band();
     else if (what == "experts") experts();
     else if (what == "matvec-bf16") matvec_bf16();
     else if (what == "matvec-q8") matvec_q8();
