@@ -132,9 +132,11 @@ __device__ __forceinline__ bool phase_gemv(const MegaArgs& a, const MegaLayer& L
             g.seg[0] = {L.wg, nullptr, a.ffn, a.kc_h}; g.seg[1] = {L.wu, nullptr, a.ffn, a.kc_h};
             g.gain = L.mlp_norm; g.y = a.h;
             break;
-        case 4:   // down projection + residual
-            g.K = a.ffn; g.KC = a.kc_f; g.epi = EPI_RESID; g.nseg = 1; g.seg[0] = {L.wd, nullptr, H, a.kc_f};
-            g.y = a.x; g.resid = a.x;
+        case 4:   // down projection: its K ranges' partial vectors join the residual stream in the next prologue; one range: + residual
+            g.K = a.ffn; g.KC = a.kc_f; g.nseg = 1; g.seg[0] = {L.wd, nullptr, H, a.kc_f};
+            g.ksplit = gemv_k_ranges(a.ffn, a.kc_f);
+            if (g.ksplit > 1) { g.epi = EPI_STORE; g.y = a.part; g.y_range_stride = a.part_ld; }
+            else { g.epi = EPI_RESID; g.y = a.x; g.resid = a.x; }
             break;
         default:  // final RMSNorm + vocabulary projection + greedy sample
             g.K = H; g.KC = a.kc_h; g.epi = EPI_ARGMAX; g.nseg = 1; g.seg[0] = {a.lm_head, nullptr, a.vocab, a.kc_h};
@@ -163,6 +165,8 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_mega(const MegaArgs a)
     unsigned long long pseq = a.gbar_base;            // running phase number: picks the job-claim counter of each phase
     bool producing = true;
     int pos = 0, tok = 0;
+    bool second = false;                              // the residual stream is in a.x2
+    int pending = 0;                                  // partial vectors that have not joined it yet
     if (is_worker) {
         pos = a.state->pos;
         tok = a.forced ? a.forced[0] : a.state->tok;
@@ -188,11 +192,11 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_mega(const MegaArgs a)
             const bool streams = phase_gemv(a, L, p, &ga);
             GemvPlan plan{};
             if (streams) plan = gemv_plan(ga, cta, ncta, 750);
-            unsigned int* ctr = a.job_ctr + (pseq % kJobCtrRing);
+            unsigned int* ctr = a.job_ctr + (pseq % kJobCtrRing) * kMaxKRanges + plan.range;
             // Re-zero the claim counter that phase pseq + 32 will use: its last user was phase pseq - 32, and no CTA can
             // be that far behind or ahead (a producer leads its consumers by at most one ring of stages, each phase
             // taking at least one).  Every phase does this, whether or not it streams weights itself.
-            if (cta == 0 && tid == 0) a.job_ctr[(pseq + kJobCtrRing / 2) % kJobCtrRing] = 0u;
+            if (cta == 0 && tid < kMaxKRanges) a.job_ctr[(pseq + kJobCtrRing / 2) % kJobCtrRing * kMaxKRanges + tid] = 0u;
             pseq++;
             if (is_producer) {
                 if (streams && elect_one() && producing) {
@@ -204,15 +208,25 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_mega(const MegaArgs a)
                 grid_barrier(a, seq, &s_abort, tid);
             } else {
                 XSource xs{};
-                if (ph == 0) { xs.table = a.embed; xs.table_kind = a.embed_kind; xs.token = tok; xs.x_out = a.x; }   // the embedding row is x
-                else xs.x = p == 2 ? a.attn : p == 4 ? a.h : a.x;
+                // the residual stream lives in a.x or a.x2, and moves to the other when partial vectors join it
+                if (ph == 0) { xs.table = a.embed; xs.table_kind = a.embed_kind; xs.token = tok; xs.x_out = a.x; second = false; pending = 0; }   // the embedding row is x
+                else xs.x = p == 2 ? a.attn : p == 4 ? a.h : second ? a.x2 : a.x;
+                if (pending && (p == 0 || p == 5)) {
+                    xs.parts = a.part; xs.n_parts = pending; xs.part_stride = a.part_ld;
+                    if (p == 0) { xs.x_out = second ? a.x : a.x2; second = !second; }
+                    pending = 0;
+                }
+                if (ga.epi == EPI_RESID) ga.y = second ? a.x2 : a.x;
+                ga.resid = ga.y;
+                if (p == 4 && ga.ksplit > 1) pending = ga.ksplit;
                 ArgBest best{-INFINITY, -1};
                 if (!s_abort) {
                     if (p == 0) attn_phase_prefetch<HD, GM, BF16>(a, L, pos, tid);
                     if (tid < kConsumers) {
                         GainRegs gr;
                         gemv_gain_preload(ga, tid, gr);
-                        gemv_consume<false, false>(ga, xs, cta == 0, plan, g, cring, tid, a.status, &best, gr);
+                        if (plan.nt > kFillTiles && plan.nt <= kJobTiles) gemv_consume<false, true>(ga, xs, cta == 0, plan, g, cring, tid, a.status, &best, gr);
+                        else gemv_consume<false, false>(ga, xs, cta == 0, plan, g, cring, tid, a.status, &best, gr);
                     }
                 }
                 if (p == 5 && tid == 0) { a.part_val[cta] = best.v; a.part_idx[cta] = best.i; }

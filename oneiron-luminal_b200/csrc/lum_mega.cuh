@@ -23,7 +23,8 @@ struct MegaArgs {
     const void* embed;
     const void* final_norm;
     const unsigned char* lm_head; // packed; for tied heads the caller keeps a packed copy
-    float *x, *qkv, *attn, *h, *logits;
+    float *x, *x2, *qkv, *attn, *h, *logits;
+    float* part; int part_ld;     // partial vectors of the down projection's K ranges (gemv_k_ranges)
     float* attn_part;
     unsigned int* attn_cnt;
     float* part_val;
@@ -35,7 +36,7 @@ struct MegaArgs {
     int head_every_token;         // 1: sample after every token (decode); 0: only after the last (prompt processing)
     int n_splits;
     int stages;
-    unsigned int* job_ctr;        // [kJobCtrRing] job-claim counters, one per phase in flight (zero before first use)
+    unsigned int* job_ctr;        // [kJobCtrRing][kMaxKRanges] job-claim counters of the phases in flight (zero before first use)
     unsigned long long* gbar;     // grid-barrier arrival counter ([0]) and completed-barrier count ([16])
     unsigned long long gbar_base; // barriers passed since the counter was zeroed
     int* abort_flag;              // kernel-wide: some wait ran out of budget

@@ -518,7 +518,7 @@ int check_status(lum_rt* rt) {
         if (rt->gbar) {   // an aborted persistent launch leaves its barrier count short: start over
             cudaMemsetAsync(rt->gbar, 0, 32 * sizeof(unsigned long long), rt->stream);
             cudaMemsetAsync(rt->abort_flag, 0, sizeof(int), rt->stream);
-            cudaMemsetAsync(rt->job_ctr, 0, kJobCtrRing * sizeof(unsigned int), rt->stream);
+            cudaMemsetAsync(rt->job_ctr, 0, (size_t)kJobCtrRing * kMaxKRanges * sizeof(unsigned int), rt->stream);
             rt->gbar_base = 0;
         }
         return fail(rt, LUM_E_DEVICE, "device status 0x%x (%s%s%s%s%s%s)", st, (st & LUM_ST_WAIT_GRID) ? "grid barrier timed out; " : "",
@@ -2023,12 +2023,16 @@ int setup_mega(lum_rt* rt) {
     a.kc_h = rt->L[0].q.kc; a.kc_o = rt->L[0].o.kc; a.kc_f = rt->L[0].down.kc;
     a.k_max = d.hidden;
     if (rt->nq_l * d.head_dim > a.k_max) a.k_max = rt->nq_l * d.head_dim;
-    if (rt->ffn_l > a.k_max) a.k_max = rt->ffn_l;
+    {   // the longest vector a CTA holds: the down projection's is a K range
+        const int tpr = rt->ffn_l / 512, r = gemv_k_ranges(rt->ffn_l, a.kc_f), f = r > 1 ? (tpr + r - 1) / r * 512 : rt->ffn_l;
+        if (f > a.k_max) a.k_max = f;
+        if (r > 1 && rt->sm_count < tpr) return 0;
+    }
     a.gain_kind = kind_of(d.embed_dtype); a.embed_kind = rt->embed.kind; a.kv_bf16 = d.kv_dtype == LUM_BF16; a.rope_style = d.rope_style;
     a.eps = rt->eps6; a.qk_eps = d.rms_eps; a.theta = d.rope_theta;
     a.c_inv_d = rt->c_inv_d; a.c_ln_theta = rt->c_ln_theta; a.c_log2e = rt->c_log2e; a.c_half_pi = rt->c_half_pi;
     a.embed = rt->embed.w; a.final_norm = rt->final_norm.w; a.lm_head = (const unsigned char*)rt->lm_head.w;
-    a.x = rt->x; a.qkv = rt->qkv; a.attn = rt->attn; a.h = rt->h; a.logits = rt->logits;
+    a.x = rt->x; a.x2 = rt->x2; a.part = rt->part; a.part_ld = rt->part_ld; a.qkv = rt->qkv; a.attn = rt->attn; a.h = rt->h; a.logits = rt->logits;
     a.attn_part = rt->attn_part; a.attn_cnt = rt->attn_cnt; a.part_val = rt->am_val; a.part_idx = rt->am_idx;
     a.state = rt->state; a.tokens_out = rt->tokens_out;
     a.n_splits = rt->n_splits;
@@ -2039,8 +2043,8 @@ int setup_mega(lum_rt* rt) {
     if (int r = dev_alloc(rt, (void**)&rt->forced_dev, (size_t)d.max_seq * sizeof(int))) return r;
     if (int r = dev_alloc(rt, (void**)&rt->gbar, 32 * sizeof(unsigned long long))) return r;   // [0] arrivals, [16] generation
     if (int r = dev_alloc(rt, (void**)&rt->abort_flag, sizeof(int))) return r;
-    if (int r = dev_alloc(rt, (void**)&rt->job_ctr, kJobCtrRing * sizeof(unsigned int))) return r;
-    CU(rt, cudaMemsetAsync(rt->job_ctr, 0, kJobCtrRing * sizeof(unsigned int), rt->stream));
+    if (int r = dev_alloc(rt, (void**)&rt->job_ctr, (size_t)kJobCtrRing * kMaxKRanges * sizeof(unsigned int))) return r;
+    CU(rt, cudaMemsetAsync(rt->job_ctr, 0, (size_t)kJobCtrRing * kMaxKRanges * sizeof(unsigned int), rt->stream));
     CU(rt, cudaMemcpyAsync(rt->mega_layers, hl.data(), hl.size() * sizeof(MegaLayer), cudaMemcpyHostToDevice, rt->stream));
     CU(rt, cudaMemsetAsync(rt->gbar, 0, 32 * sizeof(unsigned long long), rt->stream));
     CU(rt, cudaMemsetAsync(rt->abort_flag, 0, sizeof(int), rt->stream));
