@@ -306,7 +306,7 @@ bool gemv_stream_supported(const GemvArgs& a) {
     return true;
 }
 
-static cudaError_t launch_with_attrs(const void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, GemvArgs& a) {
+static cudaError_t launch_with_attrs(const void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t st, GemvArgs& a) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -316,7 +316,7 @@ static cudaError_t launch_with_attrs(const void* fn, dim3 grid, dim3 block, size
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = a.use_pdl && !a.ordered ? 1 : 0;
     void* params[] = {&a};
     return cudaLaunchKernelExC(&cfg, fn, params);
 }
@@ -374,7 +374,7 @@ cudaError_t launch_gemv(const GemvArgs& a_in, int sm_count, cudaStream_t st) {
                               : (one ? (const void*)q8_gemv_stream<false, true> : (const void*)q8_gemv_stream<false, false>);
         static std::atomic<uint64_t> raised[4] = {};
         if (const cudaError_t e = allow_smem(raised[(peer ? 2 : 0) + one], fn, (int)kAll, true)) return e;
-        return launch_with_attrs(fn, dim3(grid), dim3(kGemvThreads), smem, st, a.use_pdl != 0, a);
+        return launch_with_attrs(fn, dim3(grid), dim3(kGemvThreads), smem, st, a);
     }
 
     if (a.ksplit > 1) return cudaErrorInvalidValue;      // the caller's consumer expects several partial vectors: only the streaming kernel makes them
@@ -393,7 +393,7 @@ cudaError_t launch_gemv(const GemvArgs& a_in, int sm_count, cudaStream_t st) {
         if (e != cudaSuccess) return e;
         if (smem > 200 * 1024) return cudaErrorInvalidValue;
     }
-    return launch_with_attrs(fn, dim3(grid), dim3(256), smem, st, a.use_pdl != 0, a);
+    return launch_with_attrs(fn, dim3(grid), dim3(256), smem, st, a);
 }
 
 }  // namespace lum

@@ -75,6 +75,8 @@ struct GemvArgs {
     int k_smem;            // activations a CTA holds: K, or the longest K range (set by the launcher)
     int max_units;         // tuning override: 1 + extra jobs a CTA may claim beyond its even share (0 = default)
     int use_pdl;
+    int ordered;           // 1: starts in plain stream order behind the kernel before it, whose stores its producers then see without waiting (use_pdl still lets
+                           // its own successor come early)
     int force_direct;      // 1: never take the streaming kernel (operator tests compare the two)
     unsigned int* job_ctr; // streaming kernel: zeroed counters the producers claim pooled jobs from, one per K range (null: static split)
     int ksplit;            // > 1: EPI_STORE over one long-K matrix cut into that many K ranges, each worked on by its own CTAs (which then hold
@@ -158,8 +160,8 @@ struct EmbedArgs {
     const DecodeState* state;
     uint32_t* status;
     int use_pdl;
-    unsigned int* zero_ctr;// optional: n_zero words zeroed by this kernel (the step's job-claim counters: nothing of the previous step still runs, nothing of
-    int n_zero;            // this one starts before it is over)
+    unsigned int* zero_ctr;// optional: n_zero words zeroed by this kernel (the step's job-claim counters: nothing of the previous step still runs, and the first
+    int n_zero;            // projection is launched `ordered`: no claim of this step comes before the zeros are there)
     const double* pos_freq;// optional [ceil(H / 2)]: sin (entry 2i) and cos (2i + 1) of position * pos_freq[i] are added
 };
 // entries 2 i and 2 i + 1 of the sinusoidal position vector (angles in f64: exact to f32 rounding at any position)

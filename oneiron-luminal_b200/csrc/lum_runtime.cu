@@ -581,12 +581,13 @@ int issue_step(lum_rt* rt, bool with_head, bool pdl, int* n_launch) {
         n++;
         return 0;
     };
-    // Dynamic job claiming: projection number gi of the step claims from counters of its own, zeroed by the step's first kernel.
+    // Dynamic job claiming: projection number gi of the step claims from counters of its own, zeroed by the step's first kernel.  Producers claim without waiting
+    // for the grid dependency, which alone makes a programmatic predecessor's stores visible: the first projection starts in plain stream order, all others after it.
     const int n_proj = (d.n_experts > 0 ? 2 : 4) * d.n_layers + (with_head ? 1 : 0);     // streaming projections per step (routed experts have kernels of their own)
     int gi = 0;
     bool prev_wide = false;             // the kernel before is a projection with the wide size
     auto claim_ctr = [&](GemvArgs& g) {
-        if (rt->step_ctr) g.job_ctr = rt->step_ctr + (size_t)gi * kMaxKRanges;
+        if (rt->step_ctr) { g.job_ctr = rt->step_ctr + (size_t)gi * kMaxKRanges; g.ordered = gi == 0; }
         // Consecutive projections alternate between the two sizes of shared memory; behind a kernel of another kind the wide one
         g.wide_smem = !prev_wide;
         prev_wide = g.wide_smem != 0;
@@ -2977,8 +2978,10 @@ int32_t lum_model_init(lum_rt* rt, const lum_model_desc* dp) {
     TRY(dev_alloc(rt, (void**)&rt->attn_part, (size_t)rt->nkv_l * splits * G * (hd + 2) * 4));
     TRY(dev_alloc(rt, (void**)&rt->attn_cnt, (size_t)rt->nkv_l * 4));
     TRY(alloc_decode_state(rt));
-    TRY(dev_alloc(rt, (void**)&rt->step_ctr, ((size_t)4 * d.n_layers + 1) * kMaxKRanges * sizeof(unsigned int)));
-    cudaMemsetAsync(rt->step_ctr, 0, ((size_t)4 * d.n_layers + 1) * kMaxKRanges * sizeof(unsigned int), rt->stream);
+    if (d.weight_dtype == LUM_Q8_0) {       // (other projections claim nothing)
+        TRY(dev_alloc(rt, (void**)&rt->step_ctr, ((size_t)4 * d.n_layers + 1) * kMaxKRanges * sizeof(unsigned int)));
+        cudaMemsetAsync(rt->step_ctr, 0, ((size_t)4 * d.n_layers + 1) * kMaxKRanges * sizeof(unsigned int), rt->stream);
+    }
 #undef TRY
     cudaMemsetAsync(rt->attn_cnt, 0, (size_t)rt->nkv_l * 4, rt->stream);
 

@@ -477,6 +477,80 @@ static void matvec_q8() {
     }
 }
 
+// A step's chain: an embedding row that zeroes the claim counters, projections behind it that claim from them under programmatic launch and change places between the
+// two sizes of shared memory.  Every row of every step is there (a claim from an old count leaves rows out), and what is captured says why: the first projection
+// waits for the counters in plain stream order, the others may come early.
+static void claims() {
+    const int V = 64, H = 2560, P = 4, steps = 60;
+    const int N[P] = {2560, 1208, 4096, 264};
+    std::mt19937 rng(11);
+    Dev<float> table(normal(rng, (size_t)V * H, 1.0f)), x((size_t)H);
+    Dev<uint32_t> status(1);
+    DecodeState s{};
+    s.tok = 5; s.vocab = V;
+    Dev<DecodeState> state(std::vector<DecodeState>{s});
+    Dev<unsigned int> ctr(std::vector<unsigned int>(P * kMaxKRanges, 7u));            // (left over from a step before)
+    std::vector<Dev<unsigned char>*> packed;
+    size_t total = 0;
+    for (int n : N) {
+        std::vector<int8_t> q((size_t)n * H);
+        std::vector<__half> d((size_t)n * H / 32);
+        for (auto& v : q) v = (int8_t)((int)(rng() % 255) - 127);
+        for (auto& v : d) v = __float2half(0.001f);
+        Dev<int8_t> dq(q);
+        Dev<__half> ds(d);
+        packed.push_back(new Dev<unsigned char>(q8_packed_bytes(n, H)));
+        CK(launch_q8_pack_units(dq.p, ds.p, n, H, q8_pack_kc(n, H), packed.back()->p, nullptr));
+        CK(cudaDeviceSynchronize());
+        total += n;
+    }
+    Dev<float> y(total * (steps + 1));
+    cudaStream_t st;
+    CK(cudaStreamCreate(&st));
+    auto step = [&](int i) {
+        EmbedArgs e{};
+        e.table = table.p; e.kind = WK_F32; e.H = H; e.x = x.p; e.state = state.p; e.status = status.p; e.zero_ctr = ctr.p; e.n_zero = P * kMaxKRanges;
+        CK(launch_embed(e, st));
+        float* to = y.p + (size_t)i * total;
+        for (int p = 0; p < P; to += N[p], p++) {
+            GemvArgs a{};
+            a.nseg = 1; a.seg[0] = {packed[p]->p, nullptr, N[p], q8_pack_kc(N[p], H)}; a.K = H; a.wkind = WK_Q8; a.epi = EPI_STORE; a.x = x.p; a.y = to; a.status = status.p;
+            a.use_pdl = 1; a.job_ctr = ctr.p + p * kMaxKRanges; a.ordered = p == 0; a.wide_smem = (p & 1) == 0;
+            CK(launch_gemv(a, 148, st));
+        }
+    };
+    for (int i = 0; i < steps; i++) step(i);
+    CK(cudaStreamSynchronize(st));
+    const std::vector<float> got = y.get();
+    size_t differ = 0, zero = 0;
+    for (size_t i = 0; i < (size_t)steps * total; i++) { differ += got[i] != got[i % total]; zero += got[i] == 0.0f; }
+    report("rows of a step that differ from the first step's", (double)differ, 0);
+    report("rows that nobody wrote", (double)zero, 0);
+    report("status", status.get()[0], 0);
+
+    cudaGraph_t graph;
+    CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    step(steps);
+    CK(cudaStreamEndCapture(st, &graph));
+    size_t n = 0;
+    CK(cudaGraphGetEdges_v2(graph, nullptr, nullptr, nullptr, &n));
+    std::vector<cudaGraphNode_t> from(n), to(n);
+    std::vector<cudaGraphEdgeData> how(n);
+    CK(cudaGraphGetEdges_v2(graph, from.data(), to.data(), how.data(), &n));
+    report("edges", std::fabs((double)n - P), 0);
+    int programmatic = 0;
+    for (size_t i = 0; i < n; i++) {
+        const bool first = std::find(to.begin(), to.end(), from[i]) == to.end();          // an edge from the embedding
+        const bool pdl = how[i].type == cudaGraphDependencyTypeProgrammatic;
+        programmatic += pdl;
+        if (first) report("the first projection in plain order", pdl, 0);
+    }
+    report("the others programmatic", std::fabs(programmatic - (P - 1.0)), 0);
+    CK(cudaGraphDestroy(graph));
+    CK(cudaStreamDestroy(st));
+    for (auto* p : packed) delete p;
+}
+
 // Two to five rows: rows formed and quantised (plain, behind a norm, SwiGLU of two sums; planes, residual), then multiplied; every number of tiles, K ranges.
 static void few_rows() {
     struct Case { std::vector<int> rows; int k, m, planes; bool norm, pair; };
@@ -561,6 +635,7 @@ int main(int argc, char** argv) {
     else if (what == "experts") experts();
     else if (what == "matvec-bf16") matvec_bf16();
     else if (what == "matvec-q8") matvec_q8();
+    else if (what == "claims") claims();
     else if (what == "few-rows") few_rows();
     else { std::printf("unknown check\n"); return 2; }
     return failures ? 1 : 0;
