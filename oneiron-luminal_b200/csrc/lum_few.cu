@@ -37,12 +37,8 @@ __global__ void __launch_bounds__(256) rows_levels(const RowsArgs a, const int C
     // eight consecutive threads own a block: four of its columns each
     auto store = [&](int f4, float4 v) {
         const float e[4] = {v.x, v.y, v.z, v.w};
-        float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
         uint32_t p[3];
-        const float s1 = gemv_levels(e, amax, p);
+        const float s1 = gemv_levels(e, p);
         if (f4 < n4) {
             const int blk = s0 + (f4 >> 3), j = f4 & 7;
 #pragma unroll

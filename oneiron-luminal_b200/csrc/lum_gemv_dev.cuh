@@ -435,8 +435,13 @@ __device__ __forceinline__ GemvPlan gemv_plan(const GemvArgs& a, int cta, int n_
     return p;
 }
 
-// Four elements of a block whose largest magnitude is amax -> four bytes of each level; returns the block's scale.
-__device__ __forceinline__ float gemv_levels(const float (&e)[4], float amax, uint32_t (&p)[3]) {
+// Four elements of a block that eight consecutive threads share -> four bytes of each level; returns the block's scale.  A block with an infinite or undefined
+// element has no levels: its scale is NaN, and with it every sum that the block is part of.
+__device__ __forceinline__ float gemv_levels(const float (&e)[4], uint32_t (&p)[3]) {
+    float amax = max_nan(max_nan(fabsf(e[0]), fabsf(e[1])), max_nan(fabsf(e[2]), fabsf(e[3])));
+    amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
     const float s1 = amax * (1.0f / 127.0f);
     const float i1 = amax > 0.0f ? 127.0f / amax : 0.0f;
     const float s2 = s1 * (1.0f / 254.0f), i2 = i1 * 254.0f;
@@ -457,7 +462,7 @@ __device__ __forceinline__ float gemv_levels(const float (&e)[4], float amax, ui
         p[1] |= (__float_as_uint(t2) & 0xffu) << (8 * j);
         p[2] |= (__float_as_uint(t3) & 0xffu) << (8 * j);
     }
-    return s1;
+    return amax < INFINITY ? s1 : __int_as_float(0x7fffffff);
 }
 // Where the first level's word j (columns 4 j .. 4 j + 3) of block blk goes in the operand (gemv_load_xfrag); the other levels 16 words further on each.
 // Columns of the operand are (half of the tile, level); a block is number blk % 8 of its half.
@@ -606,12 +611,8 @@ __device__ __forceinline__ void gemv_quantize_x(const GemvArgs& a, const XSource
                     e[0] = (inv * e[0]) * gf.x; e[1] = (inv * e[1]) * gf.y; e[2] = (inv * e[2]) * gf.z; e[3] = (inv * e[3]) * gf.w;
                 }
             }
-            float amax = fmaxf(fmaxf(fabsf(e[0]), fabsf(e[1])), fmaxf(fabsf(e[2]), fabsf(e[3])));
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
             uint32_t lv[3];
-            const float s1 = gemv_levels(e, amax, lv);
+            const float s1 = gemv_levels(e, lv);
             const int blk = f4 >> 3;
             uint32_t* dst = (uint32_t*)g.xq + gemv_level_word(blk, f4 & 7);
             dst[0] = lv[0]; dst[16] = lv[1]; dst[32] = lv[2];

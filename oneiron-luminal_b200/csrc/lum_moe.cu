@@ -23,9 +23,8 @@
 namespace lum {
 
 // x[0..K) (global, f32) -> three int8 levels [3][K] and K / 32 scales in shared memory.  All `nthreads` threads (a multiple of 8)
-// call it; 8 consecutive threads own one 32-block.  Same rounding as the GEMV prologue (add-1.5*2^23 trick).
+// call it; 8 consecutive threads own one 32-block.  Same levels as the GEMV prologue's.
 __device__ __forceinline__ void x_levels_to_smem(const float* x, int K, int8_t* xq, float* xs, int tid, int nthreads) {
-    constexpr float kMagic = 12582912.0f;
     const int n4 = K >> 2;
     constexpr int kAhead = 4;                            // loads on their way before the first is used
     for (int f0 = tid; f0 < ((n4 + nthreads - 1) / nthreads) * nthreads; f0 += nthreads * kAhead) {
@@ -38,29 +37,12 @@ __device__ __forceinline__ void x_levels_to_smem(const float* x, int K, int8_t* 
         const bool in = f4 < n4;
         const float4 v = vv[u];
         const float e[4] = {v.x, v.y, v.z, v.w};
-        float amax = fmaxf(fmaxf(fabsf(e[0]), fabsf(e[1])), fmaxf(fabsf(e[2]), fabsf(e[3])));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-        const float s1 = amax * (1.0f / 127.0f);
-        const float i1 = amax > 0.0f ? 127.0f / amax : 0.0f;
-        const float s2 = s1 * (1.0f / 254.0f), i2 = i1 * 254.0f, i3 = i1 * 64516.0f;
-        uint32_t p1 = 0, p2 = 0, p3 = 0;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float t1 = fmaf(e[j], i1, kMagic);
-            const float r1 = fmaf(-s1, t1 - kMagic, e[j]);
-            const float t2 = fmaf(r1, i2, kMagic);
-            const float r2 = fmaf(-s2, t2 - kMagic, r1);
-            const float t3 = fmaf(r2, i3, kMagic);
-            p1 |= (__float_as_uint(t1) & 0xffu) << (8 * j);
-            p2 |= (__float_as_uint(t2) & 0xffu) << (8 * j);
-            p3 |= (__float_as_uint(t3) & 0xffu) << (8 * j);
-        }
+        uint32_t p[3];
+        const float s1 = gemv_levels(e, p);
         if (in) {
-            ((uint32_t*)xq)[f4] = p1;
-            ((uint32_t*)(xq + K))[f4] = p2;
-            ((uint32_t*)(xq + 2 * (size_t)K))[f4] = p3;
+            ((uint32_t*)xq)[f4] = p[0];
+            ((uint32_t*)(xq + K))[f4] = p[1];
+            ((uint32_t*)(xq + 2 * (size_t)K))[f4] = p[2];
             if ((f4 & 7) == 0) xs[f4 >> 3] = s1;
         }
       }

@@ -626,6 +626,56 @@ static void few_rows() {
     }
 }
 
+// Products on integer levels, one vector and several rows: an infinite or undefined element makes its own row undefined, as a sum over it would be, and no other.
+static void level_specials() {
+    const float inf = INFINITY, nan = std::nanf("");
+    const int N = 72;
+    for (int K : {512, 2560, 4096})
+        for (int M : {1, 2, 5}) {
+            if (M > 1 && !few_ranges(K, 148)) continue;
+            for (float special : {nan, inf, -inf}) {
+                const int nb = K / 32, bad = M - 1, at = K / 2 + 37;
+                std::mt19937 rng(K + M);
+                std::vector<float> x = normal(rng, (size_t)M * K, 1.0f);
+                x[(size_t)bad * K + at] = special;
+                std::vector<int8_t> q((size_t)N * K);
+                std::vector<__half> s((size_t)N * nb);
+                for (auto& v : q) v = (int8_t)((int)(rng() % 255) - 127);
+                for (auto& v : s) v = __float2half(0.01f);
+                std::vector<double> want((size_t)M * N);
+                for (int m = 0; m < M; m++)
+                    for (int i = 0; i < N; i++)
+                        for (int e = 0; e < K; e++) want[(size_t)m * N + i] += (double)q[(size_t)i * K + e] * x[(size_t)m * K + e] * (double)__half2float(s[(size_t)i * nb + e / 32]);
+                Dev<int8_t> dq(q);
+                Dev<__half> ds(s);
+                Dev<unsigned char> w(q8_packed_bytes(N, K));
+                CK(launch_q8_pack_units(dq.p, ds.p, N, K, q8_pack_kc(N, K), w.p, nullptr));
+                Dev<float> dx(x), y((size_t)M * N), sx(few_sx_floats(M, K));
+                Dev<int8_t> xq(few_xq_bytes(M, K));
+                Dev<uint32_t> status(1);
+                if (M == 1) {
+                    GemvArgs a{};
+                    a.nseg = 1; a.seg[0] = {w.p, nullptr, N, q8_pack_kc(N, K)}; a.K = K; a.wkind = WK_Q8; a.epi = EPI_STORE; a.x = dx.p; a.y = y.p; a.status = status.p;
+                    CK(launch_gemv(a, 148, nullptr));
+                } else {
+                    RowsArgs r{};
+                    r.a = dx.p; r.n_parts = 1; r.part_stride = (size_t)M * K; r.ld = K; r.M = M; r.K = K; r.xq = xq.p; r.sx = sx.p;
+                    CK(launch_rows_levels(r, 148, nullptr));
+                    FewArgs f{};
+                    f.nseg = 1; f.w[0] = w.p; f.rows[0] = N; f.K = K; f.M = M; f.xq = xq.p; f.sx = sx.p; f.y = y.p; f.ldy = N; f.part_stride = (size_t)M * N; f.status = status.p;
+                    CK(launch_few(f, 148, nullptr));
+                }
+                const std::vector<float> got = y.get();
+                int defined = 0;
+                for (int i = 0; i < N; i++) defined += !std::isnan(got[(size_t)bad * N + i]);
+                const std::string what = std::to_string(special) + " among " + std::to_string(K) + ", " + std::to_string(M) + " rows";
+                report(what + ": outputs of its row that look defined", defined, 0);
+                if (M > 1) report(what + ": the other rows", rel(got, std::vector<double>(want.begin(), want.begin() + (size_t)bad * N)), 16 * std::exp2(-24.0));
+                report("status", status.get()[0], 0);
+            }
+        }
+}
+
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "attention-sums") attention_sums();
@@ -637,6 +687,7 @@ int main(int argc, char** argv) {
     else if (what == "matvec-q8") matvec_q8();
     else if (what == "claims") claims();
     else if (what == "few-rows") few_rows();
+    else if (what == "level-specials") level_specials();
     else { std::printf("unknown check\n"); return 2; }
     return failures ? 1 : 0;
 }
