@@ -442,8 +442,9 @@ __device__ __forceinline__ float gemv_levels(const float (&e)[4], uint32_t (&p)[
     amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
     amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
     amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+    amax = max_nan(amax, 0x1p-104f);                     // the third level's factor, 2^23 / amax, has to stay a number (smaller elements keep an error below 2^-127)
     const float s1 = amax * (1.0f / 127.0f);
-    const float i1 = amax > 0.0f ? 127.0f / amax : 0.0f;
+    const float i1 = 127.0f / amax;
     const float s2 = s1 * (1.0f / 254.0f), i2 = i1 * 254.0f;
     const float i3 = i1 * 64516.0f;
     // Round to nearest by adding 1.5 * 2^23: the sum's low mantissa bits are the integer in two's complement,

@@ -627,17 +627,19 @@ static void few_rows() {
 }
 
 // Products on integer levels, one vector and several rows: an infinite or undefined element makes its own row undefined, as a sum over it would be, and no other.
+// A row of tiny elements (`special` 0) keeps its 24 bits, or errors below 2^-127 an element.
 static void level_specials() {
     const float inf = INFINITY, nan = std::nanf("");
     const int N = 72;
     for (int K : {512, 2560, 4096})
         for (int M : {1, 2, 5}) {
             if (M > 1 && !few_ranges(K, 148)) continue;
-            for (float special : {nan, inf, -inf}) {
+            for (float special : {nan, inf, -inf, 0.0f}) {
                 const int nb = K / 32, bad = M - 1, at = K / 2 + 37;
                 std::mt19937 rng(K + M);
                 std::vector<float> x = normal(rng, (size_t)M * K, 1.0f);
-                x[(size_t)bad * K + at] = special;
+                if (special != 0.0f) x[(size_t)bad * K + at] = special;
+                else for (int e = 0; e < K; e++) x[(size_t)bad * K + e] *= 3e-33f;
                 std::vector<int8_t> q((size_t)N * K);
                 std::vector<__half> s((size_t)N * nb);
                 for (auto& v : q) v = (int8_t)((int)(rng() % 255) - 127);
@@ -668,8 +670,11 @@ static void level_specials() {
                 const std::vector<float> got = y.get();
                 int defined = 0;
                 for (int i = 0; i < N; i++) defined += !std::isnan(got[(size_t)bad * N + i]);
-                const std::string what = std::to_string(special) + " among " + std::to_string(K) + ", " + std::to_string(M) + " rows";
-                report(what + ": outputs of its row that look defined", defined, 0);
+                const std::string what = (special == 0.0f ? "tiny ones" : std::to_string(special)) + " among " + std::to_string(K) + ", " + std::to_string(M) + " rows";
+                if (special == 0.0f)
+                    report(what, rel(std::vector<float>(got.begin() + (size_t)bad * N, got.end()), std::vector<double>(want.begin() + (size_t)bad * N, want.end())), 16 * std::exp2(-24.0) + std::exp2(-127.0) / 3e-33);
+                else
+                    report(what + ": outputs of its row that look defined", defined, 0);
                 if (M > 1) report(what + ": the other rows", rel(got, std::vector<double>(want.begin(), want.begin() + (size_t)bad * N)), 16 * std::exp2(-24.0));
                 report("status", status.get()[0], 0);
             }
