@@ -117,6 +117,11 @@ __device__ __forceinline__ bool mbar_wait_abortable(uint32_t bar, uint32_t parit
     }
 }
 
+// The same by a whole warp, with one answer for all of it: no lane is left behind at a warp instruction that the others never reach.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort) {
+    return __all_sync(0xffffffffu, mbar_wait_abortable(bar, parity, abort));
+}
+
 // ---- bulk asynchronous copy global -> shared (the untiled TMA path) -------------------------------
 // Both addresses 16-byte aligned, size a multiple of 16 bytes; completion is signalled on `bar`
 // as `bytes` of transaction count.  No multicast: every CTA fetches its own bytes.

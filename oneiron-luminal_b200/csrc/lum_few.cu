@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) q8_few(const GemvArgs a, const
     }
     __syncwarp();
     auto fail = [&](uint32_t code) { if (!s_abort) { atomicOr(a.status, code); *(volatile int*)&s_abort = 1; } };
-    if (!mbar_wait_abortable(xbar, 0u, g.abort)) fail(LUM_ST_WAIT_FULL);
+    if (!mbar_wait_warp(xbar, 0u, g.abort)) fail(LUM_ST_WAIT_FULL);
 
     const int wg = warp >> 2, wj = warp & 3, first = g.first(wg);
     constexpr int S = kFewStages;
@@ -176,8 +176,8 @@ __global__ void __launch_bounds__(kFewThreads, 1) q8_few(const GemvArgs a, const
     for (int q = grp; 2 * q < n_fill; q += 2) {
         const int f0 = 2 * q, f1 = min(f0 + 1, n_fill - 1);                   // (a last row group on its own is its own partner)
         const int st0 = f0 % S, st1 = f1 % S;
-        bool ok = mbar_wait_abortable(g.full0 + 8u * (first + st0), (uint32_t)(f0 / S) & 1u, g.abort);
-        ok = ok && mbar_wait_abortable(g.full0 + 8u * (first + st1), (uint32_t)(f1 / S) & 1u, g.abort);
+        bool ok = mbar_wait_warp(g.full0 + 8u * (first + st0), (uint32_t)(f0 / S) & 1u, g.abort);
+        ok = ok && mbar_wait_warp(g.full0 + 8u * (first + st1), (uint32_t)(f1 / S) & 1u, g.abort);
         if (!ok) fail(LUM_ST_WAIT_FULL);
         float acc[T][4];
 #pragma unroll

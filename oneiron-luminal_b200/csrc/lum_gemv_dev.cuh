@@ -591,7 +591,7 @@ __device__ __forceinline__ void gemv_quantize_x(const GemvArgs& a, const XSource
                 ss = fmaf(t.x, t.x, ss); ss = fmaf(t.y, t.y, ss); ss = fmaf(t.z, t.z, ss); ss = fmaf(t.w, t.w, ss);
             }
             if (b == nb - 1) {
-                ss = block_sum(ss, g.scratch, tid, kConsumers, 2, false);   // the prologue ends in a barrier before anything touches the scratch again
+                ss = block_sum(ss, g.scratch, tid, kConsumers, 2, false);   // (the next to use the scratch is the sampler's epilogue, behind gemv_consume's named_or)
                 const float mean = ss * (1.0f / (float)(a.k_norm > 0 ? a.k_norm : a.K));
                 inv = 1.0f / sqrtf(mean + a.eps);
             }
@@ -762,14 +762,14 @@ __device__ __forceinline__ void gemv_consume(const GemvArgs& a, const XSource& x
     if (ONE && warp < p.nt) gemv_load_xfrag(g, warp, lane, b, sx);
     auto fail = [&](uint32_t code) { if (!*g.abort) { atomicOr(status, code); *g.abort = 1; } };
     int slot = 0, slot_base = 0;
-    bool ended = false;
+    bool ended = false, gave_up = false;
 #pragma unroll 1
     while (!ended) {
         slot = 0;
 #pragma unroll 1
         for (;;) {
             const int st = first + cr.stage;
-            if (!mbar_wait_abortable(g.full0 + 8u * st, cr.par, g.abort)) { fail(LUM_ST_WAIT_FULL); ended = true; break; }
+            if (!mbar_wait_warp(g.full0 + 8u * st, cr.par, g.abort)) { fail(LUM_ST_WAIT_FULL); gave_up = true; break; }
             const int2 mm = g.meta[st];
             const uint32_t m2 = (uint32_t)mm.y;
             const bool mine = ONE ? warp < p.nt && mm.x != kMetaEnd : wj < (int)(m2 & 15u);
@@ -846,7 +846,9 @@ __device__ __forceinline__ void gemv_consume(const GemvArgs& a, const XSource& x
             }
             if (ONE ? slot == kChunkRG : (m2 & kM2JobEnd) && slot + p.sub * p.gpf > kChunkRG) break;
         }
-        ended = named_or(2, kConsumers, ended);          // (a warp that gave up takes the others along: every barrier below stays attended)
+        // A warp that gave up takes the others along: the two rings' warps then stand at different jobs, and nothing of this chunk is stored.  Otherwise every warp is
+        // here with the same jobs behind it, and every barrier below is attended by all.
+        if (named_or(2, kConsumers, gave_up)) return;
         // the warps' sums of a row, added in a fixed order, straight into the epilogue
         auto sum = [&](int i) {
             const int span = ONE ? p.nt << 8 : g.span_of[i >> 3];

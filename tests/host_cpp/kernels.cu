@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "lum_dense.cuh"
+#include "lum_gemv_dev.cuh"
 #include "lum_moe.cuh"
 #include "lum_rows.cuh"
 
@@ -681,6 +682,76 @@ static void level_specials() {
         }
 }
 
+// The consumers of a weight stream whose producer gives up: three row groups' first halves come, one row group's second half, then the abort flag and nothing more.
+// The warps of the two rings stand at different jobs by then.  All of them return, nothing is stored, no row is the best one.
+template <bool ONE>
+__global__ void __launch_bounds__(kGemvThreads) consume_short(const GemvArgs a, const int fills0, const int fills1, int* back) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ int s_abort;
+    const int tid = threadIdx.x;
+    GemvSmem g;
+    const GemvPlan plan = gemv_plan(a, 0, 1, -1);
+    gemv_carve(smem, a.K, GemvRings{a.ring_n[0], a.ring_n[1], a.ring_t[0], a.ring_t[1]}, &s_abort, &g);
+    gemv_cta_begin(g, tid, &s_abort);
+    if (tid >= kConsumers) {
+        if (elect_one()) {
+            bool ok = true;
+            for (int w = 0; w < 2; w++)
+                for (int f = 0; f < (w ? fills1 : fills0); f++) {            // (no more than the ring has stages)
+                    const int slot = g.first(w) + f;
+                    g.meta[slot] = make_int2(f, (int)m2_pack(kFillTiles, w * kFillTiles, 1, true, 0, true));
+                    mbar_arrive_expect_tx(g.full0 + 8u * slot, kFillBytes);
+                    bulk_g2s(smem_u32(g.at(w, f)), (const unsigned char*)a.seg[0].w + ((size_t)f * plan.tpr + w * kFillTiles) * kTileBytes, kFillBytes, g.full0 + 8u * slot);
+                }
+            for (int w = 0; w < 2; w++)
+                for (int f = 0; f < (w ? fills1 : fills0); f++) ok = mbar_wait(g.full0 + 8u * (g.first(w) + f), 0u) && mbar_wait(g.empty0 + 8u * (g.first(w) + f), 0u) && ok;
+            if (!ok) atomicOr(a.status, 1u << 31);
+            *(volatile int*)&s_abort = 1;
+        }
+        return;
+    }
+    XSource xs{};
+    xs.x = a.x;
+    ArgBest best{-INFINITY, -1};
+    ConsumerRing cr{0, 0u};
+    GainRegs gr;
+    gemv_gain_preload(a, tid, gr);
+    gemv_consume<false, ONE>(a, xs, false, plan, g, cr, tid, a.status, &best, gr);
+    atomicAdd(back, 1);
+    if (tid == 0) back[1] = best.i;
+}
+static void gave_up() {
+    const int K = 4096, N = 64;
+    std::mt19937 rng(3);
+    Dev<float> x(normal(rng, K, 1.0f));
+    Dev<unsigned char> w(q8_packed_bytes(N, K));          // (zeros)
+    for (bool one : {true, false})
+        for (int epi : {EPI_STORE, EPI_RESID, EPI_ARGMAX})
+            for (int fills0 : {3, 1}) {
+                Dev<float> y(std::vector<float>(N, 7.0f)), res((size_t)N);
+                Dev<int> back(2);
+                Dev<uint32_t> status(1);
+                GemvArgs a{};
+                a.nseg = 1; a.seg[0] = {w.p, nullptr, N, q8_pack_kc(N, K)}; a.K = K; a.wkind = WK_Q8; a.epi = epi; a.x = x.p; a.y = y.p; a.resid = res.p; a.status = status.p;
+                a.ring_n[0] = a.ring_n[1] = 3; a.ring_t[0] = a.ring_t[1] = kFillTiles;
+                const size_t smem = gemv_fixed_smem(K) + 6 * kFillBytes;
+                const void* fn = one ? (const void*)consume_short<true> : (const void*)consume_short<false>;
+                CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                int f0 = fills0, f1 = 4 - fills0;
+                int* bp = back.p;
+                void* params[] = {&a, &f0, &f1, &bp};
+                CK(cudaLaunchKernel(fn, dim3(1), dim3(kGemvThreads), params, smem, nullptr));
+                const std::vector<int> b = back.get();
+                const std::string what = std::string(one ? "a tile per warp" : "any K") + ", epilogue " + std::to_string(epi) + ", fills " + std::to_string(f0) + " / " + std::to_string(f1) + ": ";
+                report(what + "threads that did not return", kConsumers - b[0], 0);
+                report(what + "a best row", b[1] != -1, 0);
+                double stored = 0;
+                for (float v : y.get()) stored += v != 7.0f;
+                report(what + "rows stored", stored, 0);
+                report(what + "the producer's own waits", status.get()[0] >> 31, 0);
+            }
+}
+
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "attention-sums") attention_sums();
@@ -693,6 +764,7 @@ int main(int argc, char** argv) {
     else if (what == "claims") claims();
     else if (what == "few-rows") few_rows();
     else if (what == "level-specials") level_specials();
+    else if (what == "gave-up") gave_up();
     else { std::printf("unknown check\n"); return 2; }
     return failures ? 1 : 0;
 }
