@@ -243,6 +243,8 @@ __global__ void __launch_bounds__(kFewThreads, 1) q8_few(const GemvArgs a, const
         }
         named_sync(2 + grp, kConsumers);
     }
+    // after a run that was given up: not before the copies of x have landed (the producer sees to the ring's)
+    if (tid < 32 && elect_one() && *(volatile int*)&s_abort && !mbar_wait(xbar, 0u)) atomicOr(a.status, LUM_ST_WAIT_DRAIN);
 }
 
 // ---------------------------------------------------------------------------------------------------------------- host side
