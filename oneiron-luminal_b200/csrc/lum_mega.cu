@@ -32,10 +32,11 @@ namespace lum {
 // was last zeroed by the host) completes when the counter reaches (b + 1) * gridDim.x.  Called by all
 // consumer threads; thread 0 arrives and waits, the rest wait on the named barrier.  The wait is bounded
 // (LUM_WAIT_BUDGET_CYCLES); once it runs out the kernel-wide abort flag is raised and every later wait
-// in every CTA returns at once.
+// in every CTA returns at once.  Returns whether this CTA has given up, the same answer in all of its workers: they skip phases (and the
+// barriers inside them) together, whatever the producer warp raises meanwhile.
 constexpr int kMegaWorkers = 512;        // attention, grid barriers; the first kConsumers of them are the consumers of the weight stream
 constexpr int kMegaThreads = kMegaWorkers + 32;
-__device__ __forceinline__ void grid_barrier(const MegaArgs& a, unsigned long long& seq, volatile int* cta_abort, int tid) {
+__device__ __forceinline__ bool grid_barrier(const MegaArgs& a, unsigned long long& seq, volatile int* cta_abort, int tid) {
     named_sync(1, kMegaWorkers);                        // all of this CTA's writes of the phase are issued
     if (tid == 0) {
         __threadfence();
@@ -66,7 +67,7 @@ __device__ __forceinline__ void grid_barrier(const MegaArgs& a, unsigned long lo
         __threadfence();
     }
     seq++;
-    named_sync(1, kMegaWorkers);
+    return named_or(1, kMegaWorkers, *cta_abort != 0);
 }
 
 __device__ __forceinline__ AttnArgs attn_phase_args(const MegaArgs& a, const MegaLayer& L, bool bf16) {
@@ -163,7 +164,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_mega(const MegaArgs a)
     ConsumerRing cring{0, 0u};
     unsigned long long seq = a.gbar_base;             // grid barriers passed so far
     unsigned long long pseq = a.gbar_base;            // running phase number: picks the job-claim counter of each phase
-    bool producing = true;
+    bool producing = true, gone = false;              // gone: this CTA's workers have given up
     int pos = 0, tok = 0;
     bool second = false;                              // the residual stream is in a.x2
     int pending = 0;                                  // partial vectors that have not joined it yet
@@ -174,7 +175,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_mega(const MegaArgs a)
             // Refuse the whole launch the same way in every CTA (all read the same state): nothing was written yet.
             if (cta == 0 && tid == 0) atomicOr(a.status, pos < 0 || pos + a.n_tokens > a.max_seq ? LUM_ST_BAD_POS : LUM_ST_BAD_TOKEN);
             if (tid == 0) s_abort = 1;
-            named_sync(1, kMegaWorkers);
+            gone = true;
         }
     }
 
@@ -204,8 +205,8 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_mega(const MegaArgs a)
                 }
             } else if (!streams) {
                 // RoPE + cache append + attention
-                if (!s_abort) attn_phase<HD, GM, BF16>(a, L, (unsigned char*)g.xq, pos, tid);
-                grid_barrier(a, seq, &s_abort, tid);
+                if (!gone) attn_phase<HD, GM, BF16>(a, L, (unsigned char*)g.xq, pos, tid);
+                gone = grid_barrier(a, seq, &s_abort, tid);
             } else {
                 XSource xs{};
                 // the residual stream lives in a.x or a.x2, and moves to the other when partial vectors join it
@@ -220,7 +221,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_mega(const MegaArgs a)
                 ga.resid = ga.y;
                 if (p == 4 && ga.ksplit > 1) pending = ga.ksplit;
                 ArgBest best{-INFINITY, -1};
-                if (!s_abort) {
+                if (!gone) {
                     if (p == 0) attn_phase_prefetch<HD, GM, BF16>(a, L, pos, tid);
                     if (tid < kConsumers) {
                         GainRegs gr;
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_mega(const MegaArgs a)
                     }
                 }
                 if (p == 5 && tid == 0) { a.part_val[cta] = best.v; a.part_idx[cta] = best.i; }
-                grid_barrier(a, seq, &s_abort, tid);
+                gone = grid_barrier(a, seq, &s_abort, tid);
                 if (p == 5) {
                     // every CTA folds the per-CTA maxima itself: all of them need the token for the next embedding row
                     if (warp == 0) {
@@ -238,8 +239,8 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_mega(const MegaArgs a)
                         if (lane == 0) s_tok = fi;
                     }
                     named_sync(1, kMegaWorkers);
-                    const int sampled = s_abort ? 0 : max(0, s_tok);
-                    if (cta == 0 && tid == 0 && !s_abort) {
+                    const int sampled = gone ? 0 : max(0, s_tok);
+                    if (cta == 0 && tid == 0 && !gone) {
                         DecodeState* st = a.state;
                         const int step = st->step;
                         st->last_tok = sampled;
@@ -259,7 +260,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_mega(const MegaArgs a)
         if (elect_one() && (s_abort || !producing)) gemv_producer_drain(g, pring, a.status);
         return;
     }
-    if (cta == 0 && tid == 0 && !s_abort) {
+    if (cta == 0 && tid == 0 && !gone) {
         a.state->pos = pos;
         a.state->tok = tok;
     }
