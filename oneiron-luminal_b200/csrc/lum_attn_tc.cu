@@ -242,7 +242,8 @@ __global__ void __launch_bounds__(kApThreads, 1) attn_prompt_tc(const PromptArgs
     } else if (!softmax) {
         // K(0), K(1), V(0), K(2), V(1), ..: a tile's copies go out as soon as its buffer is no longer read, the one before is handed over when it has landed.
         // A warp's instruction takes two positions' 256 bytes.  Half a tile's positions start on a multiple of 64: one sequence slot or one page (of at least
-        // 64 rows) holds them all; rows never written (or beyond the capacity) read as zeros.
+        // 64 rows) holds them all; rows never written (or beyond the capacity) read as zeros, and so do those before `low`: a key that no row of the CTA sees may hold
+        // anything (weight 0 times infinity is no zero), and its page may be gone.
         uint32_t last = 0u;                                    // the barrier of the tile still on its way
         auto load = [&](const void* cache, int t, uint32_t dst, uint32_t full, uint32_t unread) {
             if (t >= n_tiles) return;
@@ -251,13 +252,14 @@ __global__ void __launch_bounds__(kApThreads, 1) attn_prompt_tc(const PromptArgs
             dst += (uint32_t)(t & 1) * kApOperand + ((lane >> 3) & 1) * kApHalf + k0 * 128;
 #pragma unroll 1
             for (int h = 0; h < 2; h++, dst += 64 * 128) {
-                const int j0 = (t_lo + t) * kApKT + h * 64, live = min(64, pos_max + 1 - j0);
+                const int j0 = (t_lo + t) * kApKT + h * 64, live = min(64, pos_max + 1 - j0), dead = low - j0;
                 const __nv_bfloat16* src = (const __nv_bfloat16*)cache + (size_t)kvh * kAtHD + (lane & 15) * 8;
-                if (live > 0) src += kv_phys_row(a.pg, a.seq0, a.max_seq, j0) * row_elems;
+                if (live > 0 && dead < 64) src += kv_phys_row(a.pg, a.seq0, a.max_seq, j0) * row_elems;
 #pragma unroll
                 for (int i = 0; i < (32 + kApLoaders - 1) / kApLoaders; i++) {
                     const int key = k0 + i * 2 * kApLoaders;
-                    if (key < 64) cp_async16(dst + i * 256 * kApLoaders + (((lane & 7) ^ (key & 7)) << 4), src + (key < live ? (size_t)key * row_elems : 0), key < live ? 16u : 0u);
+                    const bool in = key >= dead && key < live;
+                    if (key < 64) cp_async16(dst + i * 256 * kApLoaders + (((lane & 7) ^ (key & 7)) << 4), src + (in ? (size_t)key * row_elems : 0), in ? 16u : 0u);
                 }
             }
             cp_async_commit();

@@ -164,27 +164,39 @@ static void attention_prompt() {
     }
 }
 
-// The same kernel for layers described one by one: windows, chunks, a bias by distance, one to eight query heads per K/V head.
+// The same kernel for layers described one by one: windows, chunks, a bias by distance, one to eight query heads per K/V head.  What no row of a CTA sees, before its
+// first row's window or chunk and behind its last row, is not a number; with pages (in another order), it is on pages of its own.
 static void attention_band() {
-    struct Case { int nq, nkv, rows, first, window, chunk; bool bias; };
-    const std::vector<Case> cases = {{4, 4, 130, 0, 0, 0, true},      {8, 4, 65, 300, 128, 0, true},  {8, 2, 97, 1000, 300, 0, true}, {8, 1, 50, 255, 1, 0, true},
-                                     {8, 2, 129, 511, 512, 0, false}, {8, 1, 33, 127, 0, 100, true},  {4, 2, 200, 64, 0, 256, false}, {4, 1, 40, 900, 129, 0, true}};
+    struct Case { int nq, nkv, rows, first, window, chunk; bool bias, pages; };
+    const std::vector<Case> cases = {{4, 4, 130, 0, 0, 0, true, false},     {8, 4, 65, 300, 128, 0, true, false},     {8, 2, 97, 1000, 300, 0, true, false}, {8, 1, 50, 255, 1, 0, true, false},
+                                     {8, 2, 129, 511, 512, 0, false, true}, {8, 1, 33, 127, 0, 100, true, false},     {4, 2, 200, 64, 0, 256, false, true},  {4, 1, 40, 900, 129, 0, true, false},
+                                     {8, 2, 32, 1003, 300, 0, true, true},  {8, 1, 16, 447, 192, 0, false, false},    {8, 1, 16, 400, 0, 336, true, true},   {4, 4, 128, 765, 128, 0, true, true}};
     for (const Case& c : cases) {
         const int hd = 128, n = c.first + c.rows, max_seq = (n + 63) / 64 * 64, G = c.nq / c.nkv, chunks = c.nq * hd / 64;
         std::mt19937 rng(n * 5 + c.nq + c.window);
         const size_t ld = (size_t)c.nkv * hd, qd = (size_t)c.nq * hd;
         const std::vector<float> q = normal(rng, (size_t)c.rows * qd, 0.09f);
         const std::vector<uint16_t> k = to_bf16(normal(rng, max_seq * ld, 1.0f)), v = to_bf16(normal(rng, max_seq * ld, 1.0f, 0.5f));
+        const int low = c.window ? std::max(0, c.first + 1 - c.window) : c.chunk ? c.first / c.chunk * c.chunk : 0;
+        std::vector<uint16_t> kp = k, vp = v;
+        std::vector<int> table(max_seq / 64);
+        for (int i = 0; i < max_seq / 64; i++) table[i] = c.pages ? max_seq / 64 - 1 - i : i;
+        for (int j = 0; j < max_seq; j++)
+            for (size_t e = 0; e < ld; e++) {
+                const size_t to = ((size_t)table[j / 64] * 64 + j % 64) * ld + e;
+                kp[to] = j >= low && j < n ? k[j * ld + e] : 0x7fc0; vp[to] = j >= low && j < n ? v[j * ld + e] : 0x7fc0;
+            }
         std::vector<float> r1(c.nq), r2(c.nq);
         for (int h = 0; h < c.nq; h++) { r1[h] = 0.1f + 0.2f * h; r2[h] = 0.05f + 0.07f * h; }
         std::vector<int> pos(c.rows);
         for (int i = 0; i < c.rows; i++) pos[i] = c.first + i;
         const int rows_up = (c.rows + 127) / 128 * 128;
         Dev<float> dq(q), d1(r1), d2(r2);
-        Dev<uint16_t> kc(k), vc(v), out((size_t)rows_up * qd);
-        Dev<int> dpos(pos);
+        Dev<uint16_t> kc(kp), vc(vp), out((size_t)rows_up * qd);
+        Dev<int> dpos(pos), dtable(table);
         Dev<uint32_t> status(1);
         BandArgs a{};
+        if (c.pages) { a.pg.table = dtable.p; a.pg.lg = 6; a.pg.pages_per_seq = max_seq / 64; }
         a.p.n_q = c.nq; a.p.n_kv = c.nkv; a.p.dk = a.p.dv = a.p.dkp = a.p.dvp = hd; a.p.maps = 1;
         a.q = dq.p; a.k_cache = kc.p; a.v_cache = vc.p; a.kv_bf16 = 1; a.row_pos = dpos.p; a.M = c.rows; a.window = c.window; a.chunk = c.chunk; a.max_seq = max_seq; a.max_batch = 1;
         if (c.bias) { a.r1 = d1.p; a.r2 = d2.p; }
@@ -215,7 +227,7 @@ static void attention_band() {
             }
         // outputs are rounded to bf16: at most 2^-9 of each
         report(std::to_string(c.nq) + " / " + std::to_string(c.nkv) + " heads, rows " + std::to_string(c.first) + " + " + std::to_string(c.rows) + ", window " + std::to_string(c.window) + ", chunk " +
-               std::to_string(c.chunk) + (c.bias ? ", bias" : ""), rel(got, want), std::exp2(-9.0));
+               std::to_string(c.chunk) + (c.bias ? ", bias" : "") + (c.pages ? ", pages" : ""), rel(got, want), std::exp2(-9.0));
         report("status", status.get()[0], 0);
     }
 }
