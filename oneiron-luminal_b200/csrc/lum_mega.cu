@@ -34,10 +34,14 @@ namespace lum {
 // (LUM_WAIT_BUDGET_CYCLES); once it runs out the kernel-wide abort flag is raised and every later wait
 // in every CTA returns at once.  Returns whether this CTA has given up, the same answer in all of its workers: they skip phases (and the
 // barriers inside them) together, whatever the producer warp raises meanwhile.
-constexpr int kMegaWorkers = 512;        // attention, grid barriers; the first kConsumers of them are the consumers of the weight stream
-constexpr int kMegaThreads = kMegaWorkers + 32;
+// Threads for attention and grid barriers; the first kConsumers of them are the consumers of the weight stream.  With the producer warp 16 warps, which leaves
+// 128 registers a thread; attention without tensor cores takes 512 threads.  Measured, ms a token of the Llama-3-8B shape behind 512 / 3000 rows: 4.25 / 4.70, with
+// 512 workers (96 registers) 4.51 / 4.92.
+template <int HD, int GM, bool BF16>
+__host__ __device__ constexpr int mega_workers() { return BF16 && attn_tc_fits(HD, GM) ? 480 : kAttnThreads; }
+template <int W>
 __device__ __forceinline__ bool grid_barrier(const MegaArgs& a, unsigned long long& seq, volatile int* cta_abort, int tid) {
-    named_sync(1, kMegaWorkers);                        // all of this CTA's writes of the phase are issued
+    named_sync(1, W);                        // all of this CTA's writes of the phase are issued
     if (tid == 0) {
         __threadfence();
         // gbar[0] counts arrivals; gbar[16] (its own 128-byte line, so polls do not queue behind the atomics) holds the
@@ -67,7 +71,7 @@ __device__ __forceinline__ bool grid_barrier(const MegaArgs& a, unsigned long lo
         __threadfence();
     }
     seq++;
-    return named_or(1, kMegaWorkers, *cta_abort != 0);
+    return named_or(1, W, *cta_abort != 0);
 }
 
 __device__ __forceinline__ AttnArgs attn_phase_args(const MegaArgs& a, const MegaLayer& L, bool bf16) {
@@ -85,98 +89,120 @@ template <int HD, int GM, bool BF16>
 __device__ __forceinline__ void attn_phase_prefetch(const MegaArgs& a, const MegaLayer& L, int pos, int tid) {
     if constexpr (BF16 && attn_tc_fits(HD, GM)) {
         if ((int)blockIdx.x >= a.n_kv * a.n_splits) return;
+        constexpr int W = mega_workers<HD, GM, BF16>();
         const AttnArgs t = attn_phase_args(a, L, BF16);
         int r0, r1;
         attn_tc_range(t, (int)blockIdx.x % a.n_splits, pos, &r0, &r1);
-        attn_tc_prefetch<HD>(t, (int)blockIdx.x / a.n_splits, r0, r1, tid, kMegaWorkers);
+        attn_tc_prefetch<HD>(t, (int)blockIdx.x / a.n_splits, r0, r1, tid, W);
     }
 }
 template <int HD, int GM, bool BF16>
 __device__ __noinline__ void attn_phase(const MegaArgs& a, const MegaLayer& L, unsigned char* scratch_smem, int pos, int tid) {
     const int items = a.n_kv * a.n_splits;
     if ((int)blockIdx.x >= items) return;           // uniform per CTA: the whole CTA skips, barriers inside stay matched
+    constexpr int W = mega_workers<HD, GM, BF16>();
     const AttnArgs t = attn_phase_args(a, L, BF16);
     const int kvh = (int)blockIdx.x / a.n_splits, split = (int)blockIdx.x % a.n_splits;
     if constexpr (BF16 && attn_tc_fits(HD, GM)) {
-        // The heads are prepared and the states merged by all 512 workers, the rows (asked for in the phase before) taken by four warps.  Measured, ms a
-        // token (32 layers of 32 / 8 heads of 128) behind 512 / 3000 rows: 5.13 / 5.68 with 128 workers and nothing asked for ahead, 4.89 / 5.28 this
-        // way, 4.95 / 5.28 with a warp per key
+        // The heads are prepared and the states merged by all workers, the rows (asked for in the phase before) taken by four warps.  Of a warp per key, 128 workers
+        // and this, this was the fastest.
         AttnTile<HD> f;
-        AttnPre<HD, kMegaWorkers> pre;
-        attn_tc_pre<HD, kMegaWorkers>(t, pre, kvh, split, tid >> 5, tid & 31);
-        attn_tc_body<HD, GM / 4, false, kMegaWorkers, false>(t, scratch_smem, f, pre, kvh, split, pos, tid, 1, false);
+        AttnPre<HD, W> pre;
+        attn_tc_pre<HD, W>(t, pre, kvh, split, tid >> 5, tid & 31);
+        attn_tc_body<HD, GM / 4, false, W, false>(t, scratch_smem, f, pre, kvh, split, pos, tid, 1, false);
     } else {
         attn_decode_body<HD, GM, BF16>(t, scratch_smem, kvh, split, pos, tid, 1);
     }
 }
 
-// Phase p of layer l (p = 0..4), or the head phase (p = 5): fill in the projection's arguments.
-// Returns false for the attention phase (p == 1), which streams no weights.
-__device__ __forceinline__ bool phase_gemv(const MegaArgs& a, const MegaLayer& L, int p, GemvArgs* out) {
+// What one phase streams and where its vectors are.  Kept in shared memory and filled by one thread: as locals of 512 threads these structs (whose matrices are
+// picked by number) were a stack of 2 KB a thread, far beyond the L1 that the rings leave (7.0 / 7.5 ms a token, now 4.25 / 4.70).
+struct MegaPhase { GemvArgs ga; GemvPlan plan; XSource xs; bool streams; };
+
+// Phase p of layer l (p = 0..4), or the head phase (p = 5).  The attention phase (p == 1) streams no weights.  Where the down projection runs as K ranges, their
+// partial vectors join the residual stream in the next prologue, which moves it from one of x, x2 to the other.
+__device__ __noinline__ void mega_fill(const MegaArgs& a, int l, int p, int token, MegaPhase* out) {
     const int H = a.hidden, qd = a.n_q * a.hd, kvd = a.n_kv * a.hd;
+    const int ranges = gemv_k_ranges(a.ffn, a.kc_f);
+    const MegaLayer& L = a.layers[l];
+    auto stream = [&](int layer) { return ranges > 1 && (layer & 1) ? a.x2 : a.x; };
     GemvArgs g{};
-    g.wkind = WK_Q8; g.gain_kind = a.gain_kind; g.eps = a.eps; g.status = a.status;
+    XSource xs{};
+    g.wkind = WK_Q8; g.gain_kind = a.gain_kind; g.eps = a.eps; g.status = a.status; g.nseg = 1; g.epi = EPI_STORE;
+    const int joined = p == 0 ? l - 1 : p == 5 ? l : -1;             // the layer whose partial vectors join in this phase's prologue
+    if (joined >= 0 && ranges > 1) { xs.parts = a.part; xs.n_parts = ranges; xs.part_stride = a.part_ld; }
     switch (p) {
         case 0:   // q, k, v projections (RMSNorm in the prologue)
-            g.K = H; g.KC = a.kc_h; g.epi = EPI_STORE; g.nseg = 3;
+            g.K = H; g.KC = a.kc_h; g.nseg = 3;
             g.seg[0] = {L.wq, nullptr, qd, a.kc_h}; g.seg[1] = {L.wk, nullptr, kvd, a.kc_h}; g.seg[2] = {L.wv, nullptr, kvd, a.kc_h};
             g.gain = L.attn_norm; g.y = a.qkv;
+            if (l == 0) { xs.table = a.embed; xs.table_kind = a.embed_kind; xs.token = token; xs.x_out = a.x; }      // the embedding row is x
+            else { xs.x = stream(l - 1); if (ranges > 1) xs.x_out = stream(l); }
             break;
-        case 1:
-            return false;
         case 2:   // o projection + residual
-            g.K = qd; g.KC = a.kc_o; g.epi = EPI_RESID; g.nseg = 1; g.seg[0] = {L.wo, nullptr, H, a.kc_o};
-            g.y = a.x; g.resid = a.x;
+            g.K = qd; g.KC = a.kc_o; g.epi = EPI_RESID; g.seg[0] = {L.wo, nullptr, H, a.kc_o};
+            g.y = stream(l); g.resid = g.y; xs.x = a.attn;
             break;
         case 3:   // gate, up projections + SwiGLU (RMSNorm in the prologue)
             g.K = H; g.KC = a.kc_h; g.epi = EPI_SWIGLU; g.nseg = 2;
             g.seg[0] = {L.wg, nullptr, a.ffn, a.kc_h}; g.seg[1] = {L.wu, nullptr, a.ffn, a.kc_h};
-            g.gain = L.mlp_norm; g.y = a.h;
+            g.gain = L.mlp_norm; g.y = a.h; xs.x = stream(l);
             break;
-        case 4:   // down projection: its K ranges' partial vectors join the residual stream in the next prologue; one range: + residual
-            g.K = a.ffn; g.KC = a.kc_f; g.nseg = 1; g.seg[0] = {L.wd, nullptr, H, a.kc_f};
-            g.ksplit = gemv_k_ranges(a.ffn, a.kc_f);
-            if (g.ksplit > 1) { g.epi = EPI_STORE; g.y = a.part; g.y_range_stride = a.part_ld; }
+        case 4:   // down projection
+            g.K = a.ffn; g.KC = a.kc_f; g.seg[0] = {L.wd, nullptr, H, a.kc_f}; xs.x = a.h;
+            g.ksplit = ranges;
+            if (ranges > 1) { g.y = a.part; g.y_range_stride = a.part_ld; }
             else { g.epi = EPI_RESID; g.y = a.x; g.resid = a.x; }
             break;
-        default:  // final RMSNorm + vocabulary projection + greedy sample
-            g.K = H; g.KC = a.kc_h; g.epi = EPI_ARGMAX; g.nseg = 1; g.seg[0] = {a.lm_head, nullptr, a.vocab, a.kc_h};
-            g.gain = a.final_norm; g.y = a.logits;
+        case 5:   // final RMSNorm + vocabulary projection + greedy sample
+            g.K = H; g.KC = a.kc_h; g.epi = EPI_ARGMAX; g.seg[0] = {a.lm_head, nullptr, a.vocab, a.kc_h};
+            g.gain = a.final_norm; g.y = a.logits; xs.x = stream(l);
             break;
+        default: break;
     }
-    *out = g;
-    return true;
+    out->streams = p != 1;
+    if (p != 1) { out->ga = g; out->xs = xs; out->plan = gemv_plan(g, (int)blockIdx.x, (int)gridDim.x, 750); }
+}
+
+template <bool ONE>
+__device__ __noinline__ void mega_consume(const MegaPhase& m, const GemvSmem& g, ConsumerRing& cr, int tid, ArgBest* best) {
+    GainRegs gr;
+    gemv_gain_preload(m.ga, tid, gr);
+    gemv_consume<false, ONE>(m.ga, m.xs, blockIdx.x == 0, m.plan, g, cr, tid, m.ga.status, best, gr);
 }
 
 template <int HD, int GM, bool BF16>
-__global__ void __launch_bounds__(kMegaThreads, 1) decode_mega(const MegaArgs a) {
+__global__ void __launch_bounds__(mega_workers<HD, GM, BF16>() + 32, 1) decode_mega(const __grid_constant__ MegaArgs a) {
+    constexpr int W = mega_workers<HD, GM, BF16>();
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_abort;
     __shared__ int s_tok;
+    __shared__ MegaPhase s_phase[2], s_stream;        // the workers' phase and the next one; the producer's, which runs ahead
+    __shared__ GemvSmem g;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int cta = (int)blockIdx.x, ncta = (int)gridDim.x;
-    GemvSmem g;
-    gemv_carve(smem, a.k_max, GemvRings{(a.stages + 1) / 2, a.stages / 2, kFillTiles, kFillTiles}, &s_abort, &g, attn_smem_bytes(HD, GM));
+    if (tid == 0) gemv_carve(smem, a.k_max, GemvRings{(a.stages + 1) / 2, a.stages / 2, kFillTiles, kFillTiles}, &s_abort, &g, attn_smem_bytes(HD, GM));
+    __syncthreads();
     gemv_cta_begin(g, tid, &s_abort);
 
-    const bool is_worker = warp < kMegaWorkers / 32, is_producer = !is_worker;
+    const bool is_worker = warp < W / 32, is_producer = !is_worker;
     ProducerRing pring{};
     ConsumerRing cring{0, 0u};
     unsigned long long seq = a.gbar_base;             // grid barriers passed so far
     unsigned long long pseq = a.gbar_base;            // running phase number: picks the job-claim counter of each phase
     bool producing = true, gone = false;              // gone: this CTA's workers have given up
-    int pos = 0, tok = 0;
-    bool second = false;                              // the residual stream is in a.x2
-    int pending = 0;                                  // partial vectors that have not joined it yet
+    int pos = 0, buf = 0;
     if (is_worker) {
         pos = a.state->pos;
-        tok = a.forced ? a.forced[0] : a.state->tok;
+        const int tok = a.forced ? a.forced[0] : a.state->tok;
         if (pos < 0 || pos + a.n_tokens > a.max_seq || tok < 0 || tok >= a.vocab) {
             // Refuse the whole launch the same way in every CTA (all read the same state): nothing was written yet.
             if (cta == 0 && tid == 0) atomicOr(a.status, pos < 0 || pos + a.n_tokens > a.max_seq ? LUM_ST_BAD_POS : LUM_ST_BAD_TOKEN);
             if (tid == 0) s_abort = 1;
             gone = true;
         }
+        if (tid == 0) { mega_fill(a, 0, 0, tok, &s_phase[0]); s_tok = tok; }
+        named_sync(1, W);
     }
 
     const int per_token = 5 * a.n_layers;             // phases per token before the head
@@ -188,71 +214,61 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_mega(const MegaArgs a)
         for (int ph = 0; ph < n_phase; ph++) {
             const int l = ph < per_token ? ph / 5 : a.n_layers - 1;
             const int p = ph < per_token ? ph - l * 5 : 5;
-            const MegaLayer& L = a.layers[l];
-            GemvArgs ga;
-            const bool streams = phase_gemv(a, L, p, &ga);
-            GemvPlan plan{};
-            if (streams) plan = gemv_plan(ga, cta, ncta, 750);
-            unsigned int* ctr = a.job_ctr + (pseq % kJobCtrRing) * kMaxKRanges + plan.range;
+            const unsigned int slot = (unsigned int)(pseq % kJobCtrRing);
             // Re-zero the claim counter that phase pseq + 32 will use: its last user was phase pseq - 32, and no CTA can
             // be that far behind or ahead (a producer leads its consumers by at most one ring of stages, each phase
             // taking at least one).  Every phase does this, whether or not it streams weights itself.
-            if (cta == 0 && tid < kMaxKRanges) a.job_ctr[(pseq + kJobCtrRing / 2) % kJobCtrRing * kMaxKRanges + tid] = 0u;
+            if (cta == 0 && tid < kMaxKRanges) a.job_ctr[(slot + kJobCtrRing / 2) % kJobCtrRing * kMaxKRanges + tid] = 0u;
             pseq++;
             if (is_producer) {
-                if (streams && elect_one() && producing) {
-                    producing = gemv_produce(ga, plan, g, pring, ctr, a.status);
+                if (p != 1 && elect_one() && producing) {
+                    mega_fill(a, l, p, 0, &s_stream);
+                    producing = gemv_produce(s_stream.ga, s_stream.plan, g, pring, a.job_ctr + slot * kMaxKRanges + s_stream.plan.range, a.status);
                 }
-            } else if (!streams) {
-                // RoPE + cache append + attention
-                if (!gone) attn_phase<HD, GM, BF16>(a, L, (unsigned char*)g.xq, pos, tid);
-                gone = grid_barrier(a, seq, &s_abort, tid);
-            } else {
-                XSource xs{};
-                // the residual stream lives in a.x or a.x2, and moves to the other when partial vectors join it
-                if (ph == 0) { xs.table = a.embed; xs.table_kind = a.embed_kind; xs.token = tok; xs.x_out = a.x; second = false; pending = 0; }   // the embedding row is x
-                else xs.x = p == 2 ? a.attn : p == 4 ? a.h : second ? a.x2 : a.x;
-                if (pending && (p == 0 || p == 5)) {
-                    xs.parts = a.part; xs.n_parts = pending; xs.part_stride = a.part_ld;
-                    if (p == 0) { xs.x_out = second ? a.x : a.x2; second = !second; }
-                    pending = 0;
-                }
-                if (ga.epi == EPI_RESID) ga.y = second ? a.x2 : a.x;
-                ga.resid = ga.y;
-                if (p == 4 && ga.ksplit > 1) pending = ga.ksplit;
-                ArgBest best{-INFINITY, -1};
-                if (!gone) {
-                    if (p == 0) attn_phase_prefetch<HD, GM, BF16>(a, L, pos, tid);
+                continue;
+            }
+            const MegaPhase& m = s_phase[buf];
+            ArgBest best{-INFINITY, -1};
+            if (!gone) {
+                if (p == 1) {
+                    // RoPE + cache append + attention
+                    attn_phase<HD, GM, BF16>(a, a.layers[l], (unsigned char*)g.xq, pos, tid);
+                } else {
+                    if (p == 0) attn_phase_prefetch<HD, GM, BF16>(a, a.layers[l], pos, tid);
                     if (tid < kConsumers) {
-                        GainRegs gr;
-                        gemv_gain_preload(ga, tid, gr);
-                        if (plan.nt > kFillTiles && plan.nt <= kJobTiles) gemv_consume<false, true>(ga, xs, cta == 0, plan, g, cring, tid, a.status, &best, gr);
-                        else gemv_consume<false, false>(ga, xs, cta == 0, plan, g, cring, tid, a.status, &best, gr);
+                        if (m.plan.nt > kFillTiles && m.plan.nt <= kJobTiles) mega_consume<true>(m, g, cring, tid, &best);
+                        else mega_consume<false>(m, g, cring, tid, &best);
                     }
-                }
-                if (p == 5 && tid == 0) { a.part_val[cta] = best.v; a.part_idx[cta] = best.i; }
-                gone = grid_barrier(a, seq, &s_abort, tid);
-                if (p == 5) {
-                    // every CTA folds the per-CTA maxima itself: all of them need the token for the next embedding row
-                    if (warp == 0) {
-                        const int fi = argmax_final(a.part_val, a.part_idx, ncta, lane).i;
-                        if (lane == 0) s_tok = fi;
-                    }
-                    named_sync(1, kMegaWorkers);
-                    const int sampled = gone ? 0 : max(0, s_tok);
-                    if (cta == 0 && tid == 0 && !gone) {
-                        DecodeState* st = a.state;
-                        const int step = st->step;
-                        st->last_tok = sampled;
-                        if (st->log && a.tokens_out && step < st->max_steps) { a.tokens_out[step] = sampled; st->step = step + 1; }
-                    }
-                    tok = sampled;
-                    // part_val / part_idx are rewritten only after the next token's grid barriers, so no CTA can still
-                    // be reading them
                 }
             }
+            if (p == 5 && tid == 0) { a.part_val[cta] = best.v; a.part_idx[cta] = best.i; }
+            // the next phase's, by a thread that does not stream; handed over by the barrier
+            if (tid == W - 1) {
+                const int nx = ph + 1 < n_phase ? ph + 1 : 0, nl = nx < per_token ? nx / 5 : a.n_layers - 1;
+                mega_fill(a, nl, nx < per_token ? nx - nl * 5 : 5, nx == 0 && a.forced && t + 1 < a.n_tokens ? a.forced[t + 1] : 0, &s_phase[buf ^ 1]);
+            }
+            buf ^= 1;
+            gone = grid_barrier<W>(a, seq, &s_abort, tid);
+            if (p == 5) {
+                // every CTA folds the per-CTA maxima itself: all of them need the token for the next embedding row
+                if (warp == 0) {
+                    const int fi = argmax_final(a.part_val, a.part_idx, ncta, lane).i;
+                    if (lane == 0) {
+                        s_tok = gone ? 0 : max(0, fi);
+                        if (!a.forced) s_phase[buf].xs.token = s_tok;
+                    }
+                }
+                named_sync(1, W);
+                if (cta == 0 && tid == 0 && !gone) {
+                    DecodeState* st = a.state;
+                    const int step = st->step;
+                    st->last_tok = s_tok;
+                    if (st->log && a.tokens_out && step < st->max_steps) { a.tokens_out[step] = s_tok; st->step = step + 1; }
+                }
+                // part_val / part_idx are rewritten only after the next token's grid barriers, so no CTA can still
+                // be reading them
+            }
         }
-        if (is_worker && a.forced && t + 1 < a.n_tokens) tok = a.forced[t + 1];
         pos++;
     }
 
@@ -262,18 +278,19 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_mega(const MegaArgs a)
     }
     if (cta == 0 && tid == 0 && !gone) {
         a.state->pos = pos;
-        a.state->tok = tok;
+        a.state->tok = s_tok;
     }
 }
 
 // ------------------------------------------------------------------------------------------- host side
 
 // the attention phase borrows the activation / reduction area; it is sized for the larger of the two uses
+constexpr int kMegaSmem = 224 * 1024;      // dynamic shared memory at most: the phases' arguments are static
 static size_t mega_scratch(int hd, int groups) { return attn_smem_bytes(hd, groups <= 4 ? 4 : 8); }
 size_t mega_smem_bytes(int k_max, int stages, int hd, int groups) { return gemv_fixed_smem(k_max, mega_scratch(hd, groups)) + (size_t)stages * kFillBytes; }
 
 int mega_pick_stages(int k_max, int hd, int groups) {
-    int stages = (int)((226 * 1024 - (long)gemv_fixed_smem(k_max, mega_scratch(hd, groups))) / kFillBytes);
+    int stages = (int)((kMegaSmem - (long)gemv_fixed_smem(k_max, mega_scratch(hd, groups))) / kFillBytes);
     if (stages > kMaxStages) stages = kMaxStages;
     static const int env_stages = [] { const char* e = getenv("LUM_MEGA_STAGES"); return e ? atoi(e) : 0; }();
     if (env_stages > 0 && env_stages < stages) stages = env_stages;
@@ -297,19 +314,21 @@ cudaError_t launch_mega(const MegaArgs& a_in, int sm_count, cudaStream_t st) {
     else if (a.hd == 64) fn = g4 ? (bf ? (const void*)decode_mega<64, 4, true> : (const void*)decode_mega<64, 4, false>)
                                  : (bf ? (const void*)decode_mega<64, 8, true> : (const void*)decode_mega<64, 8, false>);
     else return cudaErrorInvalidValue;
+    const int threads = 32 + (a.hd == 128 ? (g4 ? (bf ? mega_workers<128, 4, true>() : mega_workers<128, 4, false>()) : (bf ? mega_workers<128, 8, true>() : mega_workers<128, 8, false>()))
+                                          : (g4 ? (bf ? mega_workers<64, 4, true>() : mega_workers<64, 4, false>()) : (bf ? mega_workers<64, 8, true>() : mega_workers<64, 8, false>())));
     if (a.n_kv * a.n_splits > sm_count) return cudaErrorInvalidValue;
     const size_t smem = mega_smem_bytes(a.k_max, a.stages, a.hd, a.n_q / a.n_kv);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(226 * 1024));
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kMegaSmem);
     if (e != cudaSuccess) return e;
-    if (smem > 226 * 1024) return cudaErrorInvalidValue;
+    if (smem > kMegaSmem) return cudaErrorInvalidValue;
     // every CTA must be resident at once: the grid barrier relies on it
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kMegaThreads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorLaunchOutOfResources;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sm_count);
-    cfg.blockDim = dim3(kMegaThreads);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
