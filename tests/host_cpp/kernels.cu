@@ -490,6 +490,76 @@ static void matvec_q8() {
     }
 }
 
+// The matrix-vector kernel's tensor-parallel paths, on one GPU: partial vectors as {value, completion word} pairs that are there already, rows stored as such pairs or
+// as values with a word behind them; and the sampler's epilogue, where the last of equal best rows wins.
+static void matvec_peer() {
+    struct Case { int k, n, parts, epi; bool ll; };
+    const std::vector<Case> cases = {{2560, 1208, 1, EPI_STORE, true}, {2560, 264, 2, EPI_PEER, true},   {4096, 4096, 3, EPI_STORE, true},  {4096, 1208, 5, EPI_PEER, false}, {4608, 96, 2, EPI_STORE, true},
+                                     {4608, 640, 3, EPI_PEER, true},   {1024, 72, 2, EPI_PEER, false},   {2560, 5000, 0, EPI_ARGMAX, true}, {4096, 1208, 1, EPI_ARGMAX, true}, {512, 264, 0, EPI_ARGMAX, true},
+                                     {4608, 640, 2, EPI_ARGMAX, true}, {2048, 3000, 0, EPI_PEER, false}};
+    for (const Case& c : cases) {
+        const int K = c.k, N = c.n, nb = K / 32;
+        std::mt19937 rng(K + N + c.parts);
+        Dev<uint32_t> seq(std::vector<uint32_t>{41}), status(1), flag(32);
+        const uint32_t word[2] = {peer_word(41, 7), peer_word(41, 9)};
+        const std::vector<float> x0 = normal(rng, K, 1.0f);
+        std::vector<float> x = x0;
+        std::vector<uint2> pairs((size_t)c.parts * K + 1);
+        for (int r = 0; r < c.parts; r++) {
+            const std::vector<float> v = normal(rng, K, 1.0f);
+            for (int i = 0; i < K; i++) { uint32_t b; std::memcpy(&b, &v[i], 4); pairs[(size_t)r * K + i] = make_uint2(b, word[0]); x[i] += v[i]; }
+        }
+        std::vector<int8_t> q((size_t)N * K);
+        std::vector<__half> s((size_t)N * nb, __float2half(0.001f));
+        for (auto& v : q) v = (int8_t)((int)(rng() % 255) - 127);
+        const int first = N / 3, last = N - 3;               // two equal rows that no other row comes near
+        if (c.epi == EPI_ARGMAX) for (int i = 0; i < K; i++) q[(size_t)first * K + i] = q[(size_t)last * K + i] = x[i] > 0 ? 127 : -127;
+        std::vector<double> want(N);
+        for (int n = 0; n < N; n++)
+            for (int i = 0; i < K; i++) want[n] += (double)q[(size_t)n * K + i] * x[i] * (double)__half2float(s[0]);
+        Dev<int8_t> dq(q);
+        Dev<__half> ds(s);
+        Dev<unsigned char> w(q8_packed_bytes(N, K));
+        CK(launch_q8_pack_units(dq.p, ds.p, N, K, q8_pack_kc(N, K), w.p, nullptr));
+        Dev<float> dx(x0), dxo(K), y((size_t)N), part_val(256);
+        Dev<uint2> dparts(pairs), out((size_t)N);
+        Dev<int> part_idx(256), tokens(4);
+        Dev<unsigned int> counter(1), ticket(1);
+        DecodeState st{};
+        st.max_steps = 4; st.log = 1; st.pos = 11; st.vocab = N;
+        Dev<DecodeState> state(std::vector<DecodeState>{st});
+        GemvArgs a{};
+        a.nseg = 1; a.seg[0] = {w.p, nullptr, N, q8_pack_kc(N, K)}; a.K = K; a.wkind = WK_Q8; a.epi = c.epi; a.x = dx.p; a.y = y.p; a.status = status.p; a.seq = seq.p; a.wait_cycles = 10000000;
+        if (c.parts) { a.parts = (const float*)dparts.p; a.parts_ll = 1; a.n_parts = c.parts; a.part_stride = K; a.parts_tag = 7; a.x_out = dxo.p; }
+        if (c.epi == EPI_PEER) { a.n_peers = 1; a.peer_out[0] = (float*)out.p; a.peer_flag[0] = flag.p; a.peer_ticket = ticket.p; a.peer_tag = 9; a.peer_ll = c.ll; }
+        if (c.epi == EPI_ARGMAX) { a.part_val = part_val.p; a.part_idx = part_idx.p; a.counter = counter.p; a.state = state.p; a.tokens_out = tokens.p; a.advance = 1; }
+        const std::string what = std::to_string(N) + " x " + std::to_string(K) + ", " + std::to_string(c.parts) + " parts, epilogue " + std::to_string(c.epi) + (c.ll ? "" : ", values") + ": ";
+        for (int turn = 0; turn < 2; turn++) {               // (tickets are left at zero)
+            CK(launch_gemv(a, 148, nullptr));
+            std::vector<float> got(N);
+            if (c.epi == EPI_PEER) {
+                const std::vector<uint2> o = out.get();
+                double late = 0;
+                for (int n = 0; n < N; n++) {
+                    if (c.ll) { std::memcpy(&got[n], &o[n].x, 4); late += o[n].y != word[1]; }
+                    else std::memcpy(&got[n], (const float*)o.data() + n, 4);
+                }
+                if (!c.ll) late = flag.get()[0] != word[1];
+                report(what + "words", late, 0);
+            } else {
+                got = y.get();
+            }
+            report(what + "rows", rel(got, want), 16 * std::exp2(-24.0));
+            if (c.epi == EPI_ARGMAX) {
+                const DecodeState d = state.get()[0];
+                report(what + "best row", std::fabs((double)d.last_tok - last) + std::fabs((double)tokens.get()[turn] - last) + std::fabs(d.pos - 12.0 - turn) + std::fabs(d.step - 1.0 - turn), 0);
+            }
+            report("status", status.get()[0], 0);
+        }
+        if (c.parts) report(what + "the vector itself", rel(dxo.get(), std::vector<double>(x.begin(), x.end())), std::exp2(-24.0));
+    }
+}
+
 // A step's chain: an embedding row that zeroes the claim counters, projections behind it that claim from them under programmatic launch and change places between the
 // two sizes of shared memory.  Every row of every step is there (a claim from an old count leaves rows out), and what is captured says why: the first projection
 // waits for the counters in plain stream order, the others may come early.
@@ -773,6 +843,7 @@ int main(int argc, char** argv) {
     else if (what == "experts") experts();
     else if (what == "matvec-bf16") matvec_bf16();
     else if (what == "matvec-q8") matvec_q8();
+    else if (what == "matvec-peer") matvec_peer();
     else if (what == "claims") claims();
     else if (what == "few-rows") few_rows();
     else if (what == "level-specials") level_specials();

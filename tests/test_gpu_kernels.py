@@ -20,7 +20,7 @@ def kernels(pkg, tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("check", ["attention-sums", "attention-specials", "attention-prompt", "attention-band", "experts", "matvec-bf16", "matvec-q8", "few-rows", "gave-up", "level-specials", "claims"])
+@pytest.mark.parametrize("check", ["attention-sums", "attention-specials", "attention-prompt", "attention-band", "experts", "matvec-bf16", "matvec-q8", "matvec-peer", "few-rows", "gave-up", "level-specials", "claims"])
 def test_kernels(kernels, check):
     r = subprocess.run([kernels, check], capture_output=True, text=True)
     print(r.stdout)
