@@ -223,9 +223,9 @@ __global__ void __launch_bounds__(kFewThreads, 1) q8_few(const GemvArgs a, const
                 r0[8 * LD + 8 * t] = acc[t][2]; r0[8 * LD + 8 * t + 1] = acc[t][3];
             }
         }
-        const int unit0 = s_meta[first + st0].x, unit1 = s_meta[first + st1].x;
+        const int unit0 = p.cta + f0 * p.n_cta, unit1 = p.cta + f1 * p.n_cta;      // (one row group per job: not read from the stage's words, which a refill replaces)
         __syncwarp();
-        if (lane == 0) {
+        if (lane == 0) {                                     // the tiles have been read: their sums are stored
             mbar_arrive(g.empty0 + 8u * (first + st0));
             if (f1 != f0) mbar_arrive(g.empty0 + 8u * (first + st1));
         }
