@@ -63,11 +63,13 @@ __device__ __forceinline__ void mbar_fence_init() {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// The same once `seen`, formed from loaded registers, is there: an arrival that hands shared memory back to a bulk copy has to come behind the LOADS' RETURN.  In program
-// order (and behind a fence) they have only been issued, and they queue behind copies that land in shared memory: a refill asked for by the arrival was
-// there before the last of them.  The count depends on the value for the hardware alone: bit 1 of a square is 0.
-__device__ __forceinline__ void mbar_arrive_behind(uint32_t bar, uint32_t seen) {
-    asm volatile("{\n\t.reg .b32 t;\n\tmul.lo.u32 t, %1, %1;\n\tbfe.u32 t, t, 1, 1;\n\tadd.u32 t, t, 1;\n\tmbarrier.arrive.shared::cta.b64 _, [%0], t;\n\t}" ::"r"(bar), "r"(seen) : "memory");
+// v, for an instruction that must not go out before `seen`, formed from loaded registers, is there.  Whatever lets a bulk copy overwrite shared memory (the arrival
+// that hands a stage back, the copy itself) has to come behind the RETURN of the loads from it.  In program order, and behind a fence, they have only been issued,
+// and they queue behind copies that land in shared memory: a refill was there before the last of them.  (Bit 1 of a square is 0.)
+__device__ __forceinline__ uint32_t behind(uint32_t v, uint32_t seen) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .b32 t;\n\tmul.lo.u32 t, %2, %2;\n\tbfe.u32 t, t, 1, 1;\n\tadd.u32 %0, %1, t;\n\t}" : "=r"(r) : "r"(v), "r"(seen));
+    return r;
 }
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");

@@ -793,7 +793,7 @@ __device__ __forceinline__ void gemv_consume(const GemvArgs& a, const XSource& x
                 for (int s = 0; s < 4; s++) seen ^= wx[s][0] ^ wy[s][0] ^ dw[s];
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive_behind(g.empty0 + 8u * st, seen);
+            if (lane == 0) mbar_arrive(behind(g.empty0 + 8u * st, seen));
             if (++cr.stage == S) { cr.stage = 0; cr.par ^= 1u; }
             if (mm.x == kMetaEnd) { ended = true; break; }
             if (ONE) {

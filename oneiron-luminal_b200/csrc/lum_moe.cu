@@ -65,11 +65,11 @@ __device__ __forceinline__ bool moe_stream(MoeRing& ring, int units, int K, cons
                                            Levels levels, Ready ready, Done done) {
     const int nb = K >> 5, chunks = (nb + ring.blocks - 1) / ring.blocks, total = units * chunks;
     auto count = [&](int c) { return min(ring.blocks, nb - c * ring.blocks); };
-    auto issue = [&](int i) {
+    auto issue = [&](int i, uint32_t seen) {                     // seen: see behind()
         const int u = i / chunks, c = i - u * chunks, n = count(c);
         const int8_t* src = q + rows(u) * K;
         const uint32_t st = ring.issued % ring.stages, bar = ring.bars + 8u * st;
-        const uint32_t dst = smem_u32(ring.base) + st * (uint32_t)ring.blocks * 64u;
+        const uint32_t dst = behind(smem_u32(ring.base) + st * (uint32_t)ring.blocks * 64u, seen);
         if (elect_one()) {
             mbar_arrive_expect_tx(bar, (uint32_t)n * 64u);
             if (chunks == 1) bulk_g2s(dst, src, (uint32_t)n * 64u, bar);                // both rows are one run
@@ -91,7 +91,7 @@ __device__ __forceinline__ bool moe_stream(MoeRing& ring, int units, int K, cons
         b[0] = load_gain(bias, gain_kind, (int)row);
         b[1] = load_gain(bias, gain_kind, (int)row + 1);
     };
-    for (int i = 0; i < ring.stages && i < total; i++) issue(i);
+    for (int i = 0; i < ring.stages && i < total; i++) issue(i, 0u);
     uint16_t dn[2][kMoeTrips], d[2][kMoeTrips];
     float bn[2], b[2];
     if (total > 0) scales(0, dn, bn);
@@ -133,7 +133,7 @@ __device__ __forceinline__ bool moe_stream(MoeRing& ring, int units, int K, cons
         }
         ring.taken++;
         __syncwarp();
-        if (i + ring.stages < total) issue(i + ring.stages);
+        if (i + ring.stages < total) issue(i + ring.stages, __float_as_uint(acc[0]) ^ __float_as_uint(acc[1]));      // (both rows of the chunk have been added up)
         if (c == chunks - 1) {
             done(u, warp_sum(acc[0]) + b[0], warp_sum(acc[1]) + b[1]);
             acc[0] = acc[1] = 0.0f;
