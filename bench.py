@@ -203,9 +203,9 @@ def kernel_roofline(pkg, torch, peaks, peak_kind):
     return {"bound": "hbm", "kernel": "q8_gemv_stream", "shape": f"N={n} K={k} (gate+up sized), alone, back to back",
             "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"],
             "peak_kind": f"of {peak_kind} (burst copy)", "us_per_launch": ms * 1000.0, "bytes_per_launch": bytes_per_launch,
-            # dram__bytes_read.sum + dram__bytes_write.sum of one launch of this shape under ncu (124.87 MB read + 9.17 MB
+            # dram__bytes_read.sum + dram__bytes_write.sum of one launch of this shape under ncu (124.87 MB read + 7.10 MB
             # written): a figure from a profile of this kernel, not measured by this run
-            "traffic": 134_049_024, "traffic_from": "ncu capture of this kernel on this shape (profiles/), not this run"}, launches + 4
+            "traffic": 131_967_488, "traffic_from": "ncu capture of this kernel on this shape (profiles/), not this run"}, launches + 4
 
 
 def kernel_rows_sweep(pkg, torch):

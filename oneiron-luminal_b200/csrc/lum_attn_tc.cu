@@ -111,7 +111,7 @@ __device__ __forceinline__ void split2_rn(float x0, float x1, uint32_t* hi, uint
 }  // namespace
 
 // G = query heads per KV head (1, 2, 4 or 8): MMA row r = g * QT + qi is query row q0 + qi of head kvh * G + g.
-// Measured, 32 / 8 heads of 128: 4096 rows from position 0 1278 -> 326 us (422 issued TFLOP/s), 387 rows behind 1021 positions 119 -> 36 us.  What a tile waits for now
+// Measured, 32 / 8 heads of 128: 4096 rows from position 0 1278 -> 326 us (422 useful TFLOP/s, twice that issued), 387 rows behind 1021 positions 119 -> 36 us.  What a tile waits for now
 // is its K and V: LDGSTS of 512 bytes per 24 clocks.
 //
 // BAND: the layers described one by one whose heads have this size (band_is_prompt): a window or chunks of keys, queries that carry the score's factor, a distance bias

@@ -120,7 +120,7 @@ __host__ __device__ inline FewSmem few_smem(int tiles, int k, size_t ring) {
 
 // T: groups of eight columns.  y[range][m][column] = sums of the range (planes part_stride apart, rows ldy).
 // The accumulators start at 1.5 * 2^23 as a float's bits, so that an int32 sum comes out as that float plus the sum: an addition instead of a conversion.
-// Measured, 5 rows of a Llama-3-8B layer (q8_gemm_tc_skinny / this): gate | up 45 -> 32 us, vocabulary projection 151 -> 111 us; a step of five sequences 4.08 -> 2.98 ms.
+// Measured, 5 rows of a Llama-3-8B layer (q8_gemm_tc_skinny / this): gate | up 45 -> 32 us, vocabulary projection 151 -> 111 us; a step of five sequences 4.08 -> 2.95 ms.
 // With a warp per (tile, row) instead of columns of all rows: 3.70 ms (issue slots).
 template <int T>
 __global__ void __launch_bounds__(kFewThreads, 1) q8_few(const GemvArgs a, const int M, const int8_t* xq, const float* sx, const int ldy, const size_t part_stride) {

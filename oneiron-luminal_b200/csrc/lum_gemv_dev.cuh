@@ -10,7 +10,7 @@
 //                                     sample) runs on the finished rows.
 //
 // What bounds it: HBM while weights stream, and between two phases the time from the previous one's last row to this one's
-// first: hand-over, activations, first tiles.  A CTA therefore takes half an SM (288 threads, 112 registers, 110 KB), so that
+// first: hand-over, activations, first tiles.  A CTA therefore takes half an SM (288 threads, 96 registers, 103 or 114 KB), so that
 // under programmatic dependent launch the next phase's CTA is set up and has its ring full of weights while this one still
 // works.  The form before it, tcgen05 kind::i8 over 576 threads and 512 columns of tensor memory, had an SM to itself: the next
 // phase could not ask for a byte before it was gone.  The legacy tensor path is the right one here: a tile is 8 rows, one
